@@ -65,10 +65,18 @@ class _FlatSplit(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grads):
         shape, dtype, device = ctx.meta
-        g = torch.zeros(shape, dtype=dtype, device=device)
+        g = torch.empty(shape, dtype=dtype, device=device)
+        end = 0
         for (name, (off, n)), gv in zip(ctx.layer.offsets.items(), grads):
+            if off > end:
+                g[end:off].zero_()   # padding between views
             if gv is not None:
                 g[off:off + n].copy_(gv.reshape(-1))
+            else:
+                g[off:off + n].zero_()
+            end = off + n
+        if end < g.numel():
+            g[end:].zero_()
         return g, None
 
 

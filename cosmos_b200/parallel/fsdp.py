@@ -111,10 +111,10 @@ class ShardedUnit:
             self._prefetched = None
             torch.cuda.current_stream().wait_event(ev)
             return full
-        full = torch.empty(self.n, dtype=self.dtype, device=self.device)
         if self.ws == 1:
-            full.copy_(self.shard.data)
-        elif self.fused:
+            return self.shard.detach()   # the shard is the whole tensor; nothing writes it before the optimizer step
+        full = torch.empty(self.n, dtype=self.dtype, device=self.device)
+        if self.fused:
             self._pull(full)
         else:
             dist.all_gather_into_tensor(full, self.shard.data.contiguous(), group=self.group)
@@ -256,7 +256,9 @@ class FSDP:
                 p.grad.div_(ws)
             self._avg_over_replicas(p.grad)
         inv_ws = 1.0 / ws
-        sq = torch.zeros(1, dtype=torch.float32, device=self.replicated[0].device if self.replicated else "cpu")
+        sq = torch.zeros(1, dtype=torch.float64, device=next(iter(self.parameters())).device)
+        local = self._local_kernel() and self.rep == 1
+        rep_kernel = self._rep_kernel()
         reduced: Dict[Tuple[str, int], torch.Tensor] = {}
         if self.fused:
             if self.comm is not None:
@@ -269,22 +271,13 @@ class FSDP:
             if reduced:
                 norms = torch._foreach_norm(list(reduced.values()))
                 sq += torch.stack(norms).pow(2).sum()
-        elif self._local_kernel() and self.rep == 1:
-            # gradients are already local (one rank, or the NCCL reduce-scatter ran in backward): the same
-            # optimizer kernel with this rank's gradient shard as its only source
-            ptrs: Dict[Tuple[str, int], torch.Tensor] = {}
+        elif local:
+            # gradients are already local (one rank, or the NCCL reduce-scatter ran in backward): norm and update read the
+            # bf16 gradients of all units in one launch each
             for key, u in self.units.items():
-                g = u.shard.grad
-                if g is None:
-                    continue
-                g = g.contiguous()
-                u.shard.grad = g  # keep the tensor alive until the update kernel below has read it
-                ptrs[key] = torch.tensor([g.data_ptr()], dtype=torch.int64, device=u.device)
-                # pass 1 only adds up the squares; pass 2 reads the bf16 gradient again (no fp32 copy is kept)
-                torch.ops.cosmos_b200.rs_adamw(ptrs[key], 1, 0, u.master, u.exp_avg, u.exp_avg_sq, u.shard.data, 1.0, 0.0,
-                                               b1, b2, self.eps, 0.0, self.step_count, 1, sq, None)
-                reduced[key] = g
-            sq.mul_(inv_ws * inv_ws)
+                if u.shard.grad is not None:
+                    reduced[key] = u.shard.grad.contiguous()
+            torch.ops.cosmos_b200.grad_sq_list(list(reduced.values()), inv_ws, sq)
         else:
             for key, u in self.units.items():
                 if u.shard.grad is not None:
@@ -294,15 +287,35 @@ class FSDP:
                     sq += g.pow(2).sum()
         if ws > 1:
             dist.all_reduce(sq, group=self.group)
-        rep_sq = sum(p.grad.float().pow(2).sum() for p in self.replicated) if self.replicated else 0.0
-        total = float(torch.sqrt(sq + rep_sq))
-        clip = 1.0
-        if self.max_grad_norm is not None and total > self.max_grad_norm:
-            clip = self.max_grad_norm / (total + 1e-6)
+        rep_grads = [p.grad.contiguous() for p in self.replicated]
+        if rep_kernel:
+            torch.ops.cosmos_b200.grad_sq_list(rep_grads, 1.0, sq)
+        else:
+            for g in rep_grads:
+                sq += g.float().pow(2).sum()
+        # the list kernels work the clip factor out from `sq` on the device, so where they do every update the host reads
+        # the norm only behind them
+        on_device = local and (rep_kernel or not self.replicated)
+        total, clip = None, 1.0
+        if not on_device:
+            total = float(torch.sqrt(sq))
+            if self.max_grad_norm is not None and total > self.max_grad_norm:
+                clip = self.max_grad_norm / (total + 1e-6)
+        limit = -1.0 if self.max_grad_norm is None else float(self.max_grad_norm)
+        hyper = (self.lr, b1, b2, self.eps, self.wd, self.step_count)
+        if local and reduced:
+            us = [self.units[key] for key in reduced]
+            torch.ops.cosmos_b200.adamw_list(list(reduced.values()), [u.master for u in us], [u.exp_avg for u in us],
+                                             [u.exp_avg_sq for u in us], [u.shard.data for u in us], inv_ws, sq, limit, *hyper)
+            for u in us:
+                u.shard.grad = None
+        if rep_kernel and rep_grads:
+            torch.ops.cosmos_b200.adamw_list(rep_grads, self.rep_master, self.rep_m, self.rep_v,
+                                             [p.data for p in self.replicated], 1.0, sq, limit, *hyper)
         bc1 = 1.0 - b1 ** self.step_count
         bc2 = 1.0 - b2 ** self.step_count
         for key, u in self.units.items():
-            if key not in reduced:
+            if key not in reduced or local:
                 continue
             if self.fused:
                 if u.dtype == torch.bfloat16:
@@ -313,23 +326,26 @@ class FSDP:
                            bc1, bc2)
                     u.shard.data.copy_(u.master)
                 u._has_grad = False
-            elif self._local_kernel() and self.rep == 1:
-                torch.ops.cosmos_b200.rs_adamw(ptrs[key], 1, 0, u.master, u.exp_avg, u.exp_avg_sq, u.shard.data,
-                                               clip * inv_ws, self.lr, b1, b2, self.eps, self.wd, self.step_count, 0,
-                                               None, None)
-                u.shard.grad = None
             else:
                 _adamw(u.master, u.exp_avg, u.exp_avg_sq, reduced[key] * clip, self.lr, b1, b2, self.eps, self.wd,
                        bc1, bc2)
                 u.shard.data.copy_(u.master)
                 u.shard.grad = None
         for p, mst, m, v in zip(self.replicated, self.rep_master, self.rep_m, self.rep_v):
-            _adamw(mst, m, v, p.grad.float() * clip, self.lr, b1, b2, self.eps, self.wd, bc1, bc2)
-            p.data.copy_(mst)
+            if not rep_kernel:
+                _adamw(mst, m, v, p.grad.float() * clip, self.lr, b1, b2, self.eps, self.wd, bc1, bc2)
+                p.data.copy_(mst)
             p.grad = None
         if self.fused:
             self.sg.barrier(slot=4)  # every rank's shards are updated before anyone gathers them again
-        return total
+        return float(torch.sqrt(sq)) if total is None else total
+
+    def _rep_kernel(self) -> bool:
+        """Norm and AdamW of the replicated parameters through the list kernels: CUDA, bf16, dense."""
+        from .. import ops
+        return (bool(self.replicated) and all(p.is_cuda and p.dtype == torch.bfloat16 and p.is_contiguous() and
+                                              p.grad.dtype == torch.bfloat16 for p in self.replicated)
+                and ops.load_extension(build_if_missing=False))
 
     def _local_kernel(self) -> bool:
         """AdamW through the optimizer kernel on this rank's own gradient shards (no peer reads)."""

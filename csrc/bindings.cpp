@@ -1070,6 +1070,53 @@ void rs_adamw(const Tensor& grads, int64_t world, int64_t shard_off, Tensor mast
                    (float)b1, (float)b2, (float)eps, (float)wd, (int)step, sqp, redp, cur_stream());
 }
 
+// ---- optimizer over lists of tensors (optim.cu) ----
+void check_grads(at::TensorList grads, const Tensor& sq) {
+  TORCH_CHECK(sq.is_cuda() && sq.scalar_type() == at::kDouble && sq.numel() == 1, "sq must be one fp64 value on the GPU");
+  for (const Tensor& g : grads) {
+    check_bf16_cuda(g, "gradient");
+    TORCH_CHECK(g.is_contiguous() && g.device() == sq.device(), "gradients must be contiguous and on the GPU of sq");
+  }
+}
+
+void grad_sq_list(at::TensorList grads, double scale, Tensor sq) {
+  c10::cuda::CUDAGuard guard(sq.device());
+  check_grads(grads, sq);
+  for (size_t i = 0; i < grads.size(); i += cosmos::OPT_MAX) {
+    cosmos::OptTensor t[cosmos::OPT_MAX] = {};
+    const int n = (int)std::min<size_t>(cosmos::OPT_MAX, grads.size() - i);
+    for (int j = 0; j < n; ++j) {
+      t[j].grad = grads[i + j].data_ptr();
+      t[j].n = grads[i + j].numel();
+    }
+    cosmos::grad_sq_list(t, n, (float)scale, sq.data_ptr<double>(), cur_stream());
+  }
+}
+
+void adamw_list(at::TensorList grads, at::TensorList masters, at::TensorList ms, at::TensorList vs, at::TensorList params,
+                double scale, const Tensor& sq, double max_norm, double lr, double b1, double b2, double eps, double wd,
+                int64_t step) {
+  c10::cuda::CUDAGuard guard(sq.device());
+  check_grads(grads, sq);
+  TORCH_CHECK(masters.size() == grads.size() && ms.size() == grads.size() && vs.size() == grads.size() &&
+              params.size() == grads.size(), "adamw_list: lists of one length");
+  for (size_t i = 0; i < grads.size(); i += cosmos::OPT_MAX) {
+    cosmos::OptTensor t[cosmos::OPT_MAX] = {};
+    const int n = (int)std::min<size_t>(cosmos::OPT_MAX, grads.size() - i);
+    for (int j = 0; j < n; ++j) {
+      const Tensor &g = grads[i + j], &w = masters[i + j], &m = ms[i + j], &v = vs[i + j], &p = params[i + j];
+      check_bf16_cuda(p, "parameter");
+      for (const Tensor* x : {&w, &m, &v})
+        TORCH_CHECK(x->is_cuda() && x->scalar_type() == at::kFloat && x->is_contiguous() && x->numel() == g.numel() &&
+                    x->device() == g.device(), "adamw_list: fp32 weights and moments of the gradients' sizes");
+      TORCH_CHECK(p.is_contiguous() && p.numel() == g.numel() && p.device() == g.device(), "adamw_list: parameter size mismatch");
+      t[j] = {g.data_ptr(), w.data_ptr<float>(), m.data_ptr<float>(), v.data_ptr<float>(), p.data_ptr(), g.numel(), 0};
+    }
+    cosmos::adamw_list(t, n, (float)scale, sq.data_ptr<double>(), (float)max_norm, (float)lr, (float)b1, (float)b2, (float)eps,
+                       (float)wd, (int)step, cur_stream());
+  }
+}
+
 // ---- fused communication ops (comm.cu) ----
 // grads / bufs: int64 CUDA tensors with one device address per rank; mc_ptr: NVLink multicast address of the same
 // symmetric buffer (0 = none: plain peer loads).
@@ -1250,6 +1297,8 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_set_debug", &attn_set_debug);
   m.def("bounds_check_selftest", &bounds_check_selftest);
   m.def("rs_adamw", &rs_adamw);
+  m.def("grad_sq_list", &grad_sq_list);
+  m.def("adamw_list", &adamw_list);
   m.def("allgather_pull", &allgather_pull);
   m.def("reduce_scatter_pull", &reduce_scatter_pull);
   m.def("adamw_shard", &adamw_shard);

@@ -1,0 +1,180 @@
+// Optimizer kernels over lists of tensors: global gradient norm and AdamW with clipping, one launch for a whole model.
+//
+// What bounds both is memory: the norm reads 2 bytes a parameter; the update reads 14 (bf16 gradient, fp32 weight and two
+// moments) and writes 14 (the state again, and the bf16 weight). A tensor is cut into chunks of 8192 elements and the
+// chunks of all tensors form one grid-stride loop, so that a list of many small tensors costs one launch and a large one
+// fills the chip. The clip factor is worked out from the device-side norm, so no host round trip stands between the two.
+// Measured on the 543 M parameters of a two-layer Nano generator (2 layers of 193 M, 17 tensors outside them, the largest
+// 100 M): update 2.8 ms = 5.4 TB/s, norm 0.17 ms = 6.4 TB/s. Before, the layers took a launch each (2.6 ms together) and the
+// tensors outside them a chain of about 14 elementwise launches each, 5.1 ms more.
+#include <algorithm>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace cb {
+
+constexpr int OPT_CHUNK = 8192;    // elements: 256 threads x 8 elements x 4 trips
+constexpr int OPT_THREADS = 256;
+
+struct OptList {
+  cosmos::OptTensor t[cosmos::OPT_MAX];
+  long long first_chunk[cosmos::OPT_MAX + 1];
+  int n;
+};
+
+__device__ __forceinline__ int opt_find(const OptList& l, long long chunk) {
+  int lo = 0, hi = l.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (l.first_chunk[mid] <= chunk) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+  f[0] = bf16lo(u.x); f[1] = bf16hi(u.x); f[2] = bf16lo(u.y); f[3] = bf16hi(u.y);
+  f[4] = bf16lo(u.z); f[5] = bf16hi(u.z); f[6] = bf16lo(u.w); f[7] = bf16hi(u.w);
+}
+
+// sq += scale^2 * sum of squares of all gradients. A thread's few hundred squares are added in fp32, the threads' sums in
+// fp64, so the result does not depend on the order in which blocks finish beyond the last bits of a double.
+__global__ void __launch_bounds__(OPT_THREADS)
+grad_sq_kernel(const __grid_constant__ OptList l, float scale, double* sq) {
+  __shared__ double red[OPT_THREADS / 32];
+  double sum = 0.0;
+  for (long long ch = blockIdx.x; ch < l.first_chunk[l.n]; ch += gridDim.x) {
+    const int k = opt_find(l, ch);
+    const cosmos::OptTensor& t = l.t[k];
+    const long long e0 = (ch - l.first_chunk[k]) * OPT_CHUNK;
+    const int len = (int)min((long long)OPT_CHUNK, t.n - e0);
+    const bf16* g = reinterpret_cast<const bf16*>(t.grad) + e0;
+    float s = 0.f;
+    if (t.vec && len == OPT_CHUNK) {
+      uint4 u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = reinterpret_cast<const uint4*>(g)[j * OPT_THREADS + threadIdx.x];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float f[8];
+        unpack8(u[j], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s = fmaf(f[e], f[e], s);
+      }
+    } else {
+      for (int i = threadIdx.x; i < len; i += OPT_THREADS) {
+        const float f = __bfloat162float(g[i]);
+        s = fmaf(f, f, s);
+      }
+    }
+    sum += (double)s;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < OPT_THREADS / 32; ++w) sum += red[w];
+    atomicAdd(sq, sum * (double)scale * (double)scale);
+  }
+}
+
+struct AdamWStep {
+  float lr, b1, b2, eps, wd, bc1, bc2;
+  __device__ __forceinline__ void operator()(float g, float& m, float& v, float& w) const {
+    m = b1 * m + (1.f - b1) * g;
+    v = b2 * v + (1.f - b2) * g * g;
+    w -= lr * ((m / bc1) / (sqrtf(v / bc2) + eps) + wd * w);
+  }
+};
+
+// g = grad * scale * clip with clip = min(1, max_norm / (norm + 1e-6)) from the device-side `sq`; max_norm < 0: no clipping.
+__global__ void __launch_bounds__(OPT_THREADS)
+adamw_list_kernel(const __grid_constant__ OptList l, const __grid_constant__ AdamWStep opt, float scale, const double* sq,
+                  float max_norm) {
+  float gs = scale;
+  if (max_norm >= 0.f) {
+    const double norm = sqrt(*sq);
+    if (norm > (double)max_norm) gs *= (float)((double)max_norm / (norm + 1e-6));
+  }
+  for (long long ch = blockIdx.x; ch < l.first_chunk[l.n]; ch += gridDim.x) {
+    const int k = opt_find(l, ch);
+    const cosmos::OptTensor& t = l.t[k];
+    const long long e0 = (ch - l.first_chunk[k]) * OPT_CHUNK;
+    const int len = (int)min((long long)OPT_CHUNK, t.n - e0);
+    const bf16* g = reinterpret_cast<const bf16*>(t.grad) + e0;
+    float *w = t.master + e0, *m = t.m + e0, *v = t.v + e0;
+    bf16* p = reinterpret_cast<bf16*>(t.param) + e0;
+    if (t.vec && len == OPT_CHUNK) {
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        const int i = (j * OPT_THREADS + threadIdx.x) * 8;
+        float gf[8], wf[8], mf[8], vf[8];
+        const uint4 gu = *reinterpret_cast<const uint4*>(g + i);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          *reinterpret_cast<float4*>(mf + 4 * h) = *reinterpret_cast<const float4*>(m + i + 4 * h);
+          *reinterpret_cast<float4*>(vf + 4 * h) = *reinterpret_cast<const float4*>(v + i + 4 * h);
+          *reinterpret_cast<float4*>(wf + 4 * h) = *reinterpret_cast<const float4*>(w + i + 4 * h);
+        }
+        unpack8(gu, gf);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) opt(gf[e] * gs, mf[e], vf[e], wf[e]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          *reinterpret_cast<float4*>(m + i + 4 * h) = *reinterpret_cast<float4*>(mf + 4 * h);
+          *reinterpret_cast<float4*>(v + i + 4 * h) = *reinterpret_cast<float4*>(vf + 4 * h);
+          *reinterpret_cast<float4*>(w + i + 4 * h) = *reinterpret_cast<float4*>(wf + 4 * h);
+        }
+        *reinterpret_cast<uint4*>(p + i) =
+            make_uint4(pack_bf16(wf[0], wf[1]), pack_bf16(wf[2], wf[3]), pack_bf16(wf[4], wf[5]), pack_bf16(wf[6], wf[7]));
+      }
+    } else {
+      for (int i = threadIdx.x; i < len; i += OPT_THREADS) {
+        float mi = m[i], vi = v[i], wi = w[i];
+        opt(__bfloat162float(g[i]) * gs, mi, vi, wi);
+        m[i] = mi;
+        v[i] = vi;
+        w[i] = wi;
+        p[i] = __float2bfloat16(wi);
+      }
+    }
+  }
+}
+
+static long long fill_list(const cosmos::OptTensor* t, int n, OptList& l) {
+  if (n < 1 || n > cosmos::OPT_MAX) throw std::runtime_error("optimizer list: 1 to 64 tensors per launch");
+  l.n = n;
+  l.first_chunk[0] = 0;
+  for (int i = 0; i < n; ++i) {
+    l.t[i] = t[i];
+    const auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    // 16-byte loads where every address allows them; the chunks keep that alignment
+    l.t[i].vec = al(t[i].grad) && al(t[i].master) && al(t[i].m) && al(t[i].v) && al(t[i].param);
+    l.first_chunk[i + 1] = l.first_chunk[i] + (t[i].n + OPT_CHUNK - 1) / OPT_CHUNK;
+  }
+  return l.first_chunk[n];
+}
+
+}  // namespace cb
+
+namespace cosmos {
+
+void grad_sq_list(const OptTensor* t, int n, float scale, double* sq, cudaStream_t s) {
+  cb::OptList l;
+  const long long chunks = cb::fill_list(t, n, l);
+  if (chunks == 0) return;
+  cb::grad_sq_kernel<<<(int)std::min<long long>(chunks, 148 * 8), cb::OPT_THREADS, 0, s>>>(l, scale, sq);
+}
+
+void adamw_list(const OptTensor* t, int n, float scale, const double* sq, float max_norm, float lr, float b1, float b2, float eps,
+                float wd, int step, cudaStream_t s) {
+  cb::OptList l;
+  const long long chunks = cb::fill_list(t, n, l);
+  if (chunks == 0) return;
+  const cb::AdamWStep opt{lr, b1, b2, eps, wd, 1.f - powf(b1, (float)step), 1.f - powf(b2, (float)step)};
+  cb::adamw_list_kernel<<<(int)std::min<long long>(chunks, 148 * 8), cb::OPT_THREADS, 0, s>>>(l, opt, scale, sq, max_norm);
+}
+
+}  // namespace cosmos

@@ -903,3 +903,36 @@ def test_adamw_kernels_match_the_fp32_definition(n, off):
     for got, want in ((m, m_ref), (v, v_ref), (w, w_ref)):
         assert torch.allclose(got, want, rtol=1e-5, atol=1e-6)
     assert torch.equal(p, w.bfloat16())
+
+
+@pytest.mark.parametrize("sizes", [(1,), (8191, 8192, 8193), (100_003, 16, 65_536), (257,) * 70])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_optimizer_list_kernels_match_the_definition(sizes, shift):
+    """Norm and clipped AdamW over lists: chunk edges, more tensors than one launch takes, addresses that rule 16-byte
+    accesses out (`shift`). fp32 arithmetic: a few roundings of values below 10 an element."""
+    k = torch.ops.cosmos_b200
+    g = torch.Generator(device=DEV).manual_seed(sum(sizes) + shift)
+    cut = lambda n, dt: torch.randn(n + 8, device=DEV, generator=g).to(dt)[shift:shift + n]  # noqa: E731
+    grads = [cut(n, torch.bfloat16) for n in sizes]
+    w, m = ([cut(n, torch.float32) for n in sizes] for _ in range(2))
+    v = [cut(n, torch.float32).abs() for n in sizes]
+    p = [cut(n, torch.bfloat16) for n in sizes]
+    w0, m0, v0 = ([t.double() for t in ts] for ts in (w, m, v))
+    scale, lr, b1, b2, eps, wd, step = 0.5, 1e-2, 0.9, 0.95, 1e-8, 0.1, 3
+    sq = torch.zeros(1, device=DEV, dtype=torch.float64)
+    k.grad_sq_list(grads, scale, sq)
+    norm = math.sqrt(sum(float((t.double() * scale).square().sum()) for t in grads))
+    assert abs(math.sqrt(float(sq)) - norm) <= 1e-6 * norm
+    for limit in (-1.0, 0.5 * norm, 2 * norm):
+        for ts, t0 in ((w, w0), (m, m0), (v, v0)):
+            for t, x in zip(ts, t0):
+                t.copy_(x)
+        k.adamw_list(grads, w, m, v, p, scale, sq, limit, lr, b1, b2, eps, wd, step)
+        clip = limit / (norm + 1e-6) if 0 <= limit < norm else 1.0
+        for i, gr in enumerate(grads):
+            gd = gr.double() * scale * clip
+            mr, vr = b1 * m0[i] + (1 - b1) * gd, b2 * v0[i] + (1 - b2) * gd * gd
+            wr = w0[i] - lr * ((mr / (1 - b1 ** step)) / ((vr / (1 - b2 ** step)).sqrt() + eps) + wd * w0[i])
+            for got, want in ((m[i], mr), (v[i], vr), (w[i], wr)):
+                assert (got.double() - want).abs().max() <= 1e-5 + 1e-5 * want.abs().max()
+            assert torch.equal(p[i], w[i].bfloat16())
