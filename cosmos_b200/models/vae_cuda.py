@@ -1,21 +1,23 @@
-"""Tokenizer decoder on the sm_100a kernels: activations live in zero-padded channels-last volumes
-[frames, H + 2, W + 2, C] (bf16), every 3x3x3 causal convolution is an implicit GEMM on the tensor
-cores (each filter tap is a row-shifted TMA view of the flattened volume), the channel RMS-norm +
-SiLU, the nearest upsampling and the final RGB convolution + uint8 conversion are bandwidth
-kernels. Decoding runs in temporal chunks; the causal context of every convolution (the last two
-frames of its input) is carried from chunk to chunk, so the result equals one pass over the clip.
+"""Tokenizer encoder and decoder on the sm_100a kernels: activations live in zero-bordered channels-last volumes
+[frames, H + 2, W + 2, C] (bf16) and every 3x3x3 causal convolution is an implicit GEMM on the tensor cores
+(csrc/conv_tcgen05.cu). A convolution's epilogue also does what follows it: the residual, the channel RMS-norm + SiLU, the
+nearest upsampling, the layout that a strided convolution reads, or the conversion to pixels, so that a layer is one launch.
+Clips run in temporal chunks; the causal context of every convolution (the last two frames of its input) is carried from
+chunk to chunk, so the result equals one pass over the clip.
 
 Built from a `CausalVideoVAE` (same weights); requires channel widths that are multiples of 64.
 """
 from __future__ import annotations
 
-from typing import Dict, List, Optional
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
 from .vae import CausalVideoVAE, ResBlock
 
 TPAD = 2  # context frames in front of every volume (temporal kernel 3, stride 1)
+SAME, S2D, UP, DOWN = 0, 1, 2, 3   # layouts that a convolution can write (csrc/kernels.h, ConvOut)
+NORM_WIDTHS = (64, 128, 256)       # channels that the fused norm takes: a thread of the epilogue holds a whole row
 
 
 def _pack_weight(w: torch.Tensor, cin_pad: int) -> torch.Tensor:
@@ -26,75 +28,95 @@ def _pack_weight(w: torch.Tensor, cin_pad: int) -> torch.Tensor:
     return p.reshape(cout, 27 * cin_pad).contiguous()
 
 
-class CLDecoder:
-    def __init__(self, vae: CausalVideoVAE):
-        dev = next(vae.parameters()).device
-        assert dev.type == "cuda", "the channels-last decoder runs on CUDA"
-        self.device = dev
+def _bf16_terms(w: torch.Tensor, n: int = 3) -> torch.Tensor:
+    """fp32 [rows, cols] -> [n * rows, cols] bf16 whose n blocks of rows add up to it (three terms hold all 24 bits)."""
+    out, rest = [], w.float()
+    for _ in range(n):
+        out.append(rest.to(torch.bfloat16))
+        rest = rest - out[-1].float()
+    return torch.cat(out).contiguous()
+
+
+class _CLConvs:
+    """Packed weights and the launches that encoder and decoder share."""
+
+    def __init__(self, vae: CausalVideoVAE, eps: float):
+        self.device = next(vae.parameters()).device
+        assert self.device.type == "cuda", "the channels-last tokenizer runs on CUDA"
         self.latent_channels = vae.latent_channels
+        self.eps = eps
         self.w: Dict[str, torch.Tensor] = {}
         self.b: Dict[str, torch.Tensor] = {}
         self.g: Dict[str, torch.Tensor] = {}
 
-        def conv(name, m, cin_pad=None):
-            cin = m.weight.shape[1]
-            assert m.k == (3, 3, 3) and m.stride == (1, 1, 1)
-            cp = cin_pad or cin
-            assert cp % 64 == 0 and m.weight.shape[0] % 32 == 0, "channel widths must be multiples of 64"
-            self.w[name] = _pack_weight(m.weight.data, cp)
-            self.b[name] = m.bias.data.to(torch.bfloat16).contiguous()
+    def _add_conv(self, name: str, m, cin_pad: Optional[int] = None) -> None:
+        assert m.k == (3, 3, 3)
+        cp = cin_pad or m.weight.shape[1]
+        assert cp % 64 == 0 and m.weight.shape[0] % 32 == 0, "channel widths must be multiples of 64"
+        self.w[name] = _pack_weight(m.weight.data, cp)
+        self.b[name] = m.bias.data.float().contiguous()
 
-        def res(name, blk: ResBlock):
-            assert blk.skip is None
-            self.g[name + ".n1"] = blk.n1.gamma.data.to(torch.bfloat16).contiguous()
-            self.g[name + ".n2"] = blk.n2.gamma.data.to(torch.bfloat16).contiguous()
-            conv(name + ".c1", blk.c1)
-            conv(name + ".c2", blk.c2)
+    def _add_res(self, name: str, blk: ResBlock) -> None:
+        self.g[name + ".n1"] = blk.n1.gamma.data.to(torch.bfloat16).contiguous()
+        self.g[name + ".n2"] = blk.n2.gamma.data.to(torch.bfloat16).contiguous()
+        self._add_conv(name + ".c1", blk.c1)
+        self._add_conv(name + ".c2", blk.c2)
 
-        conv("in", vae.dec_in, 64)
-        res("mid", vae.dec_mid)
+    # ------------------------------------------------------------------ launches
+    def _ctx(self, cache: Dict, key: str, vol: torch.Tensor, dim: int = 0) -> None:
+        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail."""
+        head = vol.narrow(dim, 0, TPAD)
+        if key in cache:
+            head.copy_(cache[key])
+        else:
+            head.zero_()
+        cache[key] = vol.narrow(dim, vol.shape[dim] - TPAD, TPAD).clone()
+
+    def _empty(self, *shape) -> torch.Tensor:
+        return torch.empty(*shape, dtype=torch.bfloat16, device=self.device)
+
+    def _conv(self, cache: Dict, name: str, x: torch.Tensor, resid=None, skip=None, norm: Optional[torch.Tensor] = None,
+              raw: bool = True, mode: int = SAME, a: int = 0, b: int = 0, frames: Optional[int] = None
+              ) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
+        """One convolution of `x` (context frames filled in here). Returns (result, silu(rmsnorm(result) * norm)); `raw`
+        False: the first is not wanted. `mode`, `a`, `b`: the layout written (`ops.conv3d_fused`); `frames`: its frame count."""
+        self._ctx(cache, name, x, 1 if mode == DOWN else 0)
+        w = self.w[name]
+        cout = w.shape[0]
+        if mode == DOWN:
+            shape = (frames + TPAD, x.shape[2] + 1, x.shape[3] + 1, cout)
+        elif mode == S2D:
+            shape = (4, x.shape[0], x.shape[1] // 2, x.shape[2] // 2, cout)
+        elif mode == UP:
+            shape = (frames + TPAD, 2 * x.shape[1] - 2, 2 * x.shape[2] - 2, cout)
+        else:
+            shape = (*x.shape[:3], cout)
+        fused = norm is not None and cout in NORM_WIDTHS
+        out = self._empty(*shape) if raw or not fused else None
+        out_norm = self._empty(*shape) if fused else None
+        torch.ops.cosmos_b200.conv3d_fused(x, w, self.b[name], resid, skip, out, out_norm, norm if fused else None, self.eps,
+                                           mode, a, b)
+        if norm is not None and not fused:
+            out_norm = torch.ops.cosmos_b200.rmsnorm_silu(out, norm, self.eps)
+        return out, out_norm
+
+
+class CLDecoder(_CLConvs):
+    def __init__(self, vae: CausalVideoVAE):
+        super().__init__(vae, vae.dec_norm.eps)
+        self._add_conv("in", vae.dec_in, 64)
+        self._add_res("mid", vae.dec_mid)
         self.ups: List[bool] = []
         for i, (blk, up) in enumerate(zip(vae.dec_blocks, vae.dec_up)):
-            res(f"b{i}", blk)
-            conv(f"u{i}", up.conv)
+            assert blk.skip is None
+            self._add_res(f"b{i}", blk)
+            self._add_conv(f"u{i}", up.conv)
             self.ups.append(up.temporal)
         self.g["out"] = vae.dec_norm.gamma.data.to(torch.bfloat16).contiguous()
         wo = vae.dec_out.weight.data  # [3, 64, 3, 3, 3]
         assert wo.shape[0] == 3 and wo.shape[1] == 64, "the RGB head expects 64 input channels"
-        self.w_out = wo.permute(0, 2, 3, 4, 1).reshape(3, 27, 64).float().contiguous()
+        self.w_out = _bf16_terms(wo.permute(0, 2, 3, 4, 1).reshape(3, 27 * 64))
         self.b_out = vae.dec_out.bias.data.float().contiguous()
-        self.eps = vae.dec_norm.eps
-
-    # ------------------------------------------------------------------ building blocks
-    def _ctx(self, cache: Dict, key: str, vol: torch.Tensor) -> None:
-        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail."""
-        if key in cache:
-            vol[:TPAD].copy_(cache[key])
-        else:
-            vol[:TPAD].zero_()
-        cache[key] = vol[-TPAD:].clone()
-
-    def _conv(self, cache, name, vol, resid=None):
-        self._ctx(cache, name, vol)
-        out = torch.zeros(vol.shape[0], vol.shape[1], vol.shape[2], self.w[name].shape[0], dtype=torch.bfloat16,
-                          device=self.device)
-        torch.ops.cosmos_b200.conv3d_cl(vol, self.w[name], self.b[name], resid, out, TPAD)
-        return out
-
-    def _ns(self, vol, gamma):
-        return torch.ops.cosmos_b200.rmsnorm_silu(vol, gamma, self.eps)
-
-    def _res(self, cache, name, x):
-        h = self._conv(cache, name + ".c1", self._ns(x, self.g[name + ".n1"]))
-        return self._conv(cache, name + ".c2", self._ns(h, self.g[name + ".n2"]), resid=x)
-
-    def _up(self, cache, name, x, temporal, first):
-        t_src = x.shape[0] - TPAD
-        t_dst = (2 * t_src - 1 if first else 2 * t_src) if temporal else t_src
-        hs, ws = x.shape[1] - 2, x.shape[2] - 2
-        dst = torch.zeros(t_dst + TPAD, 2 * hs + 2, 2 * ws + 2, x.shape[3], dtype=torch.bfloat16, device=self.device)
-        torch.ops.cosmos_b200.upsample_cl(x, dst, TPAD, temporal, first)
-        return self._conv(cache, name, dst)
 
     # ------------------------------------------------------------------ public
     @torch.no_grad()
@@ -103,14 +125,18 @@ class CLDecoder:
         c, tc, h, w = z.shape
         vol = torch.zeros(tc + TPAD, h + 2, w + 2, 64, dtype=torch.bfloat16, device=self.device)
         vol[TPAD:, 1:-1, 1:-1, :c] = z.permute(1, 2, 3, 0).to(torch.bfloat16)
-        x = self._conv(cache, "in", vol)
-        x = self._res(cache, "mid", x)
+        x, n = self._conv(cache, "in", vol, norm=self.g["mid.n1"])
+        _, n = self._conv(cache, "mid.c1", n, norm=self.g["mid.n2"], raw=False)
+        x, n = self._conv(cache, "mid.c2", n, resid=x, norm=self.g["b0.n1"])
+        last = len(self.ups) - 1
         for i, temporal in enumerate(self.ups):
-            x = self._res(cache, f"b{i}", x)
-            x = self._up(cache, f"u{i}", x, temporal, first)
-        x = self._ns(x, self.g["out"])
-        self._ctx(cache, "out", x)
-        return torch.ops.cosmos_b200.conv_out_rgb(x, self.w_out, self.b_out)
+            _, n = self._conv(cache, f"b{i}.c1", n, norm=self.g[f"b{i}.n2"], raw=False)
+            if temporal:
+                tc = 2 * tc - 1 if first else 2 * tc
+            x, _ = self._conv(cache, f"b{i}.c2", n, resid=x, mode=UP, a=int(temporal), b=int(first), frames=tc)
+            x, n = self._conv(cache, f"u{i}", x, norm=self.g["out" if i == last else f"b{i + 1}.n1"], raw=i < last)
+        self._ctx(cache, "out", n)
+        return torch.ops.cosmos_b200.conv3d_rgb(n, self.w_out, self.b_out)
 
     @torch.no_grad()
     def decode(self, z: torch.Tensor, chunk_latents: int = 2) -> torch.Tensor:
@@ -131,106 +157,80 @@ def even_frames(t0: int, n: int):
     return first, max(0, (n - first + 1) // 2), (t0 + 1) // 2
 
 
-class CLEncoder:
-    """Tokenizer encoder on the same kernels as `CLDecoder`: padded channels-last volumes, every 3x3x3 causal
-    convolution an implicit GEMM on the tensor cores, channel RMS-norm + SiLU as a bandwidth kernel.
+class CLEncoder(_CLConvs):
+    """Tokenizer encoder on the same kernel as `CLDecoder`.
 
-    * A strided convolution (the three down-sampling steps: stride 2 in space, the last two also in time) is the
-      stride-1 convolution evaluated everywhere followed by a strided copy of its even positions: causal padding
-      in time and `k // 2` padding in space make output (j, i) of the strided form equal output (2j, 2i) of the
-      stride-1 form. The tensor cores do 4x / 8x the minimal work on those three layers (about a third of the
-      encoder's FLOPs at 720p) in exchange for one kernel for every convolution.
-    * The 1x1x1 skip projections of the widening blocks are plain GEMMs over all positions of the padded volume;
-      the border positions (which must stay zero, they are the next convolution's padding) are cleared afterwards.
-    * The RGB input is padded to 64 channels.
+    * A strided convolution (the three down-sampling steps: stride 2 in space, the last two also in time) computes the kept
+      positions and frames alone. It reads its input split by the parity of row and column, which the block before it writes;
+      causal padding in time and `k // 2` padding in space make output (j, i) of the strided form the stride-1 form's
+      (2j, 2i).
+    * The 1x1x1 skip projections of the widening blocks are further columns of the block's second convolution: its sum runs
+      over the 27 taps of its own input and then over the channels of the block's input.
+    * The first layer's 9 spatial taps x 3 colours are packed into the 64 channels of an operand row.
 
     Frames are encoded in temporal chunks (the first frame alone, then `chunk_frames` at a time); each
     convolution's two context frames are carried over, so the result equals one pass over the clip.
     Reference behaviour: the tokenizer's causal encoder, cosmos_framework/inference (Wan2.2-style 4x8x8 VAE)."""
 
     def __init__(self, vae: CausalVideoVAE):
-        dev = next(vae.parameters()).device
-        assert dev.type == "cuda", "the channels-last encoder runs on CUDA"
-        self.device = dev
-        self.latent_channels = vae.latent_channels
-        self.w: Dict[str, torch.Tensor] = {}
-        self.b: Dict[str, torch.Tensor] = {}
-        self.g: Dict[str, torch.Tensor] = {}
-        self.eps = vae.enc_norm.eps
-
-        def conv(name, m, cin_pad=None):
-            assert m.k == (3, 3, 3)
-            cp = cin_pad or m.weight.shape[1]
-            assert cp % 64 == 0 and m.weight.shape[0] % 32 == 0, "channel widths must be multiples of 64"
-            self.w[name] = _pack_weight(m.weight.data, cp)
-            self.b[name] = m.bias.data.to(torch.bfloat16).contiguous()
+        super().__init__(vae, vae.enc_norm.eps)
+        w = vae.enc_in.weight.data   # [C, 3, 3, 3, 3]
+        assert vae.enc_in.k == (3, 3, 3) and w.shape[1] == 3 and w.shape[0] % 64 == 0, "channel widths must be multiples of 64"
+        p = torch.zeros(w.shape[0], 3, 64, dtype=torch.bfloat16, device=self.device)
+        p[:, :, :27] = w.permute(0, 2, 3, 4, 1).reshape(w.shape[0], 3, 27).to(torch.bfloat16)
+        self.w["in"] = p.reshape(w.shape[0], 192)
+        self.b["in"] = vae.enc_in.bias.data.float().contiguous()
+        self.downs: List[bool] = []
+        self.skips: Dict[str, bool] = {}
 
         def res(name, blk: ResBlock):
-            self.g[name + ".n1"] = blk.n1.gamma.data.to(torch.bfloat16).contiguous()
-            self.g[name + ".n2"] = blk.n2.gamma.data.to(torch.bfloat16).contiguous()
-            conv(name + ".c1", blk.c1)
-            conv(name + ".c2", blk.c2)
+            self._add_res(name, blk)
+            self.skips[name] = blk.skip is not None
             if blk.skip is not None:
-                self.w[name + ".skip"] = blk.skip.weight.data.reshape(blk.skip.weight.shape[0], -1).to(torch.bfloat16).contiguous()
-                self.b[name + ".skip"] = blk.skip.bias.data.to(torch.bfloat16).contiguous()
+                sw = blk.skip.weight.data.reshape(blk.skip.weight.shape[0], -1).to(torch.bfloat16)
+                self.w[name + ".c2"] = torch.cat([self.w[name + ".c2"], sw], dim=1).contiguous()
+                self.b[name + ".c2"] = blk.c2.bias.data.float() + blk.skip.bias.data.float()
 
-        conv("in", vae.enc_in, 64)
-        self.downs: List[bool] = []
         for i, (blk, down) in enumerate(zip(vae.enc_blocks, vae.enc_down)):
             res(f"b{i}", blk)
-            conv(f"d{i}", down.conv)
+            self._add_conv(f"d{i}", down.conv)
             assert down.conv.stride[1:] == (2, 2)
             self.downs.append(down.conv.stride[0] == 2)
         res("mid", vae.enc_mid)
         self.g["out"] = vae.enc_norm.gamma.data.to(torch.bfloat16).contiguous()
-        conv("out", vae.enc_out)
+        self._add_conv("out", vae.enc_out)
 
-    _ctx = CLDecoder._ctx
-    _ns = CLDecoder._ns
-
-    def _conv(self, cache, name, vol, resid=None):
-        self._ctx(cache, name, vol)
-        out = torch.zeros(vol.shape[0], vol.shape[1], vol.shape[2], self.w[name].shape[0], dtype=torch.bfloat16,
-                          device=self.device)
-        torch.ops.cosmos_b200.conv3d_cl(vol, self.w[name], self.b[name], resid, out, TPAD)
-        return out
-
-    def _res(self, cache, name, x):
-        h = self._conv(cache, name + ".c1", self._ns(x, self.g[name + ".n1"]))
-        if name + ".skip" in self.w:
-            from .. import ops
-            w = self.w[name + ".skip"]
-            r = ops.gemm(x.view(-1, x.shape[-1]), w, bias=self.b[name + ".skip"]).view(*x.shape[:3], w.shape[0])
-            r[:, 0].zero_(); r[:, -1].zero_(); r[:, :, 0].zero_(); r[:, :, -1].zero_()   # the padding ring stays zero
-        else:
-            r = x
-        return self._conv(cache, name + ".c2", self._ns(h, self.g[name + ".n2"]), resid=r)
-
-    def _down(self, cache, name, x, temporal: bool, t0: int):
-        """Stride-1 convolution, then the even positions. `t0`: index of the chunk's first frame in this level's
-        timeline (temporal steps keep the frames with an even index)."""
-        y = self._conv(cache, name, x)
-        body = y[TPAD:]
-        if temporal:
-            first, _, t0 = even_frames(t0, body.shape[0])
-            body = body[first::2]
-        hs, ws = (x.shape[1] - 2) // 2, (x.shape[2] - 2) // 2
-        dst = torch.zeros(body.shape[0] + TPAD, hs + 2, ws + 2, y.shape[3], dtype=torch.bfloat16, device=self.device)
-        dst[TPAD:, 1:-1, 1:-1] = body[:, 1:-1:2, 1:-1:2]
-        return dst, t0
+    def _res(self, cache, name, x, n, **kw):
+        """One residual block; x: its input, n: silu(rmsnorm(x))."""
+        _, n = self._conv(cache, name + ".c1", n, norm=self.g[name + ".n2"], raw=False)
+        return self._conv(cache, name + ".c2", n, **({"skip": x} if self.skips[name] else {"resid": x}), **kw)
 
     @torch.no_grad()
     def encode_chunk(self, frames: torch.Tensor, cache: Dict, t0: int) -> torch.Tensor:
         """frames [3, n, H, W] in [-1, 1] (global index of the first one: t0) -> moments [2C, n', H/8, W/8] fp32."""
-        c, n, h, w = frames.shape
-        vol = torch.zeros(n + TPAD, h + 2, w + 2, 64, dtype=torch.bfloat16, device=self.device)
-        vol[TPAD:, 1:-1, 1:-1, :c] = frames.permute(1, 2, 3, 0).to(torch.bfloat16)
-        x = self._conv(cache, "in", vol)
+        _, n, h, w = frames.shape
+        if frames.dtype not in (torch.float32, torch.bfloat16):
+            frames = frames.float()
+        if frames.stride(3) != 1 or frames.stride(2) != w or (n > 1 and frames.stride(1) != h * w):
+            frames = frames.contiguous()
+        vol = self._empty(n + TPAD, h + 2, w + 2, 64)
+        torch.ops.cosmos_b200.conv_pack_rgb(frames, vol)
+        x, y = self._conv(cache, "in", vol, norm=self.g["b0.n1"])
+        last = len(self.downs) - 1
         for i, temporal in enumerate(self.downs):
-            x = self._res(cache, f"b{i}", x)
-            x, t0 = self._down(cache, f"d{i}", x, temporal, t0)
-        x = self._res(cache, "mid", x)
-        y = self._conv(cache, "out", self._ns(x, self.g["out"]))
+            x, _ = self._res(cache, f"b{i}", x, y, mode=S2D)
+            first, step, kept = 0, 1, n
+            if temporal:
+                first, kept, t0 = even_frames(t0, n)
+                step = 2
+            if kept == 0:   # an odd frame alone: nothing of it is kept, but the next chunk needs it as context
+                self._ctx(cache, f"d{i}", x, 1)
+                return torch.empty(2 * self.latent_channels, 0, h // 8, w // 8, device=self.device)
+            x, y = self._conv(cache, f"d{i}", x, norm=self.g["mid.n1" if i == last else f"b{i + 1}.n1"], mode=DOWN, a=first,
+                              b=step, frames=kept)
+            n = kept
+        _, y = self._res(cache, "mid", x, y, norm=self.g["out"], raw=False)
+        y, _ = self._conv(cache, "out", y)
         return y[TPAD:, 1:-1, 1:-1].permute(3, 0, 1, 2).float()
 
     @torch.no_grad()

@@ -773,10 +773,84 @@ int64_t paged_decode_pick_splits(int64_t B, int64_t Hkv, int64_t max_len, int64_
                    : cosmos::paged_decode_tc_pick_splits((int)B, (int)Hkv, (int)max_len);
 }
 
-// Causal 3x3x3 convolution as an implicit GEMM. x: padded channels-last volume [F, Hp, Wp, C]
-// (C % 64 == 0; F includes `tpad` = 2 leading context frames); w: [Cout, 27 * C]; out: a padded
-// volume [F, Hp, Wp, Cout] whose interior rows are written (border rows are left untouched);
-// resid (optional) has the layout of out and is added.
+// ---- convolutions of the tokenizer (conv_tcgen05.cu) ----
+void conv_bias(cosmos::ConvArgs& a, const OptT& bias, Tensor& keep) {
+  if (!bias.has_value() || !bias->defined()) return;
+  TORCH_CHECK(bias->is_cuda() && (bias->scalar_type() == at::kFloat || bias->scalar_type() == at::kBFloat16) &&
+              bias->numel() == a.n_out && bias->is_contiguous(), "bias: one value per output channel, fp32 or bf16");
+  keep = bias->to(at::kFloat);
+  a.bias = keep.data_ptr<float>();
+}
+
+// x: padded channels-last volume [F, Hp, Wp, C] (C % 64 == 0; F includes two context frames), mode 3: its s2d form [4, F,
+// Hp / 2, Wp / 2, C]; w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only); `out` / `out_norm`: outputs (at least
+// one) in the mode's layout, written from their third frame on, border included. (a, b): mode 2 temporal doubling and first
+// chunk, mode 3 first kept frame and frame step.
+void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& resid, const OptT& skip, const OptT& out,
+                  const OptT& out_norm, const OptT& gamma, double eps, int64_t mode, int64_t ma, int64_t mb) {
+  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(mode >= 0 && mode <= 3, "conv3d_fused: unknown mode");
+  const bool down = mode == cosmos::CONV_OUT_DOWN;
+  TORCH_CHECK(x.is_contiguous() && x.dim() == (down ? 5 : 4) && (!down || x.size(0) == 4), "x must be a contiguous volume");
+  cosmos::ConvArgs a;
+  const int64_t F = x.size(down ? 1 : 0), Hp = x.size(down ? 2 : 1) * (down ? 2 : 1), Wp = x.size(down ? 3 : 2) * (down ? 2 : 1);
+  const int64_t C = x.size(-1), Cout = w.size(0);
+  TORCH_CHECK(F > 2, "x needs two context frames and at least one more");
+  TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; use shorter temporal chunks");
+  a.x = x.data_ptr(); a.w = w.data_ptr();
+  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout; a.mode = (int)mode;
+  a.f_out = (int)F - 2;
+  Tensor bias_keep;
+  conv_bias(a, bias, bias_keep);
+  if (skip.has_value() && skip->defined()) {
+    check_bf16_cuda(*skip, "skip");
+    TORCH_CHECK(!down && skip->is_contiguous() && skip->dim() == 4 && skip->size(0) == F && skip->size(1) == Hp && skip->size(2) == Wp,
+                "skip must be a volume of x's size");
+    a.skip = skip->data_ptr(); a.skip_c = (int)skip->size(3);
+  }
+  TORCH_CHECK(w.dim() == 2 && w.is_contiguous(), "w must be a contiguous matrix");
+  a.taps_t_only = w.size(1) == 3 * C && !a.skip && !down;
+  TORCH_CHECK(a.taps_t_only || w.size(1) == 27 * C + a.skip_c, "w must be [Cout, 27 * C (+ skip channels)] or [Cout, 3 * C]");
+  std::vector<int64_t> shape;
+  if (mode == cosmos::CONV_OUT_SAME) {
+    shape = {F, Hp, Wp, Cout};
+  } else if (mode == cosmos::CONV_OUT_S2D) {
+    shape = {4, F, Hp / 2, Wp / 2, Cout};
+  } else if (mode == cosmos::CONV_OUT_UP) {
+    a.up_temporal = ma != 0; a.up_first = mb != 0;
+    shape = {2 + (ma ? 2 * (F - 2) - (mb ? 1 : 0) : F - 2), 2 * (Hp - 2) + 2, 2 * (Wp - 2) + 2, Cout};
+  } else {
+    TORCH_CHECK(ma >= 0 && mb >= 1, "conv3d_fused: bad kept frames");
+    a.t_first = (int)ma; a.t_step = (int)mb;
+    a.f_out = ma < F - 2 ? (int)((F - 2 - ma + mb - 1) / mb) : 0;
+    shape = {2 + a.f_out, Hp / 2 + 1, Wp / 2 + 1, Cout};
+  }
+  if (resid.has_value() && resid->defined()) {
+    check_bf16_cuda(*resid, "resid");
+    TORCH_CHECK(resid->is_contiguous() && resid->sizes() == at::IntArrayRef({F, Hp, Wp, Cout}), "resid must have x's padded size");
+    a.resid = resid->data_ptr();
+  }
+  auto output = [&](const OptT& t, const char* name) -> void* {
+    if (!t.has_value() || !t->defined()) return nullptr;
+    check_bf16_cuda(*t, name);
+    TORCH_CHECK(t->is_contiguous() && t->sizes() == at::IntArrayRef(shape), name, " has the wrong size for this mode");
+    return t->data_ptr();
+  };
+  a.out = output(out, "out");
+  a.out_norm = output(out_norm, "out_norm");
+  if (a.out_norm) {
+    TORCH_CHECK(gamma.has_value() && gamma->defined(), "the fused norm needs gamma");
+    check_bf16_cuda(*gamma, "gamma");
+    TORCH_CHECK(gamma->is_contiguous() && gamma->numel() == Cout && reinterpret_cast<uintptr_t>(gamma->data_ptr()) % 16 == 0, "gamma: one value per channel, 16-byte aligned");
+    a.gamma = gamma->data_ptr();
+  }
+  a.eps = (float)eps;
+  a.status = status_tensor(x.get_device()).data_ptr<int>();
+  cosmos::conv3d_fused(a, cur_stream());
+}
+
+// One convolution without fusions: out and resid [F, Hp, Wp, Cout]; frames from `tpad` on are written.
 void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& resid, Tensor out, int64_t tpad) {
   check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w"); check_bf16_cuda(out, "out");
   c10::cuda::CUDAGuard guard(x.device());
@@ -784,25 +858,53 @@ void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& r
   const int64_t F = x.size(0), Hp = x.size(1), Wp = x.size(2), C = x.size(3), Cout = out.size(3);
   TORCH_CHECK(out.size(0) == F && out.size(1) == Hp && out.size(2) == Wp, "out must have the padded shape of x");
   TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == Cout && w.size(1) == 27 * C, "w must be [Cout, 27 * C]");
-  TORCH_CHECK(F * Hp * Wp < (1ll << 31), "volume too large for 32-bit row indices; decode in temporal chunks");
-  cosmos::GemmArgs g;
-  g.A = x.data_ptr(); g.B = w.data_ptr(); g.C = out.data_ptr();
-  g.M = (int)(F * Hp * Wp); g.N = (int)Cout; g.K = (int)(27 * C);
-  g.lda = C; g.ldb = 27 * C; g.ldc = Cout;
-  g.epi = EPI_CONV;
-  g.conv_c = (int)C; g.conv_hp = (int)Hp; g.conv_wp = (int)Wp; g.conv_tpad = (int)tpad;
-  if (bias.has_value() && bias->defined()) {
-    check_bf16_cuda(*bias, "bias");
-    TORCH_CHECK(bias->numel() == Cout && bias->is_contiguous());
-    g.bias = bias->data_ptr();
-  }
+  TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
+  TORCH_CHECK(tpad >= 0, "tpad must not be negative");
+  cosmos::ConvArgs a;
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
+  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout;
+  a.tpad = (int)tpad; a.f_out = (int)std::max<int64_t>(0, F - tpad);
+  Tensor bias_keep;
+  conv_bias(a, bias, bias_keep);
   if (resid.has_value() && resid->defined()) {
     check_bf16_cuda(*resid, "resid");
     TORCH_CHECK(resid->is_contiguous() && resid->sizes() == out.sizes());
-    g.R = resid->data_ptr(); g.ldr = Cout;
+    a.resid = resid->data_ptr();
   }
-  g.status = status_tensor(x.get_device()).data_ptr<int>();
-  cosmos::gemm_bf16(g, cur_stream());
+  a.status = status_tensor(x.get_device()).data_ptr<int>();
+  cosmos::conv3d_fused(a, cur_stream());
+}
+
+// Last layer of the decoder with the conversion to pixels. x: [F, Hp, Wp, C]; w [9, 27 C]: row c + 3 i = term i of channel
+// c's weights; bias [3] fp32 -> uint8 [F - 2, Hp - 2, Wp - 2, 3] = round((clamp(y, -1, 1) + 1) 127.5)
+Tensor conv3d_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
+  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(0) > 2 && x.size(1) > 2 && x.size(2) > 2, "x must be a padded volume");
+  const int64_t F = x.size(0), Hp = x.size(1), Wp = x.size(2), C = x.size(3);
+  TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == 9 && w.size(1) == 27 * C, "w must be [9, 27 * C]");
+  TORCH_CHECK(bias.is_cuda() && bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.numel() == 3);
+  TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
+  Tensor out = at::empty({F - 2, Hp - 2, Wp - 2, 3}, x.options().dtype(at::kByte));
+  cosmos::ConvArgs a;
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.bias = bias.data_ptr<float>(); a.rgb = out.data_ptr();
+  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = 9; a.f_out = (int)F - 2;
+  a.status = status_tensor(x.get_device()).data_ptr<int>();
+  cosmos::conv3d_fused(a, cur_stream());
+  return out;
+}
+
+// frames [3, n, h, w] (fp32 or bf16; channel stride free, the rest dense) -> dst [2 + n, h + 2, w + 2, 64] from frame 2 on
+void conv_pack_rgb(const Tensor& frames, Tensor dst) {
+  check_bf16_cuda(dst, "dst");
+  c10::cuda::CUDAGuard guard(dst.device());
+  TORCH_CHECK(frames.is_cuda() && (frames.scalar_type() == at::kFloat || frames.scalar_type() == at::kBFloat16) &&
+              frames.dim() == 4 && frames.size(0) == 3, "frames must be [3, n, h, w], fp32 or bf16");
+  const int64_t n = frames.size(1), h = frames.size(2), w = frames.size(3);
+  TORCH_CHECK(frames.stride(3) == 1 && frames.stride(2) == w && (n == 1 || frames.stride(1) == h * w), "frames must be dense within a channel");
+  TORCH_CHECK(dst.is_contiguous() && dst.sizes() == at::IntArrayRef({n + 2, h + 2, w + 2, 64}), "dst must be [2 + n, h + 2, w + 2, 64]");
+  cosmos::conv_pack_rgb(frames.data_ptr(), frames.scalar_type() == at::kFloat, frames.stride(0), dst.data_ptr(), (int)n, (int)h,
+                        (int)w, cur_stream());
 }
 
 Tensor rmsnorm_silu(const Tensor& x, const Tensor& gamma, double eps) {
@@ -813,33 +915,6 @@ Tensor rmsnorm_silu(const Tensor& x, const Tensor& gamma, double eps) {
   cosmos::rmsnorm_silu(x.data_ptr(), gamma.data_ptr(), y.data_ptr(), x.numel() / x.size(-1), (int)x.size(-1),
                        (float)eps, cur_stream());
   return y;
-}
-
-void upsample_cl(const Tensor& src, Tensor dst, int64_t tpad, bool temporal, bool first_chunk) {
-  check_bf16_cuda(src, "src"); check_bf16_cuda(dst, "dst");
-  c10::cuda::CUDAGuard guard(src.device());
-  TORCH_CHECK(src.dim() == 4 && dst.dim() == 4 && src.is_contiguous() && dst.is_contiguous() && src.size(3) == dst.size(3));
-  const int64_t hs = src.size(1) - 2, ws = src.size(2) - 2;
-  TORCH_CHECK(dst.size(1) == 2 * hs + 2 && dst.size(2) == 2 * ws + 2, "dst must be the x2 padded volume");
-  const int64_t t_src = src.size(0) - tpad, t_dst = dst.size(0) - tpad;
-  const int64_t want = temporal ? (first_chunk ? 2 * t_src - 1 : 2 * t_src) : t_src;
-  TORCH_CHECK(t_dst == want, "dst frame count mismatch");
-  cosmos::upsample_cl(src.data_ptr(), dst.data_ptr(), (int)t_dst, (int)hs, (int)ws, (int)src.size(3), (int)tpad,
-                      temporal ? 1 : 0, first_chunk ? 1 : 0, cur_stream());
-}
-
-// x: padded CL volume [T + 2, H + 2, W + 2, 64]; w [3, 27, 64] fp32; bias [3] fp32 -> uint8 [T, H, W, 3]
-Tensor conv_out_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
-  check_bf16_cuda(x, "x");
-  c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(3) == 64, "x must be [T+2, H+2, W+2, 64]");
-  TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kFloat && w.is_contiguous() && w.numel() == 3 * 27 * 64);
-  TORCH_CHECK(bias.is_cuda() && bias.scalar_type() == at::kFloat && bias.numel() == 3);
-  const int64_t T = x.size(0) - 2, H = x.size(1) - 2, W = x.size(2) - 2;
-  Tensor out = at::empty({T, H, W, 3}, x.options().dtype(at::kByte));
-  cosmos::conv_out_rgb(x.data_ptr(), w.data_ptr<float>(), bias.data_ptr<float>(), out.data_ptr(), (int)T, (int)H,
-                       (int)W, cur_stream());
-  return out;
 }
 
 const long long* ptr_table(const Tensor& t, const char* name) {
@@ -1274,8 +1349,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("l2_flush_", &l2_flush_);
   m.def("conv3d_cl", &conv3d_cl);
   m.def("rmsnorm_silu", &rmsnorm_silu);
-  m.def("upsample_cl", &upsample_cl);
-  m.def("conv_out_rgb", &conv_out_rgb);
+  m.def("conv3d_fused", &conv3d_fused);
+  m.def("conv3d_rgb", &conv3d_rgb);
+  m.def("conv_pack_rgb", &conv_pack_rgb);
   m.def("paged_decode", &paged_decode);
   m.def("paged_decode_pick_splits", &paged_decode_pick_splits);
   m.def("comm_barrier", &comm_barrier);

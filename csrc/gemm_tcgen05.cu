@@ -48,7 +48,6 @@ template <int NC> struct GemmCfg {
 struct GemmParams {
   int M, N, K;
   int b_row1;            // row offset in B of the second 128-row half of the tile
-  int mma_n;             // N of the MMA instruction: BN, or 64 / 128 for a convolution with that few output channels
   int n_tiles, m_tiles;  // tile counts (n_tiles counts 256-wide (or 128-wide for SWIGLU) tiles)
   bf16* C;
   long long ldc;
@@ -79,10 +78,6 @@ struct GemmParams {
   // operand majors: 0 = K-major ([rows, K] storage), 1 = MN-major ([K, rows] storage, i.e. the
   // transposed operand is read in place; used by the backward GEMMs dX = dY W and dW = dY^T X)
   int a_mn, b_mn;
-  // implicit-GEMM convolution (EPI_CONV)
-  int conv_cblocks;      // input channels / 64
-  int conv_hp, conv_wp, conv_tpad;
-  int conv_shift[27];    // row offset of each filter tap in the flattened padded volume
   // grouped by a tile map (see the file comment): {group, first row, rows, unused} per m-tile; tile rows = TILE_M
   const int4* tile_map;
   const int* n_tiles_m;  // number of m-tiles of this launch (device)
@@ -179,7 +174,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Weight prefetch (single-CTA tiles, B in its [N, K] layout): the B halves of the first tile's first stages are
     // requested here, while warp 1 still allocates tensor memory and before the dependency wait of a programmatic
     // launch; their A halves follow in the producer loop. A stage's full barrier completes when both have landed.
-    if (NC == 1 && EPI != EPI_CONV && first_tile < total_tiles && first_tile < tiles0 && !g.p[0].b_mn &&
+    if (NC == 1 && first_tile < total_tiles && first_tile < tiles0 && !g.p[0].b_mn &&
         !g.p[0].debug && !g.p[0].tile_map) {
       const GemmParams& p = g.p[0];
       const int k_blocks = (p.K + BK - 1) / BK;
@@ -260,10 +255,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // both CTAs' bytes are counted on the leader's barrier, which expects the pair's total
             const uint32_t fb = mapa(full_bar(s), 0);
             if (cta_rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * STAGE_BYTES);
-            if constexpr (EPI == EPI_CONV) {
-              const int tap = kb / p.conv_cblocks;
-              tma_load_2d_pair(sa, mA, fb, (kb - tap * p.conv_cblocks) * BK, m0 + p.conv_shift[tap]);
-            } else if (p.a_mn) {
+            if (p.a_mn) {
               tma_load_2d_pair(sa, mA, fb, m0, kb * BK);
               tma_load_2d_pair(sa + A_BYTES / 2, mA, fb, m0 + 64, kb * BK);
             } else {
@@ -279,10 +271,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             continue;
           }
           mbar_arrive_expect_tx(full_bar(s), STAGE_BYTES);
-          if constexpr (EPI == EPI_CONV) {
-            const int tap = kb / p.conv_cblocks;
-            tma_load_2d(sa, mA, full_bar(s), (kb - tap * p.conv_cblocks) * BK, m0 + p.conv_shift[tap]);
-          } else if (p.a_mn) {
+          if (p.a_mn) {
             tma_load_2d(sa, mA, full_bar(s), m0, kb * BK);
             tma_load_2d(sa + A_BYTES / 2, mA, full_bar(s), m0 + 64, kb * BK);
           } else {
@@ -333,7 +322,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + b * BN;
         const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
-        const uint32_t idesc = make_idesc_bf16(TILE_M, p.mma_n, p.a_mn, p.b_mn);
+        const uint32_t idesc = make_idesc_bf16(TILE_M, BN, p.a_mn, p.b_mn);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -586,54 +575,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 if (n + i < p.N) dst[i] = __float2bfloat16(f[i]);
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_CONV) {
-        const int plane = p.conv_hp * p.conv_wp;
-        const int frame = m / plane;
-        const int rem = m - frame * plane;
-        const int hh = rem / p.conv_wp, ww = rem - hh * p.conv_wp;
-        const bool interior = row_ok && frame >= p.conv_tpad && hh >= 1 && hh <= p.conv_hp - 2 && ww >= 1 &&
-                              ww <= p.conv_wp - 2;
-        const int n0 = tn * BN;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          const int n = n0 + c;
-          if (n >= p.N) break;  // uniform across the warp
-          uint32_t v[32];
-          tmem_ld32(t_addr + c, v);
-          tmem_wait_ld();
-          if (interior) {
-            float f[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
-            if (p.bias) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) f[i] += __bfloat162float(p.bias[n + i]);
-            }
-            if (p.R) {
-              const uint4* r4 = reinterpret_cast<const uint4*>(p.R + (long long)m * p.ldr + n);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const uint4 rv = r4[q];
-                const uint32_t ru[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  f[q * 8 + e * 2] += bf16lo(ru[e]);
-                  f[q * 8 + e * 2 + 1] += bf16hi(ru[e]);
-                }
-              }
-            }
-            uint4* d4 = reinterpret_cast<uint4*>(p.C + (long long)m * p.ldc + n);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 o;
-              o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
-              o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
-              o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
-              o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
-              d4[q] = o;
             }
           }
         }
@@ -1026,7 +967,6 @@ static void launch_epi(int epi, const CUtensorMap* maps, const cb::GemmGroup& g,
     case EPI_SWIGLU: launch<EPI_SWIGLU, NC>(maps, g, units, limit, stream); break;
     case EPI_GATED_RESID: launch<EPI_GATED_RESID, NC>(maps, g, units, limit, stream); break;
     case EPI_QKV_ROPE: launch<EPI_QKV_ROPE, NC>(maps, g, units, limit, stream); break;
-    case EPI_CONV: launch<EPI_CONV, NC>(maps, g, units, limit, stream); break;
     case EPI_ATTN_P: launch<EPI_ATTN_P, NC>(maps, g, units, limit, stream); break;
     case EPI_ATTN_DS: launch<EPI_ATTN_DS, NC>(maps, g, units, limit, stream); break;
     default: throw std::runtime_error("gemm_bf16: unknown epilogue");
@@ -1041,22 +981,15 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
     throw std::runtime_error("gemm_bf16: SwiGLU epilogue needs N/2 to be a multiple of 8");
   if (a.epi == EPI_QKV_ROPE && a.N % 128 != 0)
     throw std::runtime_error("gemm_bf16: QKV epilogue needs N to be a multiple of 128");
-  if ((a.epi == EPI_PLAIN || a.epi == EPI_GELU || a.epi == EPI_GATED_RESID || a.epi == EPI_CONV) && (a.ldc % 8 != 0))
+  if ((a.epi == EPI_PLAIN || a.epi == EPI_GELU || a.epi == EPI_GATED_RESID) && (a.ldc % 8 != 0))
     throw std::runtime_error("gemm_bf16: ldc must be a multiple of 8");
-  if (a.epi == EPI_CONV) {
-    if (a.conv_c <= 0 || a.conv_c % 64 != 0 || a.K != 27 * a.conv_c || a.N % 32 != 0 || a.conv_hp < 3 ||
-        a.conv_wp < 3 || a.ldc % 8 != 0)
-      throw std::runtime_error("gemm_bf16: conv needs C % 64 == 0, K == 27 * C, Cout % 32 == 0 and a padded volume");
-  }
-  // for the convolution the A matrix is the [rows, C] volume; the K loop revisits it once per tap
-  const uint64_t dimsA[2] = {(uint64_t)(a.epi == EPI_CONV ? a.conv_c : a.K), (uint64_t)a.M};
+  const uint64_t dimsA[2] = {(uint64_t)a.K, (uint64_t)a.M};
   const uint64_t strA[1] = {(uint64_t)a.lda * 2};
   const uint32_t boxA[2] = {cb::BK, cb::BM};
   const uint64_t dimsB[2] = {(uint64_t)a.K, (uint64_t)a.N * (uint64_t)(a.tile_map ? a.n_groups : 1)};
   const uint64_t strB[1] = {(uint64_t)a.ldb * 2};
   const uint32_t boxB[2] = {cb::BK, 128};
   if (a.a_mn) {
-    if (a.epi == EPI_CONV) throw std::runtime_error("gemm_bf16: the convolution needs a K-major A");
     const uint64_t d[2] = {(uint64_t)a.M, (uint64_t)a.K};
     const uint32_t bx[2] = {64, cb::BK};
     ta = cbh::make_tmap_bf16(a.A, 2, d, strA, bx, true);
@@ -1087,14 +1020,6 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
     p.n_tiles = (a.N + cb::BN - 1) / cb::BN;
     p.b_row1 = 128;
   }
-  p.mma_n = cb::BN;
-  if (a.epi == EPI_CONV && a.N <= 128) {
-    // a tokenizer layer with 64 or 128 output channels: a 256-column MMA would spend 3/4 or 1/2 of its cycles on
-    // zero rows of B. The tile keeps its layout (one n tile, accumulator columns 0 .. N - 1); a CTA pair splits
-    // the narrower B between its two CTAs.
-    p.mma_n = a.N <= 64 ? 64 : 128;
-    if (nc == 2) p.b_row1 = p.mma_n / 2;
-  }
   p.C = reinterpret_cast<bf16*>(a.C); p.ldc = a.ldc;
   p.bias = reinterpret_cast<const bf16*>(a.bias);
   p.R = reinterpret_cast<const bf16*>(a.R); p.ldr = a.ldr;
@@ -1116,15 +1041,6 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
         (a.epi != EPI_PLAIN && a.epi != EPI_GELU) || (long long)a.N * a.n_groups > 0x7fffffffll)
       throw std::runtime_error("gemm_bf16: bad tile-map launch");
     p.m_tiles = a.max_tiles_m;   // upper bound for the grid; the kernel reads the count
-  }
-  if (a.epi == EPI_CONV) {
-    p.conv_cblocks = a.conv_c / 64;
-    p.conv_hp = a.conv_hp; p.conv_wp = a.conv_wp; p.conv_tpad = a.conv_tpad;
-    int tap = 0;
-    for (int dt = 0; dt < 3; ++dt)
-      for (int dh = 0; dh < 3; ++dh)
-        for (int dw = 0; dw < 3; ++dw)
-          p.conv_shift[tap++] = (dt - 2) * a.conv_hp * a.conv_wp + (dh - 1) * a.conv_wp + (dw - 1);
   }
 }
 

@@ -9,7 +9,6 @@ enum GemmEpilogue : int {
   EPI_SWIGLU = 1,
   EPI_GATED_RESID = 2,
   EPI_QKV_ROPE = 3,
-  EPI_CONV = 4,  // implicit-GEMM causal 3x3x3 convolution on a zero-padded channels-last volume
   // attention backward (scores are materialised per head): C = exp(acc * scale - lse[m]) under the mask
   EPI_ATTN_P = 5,
   // C = P[m, n] * (acc - D[m]) * scale, with P passed as the residual operand
@@ -72,11 +71,6 @@ struct GemmArgs {
   const void* norm_gamma = nullptr;
   void* norm_out = nullptr;
   float norm_eps = 1e-6f;
-  // EPI_CONV: A is the padded input volume flattened to [frames * hp * wp, C] (C % 64 == 0), B the
-  // weights as [Cout, 27 * C] (tap-major: kt, kh, kw, then channel), K = 27 * C. Output rows are
-  // the same padded positions; only interior rows (frame >= conv_tpad, 1 <= h <= hp-2,
-  // 1 <= w <= wp-2) are written, so a zero border stays zero.
-  int conv_c = 0, conv_hp = 0, conv_wp = 0, conv_tpad = 0;
   // Grouped by a tile map (mixture of experts): A [M, K] holds its rows sorted by group, B [n_groups * N, K] the groups'
   // weights stacked, tile_map[max_tiles_m] (device int4: group, first row, rows, -) the m-tiles of tile_m (128 or 256)
   // rows, *n_tiles_m (device) how many of them there are. EPI_PLAIN / EPI_GELU only.
@@ -202,11 +196,34 @@ void l2_flush(void* buf, size_t bytes, cudaStream_t s);
 // y = silu(rmsnorm(x) * gamma) over rows of d channels (channels-last tokenizer activations)
 void rmsnorm_silu(const void* x, const void* gamma, void* y, long long rows, int d, float eps, cudaStream_t s);
 
-// ---- tokenizer decoder helpers on padded channels-last volumes (conv3d.cu) ----
-void upsample_cl(const void* src, void* dst, int t_dst, int hs, int ws, int c, int tpad, int temporal,
-                 int first_chunk, cudaStream_t s);
-void conv_out_rgb(const void* x, const float* wgt, const float* bias, void* out, int t_out, int h, int w,
-                  cudaStream_t s);
+// ---- causal 3x3x3 convolutions of the tokenizer on padded channels-last volumes (conv_tcgen05.cu) ----
+enum ConvOut : int {
+  CONV_OUT_SAME = 0,   // [tpad + f_out, hp, wp, n_out]
+  CONV_OUT_S2D = 1,    // [4, tpad + f_out, hp / 2, wp / 2, n_out]: parity of (row, column) of the padded volume first
+  CONV_OUT_UP = 2,     // nearest x2 in space (and in time): [tpad + frames, 2 (hp - 2) + 2, 2 (wp - 2) + 2, n_out]
+  CONV_OUT_DOWN = 3,   // stride 2: x in s2d form; kept frames t_first + i t_step; [tpad + f_out, hp / 2 + 1, wp / 2 + 1, n_out]
+};
+struct ConvArgs {
+  const void* x = nullptr;      // [frames_in, hp, wp, c] (CONV_OUT_DOWN: [4, frames_in, hp / 2, wp / 2, c])
+  const void* w = nullptr;      // [n_out, 27 c (+ skip_c)], tap-major; taps_t_only: [n_out, 3 c]
+  const float* bias = nullptr;  // [n_out]; pixels: [3]
+  const void* resid = nullptr;  // added; layout of a CONV_OUT_SAME output
+  const void* skip = nullptr;   // second input [frames_in, hp, wp, skip_c] of a 1x1x1 projection in the weights' last columns
+  void* out = nullptr;          // bf16 result (may be null)
+  void* out_norm = nullptr;     // silu(rmsnorm(bf16 result) * gamma) over 64, 128 or 256 channels, layout of out
+  const void* gamma = nullptr;
+  float eps = 1e-6f;
+  void* rgb = nullptr;          // uint8 [f_out, hp - 2, wp - 2, 3]; n_out = 9: rows of w = the 3 channels' weights in 3 bf16 terms
+  int mode = CONV_OUT_SAME;
+  int frames_in = 0, hp = 0, wp = 0, c = 0, skip_c = 0, n_out = 0, f_out = 0, tpad = 2;
+  int taps_t_only = 0;
+  int up_temporal = 0, up_first = 0;
+  int t_first = 0, t_step = 1;
+  int* status = nullptr;
+};
+void conv3d_fused(const ConvArgs& a, cudaStream_t s);
+// src [3, n, h, w] planes (fp32 or bf16) -> dst [2 + n, h + 2, w + 2, 64]: the 9 spatial taps x 3 channels as 27 channels
+void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, int n, int h, int w, cudaStream_t s);
 
 // ---- paged-KV decode attention (paged_decode.cu) ----
 struct PagedDecodeArgs {

@@ -936,3 +936,115 @@ def test_optimizer_list_kernels_match_the_definition(sizes, shift):
             for got, want in ((m[i], mr), (v[i], vr), (w[i], wr)):
                 assert (got.double() - want).abs().max() <= 1e-5 + 1e-5 * want.abs().max()
             assert torch.equal(p[i], w[i].bfloat16())
+
+
+def _volume(x):
+    """[C, T, H, W] -> zero-bordered channels-last volume behind two zero context frames."""
+    c, t, h, w = x.shape
+    vol = torch.zeros(t + 2, h + 2, w + 2, c, device=DEV, dtype=torch.bfloat16)
+    vol[2:, 1:-1, 1:-1] = x.permute(1, 2, 3, 0)
+    return vol
+
+
+@pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 6, 10), (2, 34, 62)])
+@pytest.mark.parametrize("cin,cout", [(64, 64), (64, 128), (128, 128), (256, 256), (320, 96), (128, 320)])
+def test_conv3d_fused_forms(cin, cout, t, h, w):
+    """Every layout a convolution writes, with residual, skip projection and norm, against fp64 convolutions of the same
+    bf16 inputs: volumes smaller than a tile and with a remainder, channels in several blocks and output tiles. Bound:
+    one bf16 rounding of the result (2^-9 relative), twice with the norm."""
+    import torch.nn.functional as F
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(cin + cout + t)
+    x = _rand(cin, t, h, w)
+    wt = _rand(cout, cin, 3, 3, 3, scale=1 / math.sqrt(27 * cin))
+    b = torch.randn(cout, device=DEV)
+    r, sk, sw = _rand(cout, t, h, w), _rand(64, t, h, w), _rand(cout, 64, scale=0.125)
+    g = (1 + 0.1 * torch.randn(cout, device=DEV)).bfloat16()
+    y = F.conv3d(F.pad(x[None].double(), (1, 1, 1, 1, 2, 0)), wt.double(), b.double())[0]
+    wp = wt.permute(0, 2, 3, 4, 1).reshape(cout, 27 * cin).contiguous()
+    vol = _volume(x)
+    nan = lambda *s: torch.full(s, float("nan"), device=DEV, dtype=torch.bfloat16)  # noqa: E731
+
+    def check(got, want, what, rel=2 ** -8):
+        got, want = got.double(), want.permute(1, 2, 3, 0)
+        assert (got - want).abs().max() <= rel * max(1.0, want.abs().max().item()), what
+
+    def norm(v):
+        v = v.bfloat16().double()
+        z = v * torch.rsqrt(v.square().mean(0, keepdim=True) + 1e-6) * g.double()[:, None, None, None]
+        return z * torch.sigmoid(z)
+
+    def border(v):
+        assert v[:, 0].abs().max() == 0 and v[:, -1].abs().max() == 0 and v[:, :, 0].abs().max() == 0 and v[:, :, -1].abs().max() == 0
+
+    fused = cout in (64, 128, 256)
+    out, on = nan(t + 2, h + 2, w + 2, cout), nan(t + 2, h + 2, w + 2, cout) if fused else None
+    k.conv3d_fused(vol, wp, b, _volume(r), None, out, on, g if fused else None, 1e-6, 0, 0, 0)
+    check(out[2:, 1:-1, 1:-1], y + r.double(), "residual")
+    border(out[2:])
+    assert out[:2].isnan().all()
+    if fused:
+        check(on[2:, 1:-1, 1:-1], norm(y + r.double()), "norm", 2 ** -6)
+        border(on[2:])
+        only = nan(*on.shape)
+        k.conv3d_fused(vol, wp, b, _volume(r), None, None, only, g, 1e-6, 0, 0, 0)
+        assert torch.equal(only[2:], on[2:])
+    # skip projection, s2d layout
+    s2d = nan(4, t + 2, h // 2 + 1, w // 2 + 1, cout)
+    k.conv3d_fused(vol, torch.cat([wp, sw], 1).contiguous(), b, None, _volume(sk), s2d, None, None, 1e-6, 1, 0, 0)
+    flat = torch.empty(t, h + 2, w + 2, cout, device=DEV, dtype=torch.bfloat16)
+    for i in range(4):
+        flat[:, i >> 1::2, i & 1::2] = s2d[i, 2:]
+    check(flat[:, 1:-1, 1:-1], y + torch.einsum("oc,cthw->othw", sw.double(), sk.double()), "skip")
+    border(flat)
+    # nearest upsampling
+    for tem, first in ((0, 0), (1, 0), (1, 1)):
+        want = y.repeat_interleave(2, 2).repeat_interleave(2, 3)
+        want = want.repeat_interleave(2, 1)[:, first:] if tem else want
+        up = nan(want.shape[1] + 2, 2 * h + 2, 2 * w + 2, cout)
+        k.conv3d_fused(vol, wp, b, None, None, up, None, None, 1e-6, 2, tem, first)
+        check(up[2:, 1:-1, 1:-1], want, "upsampling")
+        border(up[2:])
+    # stride 2 over the s2d form of the input
+    xs = torch.empty(4, t + 2, h // 2 + 1, w // 2 + 1, cin, device=DEV, dtype=torch.bfloat16)
+    for i in range(4):
+        xs[i] = vol[:, i >> 1::2, i & 1::2]
+    for first, step in ((0, 1), (0, 2), (1, 2)):
+        want = y[:, first::step, ::2, ::2]
+        if want.shape[1] == 0:
+            continue
+        down = nan(want.shape[1] + 2, h // 2 + 2, w // 2 + 2, cout)
+        dn = nan(*down.shape) if fused else None
+        k.conv3d_fused(xs, wp, b, None, None, down, dn, g if fused else None, 1e-6, 3, first, step)
+        check(down[2:, 1:-1, 1:-1], want, "stride 2")
+        border(down[2:])
+        if fused:
+            check(dn[2:, 1:-1, 1:-1], norm(want), "stride 2, norm", 2 ** -6)
+            border(dn[2:])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 10, 22)])
+def test_conv3d_of_colours(dtype, t, h, w):
+    """First layer of the encoder (packed taps) and last layer of the decoder (fp32 weights in three bf16 terms)."""
+    import torch.nn.functional as F
+    from cosmos_b200.models.vae_cuda import _bf16_terms
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(t)
+    src = torch.randn(3, t + 1, h, w, device=DEV).to(dtype)[:, 1:]      # channel stride of a slice
+    wt = _rand(64, 3, 3, 3, 3, scale=1 / 9)
+    p = torch.zeros(64, 3, 64, device=DEV, dtype=torch.bfloat16)
+    p[:, :, :27] = wt.permute(0, 2, 3, 4, 1).reshape(64, 3, 27)
+    vol = torch.zeros(t + 2, h + 2, w + 2, 64, device=DEV, dtype=torch.bfloat16)
+    k.conv_pack_rgb(src, vol)
+    out = torch.empty(t + 2, h + 2, w + 2, 64, device=DEV, dtype=torch.bfloat16)
+    k.conv3d_fused(vol, p.view(64, 192), None, None, None, out, None, None, 1e-6, 0, 0, 0)
+    want = F.conv3d(F.pad(src.bfloat16()[None].double(), (1, 1, 1, 1, 2, 0)), wt.double())[0].permute(1, 2, 3, 0)
+    assert (out[2:, 1:-1, 1:-1].double() - want).abs().max() <= 2 ** -8 * max(1.0, want.abs().max().item())
+    x, wo, b = _rand(64, t, h, w), torch.randn(3, 64, 3, 3, 3, device=DEV) / 40, torch.randn(3, device=DEV) * 0.1
+    terms = _bf16_terms(wo.permute(0, 2, 3, 4, 1).reshape(3, 27 * 64))
+    assert torch.equal(terms.float().view(3, 3, -1).sum(0), wo.permute(0, 2, 3, 4, 1).reshape(3, -1))
+    got = k.conv3d_rgb(_volume(x), terms, b)
+    y = F.conv3d(F.pad(x[None].double(), (1, 1, 1, 1, 2, 0)), wo.double(), b.double())[0]
+    pix = ((y.clamp(-1, 1) + 1) * 127.5).permute(1, 2, 3, 0)
+    assert (got.double() - pix).abs().max() <= 0.5 + 1e-3      # rounding, and fp32 sums of 1728 products below 4
