@@ -63,14 +63,14 @@ class _CLConvs:
         self._add_conv(name + ".c2", blk.c2)
 
     # ------------------------------------------------------------------ launches
-    def _ctx(self, cache: Dict, key: str, vol: torch.Tensor, dim: int = 0) -> None:
-        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail."""
-        head = vol.narrow(dim, 0, TPAD)
+    def _ctx(self, cache: Dict, key: str, vol: torch.Tensor) -> None:
+        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail (a view: nothing writes
+        a volume again once the next chunk has begun, and it is let go when that one takes its place)."""
         if key in cache:
-            head.copy_(cache[key])
+            vol[:TPAD].copy_(cache[key])
         else:
-            head.zero_()
-        cache[key] = vol.narrow(dim, vol.shape[dim] - TPAD, TPAD).clone()
+            vol[:TPAD].zero_()
+        cache[key] = vol[-TPAD:]
 
     def _empty(self, *shape) -> torch.Tensor:
         return torch.empty(*shape, dtype=torch.bfloat16, device=self.device)
@@ -80,13 +80,13 @@ class _CLConvs:
               ) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
         """One convolution of `x` (context frames filled in here). Returns (result, silu(rmsnorm(result) * norm)); `raw`
         False: the first is not wanted. `mode`, `a`, `b`: the layout written (`ops.conv3d_fused`); `frames`: its frame count."""
-        self._ctx(cache, name, x, 1 if mode == DOWN else 0)
+        self._ctx(cache, name, x)
         w = self.w[name]
         cout = w.shape[0]
         if mode == DOWN:
             shape = (frames + TPAD, x.shape[2] + 1, x.shape[3] + 1, cout)
         elif mode == S2D:
-            shape = (4, x.shape[0], x.shape[1] // 2, x.shape[2] // 2, cout)
+            shape = (x.shape[0], 4, x.shape[1] // 2, x.shape[2] // 2, cout)
         elif mode == UP:
             shape = (frames + TPAD, 2 * x.shape[1] - 2, 2 * x.shape[2] - 2, cout)
         else:
@@ -147,6 +147,42 @@ class CLDecoder(_CLConvs):
         for s in range(0, z.shape[2], chunk_latents):
             outs.append(self.decode_chunk(z[0, :, s:s + chunk_latents], cache, s == 0))
         return torch.cat(outs, dim=0)[None]
+
+    @torch.no_grad()
+    def decode_to_host(self, z: torch.Tensor, chunk_latents: int = 2) -> torch.Tensor:
+        """`decode` with the frames on the host: a chunk's frames go through one of two pinned buffers on a stream of their
+        own and from there into the result while the next chunk is computed."""
+        assert z.shape[0] == 1
+        t = z.shape[2]
+        out = torch.empty(1 + 4 * (t - 1), 8 * z.shape[3], 8 * z.shape[4], 3, dtype=torch.uint8)
+        stage = [torch.empty(min(4 * chunk_latents, out.shape[0]), *out.shape[1:], dtype=torch.uint8, pin_memory=True)
+                 for _ in range(2)]
+        cur, side = torch.cuda.current_stream(self.device), torch.cuda.Stream(self.device)
+        cache: Dict = {}
+        done, waiting = 0, []
+
+        def drain():
+            nonlocal done
+            ev, buf = waiting.pop(0)
+            ev.synchronize()
+            out[done:done + buf.shape[0]].copy_(buf)
+            done += buf.shape[0]
+
+        for i, s in enumerate(range(0, t, chunk_latents)):
+            frames = self.decode_chunk(z[0, :, s:s + chunk_latents], cache, s == 0)
+            buf = stage[i % 2][:frames.shape[0]]
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                buf.copy_(frames, non_blocking=True)
+                ev = torch.cuda.Event()
+                ev.record(side)
+            frames.record_stream(side)
+            waiting.append((ev, buf))
+            if len(waiting) == 2:   # the older buffer is free again before the next chunk asks for it
+                drain()
+        while waiting:
+            drain()
+        return out
 
 
 def even_frames(t0: int, n: int):
@@ -224,7 +260,7 @@ class CLEncoder(_CLConvs):
                 first, kept, t0 = even_frames(t0, n)
                 step = 2
             if kept == 0:   # an odd frame alone: nothing of it is kept, but the next chunk needs it as context
-                self._ctx(cache, f"d{i}", x, 1)
+                self._ctx(cache, f"d{i}", x)
                 return torch.empty(2 * self.latent_channels, 0, h // 8, w // 8, device=self.device)
             x, y = self._conv(cache, f"d{i}", x, norm=self.g["mid.n1" if i == last else f"b{i + 1}.n1"], mode=DOWN, a=first,
                               b=step, frames=kept)

@@ -779,10 +779,11 @@ void conv_bias(cosmos::ConvArgs& a, const OptT& bias, Tensor& keep) {
   TORCH_CHECK(bias->is_cuda() && (bias->scalar_type() == at::kFloat || bias->scalar_type() == at::kBFloat16) &&
               bias->numel() == a.n_out && bias->is_contiguous(), "bias: one value per output channel, fp32 or bf16");
   keep = bias->to(at::kFloat);
+  if (reinterpret_cast<uintptr_t>(keep.data_ptr()) % 16) keep = keep.clone();   // read in 16-byte vectors
   a.bias = keep.data_ptr<float>();
 }
 
-// x: padded channels-last volume [F, Hp, Wp, C] (C % 64 == 0; F includes two context frames), mode 3: its s2d form [4, F,
+// x: padded channels-last volume [F, Hp, Wp, C] (C % 64 == 0; F includes two context frames), mode 3: its s2d form [F, 4,
 // Hp / 2, Wp / 2, C]; w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only); `out` / `out_norm`: outputs (at least
 // one) in the mode's layout, written from their third frame on, border included. (a, b): mode 2 temporal doubling and first
 // chunk, mode 3 first kept frame and frame step.
@@ -792,9 +793,9 @@ void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(mode >= 0 && mode <= 3, "conv3d_fused: unknown mode");
   const bool down = mode == cosmos::CONV_OUT_DOWN;
-  TORCH_CHECK(x.is_contiguous() && x.dim() == (down ? 5 : 4) && (!down || x.size(0) == 4), "x must be a contiguous volume");
+  TORCH_CHECK(x.is_contiguous() && x.dim() == (down ? 5 : 4) && (!down || x.size(1) == 4), "x must be a contiguous volume");
   cosmos::ConvArgs a;
-  const int64_t F = x.size(down ? 1 : 0), Hp = x.size(down ? 2 : 1) * (down ? 2 : 1), Wp = x.size(down ? 3 : 2) * (down ? 2 : 1);
+  const int64_t F = x.size(0), Hp = x.size(down ? 2 : 1) * (down ? 2 : 1), Wp = x.size(down ? 3 : 2) * (down ? 2 : 1);
   const int64_t C = x.size(-1), Cout = w.size(0);
   TORCH_CHECK(F > 2, "x needs two context frames and at least one more");
   TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; use shorter temporal chunks");
@@ -816,7 +817,7 @@ void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT
   if (mode == cosmos::CONV_OUT_SAME) {
     shape = {F, Hp, Wp, Cout};
   } else if (mode == cosmos::CONV_OUT_S2D) {
-    shape = {4, F, Hp / 2, Wp / 2, Cout};
+    shape = {F, 4, Hp / 2, Wp / 2, Cout};
   } else if (mode == cosmos::CONV_OUT_UP) {
     a.up_temporal = ma != 0; a.up_first = mb != 0;
     shape = {2 + (ma ? 2 * (F - 2) - (mb ? 1 : 0) : F - 2), 2 * (Hp - 2) + 2, 2 * (Wp - 2) + 2, Cout};

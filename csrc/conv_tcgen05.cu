@@ -13,7 +13,7 @@
 //     activation tile for three.
 // Per 64 channels and tap a CTA of the pair stages 5.7 + 8 KB in place of 32 KB at 128 output channels.
 //
-// A strided convolution reads its input split into the four parities of (row, column) ("s2d": [4, frames, (H + 2) / 2,
+// A strided convolution reads its input split into the four parities of (row, column) ("s2d": [frames, 4, (H + 2) / 2,
 // (W + 2) / 2, C]), which the layer before it writes; each tap is then again a row offset, taps of equal column parity share
 // a tile, and only the kept positions and frames are computed.
 //
@@ -21,6 +21,10 @@
 // x2 / x4 / x8 upsampling that the next convolution reads, and / or silu(rmsnorm(.)) over the channels (a thread holds a
 // whole row); or, for the 3 output channels of the decoder, uint8 pixels.
 //
+// Measured (480p, chunks of 8 frames at full resolution): 128 -> 128 channels with skip projection 1.95 ms = 1.47 PFLOP/s,
+// 256 -> 256 at half resolution 1.74 ms = 1.62, 128 -> 64 upsampled 1.57 ms = 0.90 (at 64 columns the reads of A from shared
+// memory bound the product). The one-tile-per-tap form with its separate passes took 48 ms a chunk of the encoder's
+// convolutions and norms where this takes 9.5.
 // Order of the sum: filter taps, then channel blocks of 64 (of up to 256 channels at a time). Waits are bounded as
 // everywhere (common.cuh).
 #include <algorithm>
@@ -31,12 +35,12 @@
 namespace cb {
 using namespace cosmos;   // ConvOut
 
-constexpr int CV_THREADS = 192;
 constexpr int CV_HALO_ROWS = 136;              // rows of the first box of a tile: 128 and the 2 rows that shifted taps need
 constexpr int CV_MAX_GROUPS = 18;
 constexpr int CV_CHUNK = 4;                    // channel blocks of 64 whose tiles are staged together
 constexpr int CV_SMEM_MAX = 227 * 1024;
 constexpr int CV_BARS = 512;                   // bytes for barriers, tensor-memory slot and abort flag
+constexpr int CV_SUMS = 8192;                  // row sums of the norm: [2 tiles][2 row tiles][2 column halves][128 rows][2] floats
 
 // Taps that read one staged tile: row offset of the tile, and per tap its shift inside the tile and its index in the weights.
 struct ConvGroup {
@@ -75,14 +79,26 @@ struct ConvCfg {
   static constexpr int A_ROWS = 128 * R + 8;
   static constexpr int A_SLOT = A_ROWS * 128;
   static constexpr int ACC_COLS = 256 / R;     // tensor-memory columns of one accumulator
+  static constexpr int THREADS = 64 + 256 * R; // producer, MMA issuer, eight epilogue warps per row tile
 };
 
-__device__ __forceinline__ void cv_store32(bf16* dst, const uint32_t (&pk)[16], int cols) {
-  if (cols >= 32) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      reinterpret_cast<uint4*>(dst)[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-  }
+__device__ __forceinline__ void cv_store16(bf16* dst, const uint32_t (&pk)[8]) {
+  reinterpret_cast<uint4*>(dst)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  reinterpret_cast<uint4*>(dst)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+}
+
+// Meeting of the two warps that share the rows of a quadrant; true when both say so.
+__device__ __forceinline__ bool cv_pair_and(int id, bool ok) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 q, %1, 0;\n\t"
+      "barrier.cta.red.and.pred p, %2, 64, q;\n\t"
+      "selp.s32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)
+      : "r"(ok ? 1 : 0), "r"(id)
+      : "memory");
+  return r != 0;
 }
 
 // Where a row of the result goes: `n_t` x `n_y` x `n_x` rows starting at `row` (one row except for the upsampled form).
@@ -97,7 +113,7 @@ __device__ __forceinline__ ConvDest conv_dest(const ConvParams& p, int f, int y,
     d.row = (long long)(f + p.tpad) * p.plane + y * p.pw + x;
   } else if (p.mode == CONV_OUT_S2D) {
     const int q = (p.hp >> 1) * (p.wp >> 1);
-    d.row = ((long long)((y & 1) * 2 + (x & 1)) * (p.f_out + p.tpad) + f + p.tpad) * q + (y >> 1) * (p.wp >> 1) + (x >> 1);
+    d.row = ((long long)(f + p.tpad) * 4 + (y & 1) * 2 + (x & 1)) * q + (y >> 1) * (p.wp >> 1) + (x >> 1);
   } else if (p.mode == CONV_OUT_DOWN) {
     d.row = ((long long)(f + p.tpad) * (p.hp + 1) + y + 1) * (p.wp + 1) + x + 1;
   } else {  // CONV_OUT_UP: interior position (y, x) -> rows 2y - 1, 2y and columns 2x - 1, 2x; the border stays one wide
@@ -117,19 +133,9 @@ __device__ __forceinline__ ConvDest conv_dest(const ConvParams& p, int f, int y,
   return d;
 }
 
-// Sum over the 8-element partial sums of a row in the order of a warp's butterfly (the separate norm kernel's order).
-template <int NV>
-__device__ __forceinline__ float conv_tree_sum(float (&s)[NV]) {
-#pragma unroll
-  for (int o = NV / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int i = 0; i < o; ++i) s[i] += s[i + o];
-  return s[0];
-}
-
 // R row tiles per CTA; NC = channels of the fused norm (64, 128, 256) or 0; RGB: pixels.
 template <int R, int NC, bool RGB>
-__global__ void __launch_bounds__(CV_THREADS, 1)
+__global__ void __launch_bounds__(ConvCfg<R>::THREADS, 1)
 conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
             const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmX2,
             const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ConvParams p) {
@@ -152,6 +158,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint8_t* gen = smem_raw + (tmem_slot - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 8);
+  float2* row_sums = reinterpret_cast<float2*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
 
   const uint32_t rank = cluster_ctarank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -161,7 +168,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (threadIdx.x == 0) {
     for (int s = 0; s < NA; ++s) { mbar_init(full_a(s), 1); mbar_init(empty_a(s), 1); }
     for (int s = 0; s < NB; ++s) { mbar_init(full_b(s), 1); mbar_init(empty_b(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 16 * R); }
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmA);
@@ -298,134 +305,169 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
     }
   } else {
-    // ---------------- epilogue warps 2..5; tensor-memory lane quadrant = warp % 4
-    const int quad = warp & 3;
+    // ---------------- epilogue: eight warps per row tile; tensor-memory lane quadrant = warp % 4, and the two warps of a
+    // quadrant take every other group of 16 columns. The loops over these groups stay rolled: unrolled over 256 columns the
+    // code left the instruction cache and a tile took 67 us. Latency bounds what is left (the divisions of the SiLU most of
+    // all, which are exact so that the result is the separate norm kernel's), hence the number of warps.
+    const int quad = warp & 3, half = ((warp - 2) >> 2) & 1, r = (warp - 2) >> 3;
+    const int pair_id = 1 + r * 4 + quad;
     int tcount = 0;
     for (int t = first_tile; t < total; t += tile_step, ++tcount) {
       const int buf = tcount & 1;
       const int nt = t % p.n_tiles, mt = t / p.n_tiles;
       const int seg = mt / p.tiles_per_seg, tile = mt - seg * p.tiles_per_seg;
-      if (!mbar_wait(tfull(buf), (tcount >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EPI)) break;
+      const int q = tile * TILE_M + int(rank) * (128 * R) + r * 128 + quad * 32 + lane;
+      const uint32_t ta = tmem_base + (uint32_t(quad * 32) << 16) + buf * 256 + r * Cfg::ACC_COLS;
+      const bool row_ok = q < p.seg_rows;
+      const int f0 = q / p.plane, rem = q - f0 * p.plane;
+      const int f = f0 + seg, y = rem / p.pw, x = rem - y * p.pw;   // several segments: one frame each
+      const bool down = p.mode == CONV_OUT_DOWN;
+      const bool inside = row_ok && (down ? (y < p.hp - 1 && x < p.wp - 1) : (y >= 1 && y <= p.hp - 2 && x >= 1 && x <= p.wp - 2));
+      bool go = mbar_wait(tfull(buf), (tcount >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EPI);
+      // warps that meet below leave together: a wait that one of them gave up is given up by both
+      go = NC > 0 ? cv_pair_and(pair_id, go) : __all_sync(0xffffffffu, go);
+      if (!go) break;
       tc_fence_after();
+      if constexpr (RGB) {
+        uint32_t v[16];
+        tmem_ld16(ta, v);
+        tmem_wait_ld();
+        if (inside && half == 0) {
+          uint8_t* o = p.rgb + (((long long)f * (p.hp - 2) + y - 1) * (p.wp - 2) + x - 1) * 3;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            // columns 3 .. 8: the low parts of fp32 weights, exact in three bf16 terms
+            const float a = ((__uint_as_float(v[6 + c]) + __uint_as_float(v[3 + c])) + __uint_as_float(v[c])) + p.bias[c];
+            o[c] = (uint8_t)__float2int_rn((fminf(fmaxf(a, -1.f), 1.f) + 1.f) * 127.5f);
+          }
+        }
+      } else {
+        const ConvDest dst = conv_dest(p, f, y, x);
+        const int n_base = nt * 256, n_end = min(256, p.n_out - n_base);
+        const long long ld = p.n_out;
+        if (down && row_ok && half == 0 && (x == 0 || y == 0)) {
+          // border cells that no position of the plane maps to: left column, top row
+          for (int k = 0; k < 3; ++k) {
+            if ((k == 0 && x != 0) || (k == 1 && y != 0) || (k == 2 && (x != 0 || y != 0))) continue;
+            const long long cell = dst.row - (k == 1 ? 0 : 1) - (k == 0 ? 0 : p.wp + 1);
+            for (int c = 0; c < n_end; c += 8) {
+              if (p.out) *reinterpret_cast<uint4*>(p.out + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+              if (p.out_norm) *reinterpret_cast<uint4*>(p.out_norm + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+            }
+          }
+        }
+        __syncwarp();
+        const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
+        // Squares are added per 8 channels and these sums in the order of a warp's butterfly: groups in bit-reversed order,
+        // summed like a binary counter.
+        float lvl[3][2], sum[2] = {0.f, 0.f};
+        const int groups = (NC > 0 ? NC : n_end) >> 5;   // of this warp
 #pragma unroll 1
-      for (int r = 0; r < R; ++r) {
-        const int q = tile * TILE_M + int(rank) * (128 * R) + r * 128 + quad * 32 + lane;
-        const uint32_t ta = tmem_base + (uint32_t(quad * 32) << 16) + buf * 256 + r * Cfg::ACC_COLS;
-        const bool row_ok = q < p.seg_rows;
-        const int f0 = q / p.plane, rem = q - f0 * p.plane;
-        const int f = f0 + seg, y = rem / p.pw, x = rem - y * p.pw;   // several segments: one frame each
-        const bool down = p.mode == CONV_OUT_DOWN;
-        const bool inside = down ? (y < p.hp - 1 && x < p.wp - 1) : (y >= 1 && y <= p.hp - 2 && x >= 1 && x <= p.wp - 2);
-        if constexpr (RGB) {
-          uint32_t v[32];
-          tmem_ld32(ta, v);
+        for (int i = 0; i < groups; ++i) {
+          const int ri = NC == 256 ? ((i & 1) << 2 | (i & 2) | i >> 2) : NC == 128 ? ((i & 1) << 1 | i >> 1) : i;
+          const int c = 32 * ri + 16 * half;
+          uint32_t v[16], pk[8];
+          tmem_ld16(ta + c, v);
+          uint4 ru[2];
+          if (res && inside) {
+            ru[0] = reinterpret_cast<const uint4*>(res + c)[0];
+            ru[1] = reinterpret_cast<const uint4*>(res + c)[1];
+          }
           tmem_wait_ld();
-          if (row_ok && inside) {
-            uint8_t* o = p.rgb + (((long long)f * (p.hp - 2) + y - 1) * (p.wp - 2) + x - 1) * 3;
+          if (inside) {
+            float a[16];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              // columns 3, 6 ..: the low parts of fp32 weights, exact in three bf16 terms
-              const float a = ((__uint_as_float(v[6 + c]) + __uint_as_float(v[3 + c])) + __uint_as_float(v[c])) + p.bias[c];
-              o[c] = (uint8_t)__float2int_rn((fminf(fmaxf(a, -1.f), 1.f) + 1.f) * 127.5f);
-            }
-          }
-        } else {
-          const ConvDest dst = conv_dest(p, f, y, x);
-          const int n_base = nt * 256, n_end = min(256, p.n_out - n_base);
-          const long long ld = p.n_out;
-          if (down && row_ok && (x == 0 || y == 0)) {
-            // border cells that no position of the plane maps to: left column, top row
-            for (int k = 0; k < 3; ++k) {
-              if ((k == 0 && x != 0) || (k == 1 && y != 0) || (k == 2 && (x != 0 || y != 0))) continue;
-              const long long cell = dst.row - (k == 1 ? 0 : 1) - (k == 0 ? 0 : p.wp + 1);
-              for (int c = 0; c < n_end; c += 8) {
-                if (p.out) *reinterpret_cast<uint4*>(p.out + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
-                if (p.out_norm) *reinterpret_cast<uint4*>(p.out_norm + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+            for (int k = 0; k < 16; ++k) a[k] = __uint_as_float(v[k]);
+            if (p.bias) {
+              const float4* b4 = reinterpret_cast<const float4*>(p.bias + n_base + c);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float4 b = b4[k];
+                a[4 * k] += b.x; a[4 * k + 1] += b.y; a[4 * k + 2] += b.z; a[4 * k + 3] += b.w;
               }
             }
+            if (res) {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const uint32_t w[4] = {ru[k].x, ru[k].y, ru[k].z, ru[k].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { a[k * 8 + 2 * e] += bf16lo(w[e]); a[k * 8 + 2 * e + 1] += bf16hi(w[e]); }
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) pk[k] = pack_bf16(a[2 * k], a[2 * k + 1]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) pk[k] = 0u;
           }
-          const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
-          __syncwarp();
-          uint32_t keep[NC > 0 ? NC / 2 : 1];
-          float part[NC > 0 ? NC / 8 : 1];
-#pragma unroll
-          for (int c = 0; c < (NC > 0 ? NC : 256); c += 32) {
-            if (NC == 0 && c >= n_end) break;   // uniform
-            uint32_t v[32], pk[16];
-            tmem_ld32(ta + c, v);
-            tmem_wait_ld();
-            if (row_ok) {
-              if (inside) {
-                float a[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) a[i] = __uint_as_float(v[i]);
-                if (p.bias) {
-                  const float* b = p.bias + n_base + c;
-#pragma unroll
-                  for (int i = 0; i < 32; ++i) a[i] += b[i];
-                }
-                if (res) {
-                  const uint4* r4 = reinterpret_cast<const uint4*>(res + c);
-#pragma unroll
-                  for (int k = 0; k < 4; ++k) {
-                    const uint4 u = r4[k];
-                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) { a[k * 8 + 2 * e] += bf16lo(w[e]); a[k * 8 + 2 * e + 1] += bf16hi(w[e]); }
-                  }
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(a[2 * i], a[2 * i + 1]);
-              } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) pk[i] = 0u;
-              }
-              if (p.out) {
-                if (p.mode != CONV_OUT_UP) {
-                  cv_store32(p.out + dst.row * ld + n_base + c, pk, 32);
-                } else {
-                  for (int tt = 0; tt < dst.n_t; ++tt)
-                    for (int yy = 0; yy < dst.n_y; ++yy)
-                      for (int xx = 0; xx < dst.n_x; ++xx)
-                        cv_store32(p.out + (dst.row + tt * dst.st + yy * dst.sy + xx) * ld + n_base + c, pk, 32);
-                }
-              }
-              if constexpr (NC > 0) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) keep[c / 2 + i] = pk[i];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  float s = 0.f;
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const float lo = bf16lo(pk[4 * k + e]), hi = bf16hi(pk[4 * k + e]);
-                    s += lo * lo;
-                    s += hi * hi;
-                  }
-                  part[c / 8 + k] = s;
-                }
-              }
+          if (p.out && row_ok) {
+            bf16* o = p.out + dst.row * ld + n_base + c;
+            if (p.mode != CONV_OUT_UP) {
+              cv_store16(o, pk);
+            } else {
+              for (int tt = 0; tt < dst.n_t; ++tt)
+                for (int yy = 0; yy < dst.n_y; ++yy)
+                  for (int xx = 0; xx < dst.n_x; ++xx) cv_store16(o + (tt * dst.st + yy * dst.sy + xx) * ld, pk);
             }
           }
           if constexpr (NC > 0) {
-            if (row_ok) {
-              const float rinv = rsqrtf(conv_tree_sum<NC / 8>(part) / (float)NC + p.eps);
-              uint4* o4 = reinterpret_cast<uint4*>(p.out_norm + dst.row * ld);
-              const uint4* g4 = reinterpret_cast<const uint4*>(p.gamma);
 #pragma unroll
-              for (int k = 0; k < NC / 8; ++k) {
-                const uint4 gu = g4[k];
-                const uint32_t gw[4] = {gu.x, gu.y, gu.z, gu.w};
-                uint32_t o[4];
+            for (int k = 0; k < 2; ++k) {
+              float s = 0.f;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const uint32_t u = keep[4 * k + e];
-                  const float lo = bf16lo(u) * rinv * bf16lo(gw[e]), hi = bf16hi(u) * rinv * bf16hi(gw[e]);
-                  o[e] = pack_bf16(lo / (1.f + __expf(-lo)), hi / (1.f + __expf(-hi)));   // zero on the border
+              for (int e = 0; e < 4; ++e) {
+                const float lo = bf16lo(pk[4 * k + e]), hi = bf16hi(pk[4 * k + e]);
+                s += lo * lo;
+                s += hi * hi;
+              }
+              if (i & 1) {
+                s = lvl[0][k] + s;
+                if (i & 2) {
+                  s = lvl[1][k] + s;
+                  if (i & 4) s = lvl[2][k] + s; else lvl[2][k] = s;
+                } else {
+                  lvl[1][k] = s;
                 }
-                o4[k] = make_uint4(o[0], o[1], o[2], o[3]);
+              } else {
+                lvl[0][k] = s;
+              }
+              sum[k] = s;
+            }
+            __syncwarp();
+            tmem_st8(ta + c, pk);   // the rounded values wait in place of their accumulators
+          }
+          __syncwarp();
+        }
+        if constexpr (NC > 0) {
+          // the other half's sums (two buffers: a warp is at most one meeting ahead of its partner)
+          float2* mine = row_sums + ((buf * 2 + r) * 2 + half) * 128 + quad * 32 + lane;
+          *mine = make_float2(sum[0], sum[1]);
+          tmem_wait_st();
+          cv_pair_and(pair_id, true);
+          const float2 other = row_sums[((buf * 2 + r) * 2 + (half ^ 1)) * 128 + quad * 32 + lane];
+          const float s0 = half ? other.x + sum[0] : sum[0] + other.x, s1 = half ? other.y + sum[1] : sum[1] + other.y;
+          const float rinv = rsqrtf((s0 + s1) / (float)NC + p.eps);
+          bf16* o = p.out_norm + dst.row * ld;
+#pragma unroll 1
+          for (int c = 16 * half; c < NC; c += 32) {
+            uint32_t pk[8], on[8];
+            tmem_ld8(ta + c, pk);
+            uint4 gu[2];
+            gu[0] = reinterpret_cast<const uint4*>(p.gamma + c)[0];
+            gu[1] = reinterpret_cast<const uint4*>(p.gamma + c)[1];
+            tmem_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const uint32_t gw[4] = {gu[k].x, gu[k].y, gu[k].z, gu[k].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint32_t u = pk[4 * k + e];
+                const float lo = bf16lo(u) * rinv * bf16lo(gw[e]), hi = bf16hi(u) * rinv * bf16hi(gw[e]);
+                on[4 * k + e] = pack_bf16(lo / (1.f + __expf(-lo)), hi / (1.f + __expf(-hi)));   // zero on the border
               }
             }
+            if (row_ok) cv_store16(o + c, on);
+            __syncwarp();
           }
         }
       }
@@ -503,7 +545,7 @@ void conv_launch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, int smem
   auto kern = cb::conv_kernel<R, NC, RGB>;
   static int pairs = 0;   // of this kernel, at its largest shared-memory size
   cudaLaunchConfig_t cfg{};
-  cfg.blockDim = dim3(cb::CV_THREADS);
+  cfg.blockDim = dim3(cb::ConvCfg<R>::THREADS);
   cfg.dynamicSmemBytes = cb::CV_SMEM_MAX;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -595,16 +637,16 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
     // segment = kept frame; the kept position (j, i) of a frame sits at padded (2 j + kh, 2 i + kw) for tap (kh, kw)
     p.n_seg = a.f_out;
     p.seg_rows = sub;
-    p.a_row0 = a.t_first * sub;
-    p.a_seg_stride = a.t_step * sub;
+    p.a_row0 = a.t_first * 4 * sub;
+    p.a_seg_stride = a.t_step * 4 * sub;
     p.plane = sub;
     p.pw = a.wp / 2; p.hp = a.hp / 2; p.wp = a.wp / 2;
     for (int kt = 0; kt < 3; ++kt)
       for (int kh = 0; kh < 3; ++kh) {
-        const int base = ((kh & 1) * 2 * a.frames_in + kt) * sub + (kh >> 1) * (a.wp / 2);
+        const int base = (kt * 4 + (kh & 1) * 2) * sub + (kh >> 1) * (a.wp / 2);
         const short t0 = (short)((kt * 3 + kh) * 3);
         p.g[p.n_groups++] = {base, 2, {0, 1, 0}, {t0, (short)(t0 + 2), 0}};
-        p.g[p.n_groups++] = {base + a.frames_in * sub, 1, {0, 0, 0}, {(short)(t0 + 1), 0, 0}};
+        p.g[p.n_groups++] = {base + sub, 1, {0, 0, 0}, {(short)(t0 + 1), 0, 0}};
       }
   }
   if (a.skip) {
@@ -616,7 +658,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   const int R = p.mma_n <= 128 ? 2 : 1;
   p.tiles_per_seg = (p.seg_rows + 256 * R - 1) / (256 * R);
   const int a_slot = (128 * R + 8) * 128, b_slot = p.mma_n * 64;
-  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_BARS;
+  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_BARS - cb::CV_SUMS;
   const int chunk = std::min(cb::CV_CHUNK, std::max(p.cblocks, p.skip_cblocks));
   // activations: one group's tiles and as many of the next one as fit beside the weight tiles: eight of those, or six where
   // four channel blocks meet 256 output channels

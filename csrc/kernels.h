@@ -199,12 +199,12 @@ void rmsnorm_silu(const void* x, const void* gamma, void* y, long long rows, int
 // ---- causal 3x3x3 convolutions of the tokenizer on padded channels-last volumes (conv_tcgen05.cu) ----
 enum ConvOut : int {
   CONV_OUT_SAME = 0,   // [tpad + f_out, hp, wp, n_out]
-  CONV_OUT_S2D = 1,    // [4, tpad + f_out, hp / 2, wp / 2, n_out]: parity of (row, column) of the padded volume first
+  CONV_OUT_S2D = 1,    // [tpad + f_out, 4, hp / 2, wp / 2, n_out]: a plane per parity of (row, column) of the padded volume
   CONV_OUT_UP = 2,     // nearest x2 in space (and in time): [tpad + frames, 2 (hp - 2) + 2, 2 (wp - 2) + 2, n_out]
   CONV_OUT_DOWN = 3,   // stride 2: x in s2d form; kept frames t_first + i t_step; [tpad + f_out, hp / 2 + 1, wp / 2 + 1, n_out]
 };
 struct ConvArgs {
-  const void* x = nullptr;      // [frames_in, hp, wp, c] (CONV_OUT_DOWN: [4, frames_in, hp / 2, wp / 2, c])
+  const void* x = nullptr;      // [frames_in, hp, wp, c] (CONV_OUT_DOWN: [frames_in, 4, hp / 2, wp / 2, c])
   const void* w = nullptr;      // [n_out, 27 c (+ skip_c)], tap-major; taps_t_only: [n_out, 3 c]
   const float* bias = nullptr;  // [n_out]; pixels: [3]
   const void* resid = nullptr;  // added; layout of a CONV_OUT_SAME output

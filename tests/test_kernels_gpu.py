@@ -990,11 +990,11 @@ def test_conv3d_fused_forms(cin, cout, t, h, w):
         k.conv3d_fused(vol, wp, b, _volume(r), None, None, only, g, 1e-6, 0, 0, 0)
         assert torch.equal(only[2:], on[2:])
     # skip projection, s2d layout
-    s2d = nan(4, t + 2, h // 2 + 1, w // 2 + 1, cout)
+    s2d = nan(t + 2, 4, h // 2 + 1, w // 2 + 1, cout)
     k.conv3d_fused(vol, torch.cat([wp, sw], 1).contiguous(), b, None, _volume(sk), s2d, None, None, 1e-6, 1, 0, 0)
     flat = torch.empty(t, h + 2, w + 2, cout, device=DEV, dtype=torch.bfloat16)
     for i in range(4):
-        flat[:, i >> 1::2, i & 1::2] = s2d[i, 2:]
+        flat[:, i >> 1::2, i & 1::2] = s2d[2:, i]
     check(flat[:, 1:-1, 1:-1], y + torch.einsum("oc,cthw->othw", sw.double(), sk.double()), "skip")
     border(flat)
     # nearest upsampling
@@ -1006,9 +1006,9 @@ def test_conv3d_fused_forms(cin, cout, t, h, w):
         check(up[2:, 1:-1, 1:-1], want, "upsampling")
         border(up[2:])
     # stride 2 over the s2d form of the input
-    xs = torch.empty(4, t + 2, h // 2 + 1, w // 2 + 1, cin, device=DEV, dtype=torch.bfloat16)
+    xs = torch.empty(t + 2, 4, h // 2 + 1, w // 2 + 1, cin, device=DEV, dtype=torch.bfloat16)
     for i in range(4):
-        xs[i] = vol[:, i >> 1::2, i & 1::2]
+        xs[:, i] = vol[:, i >> 1::2, i & 1::2]
     for first, step in ((0, 1), (0, 2), (1, 2)):
         want = y[:, first::step, ::2, ::2]
         if want.shape[1] == 0:
@@ -1048,3 +1048,17 @@ def test_conv3d_of_colours(dtype, t, h, w):
     y = F.conv3d(F.pad(x[None].double(), (1, 1, 1, 1, 2, 0)), wo.double(), b.double())[0]
     pix = ((y.clamp(-1, 1) + 1) * 127.5).permute(1, 2, 3, 0)
     assert (got.double() - pix).abs().max() <= 0.5 + 1e-3      # rounding, and fp32 sums of 1728 products below 4
+
+
+@pytest.mark.parametrize("t,chunk", [(1, 2), (2, 2), (5, 2), (6, 1), (4, 8)])
+def test_vae_decode_to_host_is_the_decode(t, chunk):
+    from cosmos_b200.models.vae import CausalVideoVAE
+    from cosmos_b200.models.vae_cuda import CLDecoder
+    torch.manual_seed(t)
+    dec = CLDecoder(CausalVideoVAE(16, (64, 128, 128, 128)).to(device=DEV, dtype=torch.bfloat16).eval())
+    z = torch.randn(1, 16, t, 4, 6, device=DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = dec.decode_to_host(z, chunk_latents=chunk)
+    assert torch.equal(got, dec.decode(z, chunk_latents=chunk)[0].cpu())
