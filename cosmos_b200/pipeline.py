@@ -412,7 +412,7 @@ class Cosmos3OmniPipeline:
         cl = self._cl_decoder()
         if cl is not None:
             # tensor-core implicit-GEMM decoder on padded channels-last volumes (2 latent frames per chunk)
-            frames = cl.decode(z, chunk_latents=2)[0].cpu().numpy()
+            frames = cl.decode_to_host(z, chunk_latents=2).numpy()
         else:
             video = self.vae.decode(z, chunk_latents=chunk_latents if st.grid[0] > (chunk_latents or 0) else None)
             frames = CausalVideoVAE.to_uint8(video)[0].cpu().numpy()
