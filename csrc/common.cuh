@@ -407,6 +407,11 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
                    cluster_bar)
                : "memory");
 }
+// The same for the barriers at shared-memory offset `bar` of both CTAs; called by the leader (rank 0).
+__device__ __forceinline__ void tc_commit_both(uint32_t bar) {
+  tc_commit_pair(bar);
+  tc_commit_pair(mapa(bar, 1));
+}
 __device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(

@@ -1,11 +1,11 @@
 // K1: persistent bf16 GEMM  C[M,N] = A[M,K] * B[N,K]^T  on tcgen05 tensor cores.
 //
-// Layout of one CTA (192 threads):
+// Layout of one CTA (320 threads):
 //   warp 0      TMA producer  (A 128x64 and B 256x64 tiles, 128-byte swizzle, 4-stage ring)
 //   warp 1      MMA issuer    (tcgen05.mma M=128 N=256 K=16, fp32 accumulators in TMEM,
 //                              two 256-column accumulator buffers so the epilogue of tile i
 //                              overlaps the main loop of tile i+1)
-//   warps 2..5  epilogue      (tcgen05.ld -> registers -> fused epilogue -> global / peer stores)
+//   warps 2..9  epilogue      (tcgen05.ld -> registers -> fused epilogue -> global / peer stores)
 //
 // Fused epilogues (template parameter EPI):
 //   EPI_PLAIN        C = acc (+ bias)
@@ -33,22 +33,30 @@ namespace cb {
 
 constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;      // 16 KB
-constexpr int GEMM_THREADS = 192;
 // NC = 1: one CTA per 128x256 tile, 4 stages of A 16 KB + B 32 KB.
 // NC = 2: a CTA pair per 256x256 tile (tcgen05 cta_group::2, M = 256): each CTA stages its own 128 rows
 // of A and its own 128 of the tile's 256 B rows, so a stage is 32 KB per CTA and the B operand crosses
 // shared memory once per pair instead of once per CTA; 6 stages.
-template <int NC> struct GemmCfg {
-  static constexpr int STAGES = NC == 2 ? 6 : 4;
-  static constexpr int B_BYTES = (BN / NC) * BK * 2;
+// NW = 2 (pairs only): a pair computes 256 x 512, two neighbouring 256-column tiles of one A tile. What bounds a tall
+// GEMM is the delivery of operands from L2 into shared memory, about 45 B per clock and SM: a 256x256 tile stages 32 KB per
+// CTA and 512 clocks of MMA (64 B per clock), a 256x512 tile 48 KB per 1024 clocks (48 B per clock). The two accumulators
+// fill tensor memory, so they are not double-buffered: the first and last k-blocks of a tile are issued accumulator by
+// accumulator, so that one is drained while the other is computed. 4 stages.
+constexpr int EPI_WARPS = 8;   // two per quadrant of accumulator rows, each with half of the columns
+constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int gamma_smem(int epi) { return epi == EPI_QKV_ROPE ? 1024 : 0; }  // both norms' weights as fp32, behind the barriers
+template <int NC, int NW = 1> struct GemmCfg {
+  static constexpr int STAGES = NW == 2 ? 4 : NC == 2 ? 6 : 4;
+  static constexpr int B_BYTES = NW * (BN / NC) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SLABS = EPI_WARPS * 4096;  // one per epilogue warp (see Slab)
+  static constexpr int SMEM = STAGES * STAGE_BYTES + SLABS + 1024 /*align*/ + 256 /*barriers*/;
 };
 
 struct GemmParams {
   int M, N, K;
   int b_row1;            // row offset in B of the second 128-row half of the tile
-  int n_tiles, m_tiles;  // tile counts (n_tiles counts 256-wide (or 128-wide for SWIGLU) tiles)
+  int n_tiles, m_tiles;  // tile counts (n_tiles counts tiles of 256 * NW columns, 128 * NW for SWIGLU)
   bf16* C;
   long long ldc;
   const bf16* bias;      // [N] or null
@@ -117,18 +125,439 @@ __device__ __forceinline__ TileRows tile_rows(const GemmParams& p, int tm) {
   return {tm * TILE_M, p.M, 0};
 }
 
-template <int EPI, int NC>
+// A warp's staging area: 32 rows of 128 bytes, the 16-byte chunk c of row r at position c ^ (r & 7). In the accumulator's
+// layout a lane holds a row, so a direct access of global memory touches 32 lines per instruction, and those wavefronts
+// compete with the operand copies and the tensor core's reads for the shared memory's bandwidth; through the slab an
+// instruction touches 4 whole lines.
+struct Slab {
+  uint32_t base;
+  int lane;
+  __device__ __forceinline__ uint32_t at(int r, int c) const { return base + r * 128 + ((c ^ (r & 7)) << 4); }
+  __device__ __forceinline__ void put(int r, int c, uint4 v) const {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at(r, c)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+  }
+  __device__ __forceinline__ uint4 get(int r, int c) const {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at(r, c)) : "memory");
+    return v;
+  }
+  // 8 columns f[0..7] of this lane's row
+  __device__ __forceinline__ void put_bf16(int c, const float* f) const {
+    put(lane, c, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
+  }
+  // Coalesced order: lane's i-th chunk is chunk (lane & 7) of row 4 i + lane / 8. rows x 64 columns of `src` (row stride
+  // ld) in that order; what lies beyond is zero.
+  __device__ __forceinline__ void fetch(uint4 (&v)[8], const bf16* src, long long ld, int rows, int cols) const {
+    const int c = (lane & 7) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      v[i] = make_uint4(0, 0, 0, 0);
+      if (r < rows && c < cols) {
+        const bf16* s = src + r * ld + c;
+        if (c + 8 <= cols) {
+          v[i] = *reinterpret_cast<const uint4*>(s);
+        } else {
+          uint32_t u[4] = {0, 0, 0, 0};
+          const unsigned short* h = reinterpret_cast<const unsigned short*>(s);
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (c + e < cols) u[e >> 1] |= uint32_t(h[e]) << (16 * (e & 1));
+          v[i] = make_uint4(u[0], u[1], u[2], u[3]);
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void fill(const uint4 (&v)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) put(i * 4 + (lane >> 3), lane & 7, v[i]);
+    __syncwarp();
+  }
+  // slab -> rows x 64 columns of `dst` (bf16) or rows x 32 (fp32)
+  template <class T>
+  __device__ __forceinline__ void store(T* dst, long long ld, int rows, int cols) const {
+    constexpr int PER = 16 / sizeof(T);
+    __syncwarp();
+    const int c = (lane & 7) * PER;
+    if (c < cols) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3);
+        if (r < rows) {
+          const uint4 v = get(r, lane & 7);
+          T* d = dst + r * ld + c;
+          if (c + PER <= cols) {
+            *reinterpret_cast<uint4*>(d) = v;
+          } else {
+            const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+            for (int j = 0; j < PER; ++j)
+              if (c + j < cols) d[j] = e[j];
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+};
+
+// Epilogue of a warp: its 32 rows m0 .. (those below m_end) and one half of the 256 columns of accumulator tile tn. `wait`
+// waits for the accumulator, `release` hands it back once it has been read. The loops over columns stay rolled: unrolled,
+// the code of one tile does not fit the instruction cache and fetching it takes longer than the work.
+template <int EPI, class Wait, class Release>
+__device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& slab, uint32_t t_addr, int half, int m0, int m_end,
+                                            int tn, int ks, const float* sgamma, Wait wait, Release release) {
+  const int lane = slab.lane, m = min(m0 + lane, m_end - 1), rows = m_end - m0;
+  const int n0 = EPI == EPI_SWIGLU ? tn * 128 + half * 64 : tn * BN + half * 128;   // first output column
+  const int n_out = EPI == EPI_SWIGLU ? p.N / 2 : p.N;
+  if (rows <= 0 || n0 >= n_out) {   // nothing to store
+    if (!wait()) return false;
+    release();
+    return true;
+  }
+  if (p.partial) {   // raw fp32 sums of a K range, the columns of B
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      uint32_t v[32];
+      const int at = EPI == EPI_SWIGLU ? (c >> 1) * 128 + half * 64 + (c & 1) * 32 : half * 128 + c * 32;
+      tmem_ld32(t_addr + at, v);
+      tmem_wait_ld();
+      if (c == 3) release();
+      const int n = EPI == EPI_SWIGLU ? n0 + (c & 1) * 32 : n0 + c * 32;
+      if (rows <= 8 && n + 32 <= n_out) {   // few rows (decode): a lane's own stores touch no more lines, and need no staging
+        if (lane < rows) {
+          uint4* d = reinterpret_cast<uint4*>(p.partial + ((long long)ks * p.M + m) * p.N + n + (EPI == EPI_SWIGLU && c >= 2 ? n_out : 0));
+#pragma unroll
+          for (int q = 0; q < 8; ++q) d[q] = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+        }
+        __syncwarp();
+        continue;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) slab.put(lane, q, make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]));
+      float* dst = p.partial + ((long long)ks * p.M + m0) * p.N + n + (EPI == EPI_SWIGLU && c >= 2 ? n_out : 0);
+      slab.store(dst, p.N, rows, n_out - n);
+    }
+    return true;
+  }
+  if constexpr (EPI == EPI_SWIGLU) {
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      uint32_t g[16], u[16];
+      tmem_ld16(t_addr + half * 64 + c * 16, g);
+      tmem_ld16(t_addr + 128 + half * 64 + c * 16, u);
+      tmem_wait_ld();
+      if (c == 3) release();
+      // silu(g) = g / (1 + exp(-g)). A division has a branch, so that 16 of them run one after another (M 240 of the 24576-wide
+      // projection: 74 us with them, 55 without): the quotient is g times the approximate reciprocal, corrected once by its
+      // residual (Newton's step; the result differs from the division's in about one of 2^22 cases, by one ulp of fp32),
+      // and values whose residual could overflow or underflow are divided.
+      float o[16];
+      bool odd = false;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float gv = __uint_as_float(g[i]), den = 1.f + __expf(-gv);
+        float rc;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(den));
+        const float q = gv * rc;
+        o[i] = fmaf(fmaf(-q, den, gv), rc, q);
+        odd |= !(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-30f && gv != 0.f);
+      }
+      if (odd) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float gv = __uint_as_float(g[i]);
+          if (!(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-30f && gv != 0.f)) o[i] = gv / (1.f + __expf(-gv));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i] *= __uint_as_float(u[i]);
+      slab.put_bf16(c * 2, o);
+      slab.put_bf16(c * 2 + 1, o + 8);
+    }
+    slab.store(p.C + (long long)m0 * p.ldc + n0, p.ldc, rows, n_out - n0);
+    return true;
+  }
+  if constexpr (EPI == EPI_QKV_ROPE) {
+    const int chunk = tn * 2 + half;
+    bf16* dst = p.route_ptr ? reinterpret_cast<bf16*>(p.route_ptr[chunk]) : p.C + n0;
+    const long long ld = p.route_ptr ? p.route_ld[chunk] : p.ldc;
+    if (chunk < p.n_q_heads + p.n_k_heads && (p.gamma_q || p.gamma_k || p.cos_tab)) {
+      // Norm and rotary embedding of one head. 16 columns of both tables at a time go through the slab (chunks 0-3 of a row
+      // cosines, 4-7 sines), requested two steps ahead: their latency would otherwise hold the accumulator. The norm's
+      // weights are in shared memory for the same reason.
+      const bool is_q = chunk < p.n_q_heads;
+      const bool normed = (is_q ? p.gamma_q : p.gamma_k) != nullptr, rope = p.cos_tab != nullptr;
+      const float* gam = sgamma + (is_q ? 0 : 128);
+      const bf16* bias = p.bias ? p.bias + n0 : nullptr;
+      const float* tab = (lane & 4 ? p.sin_tab : p.cos_tab) + (lane & 3) * 4;
+      const int rr = p.rope_rows, row0 = m0 % rr;
+      uint4 t0[8], t1[8];
+      auto fetch_tab = [&](uint4 (&t)[8], int q) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = i * 4 + (lane >> 3);
+          t[i] = make_uint4(0, 0, 0, 0);
+          int row = row0 + r;
+          if (row >= rr) row = rr >= 32 ? row - rr : row % rr;
+          if (r < rows) t[i] = *reinterpret_cast<const uint4*>(tab + (long long)row * 64 + q * 16);
+        }
+      };
+      if (rope) {
+        fetch_tab(t0, 0);
+        fetch_tab(t1, 1);
+      }
+      if (!wait()) return false;
+      t_addr += half * 128;
+      float rinv = 1.f;
+      if (normed) {
+        float ss = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(t_addr + c * 32, v);
+          tmem_wait_ld();
+          if (bias) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __bfloat162float(bias[c * 32 + i]));
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) ss += __uint_as_float(v[i]) * __uint_as_float(v[i]);
+        }
+        rinv = rsqrtf(ss * (1.f / 128.f) + p.eps);
+      }
+      auto step = [&](uint4 (&t)[8], int q) {
+        uint32_t va[16], vb[16];
+        tmem_ld16(t_addr + q * 16, va);
+        tmem_ld16(t_addr + 64 + q * 16, vb);
+        tmem_wait_ld();
+        if (q == 3) release();
+        float a[16], b[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          a[i] = __uint_as_float(va[i]);
+          b[i] = __uint_as_float(vb[i]);
+        }
+        if (bias) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            a[i] += __bfloat162float(bias[q * 16 + i]);
+            b[i] += __bfloat162float(bias[64 + q * 16 + i]);
+          }
+        }
+        if (normed) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            a[i] = a[i] * rinv * gam[q * 16 + i];
+            b[i] = b[i] * rinv * gam[64 + q * 16 + i];
+          }
+        }
+        if (rope) {
+          slab.fill(t);
+          if (q < 2) fetch_tab(t, q + 2);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint4 cu = slab.get(lane, j), su = slab.get(lane, 4 + j);
+            const uint32_t c4[4] = {cu.x, cu.y, cu.z, cu.w}, s4[4] = {su.x, su.y, su.z, su.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float x = a[j * 4 + e], y = b[j * 4 + e], cc = __uint_as_float(c4[e]), sn = __uint_as_float(s4[e]);
+              a[j * 4 + e] = fmaf(x, cc, -__fmul_rn(y, sn));
+              b[j * 4 + e] = fmaf(x, sn, __fmul_rn(y, cc));
+            }
+          }
+          __syncwarp();
+        }
+        slab.put_bf16(0, a);
+        slab.put_bf16(1, a + 8);
+        slab.put_bf16(2, b);
+        slab.put_bf16(3, b + 8);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {   // 8 rows of 2 x 32 bytes per instruction
+          const int r = i * 8 + (lane >> 2), c = lane & 3;
+          const uint4 v = slab.get(r, c);
+          if (r < rows) *reinterpret_cast<uint4*>(dst + (m0 + r) * ld + (c >> 1) * 64 + q * 16 + (c & 1) * 8) = v;
+        }
+        __syncwarp();
+      };
+#pragma unroll 1
+      for (int q = 0; q < 4; q += 2) {
+        step(t0, q);
+        step(t1, q + 1);
+      }
+      return true;
+    }
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      uint32_t v[32];
+      tmem_ld32(t_addr + half * 128 + c * 32, v);
+      tmem_wait_ld();
+      if (c == 3) release();
+      float f[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        f[i] = __uint_as_float(v[i]);
+        if (p.bias) f[i] += __bfloat162float(p.bias[n0 + c * 32 + i]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) slab.put_bf16((c & 1) * 4 + q, f + q * 8);
+      if (c & 1) slab.store(dst + (long long)m0 * ld + (c >> 1) * 64, ld, rows, 64);
+    }
+    return true;
+  }
+  if constexpr (EPI == EPI_PLAIN || EPI == EPI_GELU || EPI == EPI_GATED_RESID) {
+    // the residual of both 64-column steps is on its way before the accumulator is waited for
+    uint4 r1[8];
+    if constexpr (EPI == EPI_GATED_RESID) {
+      const bf16* r = p.R + (long long)m0 * p.ldr + n0;
+      slab.fetch(r1, r, p.ldr, rows, p.N - n0);
+      slab.fill(r1);
+      slab.fetch(r1, r + 64, p.ldr, rows, p.N - n0 - 64);
+    }
+    if (!wait()) return false;
+    const bf16* gate = EPI == EPI_GATED_RESID && p.gate ? p.gate + (long long)(m / p.rows_per_batch) * p.N : nullptr;
+#pragma unroll 1
+    for (int c = 0; c < 8; ++c) {   // 16 columns at a time
+      const int n = n0 + c * 16;
+      uint32_t v[16];
+      tmem_ld16(t_addr + half * 128 + c * 16, v);
+      tmem_wait_ld();
+      if (c == 7) release();
+      if (c == 4) {
+        slab.store(p.C + (long long)m0 * p.ldc + n0, p.ldc, rows, p.N - n0);
+        if constexpr (EPI == EPI_GATED_RESID) slab.fill(r1);
+      }
+      float f[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+      if (p.bias) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (n + i < p.N) f[i] += __bfloat162float(p.bias[n + i]);
+      }
+      if constexpr (EPI == EPI_GELU) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = gelu_erf(f[i]);
+      }
+      if constexpr (EPI == EPI_GATED_RESID) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint4 rv = slab.get(lane, (c & 3) * 2 + q);
+          const uint32_t ru[4] = {rv.x, rv.y, rv.z, rv.w};
+          uint32_t gu[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
+          if (gate && (p.N & 7) == 0) {
+            if (n + q * 8 < p.N) {
+              const uint4 gv = *reinterpret_cast<const uint4*>(gate + n + q * 8);
+              gu[0] = gv.x; gu[1] = gv.y; gu[2] = gv.z; gu[3] = gv.w;
+            }
+          } else if (gate) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (n + q * 8 + e < p.N)
+                gu[e >> 1] = (gu[e >> 1] & (e & 1 ? 0x0000ffffu : 0xffff0000u)) |
+                             (uint32_t(reinterpret_cast<const unsigned short*>(gate)[n + q * 8 + e]) << (16 * (e & 1)));
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            f[q * 8 + e * 2] = bf16lo(ru[e]) + bf16lo(gu[e]) * f[q * 8 + e * 2];
+            f[q * 8 + e * 2 + 1] = bf16hi(ru[e]) + bf16hi(gu[e]) * f[q * 8 + e * 2 + 1];
+          }
+        }
+      }
+      slab.put_bf16((c & 3) * 2, f);
+      slab.put_bf16((c & 3) * 2 + 1, f + 8);
+    }
+    slab.store(p.C + (long long)m0 * p.ldc + n0 + 64, p.ldc, rows, p.N - n0 - 64);
+    return true;
+  }
+  if constexpr (EPI == EPI_ATTN_P || EPI == EPI_ATTN_DS) {
+    if (!wait()) return false;
+    const bool row_ok = lane < rows;
+    const float rv = p.rowvec[m];
+    int lim = p.N;
+    if (p.attn_mask == MASK_CAUSAL) lim = min(p.N, m + 1 + (p.N - p.M));
+    if (p.attn_mask == MASK_MOT) lim = m < p.attn_n_ar ? m + 1 : p.N;
+    const float sl2 = p.attn_scale * 1.4426950408889634f;
+    const float rv2 = rv * 1.4426950408889634f;
+#pragma unroll 1
+    for (int c = 0; c < 128; c += 32) {
+      const int n = n0 + c;
+      if (n >= p.N) break;
+      uint32_t v[32];
+      tmem_ld32(t_addr + half * 128 + c, v);
+      tmem_wait_ld();
+      if (row_ok) {
+        float f[32];
+        const bool full32 = (n + 32 <= p.N);
+        if constexpr (EPI == EPI_ATTN_P) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            f[i] = (n + i < lim) ? exp2f(fmaf(__uint_as_float(v[i]), sl2, -rv2)) : 0.f;
+        } else {
+          const bf16* pr = p.R + (long long)m * p.ldr + n;
+          if (full32) {
+            const uint4* r4 = reinterpret_cast<const uint4*>(pr);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint4 rr = r4[q];
+              const uint32_t ru[4] = {rr.x, rr.y, rr.z, rr.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                f[q * 8 + 2 * e] = bf16lo(ru[e]) * (__uint_as_float(v[q * 8 + 2 * e]) - rv) * p.attn_scale;
+                f[q * 8 + 2 * e + 1] = bf16hi(ru[e]) * (__uint_as_float(v[q * 8 + 2 * e + 1]) - rv) * p.attn_scale;
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              f[i] = (n + i < p.N) ? __bfloat162float(pr[i]) * (__uint_as_float(v[i]) - rv) * p.attn_scale : 0.f;
+          }
+        }
+        bf16* dst = p.C + (long long)m * p.ldc + n;
+        if (full32) {
+          uint4* d4 = reinterpret_cast<uint4*>(dst);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint4 o;
+            o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
+            o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
+            o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
+            o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
+            d4[q] = o;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (n + i < p.N) dst[i] = __float2bfloat16(f[i]);
+        }
+      }
+    }
+    release();
+    return true;
+  }
+  return false;
+}
+
+template <int EPI, int NC, int NW>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmB1,
                  const __grid_constant__ GemmGroup g) {
-  constexpr int STAGES = GemmCfg<NC>::STAGES;
-  constexpr int B_BYTES = GemmCfg<NC>::B_BYTES;
-  constexpr int STAGE_BYTES = GemmCfg<NC>::STAGE_BYTES;
+  static_assert(NW == 1 || NC == 2, "two column tiles per item need a CTA pair");
+  using Cfg = GemmCfg<NC, NW>;
+  constexpr int STAGES = Cfg::STAGES;
+  constexpr int B_BYTES = Cfg::B_BYTES;
+  constexpr int STAGE_BYTES = Cfg::STAGE_BYTES;
+  constexpr int TN = BN / NC * BK * 2;  // bytes of one column tile's B in this CTA
+  constexpr int BARS = STAGES * STAGE_BYTES + Cfg::SLABS;  // offset of the barriers
   constexpr int TILE_M = BM * NC;  // rows of one output tile (of the CTA pair when NC == 2)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t bar_base = smem_base + BARS;
   // CTA pair: rank 0 (the leader) issues the MMAs and owns the `full` and `tempty` barriers that
   // both CTAs signal; `empty` and `tfull` exist in both CTAs and the leader's commits reach both.
   const uint32_t cta_rank = NC == 2 ? cluster_ctarank() : 0u;
@@ -142,9 +571,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 4);
   uint8_t* gen_base = smem_raw + (smem_base - smem_u32(smem_raw));
   volatile int* abort_flag =
-      reinterpret_cast<volatile int*>(gen_base + STAGES * STAGE_BYTES + 8 * (2 * STAGES + 4) + 8);
+      reinterpret_cast<volatile int*>(gen_base + BARS + 8 * (2 * STAGES + 4) + 8);
   volatile uint32_t* tmem_slot_ptr =
-      reinterpret_cast<volatile uint32_t*>(gen_base + STAGES * STAGE_BYTES + 8 * (2 * STAGES + 4));
+      reinterpret_cast<volatile uint32_t*>(gen_base + BARS + 8 * (2 * STAGES + 4));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -161,7 +590,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 4 * NC);
+      mbar_init(tempty_bar(b), EPI_WARPS * NC);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -231,7 +660,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tile_coords(tl / p.k_splits, second ? p.m_tiles : m_tiles0, p.n_tiles, tm, tn);
         const TileRows tr = tile_rows<TILE_M>(p, tm);
         const int m0 = (p.debug & 1) ? 0 : tr.m0 + int(cta_rank) * BM;
-        const int n0 = (p.debug & 1) ? 0 : tr.b_row + ((EPI == EPI_SWIGLU) ? tn * 128 : tn * BN);
+        const int n0 = (p.debug & 1) ? 0 : tr.b_row + ((EPI == EPI_SWIGLU) ? tn * NW * 128 : tn * NW * BN);
         if (p.debug & 2) continue;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
@@ -261,12 +690,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             } else {
               tma_load_2d_pair(sa, mA, fb, kb * BK, m0);
             }
-            const int nb = n0 + int(cta_rank) * p.b_row1;  // this CTA's 128 B rows (N columns of the tile)
-            if (p.b_mn) {
-              tma_load_2d_pair(sa + A_BYTES, mB, fb, nb, kb * BK);
-              tma_load_2d_pair(sa + A_BYTES + B_BYTES / 2, mB, fb, nb + 64, kb * BK);
-            } else {
-              tma_load_2d_pair(sa + A_BYTES, mB, fb, kb * BK, nb);
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+              // this CTA's 128 B rows (N columns) of each column tile
+              const int nb = n0 + w * (EPI == EPI_SWIGLU ? 128 : BN) + int(cta_rank) * p.b_row1;
+              const uint32_t sb = sa + A_BYTES + w * TN;
+              if (p.b_mn) {
+                tma_load_2d_pair(sb, mB, fb, nb, kb * BK);
+                tma_load_2d_pair(sb + TN / 2, mB, fb, nb + 64, kb * BK);
+              } else {
+                tma_load_2d_pair(sb, mB, fb, kb * BK, nb);
+              }
             }
             continue;
           }
@@ -316,345 +750,131 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int k_blocks = (p.K + BK - 1) / BK;
         const int ks = (second ? t - tiles0 : t) % p.k_splits;
         const int kb0 = ks * k_blocks / p.k_splits, kb1 = (ks + 1) * k_blocks / p.k_splits;
-        const int b = tcount & 1;
-        const uint32_t bph = (tcount >> 1) & 1;
+        const int b = NW == 2 ? 0 : tcount & 1;
+        const uint32_t bph = NW == 2 ? tcount & 1 : (tcount >> 1) & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(b), bph ^ 1, abort_flag, p.status, ST_TIMEOUT_MMA))) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + b * BN;
         const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;
         const uint32_t idesc = make_idesc_bf16(TILE_M, BN, p.a_mn, p.b_mn);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!(p.debug & 2) &&
-              !__all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, abort_flag, p.status, ST_TIMEOUT_MMA))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_base + s * STAGE_BYTES;
+        // the products of one stage with one column tile
+        auto issue = [&](uint32_t sa, int w, bool first) {
           // K-major: 128-byte rows along K, +32 B per k-step. MN-major: 64-element chunks along M/N
           // 8 KB apart (LBO), k advances by rows of 128 B, +2048 B per k-step of 16.
+          const uint32_t d_tmem = tmem_base + (NW == 2 ? w : b) * BN, sb = sa + A_BYTES + w * TN;
           const uint64_t adesc = p.a_mn ? make_smem_desc_sw128(sa, 8192, 1024) : make_smem_desc_sw128(sa, 16, 1024);
-          const uint64_t bdesc = p.b_mn ? make_smem_desc_sw128(sa + A_BYTES, 8192, 1024)
-                                        : make_smem_desc_sw128(sa + A_BYTES, 16, 1024);
-          if (elect_one()) {
+          const uint64_t bdesc = p.b_mn ? make_smem_desc_sw128(sb, 8192, 1024) : make_smem_desc_sw128(sb, 16, 1024);
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-              // advance 32 bytes (16 bf16) along K inside the 128-byte swizzle row: +2 in >>4 units
-              if constexpr (NC == 2)
-                mma_ss_pair(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-              else
-                mma_ss(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-            }
-            if constexpr (NC == 2) {
-              tc_commit_pair(empty_bar(s));            // frees the stage in this CTA ...
-              tc_commit_pair(mapa(empty_bar(s), 1));   // ... and in the peer
-            } else {
-              tc_commit(empty_bar(s));
-            }
+          for (int k = 0; k < BK / 16; ++k) {
+            // advance 32 bytes (16 bf16) along K inside the 128-byte swizzle row: +2 in >>4 units
+            if constexpr (NC == 2)
+              mma_ss_pair(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, (!first || k > 0) ? 1u : 0u);
+            else
+              mma_ss(d_tmem, adesc + a_step * k, bdesc + b_step * k, idesc, (!first || k > 0) ? 1u : 0u);
           }
-          __syncwarp();
+        };
+        for (int kb = kb0; kb < kb1;) {
+          // k-blocks issued together: at the two ends of a 256x512 tile EDGE of them, first for one accumulator and then
+          // for the other, so that a drain has EDGE x 512 clocks of the other accumulator's products to hide behind
+          constexpr int EDGE = 2;
+          const int nk = (NW == 2 && (kb == kb0 || kb + EDGE >= kb1)) ? min(EDGE, kb1 - kb) : 1;
+          for (int j = 0; j < nk; ++j) {
+            const int s = (it + j) % STAGES;
+            const uint32_t ph = ((it + j) / STAGES) & 1;
+            if (!(p.debug & 2) &&
+                !__all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, abort_flag, p.status, ST_TIMEOUT_MMA))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            if (elect_one()) {
+              issue(smem_base + s * STAGE_BYTES, 0, kb + j == kb0);
+              if constexpr (NW == 1) {
+                if constexpr (NC == 2) tc_commit_both(empty_bar(s));  // frees the stage in both CTAs
+                else tc_commit(empty_bar(s));
+              }
+            }
+            __syncwarp();
+          }
+          if (!ok) break;
+          if constexpr (NW == 2) {
+            if (kb + nk == kb1) {
+              if (elect_one()) tc_commit_both(tfull_bar(0));
+              __syncwarp();
+            }
+            if (kb == kb0) {
+              if (!__all_sync(0xffffffffu, mbar_wait(tempty_bar(1), bph ^ 1, abort_flag, p.status, ST_TIMEOUT_MMA))) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+            }
+            if (elect_one()) {
+              for (int j = 0; j < nk; ++j) {
+                const int s = (it + j) % STAGES;
+                issue(smem_base + s * STAGE_BYTES, 1, kb + j == kb0);
+                tc_commit_both(empty_bar(s));
+              }
+            }
+            __syncwarp();
+          }
+          kb += nk;
+          it += nk;
         }
         if (ok) {
           if (elect_one()) {
-            if constexpr (NC == 2) {
-              tc_commit_pair(tfull_bar(b));
-              tc_commit_pair(mapa(tfull_bar(b), 1));
-            } else {
-              tc_commit(tfull_bar(b));
-            }
+            if constexpr (NC == 2) tc_commit_both(tfull_bar(NW == 2 ? 1 : b));
+            else tc_commit(tfull_bar(b));
           }
           __syncwarp();
         }
       }
     }
   } else {
-    // ---------------- epilogue warps (2..5); TMEM lane quadrant = warp % 4
+    // ---------------- epilogue warps (2..9); TMEM lane quadrant = warp % 4
     const int quad = warp & 3;
-    const int row_in_tile = quad * 32 + lane;
+    const Slab slab{smem_base + STAGES * STAGE_BYTES + uint32_t(warp - 2) * 4096u, lane};
+    float* sgamma = reinterpret_cast<float*>(gen_base + BARS + 256);
+    if constexpr (EPI == EPI_QKV_ROPE) {   // one problem per launch (checked on the host)
+      for (int i = threadIdx.x - 64; i < 256; i += EPI_WARPS * 32) {
+        const bf16* gam = i < 128 ? g.p[0].gamma_q : g.p[0].gamma_k;
+        sgamma[i] = gam ? __bfloat162float(gam[i & 127]) : 1.f;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+    }
     int tcount = 0;
     for (int t = first_tile; t < total_tiles; t += tile_step, ++tcount) {
-      const int b = tcount & 1;
-      const uint32_t bph = (tcount >> 1) & 1;
       const int second = t >= tiles0;
       const GemmParams& p = g.p[second];
       const int tl = second ? t - tiles0 : t;
       int tm, tn;
       tile_coords(tl / p.k_splits, second ? p.m_tiles : m_tiles0, p.n_tiles, tm, tn);
       const TileRows tr = tile_rows<TILE_M>(p, tm);
-      const int m = tr.m0 + int(cta_rank) * BM + row_in_tile;
-      if (!mbar_wait(tfull_bar(b), bph, abort_flag, p.status, ST_TIMEOUT_EPI)) break;
-      tc_fence_after();
-      const uint32_t t_addr = tmem_base + (uint32_t(quad * 32) << 16) + b * BN;
-      const bool row_ok = m < tr.m_end;
-
-      if ((EPI == EPI_PLAIN || EPI == EPI_SWIGLU || EPI == EPI_GATED_RESID || EPI == EPI_GELU) && p.partial) {
-        // raw fp32 partial sums; accumulator column c maps to output column col(c)
-        float* dst_row = p.partial + ((long long)(tl % p.k_splits) * p.M + m) * p.N;
+      const int m0 = tr.m0 + int(cta_rank) * BM + quad * 32;
+      bool ok = true;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t v[32];
-          tmem_ld32(t_addr + c, v);
-          tmem_wait_ld();
-          const int col = (EPI == EPI_SWIGLU) ? (c < 128 ? tn * 128 + c : p.N / 2 + tn * 128 + (c - 128))
-                                              : tn * BN + c;
-          const int col_end = (EPI == EPI_SWIGLU) ? (c < 128 ? p.N / 2 : p.N) : p.N;
-          if (row_ok && col < col_end) {
-            if (col + 32 <= col_end) {
-              float4* d4 = reinterpret_cast<float4*>(dst_row + col);
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                d4[q] = make_float4(__uint_as_float(v[q * 4]), __uint_as_float(v[q * 4 + 1]),
-                                    __uint_as_float(v[q * 4 + 2]), __uint_as_float(v[q * 4 + 3]));
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (col + i < col_end) dst_row[col + i] = __uint_as_float(v[i]);
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_PLAIN || EPI == EPI_GATED_RESID || EPI == EPI_GELU) {
-        const int n0 = tn * BN;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t v[32];
-          tmem_ld32(t_addr + c, v);
-          tmem_wait_ld();
-          const int n = n0 + c;
-          if (row_ok && n < p.N) {
-            float f[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
-            const bool full32 = (n + 32 <= p.N);
-            if (p.bias) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (full32 || n + i < p.N) f[i] += __bfloat162float(p.bias[n + i]);
-            }
-            if constexpr (EPI == EPI_GELU) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) f[i] = gelu_erf(f[i]);
-            }
-            if constexpr (EPI == EPI_GATED_RESID) {
-              const bf16* g = p.gate ? p.gate + (long long)(m / p.rows_per_batch) * p.N + n : nullptr;
-              const bf16* r = p.R + (long long)m * p.ldr + n;
-              if (full32) {
-                const uint4* r4 = reinterpret_cast<const uint4*>(r);
-                const uint4* g4 = reinterpret_cast<const uint4*>(g);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint4 rv = r4[q];
-                  const uint32_t ru[4] = {rv.x, rv.y, rv.z, rv.w};
-                  uint32_t gu[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
-                  if (g) {
-                    const uint4 gv = g4[q];
-                    gu[0] = gv.x; gu[1] = gv.y; gu[2] = gv.z; gu[3] = gv.w;
-                  }
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    f[q * 8 + e * 2] = bf16lo(ru[e]) + bf16lo(gu[e]) * f[q * 8 + e * 2];
-                    f[q * 8 + e * 2 + 1] = bf16hi(ru[e]) + bf16hi(gu[e]) * f[q * 8 + e * 2 + 1];
-                  }
-                }
-              } else {
-                for (int i = 0; i < 32 && n + i < p.N; ++i) {
-                  const float gg = g ? __bfloat162float(g[i]) : 1.f;
-                  f[i] = __bfloat162float(r[i]) + gg * f[i];
-                }
+      for (int w = 0; w < NW && ok; ++w) {
+        const int half = (warp - 2) >> 2;
+        const int b = NW == 2 ? w : tcount & 1;
+        const uint32_t bph = NW == 2 ? tcount & 1 : (tcount >> 1) & 1;
+        ok = finish_half<EPI>(
+            p, slab, tmem_base + (uint32_t(quad * 32) << 16) + b * BN, half, m0, tr.m_end, tn * NW + w,
+            tl % p.k_splits, sgamma,
+            [&] {
+              const bool up = __all_sync(0xffffffffu, mbar_wait(tfull_bar(b), bph, abort_flag, p.status, ST_TIMEOUT_EPI));
+              tc_fence_after();
+              return up;
+            },
+            [&] {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                // the leader's MMA warp waits for both CTAs' epilogues
+                if (NC == 2 && cta_rank != 0) mbar_arrive_cluster(mapa(tempty_bar(b), 0));
+                else mbar_arrive(tempty_bar(b));
               }
-            }
-            bf16* dst = p.C + (long long)m * p.ldc + n;
-            if (full32) {
-              uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
-                o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
-                o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
-                o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
-                d4[q] = o;
-              }
-            } else {
-              for (int i = 0; i < 32 && n + i < p.N; ++i) dst[i] = __float2bfloat16(f[i]);
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_SWIGLU) {
-        // accumulator columns [0,128) = gate, [128,256) = up, for output columns tn*128 ...
-        const int n0 = tn * 128;
-        const int n_out = p.N / 2;
-#pragma unroll 1
-        for (int c = 0; c < 128; c += 32) {
-          uint32_t g[32], u[32];
-          tmem_ld32(t_addr + c, g);
-          tmem_ld32(t_addr + 128 + c, u);
-          tmem_wait_ld();
-          const int n = n0 + c;
-          if (row_ok && n < n_out) {
-            float f[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float gv = __uint_as_float(g[i]);
-              const float uv = __uint_as_float(u[i]);
-              f[i] = gv / (1.f + __expf(-gv)) * uv;
-            }
-            bf16* dst = p.C + (long long)m * p.ldc + n;
-            if (n + 32 <= n_out) {
-              uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
-                o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
-                o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
-                o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
-                d4[q] = o;
-              }
-            } else {
-              for (int i = 0; i < 32 && n + i < n_out; ++i) dst[i] = __float2bfloat16(f[i]);
-            }
-          }
-        }
-      } else if constexpr (EPI == EPI_ATTN_P || EPI == EPI_ATTN_DS) {
-        const int n0 = tn * BN;
-        const float rv = row_ok ? p.rowvec[m] : 0.f;
-        int lim = p.N;
-        if (p.attn_mask == MASK_CAUSAL) lim = min(p.N, m + 1 + (p.N - p.M));
-        if (p.attn_mask == MASK_MOT) lim = m < p.attn_n_ar ? m + 1 : p.N;
-        const float sl2 = p.attn_scale * 1.4426950408889634f;
-        const float rv2 = rv * 1.4426950408889634f;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          const int n = n0 + c;
-          if (n >= p.N) break;
-          uint32_t v[32];
-          tmem_ld32(t_addr + c, v);
-          tmem_wait_ld();
-          if (row_ok) {
-            float f[32];
-            const bool full32 = (n + 32 <= p.N);
-            if constexpr (EPI == EPI_ATTN_P) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                f[i] = (n + i < lim) ? exp2f(fmaf(__uint_as_float(v[i]), sl2, -rv2)) : 0.f;
-            } else {
-              const bf16* pr = p.R + (long long)m * p.ldr + n;
-              if (full32) {
-                const uint4* r4 = reinterpret_cast<const uint4*>(pr);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint4 rr = r4[q];
-                  const uint32_t ru[4] = {rr.x, rr.y, rr.z, rr.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    f[q * 8 + 2 * e] = bf16lo(ru[e]) * (__uint_as_float(v[q * 8 + 2 * e]) - rv) * p.attn_scale;
-                    f[q * 8 + 2 * e + 1] = bf16hi(ru[e]) * (__uint_as_float(v[q * 8 + 2 * e + 1]) - rv) * p.attn_scale;
-                  }
-                }
-              } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  f[i] = (n + i < p.N) ? __bfloat162float(pr[i]) * (__uint_as_float(v[i]) - rv) * p.attn_scale : 0.f;
-              }
-            }
-            bf16* dst = p.C + (long long)m * p.ldc + n;
-            if (full32) {
-              uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
-                o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
-                o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
-                o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
-                d4[q] = o;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (n + i < p.N) dst[i] = __float2bfloat16(f[i]);
-            }
-          }
-        }
-      } else {  // EPI_QKV_ROPE: two heads (128-column chunks) per tile
-#pragma unroll 1
-        for (int hc = 0; hc < 2; ++hc) {
-          const int chunk = tn * 2 + hc;
-          const int n = chunk * 128;
-          float f[128];
-#pragma unroll
-          for (int c = 0; c < 128; c += 32) {
-            uint32_t v[32];
-            tmem_ld32(t_addr + hc * 128 + c, v);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) f[c + i] = __uint_as_float(v[i]);
-          }
-          if (row_ok && n < p.N) {
-            if (p.bias) {
-#pragma unroll
-              for (int i = 0; i < 128; ++i) f[i] += __bfloat162float(p.bias[n + i]);
-            }
-            const int kind = chunk < p.n_q_heads ? 1 : (chunk < p.n_q_heads + p.n_k_heads ? 2 : 0);
-            if (kind != 0) {
-              const bf16* gam = kind == 1 ? p.gamma_q : p.gamma_k;
-              if (gam) {
-                float ss = 0.f;
-#pragma unroll
-                for (int i = 0; i < 128; ++i) ss += f[i] * f[i];
-                const float rinv = rsqrtf(ss * (1.f / 128.f) + p.eps);
-#pragma unroll
-                for (int i = 0; i < 128; ++i) f[i] = f[i] * rinv * __bfloat162float(gam[i]);
-              }
-              if (p.cos_tab) {
-                const float4* ct =
-                    reinterpret_cast<const float4*>(p.cos_tab + (long long)(m % p.rope_rows) * 64);
-                const float4* st =
-                    reinterpret_cast<const float4*>(p.sin_tab + (long long)(m % p.rope_rows) * 64);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                  const float4 c4 = ct[q], s4 = st[q];
-                  const float cc[4] = {c4.x, c4.y, c4.z, c4.w};
-                  const float sn[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const int i = q * 4 + e;
-                    const float a = f[i], bb = f[i + 64];
-                    f[i] = a * cc[e] - bb * sn[e];
-                    f[i + 64] = bb * cc[e] + a * sn[e];
-                  }
-                }
-              }
-            }
-            bf16* dst;
-            if (p.route_ptr) {
-              dst = reinterpret_cast<bf16*>(p.route_ptr[chunk]) + (long long)m * p.route_ld[chunk];
-            } else {
-              dst = p.C + (long long)m * p.ldc + n;
-            }
-            uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              uint4 o;
-              o.x = pack_bf16(f[q * 8 + 0], f[q * 8 + 1]);
-              o.y = pack_bf16(f[q * 8 + 2], f[q * 8 + 3]);
-              o.z = pack_bf16(f[q * 8 + 4], f[q * 8 + 5]);
-              o.w = pack_bf16(f[q * 8 + 6], f[q * 8 + 7]);
-              d4[q] = o;
-            }
-          }
-        }
+            });
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (NC == 2 && cta_rank != 0)
-          mbar_arrive_cluster(mapa(tempty_bar(b), 0));  // the leader's MMA warp waits for both CTAs' epilogues
-        else
-          mbar_arrive(tempty_bar(b));
-      }
+      if (!ok) break;
     }
   }
 
@@ -903,13 +1123,13 @@ static bool pair_enabled() {
   return g_pair == 1;
 }
 
-template <int EPI, int NC>
+template <int EPI, int NC, int NW>
 static int max_grid() {
   // NC == 1: one CTA per SM. NC == 2: as many CTA pairs as the device can hold at once.
   static int n = 0;
   if (n) return n;
-  cudaFuncSetAttribute(cb::gemm_bf16_kernel<EPI, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       cb::GemmCfg<NC>::SMEM);
+  cudaFuncSetAttribute(cb::gemm_bf16_kernel<EPI, NC, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (cb::GemmCfg<NC, NW>::SMEM + cb::gamma_smem(EPI)));
   if (NC == 1) {
     n = sm_count();
     return n;
@@ -917,13 +1137,13 @@ static int max_grid() {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
   cfg.blockDim = dim3(cb::GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = cb::GemmCfg<NC>::SMEM;
+  cfg.dynamicSmemBytes = (cb::GemmCfg<NC, NW>::SMEM + cb::gamma_smem(EPI));
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, cb::gemm_bf16_kernel<EPI, NC>, &cfg) != cudaSuccess || clusters < 1) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, cb::gemm_bf16_kernel<EPI, NC, NW>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
     clusters = sm_count() / 2;
   }
@@ -933,9 +1153,9 @@ static int max_grid() {
 }
 
 // `units` = number of tiles (of CTA pairs when NC == 2); `limit` caps the number of CTAs (0 = none).
-template <int EPI, int NC>
+template <int EPI, int NC, int NW = 1>
 static void launch(const CUtensorMap* maps, const cb::GemmGroup& g, int units, int limit, cudaStream_t stream) {
-  int grid = max_grid<EPI, NC>();
+  int grid = max_grid<EPI, NC, NW>();
   if (limit > 0 && grid > limit) grid = limit;
   if (NC == 2) {
     grid &= ~1;
@@ -947,7 +1167,7 @@ static void launch(const CUtensorMap* maps, const cb::GemmGroup& g, int units, i
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(cb::GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = cb::GemmCfg<NC>::SMEM;
+  cfg.dynamicSmemBytes = (cb::GemmCfg<NC, NW>::SMEM + cb::gamma_smem(EPI));
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -955,7 +1175,7 @@ static void launch(const CUtensorMap* maps, const cb::GemmGroup& g, int units, i
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = (NC == 1 && pdl_on() && !g.p[0].tile_map) ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, cb::gemm_bf16_kernel<EPI, NC>, maps[0], maps[1], maps[2], maps[3], g);
+  cudaLaunchKernelEx(&cfg, cb::gemm_bf16_kernel<EPI, NC, NW>, maps[0], maps[1], maps[2], maps[3], g);
 }
 
 template <int NC>
@@ -973,7 +1193,22 @@ static void launch_epi(int epi, const CUtensorMap* maps, const cb::GemmGroup& g,
   }
 }
 
-static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, int nc = 1) {
+// Epilogues that exist for the 256x512 tile.
+static void launch_wide(int epi, const CUtensorMap* maps, const cb::GemmGroup& g, int units, int limit, cudaStream_t stream) {
+  switch (epi) {
+    case EPI_PLAIN: launch<EPI_PLAIN, 2, 2>(maps, g, units, limit, stream); break;
+    case EPI_GELU: launch<EPI_GELU, 2, 2>(maps, g, units, limit, stream); break;
+    case EPI_SWIGLU: launch<EPI_SWIGLU, 2, 2>(maps, g, units, limit, stream); break;
+    case EPI_GATED_RESID: launch<EPI_GATED_RESID, 2, 2>(maps, g, units, limit, stream); break;
+    case EPI_QKV_ROPE: launch<EPI_QKV_ROPE, 2, 2>(maps, g, units, limit, stream); break;
+    default: throw std::runtime_error("gemm_bf16: unknown epilogue");
+  }
+}
+static bool wide_epi(int epi) {
+  return epi == EPI_PLAIN || epi == EPI_GELU || epi == EPI_SWIGLU || epi == EPI_GATED_RESID || epi == EPI_QKV_ROPE;
+}
+
+static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, CUtensorMap& tb, int nc = 1, int nw = 1) {
   // TMA needs 16-byte row strides; a ragged K is fine (out-of-range columns are zero-filled)
   if (a.lda % 8 != 0 || a.ldb % 8 != 0)
     throw std::runtime_error("gemm_bf16: leading dimensions must be multiples of 8");
@@ -1014,10 +1249,10 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.m_tiles = (a.M + cb::BM * nc - 1) / (cb::BM * nc);
   if (a.epi == EPI_SWIGLU) {
-    p.n_tiles = (a.N / 2 + 127) / 128;
+    p.n_tiles = (a.N / 2 + 128 * nw - 1) / (128 * nw);
     p.b_row1 = a.N / 2;
   } else {
-    p.n_tiles = (a.N + cb::BN - 1) / cb::BN;
+    p.n_tiles = (a.N + cb::BN * nw - 1) / (cb::BN * nw);
     p.b_row1 = 128;
   }
   p.C = reinterpret_cast<bf16*>(a.C); p.ldc = a.ldc;
@@ -1081,35 +1316,63 @@ int gemm_pick_k_splits(int M, int N, int K, int epi) {
   return best;
 }
 
+// Tile of a problem taller than 128 rows: 128x256 on single CTAs (only for SwiGLU, whose pairs of 256x256 are slower), 256x256
+// or 256x512 on CTA pairs. All three are bound by the bytes that a CTA stages per k-block (48, 32 and 48 KB), so the cost
+// of a launch is its rounds of the persistent CTAs times those bytes; ties go to the larger tile where that does not pad more
+// rows. The norm and rotary epilogue holds an accumulator for about 3 us, which 256x512 tiles hide only in part: counted
+// like 10 k-blocks.
+// Measured, 256x256 (SwiGLU: 128x256) -> 256x512, us: N x K = 24576 x 4096 SwiGLU M 14080 2291 -> 1821, M 1920 319 -> 290;
+// 4096 x 12288 residual M 14080 1143 -> 924, M 3600 352 -> 272; 4096 x 4096 residual M 3600 124 -> 103; 6144 x 4096 with
+// norm and rotary embedding M 14080 577 -> 550, but M 1920 101 -> 118.
+static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) {
+  const int ctas = limit > 0 && limit < sm_count() ? limit : sm_count();
+  const int epi = args[0].epi, k_blocks = (args[0].K + cb::BK - 1) / cb::BK;
+  auto cost = [&](int c, int w, int kb_bytes) {
+    long long tiles = 0;
+    for (int i = 0; i < n; ++i) {
+      const int cols = epi == EPI_SWIGLU ? args[i].N / 2 : args[i].N;
+      const int tile_n = (epi == EPI_SWIGLU ? 128 : cb::BN) * w;
+      tiles += (long long)((args[i].M + cb::BM * c - 1) / (cb::BM * c)) * ((cols + tile_n - 1) / tile_n);
+    }
+    const int at_once = ctas / c > 0 ? ctas / c : 1;
+    return (tiles + at_once - 1) / at_once * kb_bytes * (k_blocks + (w == 2 && epi == EPI_QKV_ROPE ? 10 : 0));
+  };
+  const bool single = epi == EPI_SWIGLU;
+  nc = single ? 1 : 2;
+  nw = 1;
+  if (wide_epi(epi) && cost(2, 2, 48) <= (single ? cost(1, 1, 48) - 1 : cost(2, 1, 32))) nc = nw = 2;
+}
+
 // One launch for one or two problems that share the epilogue kind.
 void gemm_bf16_grouped(const GemmArgs* args, int n, cudaStream_t stream) {
   if (n < 1 || n > 2) throw std::runtime_error("gemm_bf16_grouped: 1 or 2 problems per launch");
   if (n == 2 && args[0].epi != args[1].epi)
     throw std::runtime_error("gemm_bf16_grouped: both problems must use the same epilogue");
-  // CTA pairs (256-row tiles) as soon as a problem has more than one 128-row tile
   const bool two = n == 2 && args[1].M > 0;
-  // (not for the SwiGLU epilogue: measured 3 - 10 % slower on pairs at 16384 x 24576 x 4096)
+  if (args[0].epi == EPI_QKV_ROPE && two) throw std::runtime_error("gemm_bf16_grouped: the QKV epilogue takes one problem");
   if (args[0].tile_map && two) throw std::runtime_error("gemm_bf16_grouped: a tile map takes one problem");
-  const int nc = args[0].tile_map ? args[0].tile_m / cb::BM
-                 : (pair_enabled() && args[0].epi != EPI_SWIGLU && (args[0].M > cb::BM || (two && args[1].M > cb::BM)))
-                     ? 2 : 1;
+  int limit = args[0].max_ctas > 0 ? args[0].max_ctas : 0;
+  if (g_grid_limit > 0 && (limit == 0 || limit > g_grid_limit)) limit = g_grid_limit;
+  int nc = args[0].tile_map ? args[0].tile_m / cb::BM : 1, nw = 1;
+  if (!args[0].tile_map && pair_enabled() && (args[0].M > cb::BM || (two && args[1].M > cb::BM)))
+    pick_tile(args, two ? 2 : 1, limit, nc, nw);
   if (nc != 1 && nc != 2) throw std::runtime_error("gemm_bf16_grouped: tile rows must be 128 or 256");
   cb::GemmGroup g{};
   CUtensorMap maps[4];
-  fill_problem(args[0], g.p[0], maps[0], maps[1], nc);
+  fill_problem(args[0], g.p[0], maps[0], maps[1], nc, nw);
   g.tiles0 = g.p[0].m_tiles * g.p[0].n_tiles;
   g.total = g.tiles0;
   if (two) {
-    fill_problem(args[1], g.p[1], maps[2], maps[3], nc);
+    fill_problem(args[1], g.p[1], maps[2], maps[3], nc, nw);
     g.total += g.p[1].m_tiles * g.p[1].n_tiles;
   } else {
     maps[2] = maps[0];
     maps[3] = maps[1];
   }
   if (g.total == 0) return;
-  int limit = args[0].max_ctas > 0 ? args[0].max_ctas : 0;
-  if (g_grid_limit > 0 && (limit == 0 || limit > g_grid_limit)) limit = g_grid_limit;
-  if (nc == 2)
+  if (nw == 2)
+    launch_wide(args[0].epi, maps, g, g.total, limit, stream);
+  else if (nc == 2)
     launch_epi<2>(args[0].epi, maps, g, g.total, limit, stream);
   else
     launch_epi<1>(args[0].epi, maps, g, g.total, limit, stream);

@@ -1062,3 +1062,67 @@ def test_vae_decode_to_host_is_the_decode(t, chunk):
     with torch.cuda.stream(side):
         got = dec.decode_to_host(z, chunk_latents=chunk)
     assert torch.equal(got, dec.decode(z, chunk_latents=chunk)[0].cpu())
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 512, 64), (300, 768, 136), (513, 1032, 320), (700, 1536, 1088), (1024, 2048, 192),
+                                    (257, 1024, 2048)])
+def test_gemm_wide_tiles(m, n, k):
+    """256x512 tiles (a launch of one or two CTA pairs takes them at these sizes) against the fp32 definition, for each
+    epilogue and operand order; ragged rows, columns, k-blocks and an odd number of 256-column tiles. A tile's products are
+    summed in the same order whichever pair computes it, so both launches give the same bits."""
+    torch.manual_seed(41)
+    kern = torch.ops.cosmos_b200
+    a, w, r = _rand(m, k), _rand(n, k, scale=1 / math.sqrt(k)), _rand(m, n)
+    bias, gate = _rand(n), _rand(2, n)
+    rpb = (m + 1) // 2
+    wt = w.t().contiguous()
+    ang = torch.rand(m, 64, device=DEV) * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    gamma = (1 + 0.1 * torch.randn(128, device=DEV)).bfloat16()
+    calls = {
+        "plain": lambda: ops.gemm(a, w, bias),
+        "resid": lambda: ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, gate, rpb),
+        "b_mn": lambda: kern.gemm_ex(a, wt, False, True, None),
+    }
+    want = {"plain": a.float() @ w.float().t() + bias.float(),
+            "resid": ref.gemm(a.float(), w.float(), None, ops.EPI_GATED_RESID, r.float(), gate.float(), rpb),
+            "b_mn": a.float() @ w.float().t()}
+    if n % 16 == 0:
+        calls["swiglu"] = lambda: ops.gemm(a, w, epi=ops.EPI_SWIGLU)
+        want["swiglu"] = ref.gemm(a.float(), w.float(), epi=ops.EPI_SWIGLU)
+    if n % 128 == 0:
+        hq, gf = n // 128 - 2, gamma.float()
+        calls["qkv"] = lambda: ops.gemm_qkv_rope(a, w, bias, cos, sin, gamma, gamma, hq, 1, 1e-6)
+        want["qkv"] = ref.gemm_qkv_rope(a.float(), w.float(), bias.float(), cos, sin, gf, gf, hq, 1, 1e-6)
+        calls["qkv plain"] = lambda: ops.gemm_qkv_rope(a, w, None, None, None, None, None, hq, 1, 1e-6)
+        want["qkv plain"] = want["b_mn"]
+    if m % 8 == 0:
+        at = a.t().contiguous()
+        calls["a_mn"] = lambda: kern.gemm_ex(at, wt, True, True, None)
+        want["a_mn"] = want["b_mn"]
+    try:
+        for name, call in calls.items():
+            got = {}
+            for limit in (2, 4):
+                kern.gemm_set_grid_limit(limit)
+                got[limit] = call().clone()
+            _close(got[2], want[name], 3e-2, 2e-2, f"{name} {m}x{n}x{k}")
+            assert torch.equal(got[2], got[4]), name
+    finally:
+        kern.gemm_set_grid_limit(0)
+
+
+def test_gemm_swiglu_keeps_the_limits_of_silu():
+    """Gates beyond the range in which the quotient of silu is corrected: large of both signs, tiny, zero, infinite."""
+    k = 64
+    g = torch.tensor([0.0, 1e-38, -1e-38, 1e-30, 79.0, -79.0, 81.0, -81.0, -87.0, -88.0, -89.0, -200.0, 3e38, -3e38, math.inf, 1.0])
+    a = torch.zeros(300, k, device=DEV, dtype=torch.bfloat16)
+    a[:, 0] = 1
+    w = torch.zeros(32, k, device=DEV, dtype=torch.bfloat16)
+    w[:16, 0] = g.to(DEV).bfloat16()
+    w[16:, 0] = 1
+    got = ops.gemm(a, w, epi=ops.EPI_SWIGLU)
+    want = torch.nn.functional.silu(w[:16, 0].double())
+    fin = torch.isfinite(want)
+    _close(got[:, fin], want[fin].expand(300, -1), 1e-35, 8e-3, "silu")
+    assert (got[:, ~fin] == math.inf).all()
