@@ -180,14 +180,14 @@ class WorkspaceAttn(AttnContext):
             qb = torch.empty(b, s, hq, hd, dtype=like.dtype, device=like.device)
             kb = torch.empty(b, n_pre + s, hk, hd, dtype=like.dtype, device=like.device)
             vb = torch.empty_like(kb)
-            routes = []
+            ptrs, lds = [], []
             for bi in range(b):
-                ptrs = ([qb[bi].data_ptr() + j * hd * 2 for j in range(hq)]
+                ptrs += ([qb[bi].data_ptr() + j * hd * 2 for j in range(hq)]
                         + [kb[bi, n_pre:].data_ptr() + j * hd * 2 for j in range(hk)]
                         + [vb[bi, n_pre:].data_ptr() + j * hd * 2 for j in range(hk)])
-                lds = [hq * hd] * hq + [hk * hd] * (2 * hk)
-                routes.append((torch.tensor(ptrs, dtype=torch.int64, device=like.device),
-                               torch.tensor(lds, dtype=torch.int64, device=like.device)))
+                lds += [hq * hd] * hq + [hk * hd] * (2 * hk)
+            routes = (torch.tensor(ptrs, dtype=torch.int64, device=like.device),
+                      torch.tensor(lds, dtype=torch.int64, device=like.device))
             self._ws[key] = (qb, kb, vb, routes)
         return self._ws[key]
 
@@ -203,9 +203,10 @@ class WorkspaceAttn(AttnContext):
             vb[:, :n_pre].copy_(prefix[1])
         gq = q_norm if cfg.qk_norm else None
         gk = k_norm if cfg.qk_norm else None
-        for bi in range(b):
-            ops.gemm_qkv_rope(h[bi], w, None, cos, sin, gq, gk, cfg.n_heads, cfg.n_kv_heads, cfg.rms_eps,
-                              routes[bi][0], routes[bi][1])
+        # all batch entries in one launch, each through its own routing table (guided steps: two branches; at 240 tokens a
+        # branch, where 24 pairs of CTAs have a tile each, the two launches took 79 us and one takes 42)
+        ops.gemm_qkv_rope(h.reshape(b * s, -1), w, None, cos, sin, gq, gk, cfg.n_heads, cfg.n_kv_heads, cfg.rms_eps,
+                          *routes, route_rows=s)
         return qb, kb, vb
 
 
@@ -239,6 +240,10 @@ def dm_modulation(t_mod: torch.Tensor, mod_table: torch.Tensor) -> List[torch.Te
     -> six [B, d] tensors: shift1, scale1, gate1, shift2, scale2, gate2."""
     b = t_mod.shape[0]
     d = mod_table.shape[-1]
+    if t_mod.dtype == mod_table.dtype and not torch.is_grad_enabled():
+        # one sum and (b > 1) one copy in place of three casts, the sum and six copies; an addition of two bf16 tensors is
+        # rounded once, as the fp32 sum's cast is
+        return list((t_mod.view(b, 6, d).transpose(0, 1) + mod_table[:, None]).contiguous().unbind(0))
     m = (t_mod.view(b, 6, d).float() + mod_table.float()[None]).to(t_mod.dtype)
     return [m[:, i].contiguous() for i in range(6)]
 

@@ -15,11 +15,11 @@ from typing import Optional, Sequence, Tuple
 import torch
 
 
-def axis_of_frequency(half_dim: int, section: Sequence[int]) -> torch.Tensor:
+def axis_of_frequency(half_dim: int, section: Sequence[int], device=None) -> torch.Tensor:
     """For each of the half_dim rotary frequencies: which axis (0=t, 1=h, 2=w) drives it."""
     st, sh, sw = section
     assert st + sh + sw == half_dim, f"mrope_section {section} must sum to {half_dim}"
-    axis = torch.zeros(half_dim, dtype=torch.long)
+    axis = torch.zeros(half_dim, dtype=torch.long, device=device)
     axis[1:sh * 3:3] = 1
     axis[2:sw * 3:3] = 2
     return axis
@@ -30,7 +30,7 @@ def rope_tables(pos: torch.Tensor, head_dim: int, theta: float, section: Sequenc
     """pos [3, S] (t, h, w) -> cos, sin [S, head_dim/2] fp32 (rotate-half convention)."""
     half = head_dim // 2
     inv_freq = 1.0 / (theta ** (torch.arange(0, half, dtype=torch.float64, device=pos.device) * 2.0 / head_dim))
-    axis = axis_of_frequency(half, section).to(pos.device)
+    axis = axis_of_frequency(half, section, pos.device)   # filled on the device: a copy from the host would wait for the stream
     p = pos.to(torch.float64)[axis, :]            # [half, S]
     ang = (p * inv_freq[:, None]).t().contiguous()  # [S, half]
     return ang.cos().float().contiguous(), ang.sin().float().contiguous()

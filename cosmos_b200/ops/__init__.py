@@ -208,10 +208,12 @@ def linear(x, w, bias=None):
 
 
 def gemm_qkv_rope(a, w, bias, cos, sin, gamma_q, gamma_k, n_q_heads: int, n_k_heads: int,
-                  eps: float = 1e-6, route_ptr=None, route_ld=None, out=None):
+                  eps: float = 1e-6, route_ptr=None, route_ld=None, out=None, route_rows: int = 0):
+    """QKV projection with per-head norm and rotary embedding. `route_ptr` / `route_ld` (one entry per head) send each
+    head's columns to buffers of their own; with `route_rows`, one such table for every route_rows rows of a."""
     if _use_cuda(a, w, bias, gamma_q, gamma_k):
         return _k().gemm_qkv_rope(a, w, bias, cos, sin, gamma_q, gamma_k, n_q_heads, n_k_heads, eps,
-                                  route_ptr, route_ld, out)
+                                  route_ptr, route_ld, out, route_rows)
     assert route_ptr is None, "routed epilogue is CUDA-only"
     if _library(a):
         from . import library as lib

@@ -277,7 +277,7 @@ std::tuple<Tensor, Tensor> gemm_grouped2(const Tensor& A0_, const Tensor& W0, co
 Tensor gemm_qkv_rope(const Tensor& A_, const Tensor& W, const OptT& bias, const OptT& cos_t,
                      const OptT& sin_t, const OptT& gamma_q, const OptT& gamma_k, int64_t n_q_heads,
                      int64_t n_k_heads, double eps, const OptT& route_ptr, const OptT& route_ld,
-                     const OptT& out) {
+                     const OptT& out, int64_t route_rows) {
   check_bf16_cuda(A_, "A");
   check_bf16_cuda(W, "W");
   c10::cuda::CUDAGuard guard(A_.device());
@@ -291,8 +291,12 @@ Tensor gemm_qkv_rope(const Tensor& A_, const Tensor& W, const OptT& bias, const 
   if (routed) {
     TORCH_CHECK(route_ld.has_value() && route_ptr->scalar_type() == at::kLong &&
                     route_ld->scalar_type() == at::kLong && route_ptr->is_cuda() &&
-                    route_ptr->numel() == N / 128 && route_ld->numel() == N / 128,
-                "route tables must be int64 CUDA tensors with one entry per head");
+                    route_rows >= 0 && (route_rows == 0 || M % route_rows == 0) &&
+                    route_ptr->numel() == N / 128 * (route_rows ? M / route_rows : 1) &&
+                    route_ld->numel() == route_ptr->numel() &&
+                    (!route_rows || (route_ptr->is_contiguous() && route_ld->is_contiguous())),
+                "route tables must be int64 CUDA tensors with one entry per head (and per route_rows rows)");
+    g.route_rows = (int)route_rows;
     g.route_ptr = reinterpret_cast<const long long*>(route_ptr->data_ptr<int64_t>());
     g.route_ld = reinterpret_cast<const long long*>(route_ld->data_ptr<int64_t>());
     C = out.has_value() && out->defined() ? *out : at::empty({0}, A.options());
@@ -1327,7 +1331,9 @@ void allgather_pull(const Tensor& srcs, int64_t world, Tensor dst, int64_t bytes
 TORCH_LIBRARY(cosmos_b200, m) {
   m.def("status_word", &status_word);
   m.def("gemm", &gemm);
-  m.def("gemm_qkv_rope", &gemm_qkv_rope);
+  m.def("gemm_qkv_rope(Tensor a, Tensor w, Tensor? bias, Tensor? cos, Tensor? sin, Tensor? gamma_q, Tensor? gamma_k, "
+        "int n_q_heads, int n_k_heads, float eps, Tensor? route_ptr, Tensor? route_ld, Tensor? out, int route_rows=0) -> Tensor",
+        &gemm_qkv_rope);
   m.def("gemm_grouped2", &gemm_grouped2);
   m.def("gemm_ex", &gemm_ex);
   m.def("gemm_reduce_rmsnorm", &gemm_reduce_rmsnorm);

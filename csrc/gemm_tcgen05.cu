@@ -67,6 +67,7 @@ struct GemmParams {
   // EPI_QKV_ROPE
   const long long* route_ptr;  // per 128-col chunk: destination base address (bf16*)
   const long long* route_ld;   // per chunk: row stride in elements
+  int route_rows;              // rows per routing table: row m goes through table m / route_rows, as its row m % route_rows
   const float* cos_tab;        // [rope_rows, 64]
   const float* sin_tab;
   int rope_rows;
@@ -282,8 +283,26 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
   }
   if constexpr (EPI == EPI_QKV_ROPE) {
     const int chunk = tn * 2 + half;
-    bf16* dst = p.route_ptr ? reinterpret_cast<bf16*>(p.route_ptr[chunk]) : p.C + n0;
-    const long long ld = p.route_ptr ? p.route_ld[chunk] : p.ldc;
+    // This warp's rows lie in one routing table or, from row `next` on, in the one after it (any, with short tables).
+    const int t_rows = p.route_rows, tab0 = p.route_ptr ? m0 / t_rows : 0, next = p.route_ptr ? (tab0 + 1) * t_rows - m0 : 32;
+    const int chunks = p.N >> 7;
+    const bool crosses = p.route_ptr && next < min(rows, 32);
+    long long ld = p.ldc, ld1 = 0;
+    bf16 *dst = p.C + n0, *dst1 = nullptr;   // where row m0 = 0 of either table would lie
+    if (p.route_ptr) {
+      ld = p.route_ld[tab0 * chunks + chunk];
+      dst = reinterpret_cast<bf16*>(p.route_ptr[tab0 * chunks + chunk]) - (long long)tab0 * t_rows * ld;
+    }
+    if (crosses) {
+      ld1 = p.route_ld[(tab0 + 1) * chunks + chunk];
+      dst1 = reinterpret_cast<bf16*>(p.route_ptr[(tab0 + 1) * chunks + chunk]) - (long long)(tab0 + 1) * t_rows * ld1;
+    }
+    auto row_at = [&](int r) -> bf16* {
+      if (!crosses || r < next) return dst + (m0 + r) * ld;
+      if (r < next + t_rows) return dst1 + (m0 + r) * ld1;
+      const int t = (m0 + r) / t_rows;
+      return reinterpret_cast<bf16*>(p.route_ptr[t * chunks + chunk]) + (long long)(m0 + r - t * t_rows) * p.route_ld[t * chunks + chunk];
+    };
     if (chunk < p.n_q_heads + p.n_k_heads && (p.gamma_q || p.gamma_k || p.cos_tab)) {
       // Norm and rotary embedding of one head. 16 columns of both tables at a time go through the slab (chunks 0-3 of a row
       // cosines, 4-7 sines), requested two steps ahead: their latency would otherwise hold the accumulator. The norm's
@@ -379,7 +398,7 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
         for (int i = 0; i < 4; ++i) {   // 8 rows of 2 x 32 bytes per instruction
           const int r = i * 8 + (lane >> 2), c = lane & 3;
           const uint4 v = slab.get(r, c);
-          if (r < rows) *reinterpret_cast<uint4*>(dst + (m0 + r) * ld + (c >> 1) * 64 + q * 16 + (c & 1) * 8) = v;
+          if (r < rows) *reinterpret_cast<uint4*>(row_at(r) + (c >> 1) * 64 + q * 16 + (c & 1) * 8) = v;
         }
         __syncwarp();
       };
@@ -405,7 +424,16 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) slab.put_bf16((c & 1) * 4 + q, f + q * 8);
-      if (c & 1) slab.store(dst + (long long)m0 * ld + (c >> 1) * 64, ld, rows, 64);
+      if (c & 1) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = i * 4 + (lane >> 3);
+          const uint4 o = slab.get(r, lane & 7);
+          if (r < rows) *reinterpret_cast<uint4*>(row_at(r) + (c >> 1) * 64 + (lane & 7) * 8) = o;
+        }
+        __syncwarp();
+      }
     }
     return true;
   }
@@ -1261,6 +1289,7 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
   p.gate = reinterpret_cast<const bf16*>(a.gate);
   p.rows_per_batch = a.rows_per_batch > 0 ? a.rows_per_batch : (a.M > 0 ? a.M : 1);
   p.route_ptr = a.route_ptr; p.route_ld = a.route_ld;
+  p.route_rows = a.route_rows > 0 ? a.route_rows : (a.M > 0 ? a.M : 1);
   p.cos_tab = a.cos_tab; p.sin_tab = a.sin_tab; p.rope_rows = a.rope_rows > 0 ? a.rope_rows : 1;
   p.gamma_q = reinterpret_cast<const bf16*>(a.gamma_q);
   p.gamma_k = reinterpret_cast<const bf16*>(a.gamma_k);

@@ -46,6 +46,7 @@ struct GemmArgs {
   int rows_per_batch = 0;
   const long long* route_ptr = nullptr;  // device arrays, one entry per 128-column chunk
   const long long* route_ld = nullptr;
+  int route_rows = 0;  // > 0: row m goes through the (m / route_rows)-th table of such entries, as its row m % route_rows
   const float* cos_tab = nullptr;  // [rope_rows, 64]
   const float* sin_tab = nullptr;
   int rope_rows = 0;

@@ -1126,3 +1126,33 @@ def test_gemm_swiglu_keeps_the_limits_of_silu():
     fin = torch.isfinite(want)
     _close(got[:, fin], want[fin].expand(300, -1), 1e-35, 8e-3, "silu")
     assert (got[:, ~fin] == math.inf).all()
+
+
+@pytest.mark.parametrize("batch,rows", [(1, 40), (2, 240), (3, 100), (5, 33), (9, 20), (40, 7)])
+def test_gemm_qkv_rope_routed_by_batch(batch, rows):
+    """One routing table per batch entry: the same bits in every buffer as one launch per entry, whichever tables a tile or
+    a warp's 32 rows cross; rows that belong to nobody stay untouched."""
+    torch.manual_seed(43)
+    k, hq, hk, pre = 256, 4, 2, 3
+    a = _rand(batch, rows, k)
+    w = _rand((hq + 2 * hk) * 128, k, scale=1 / math.sqrt(k))
+    ang = torch.rand(rows, 64, device=DEV) * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    gamma = (1 + 0.1 * torch.randn(128, device=DEV)).bfloat16()
+    outs = []
+    for merged in (False, True):
+        q = torch.full((batch, rows, hq, 128), 7.0, device=DEV, dtype=torch.bfloat16)
+        kv = torch.full((2, batch, pre + rows, hk, 128), 7.0, device=DEV, dtype=torch.bfloat16)
+        ptr = torch.tensor([[q[b, :, j].data_ptr() for j in range(hq)] + [kv[i, b, pre:, j].data_ptr() for i in (0, 1) for j in range(hk)]
+                            for b in range(batch)], device=DEV)
+        ld = torch.tensor([[hq * 128] * hq + [hk * 128] * 2 * hk] * batch, device=DEV)
+        if merged:
+            ops.gemm_qkv_rope(a.view(batch * rows, k), w, None, cos, sin, gamma, gamma, hq, hk, 1e-6, ptr, ld, route_rows=rows)
+        else:
+            for b in range(batch):
+                ops.gemm_qkv_rope(a[b], w, None, cos, sin, gamma, gamma, hq, hk, 1e-6, ptr[b].contiguous(), ld[b].contiguous())
+        outs.append((q, kv))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert (outs[1][1][:, :, :pre] == 7).all()
+    want = ref.gemm_qkv_rope(a[-1].float(), w.float(), None, cos, sin, gamma.float(), gamma.float(), hq, hk, 1e-6)
+    _close(outs[1][0][-1].reshape(rows, -1), want[:, :hq * 128], 3e-2, 2e-2, "routed by batch")
