@@ -87,6 +87,12 @@ struct GemmParams {
   // operand majors: 0 = K-major ([rows, K] storage), 1 = MN-major ([K, rows] storage, i.e. the
   // transposed operand is read in place; used by the backward GEMMs dX = dY W and dW = dY^T X)
   int a_mn, b_mn;
+  // Rows of A that a single CTA's stage receives: 128, or 8 or 16 in a decode step of so few sequences. The rows behind them
+  // keep what was there before: products of theirs land in accumulator rows that nobody reads. Zero-filling them took a
+  // third of the bytes that reach a CTA, and these launches are bound by that, not by HBM: with the weights resident in L2
+  // they took as long. M 1, with the reduction, us: 24576 x 4096 SwiGLU 42.3 -> 38.2, 6144 x 4096 15.9 -> 14.3, 151936 x 4096
+  // 229 -> 212. With 32 rows nothing is gained (43.0 -> 43.1): there the fp32 partial sums weigh more.
+  int a_rows;
   // grouped by a tile map (see the file comment): {group, first row, rows, unused} per m-tile; tile rows = TILE_M
   const int4* tile_map;
   const int* n_tiles_m;  // number of m-tiles of this launch (device)
@@ -642,7 +648,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int n0 = (EPI == EPI_SWIGLU) ? tn * 128 : tn * BN;
       for (int kb = kb0; kb < kb1 && prefetched < STAGES; ++kb, ++prefetched) {
         const uint32_t sa = smem_base + prefetched * STAGE_BYTES;
-        mbar_arrive_expect_tx(full_bar(prefetched), STAGE_BYTES);
+        mbar_arrive_expect_tx(full_bar(prefetched), B_BYTES + p.a_rows * BK * 2);
         tma_load_2d(sa + A_BYTES, &tmB, full_bar(prefetched), kb * BK, n0);
         tma_load_2d(sa + A_BYTES + B_BYTES / 2, &tmB, full_bar(prefetched), kb * BK, n0 + p.b_row1);
       }
@@ -732,7 +738,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             continue;
           }
-          mbar_arrive_expect_tx(full_bar(s), STAGE_BYTES);
+          mbar_arrive_expect_tx(full_bar(s), B_BYTES + p.a_rows * BK * 2);
           if (p.a_mn) {
             tma_load_2d(sa, mA, full_bar(s), m0, kb * BK);
             tma_load_2d(sa + A_BYTES / 2, mA, full_bar(s), m0 + 64, kb * BK);
@@ -1248,7 +1254,8 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
     throw std::runtime_error("gemm_bf16: ldc must be a multiple of 8");
   const uint64_t dimsA[2] = {(uint64_t)a.K, (uint64_t)a.M};
   const uint64_t strA[1] = {(uint64_t)a.lda * 2};
-  const uint32_t boxA[2] = {cb::BK, cb::BM};
+  const int a_rows = nc == 1 && a.M <= 16 && !a.a_mn && !a.tile_map ? (a.M + 7) / 8 * 8 : cb::BM;
+  const uint32_t boxA[2] = {cb::BK, (uint32_t)a_rows};
   const uint64_t dimsB[2] = {(uint64_t)a.K, (uint64_t)a.N * (uint64_t)(a.tile_map ? a.n_groups : 1)};
   const uint64_t strB[1] = {(uint64_t)a.ldb * 2};
   const uint32_t boxB[2] = {cb::BK, 128};
@@ -1272,6 +1279,7 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
     throw std::runtime_error("gemm_bf16: attention-backward epilogues need a row vector and ldc % 8 == 0");
   if (a.epi == EPI_ATTN_DS && (!a.R || a.ldr % 8 != 0))
     throw std::runtime_error("gemm_bf16: the dS epilogue needs P as the residual operand");
+  p.a_rows = a_rows;
   p.a_mn = a.a_mn ? 1 : 0;
   p.b_mn = a.b_mn ? 1 : 0;
   p.M = a.M; p.N = a.N; p.K = a.K;

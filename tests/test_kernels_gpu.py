@@ -1156,3 +1156,16 @@ def test_gemm_qkv_rope_routed_by_batch(batch, rows):
     assert (outs[1][1][:, :, :pre] == 7).all()
     want = ref.gemm_qkv_rope(a[-1].float(), w.float(), None, cos, sin, gamma.float(), gamma.float(), hq, hk, 1e-6)
     _close(outs[1][0][-1].reshape(rows, -1), want[:, :hq * 128], 3e-2, 2e-2, "routed by batch")
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 100, 128])
+@pytest.mark.parametrize("n,k", [(272, 72), (1024, 4096), (40000, 512)])
+def test_gemm_of_a_partly_filled_row_tile(m, n, k):
+    """Up to 16 rows only the rows that exist are staged, in eights: launches with and without split-K, one and several tiles a CTA. What lies
+    behind the rows, infinities among it, reaches no result."""
+    torch.manual_seed(53)
+    big = torch.full((200, k), math.inf, device=DEV, dtype=torch.bfloat16)
+    ops.gemm(big, _rand(1024, k))     # leaves infinities in shared memory
+    a, w = _rand(m, k), _rand(n, k, scale=1 / math.sqrt(k))
+    _close(ops.gemm(a, w), a.float() @ w.float().t(), 2e-2, 2e-2, f"gemm {m}x{n}x{k}")
+    _close(ops.gemm(a, w, epi=ops.EPI_SWIGLU), ref.gemm(a.float(), w.float(), epi=ops.EPI_SWIGLU), 2e-2, 2e-2, "swiglu")
