@@ -1103,6 +1103,15 @@ void gemm_set_debug(int64_t bits) { cosmos::gemm_set_debug((int)bits); }
 int64_t gemm_pick_k_splits(int64_t M, int64_t N, int64_t K, int64_t epi) {
   return cosmos::gemm_pick_k_splits((int)M, (int)N, (int)K, (int)epi);
 }
+// The number of gates among the `count` bit patterns from `first` on (`count` a multiple of 16) whose silu in the SwiGLU epilogue
+// is not the division's.
+Tensor silu_selftest(int64_t first, int64_t count, const Tensor& like) {
+  TORCH_CHECK(like.is_cuda() && first >= 0 && count >= 0 && count % 16 == 0 && first + count <= (1ll << 32), "bad range of gates");
+  c10::cuda::CUDAGuard guard(like.device());
+  Tensor differ = at::zeros({1}, like.options().dtype(at::kLong));
+  cosmos::silu_selftest((uint32_t)first, count / 16, reinterpret_cast<unsigned long long*>(differ.data_ptr<int64_t>()), cur_stream());
+  return differ;
+}
 void set_pdl(bool on) { cosmos::set_pdl(on); }
 void attn_set_cta_pair(bool on) { cosmos::attn_set_cta_pair(on); }
 void attn_set_exp_emulation(int64_t v) { attn_exp_emu() = (int)v; }
@@ -1379,6 +1388,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_set_exp_emulation", &attn_set_exp_emulation);
   m.def("attn_set_debug", &attn_set_debug);
   m.def("bounds_check_selftest", &bounds_check_selftest);
+  m.def("silu_selftest", &silu_selftest);
   m.def("rs_adamw", &rs_adamw);
   m.def("grad_sq_list", &grad_sq_list);
   m.def("adamw_list", &adamw_list);

@@ -436,6 +436,32 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&t);
 }
 __device__ __forceinline__ float gelu_erf(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
+// silu(g) = g / (1 + exp(-g)) of 16 values, in the bits that the division gives. A division has a branch, so that 16 of them run
+// one after another: SwiGLU of 240 x 24576 x 4096 takes 74 us with them and 55 without. The quotient here is g times an approximate
+// reciprocal, refined twice by its residual g - q den (exact in a fused multiply-add; each step of this iterative refinement
+// multiplies the error by that of the reciprocal, about 2^-23). Residuals that could underflow or overflow are left to the
+// division. Compared with it for every one of the 2^32 gates (silu_selftest): no bit differs; after one step two results do.
+__device__ __forceinline__ void silu16(const uint32_t (&g)[16], float (&o)[16]) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float gv = __uint_as_float(g[i]), den = 1.f + __expf(-gv);
+    float rc;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(den));
+    float q = gv * rc;
+    q = fmaf(fmaf(-q, den, gv), rc, q);
+    q = fmaf(fmaf(-q, den, gv), rc, q);
+    o[i] = copysignf(q, gv);   // den > 0; a gate of -0 keeps its sign
+    odd |= !(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-20f && gv != 0.f);
+  }
+  if (odd) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float gv = __uint_as_float(g[i]);
+      if (!(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-20f && gv != 0.f)) o[i] = gv / (1.f + __expf(-gv));
+    }
+  }
+}
 __device__ __forceinline__ float bf16lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
 

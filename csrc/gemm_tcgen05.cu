@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.cuh"
+#include <algorithm>
 #include <cstdlib>
 
 namespace cb {
@@ -257,28 +258,8 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
       tmem_ld16(t_addr + 128 + half * 64 + c * 16, u);
       tmem_wait_ld();
       if (c == 3) release();
-      // silu(g) = g / (1 + exp(-g)). A division has a branch, so that 16 of them run one after another (M 240 of the 24576-wide
-      // projection: 74 us with them, 55 without): the quotient is g times the approximate reciprocal, corrected once by its
-      // residual (Newton's step; the result differs from the division's in about one of 2^22 cases, by one ulp of fp32),
-      // and values whose residual could overflow or underflow are divided.
       float o[16];
-      bool odd = false;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float gv = __uint_as_float(g[i]), den = 1.f + __expf(-gv);
-        float rc;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(den));
-        const float q = gv * rc;
-        o[i] = fmaf(fmaf(-q, den, gv), rc, q);
-        odd |= !(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-30f && gv != 0.f);
-      }
-      if (odd) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float gv = __uint_as_float(g[i]);
-          if (!(fabsf(gv) < 80.f) || (fabsf(gv) < 1e-30f && gv != 0.f)) o[i] = gv / (1.f + __expf(-gv));
-        }
-      }
+      silu16(g, o);
 #pragma unroll
       for (int i = 0; i < 16; ++i) o[i] *= __uint_as_float(u[i]);
       slab.put_bf16(c * 2, o);
@@ -1055,6 +1036,25 @@ splitk_reduce_kernel(const float* __restrict__ partial, int k_splits, int M, int
   }
 }
 
+// Gates with the bit patterns first .. first + 16 n - 1: how many results of silu16 differ from the division's.
+__global__ void __launch_bounds__(256)
+silu_selftest_kernel(uint32_t first, long long n, unsigned long long* differ) {
+  unsigned long long bad = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    uint32_t g[16];
+    float o[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) g[e] = first + (uint32_t)(i * 16) + e;
+    silu16(g, o);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float gv = __uint_as_float(g[e]), want = gv / (1.f + __expf(-gv));
+      bad += __float_as_uint(o[e]) != __float_as_uint(want) && !(isnan(o[e]) && isnan(want));
+    }
+  }
+  if (bad) atomicAdd(differ, bad);
+}
+
 }  // namespace cb
 
 // ====================================================================== host
@@ -1319,6 +1319,10 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
 void gemm_set_grid_limit(int max_ctas) { g_grid_limit = max_ctas > 0 ? max_ctas : 0; }
 void gemm_set_cta_pair(bool on) { g_pair = on ? 1 : 0; }
 void gemm_set_debug(int bits) { g_debug = bits; }
+
+void silu_selftest(uint32_t first, long long n, unsigned long long* differ, cudaStream_t stream) {
+  if (n > 0) cb::silu_selftest_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, stream>>>(first, n, differ);
+}
 
 int gemm_pick_k_splits(int M, int N, int K, int epi) {
   if (epi != EPI_PLAIN && epi != EPI_SWIGLU && epi != EPI_GATED_RESID && epi != EPI_GELU) return 1;

@@ -89,6 +89,9 @@ void gemm_set_cta_pair(bool on);
 // Timing experiments (results are wrong): bit 0 = every tile loads the operand tiles at (0, 0) (all loads hit L2),
 // bit 1 = no operand loads at all (the MMA issue rate alone).
 void gemm_set_debug(int bits);
+// Compares the SwiGLU epilogue's silu with the division for the 16 n gates whose bit patterns follow `first`; the results that
+// differ are added to *differ (device).
+void silu_selftest(uint32_t first, long long n, unsigned long long* differ, cudaStream_t stream);
 void gemm_bf16(const GemmArgs& a, cudaStream_t stream);
 // K12: one persistent launch over one or two problems with the same epilogue kind (per-modality
 // weight routing: tokens are already grouped into an AR segment and a DM segment).

@@ -1113,7 +1113,8 @@ def test_gemm_wide_tiles(m, n, k):
 
 
 def test_gemm_swiglu_keeps_the_limits_of_silu():
-    """Gates beyond the range in which the quotient of silu is corrected: large of both signs, tiny, zero, infinite."""
+    """Gates beyond the range in which the quotient of silu is refined: large of both signs, tiny, zero, infinite. Two spacings of
+    subnormal bf16 (9.2e-41) absolutely, far below every value that is checked."""
     k = 64
     g = torch.tensor([0.0, 1e-38, -1e-38, 1e-30, 79.0, -79.0, 81.0, -81.0, -87.0, -88.0, -89.0, -200.0, 3e38, -3e38, math.inf, 1.0])
     a = torch.zeros(300, k, device=DEV, dtype=torch.bfloat16)
@@ -1123,9 +1124,16 @@ def test_gemm_swiglu_keeps_the_limits_of_silu():
     w[16:, 0] = 1
     got = ops.gemm(a, w, epi=ops.EPI_SWIGLU)
     want = torch.nn.functional.silu(w[:16, 0].double())
+    want[w[:16, 0].double() < -88.8] = 0.0    # exp(-gate) is beyond fp32
     fin = torch.isfinite(want)
-    _close(got[:, fin], want[fin].expand(300, -1), 1e-35, 8e-3, "silu")
+    _close(got[:, fin], want[fin].float().expand(300, -1), 2e-40, 8e-3, "silu")
     assert (got[:, ~fin] == math.inf).all()
+
+
+@pytest.mark.parametrize("first", range(0, 2 ** 32, 2 ** 30))
+def test_silu_of_the_swiglu_epilogue_is_the_division(first):
+    """Every fp32 gate: the epilogue's quotient has the bits of CUDA's division, signed zeros and both limits among them."""
+    assert torch.ops.cosmos_b200.silu_selftest(first, 2 ** 30, torch.empty(0, device=DEV)).item() == 0
 
 
 @pytest.mark.parametrize("batch,rows", [(1, 40), (2, 240), (3, 100), (5, 33), (9, 20), (40, 7)])
