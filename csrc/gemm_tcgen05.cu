@@ -153,17 +153,23 @@ struct Slab {
   __device__ __forceinline__ void put_bf16(int c, const float* f) const {
     put(lane, c, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
   }
+  // Whether rows of `ld` elements from `p` on take 16-byte accesses: callers may pass views that start at any element.
+  template <class T>
+  static __device__ __forceinline__ bool aligned(const T* p, long long ld) {
+    return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(ld * (long long)sizeof(T))) & 15) == 0;
+  }
   // Coalesced order: lane's i-th chunk is chunk (lane & 7) of row 4 i + lane / 8. rows x 64 columns of `src` (row stride
   // ld) in that order; what lies beyond is zero.
   __device__ __forceinline__ void fetch(uint4 (&v)[8], const bf16* src, long long ld, int rows, int cols) const {
     const int c = (lane & 7) * 8;
+    const int vec_cols = aligned(src, ld) ? cols : 0;   // the rest goes by element
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = i * 4 + (lane >> 3);
       v[i] = make_uint4(0, 0, 0, 0);
       if (r < rows && c < cols) {
         const bf16* s = src + r * ld + c;
-        if (c + 8 <= cols) {
+        if (c + 8 <= vec_cols) {
           v[i] = *reinterpret_cast<const uint4*>(s);
         } else {
           uint32_t u[4] = {0, 0, 0, 0};
@@ -187,6 +193,7 @@ struct Slab {
     constexpr int PER = 16 / sizeof(T);
     __syncwarp();
     const int c = (lane & 7) * PER;
+    const int vec_cols = aligned(dst, ld) ? cols : 0;
     if (c < cols) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -194,7 +201,7 @@ struct Slab {
         if (r < rows) {
           const uint4 v = get(r, lane & 7);
           T* d = dst + r * ld + c;
-          if (c + PER <= cols) {
+          if (c + PER <= vec_cols) {
             *reinterpret_cast<uint4*>(d) = v;
           } else {
             const T* e = reinterpret_cast<const T*>(&v);
@@ -435,6 +442,7 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
     }
     if (!wait()) return false;
     const bf16* gate = EPI == EPI_GATED_RESID && p.gate ? p.gate + (long long)(m / p.rows_per_batch) * p.N : nullptr;
+    const bool gate_vec = (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.gate) & 15) == 0;   // rows of whole 16-byte vectors
 #pragma unroll 1
     for (int c = 0; c < 8; ++c) {   // 16 columns at a time
       const int n = n0 + c * 16;
@@ -464,7 +472,7 @@ __device__ __forceinline__ bool finish_half(const GemmParams& p, const Slab& sla
           const uint4 rv = slab.get(lane, (c & 3) * 2 + q);
           const uint32_t ru[4] = {rv.x, rv.y, rv.z, rv.w};
           uint32_t gu[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
-          if (gate && (p.N & 7) == 0) {
+          if (gate && gate_vec) {
             if (n + q * 8 < p.N) {
               const uint4 gv = *reinterpret_cast<const uint4*>(gate + n + q * 8);
               gu[0] = gv.x; gu[1] = gv.y; gu[2] = gv.z; gu[3] = gv.w;

@@ -1136,6 +1136,34 @@ def test_silu_of_the_swiglu_epilogue_is_the_division(first):
     assert torch.ops.cosmos_b200.silu_selftest(first, 2 ** 30, torch.empty(0, device=DEV)).item() == 0
 
 
+@pytest.mark.parametrize("m", [5, 300])
+@pytest.mark.parametrize("n", [8, 24, 40, 264])
+@pytest.mark.parametrize("shift", [1, 4])
+def test_gemm_epilogues_take_views_that_start_anywhere(m, n, shift):
+    """Residual, gate and output as views that rule 16-byte accesses out, and SwiGLU rows of an odd stride: the same bits as with
+    aligned tensors, and nothing beside the view is written."""
+    torch.manual_seed(59)
+    a, w, w2 = _rand(m, 64), _rand(n, 64, scale=0.125), _rand(2 * n, 64, scale=0.125)
+    r, gate, rpb = _rand(m, n), _rand(2, n), (m + 1) // 2
+    ld = (n + shift + 7) // 8 * 8 + 8
+
+    def moved(t):
+        v = torch.empty(t.shape[0], ld, device=DEV, dtype=torch.bfloat16)[:, shift:shift + n]
+        return v.copy_(t)
+
+    flat = torch.empty(2 * n + 8, device=DEV, dtype=torch.bfloat16)[shift:shift + 2 * n].view(2, n).copy_(gate)
+    for name, call in {"plain": lambda r, g, **o: ops.gemm(a, w, **o),
+                       "gelu": lambda r, g, **o: ops.gemm(a, w, epi=7, **o),     # EPI_GELU of the kernels
+                       "resid": lambda r, g, **o: ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, g, rpb, **o),
+                       "swiglu": lambda r, g, **o: ops.gemm(a, w2, epi=ops.EPI_SWIGLU, **o)}.items():
+        want = call(r, gate)
+        for stride in (ld, ld + 3) if name == "swiglu" else (ld,):
+            big = torch.full((m, stride), 7.0, device=DEV, dtype=torch.bfloat16)
+            call(moved(r), flat, out=big[:, shift:shift + n])
+            assert torch.equal(big[:, shift:shift + n], want), (name, stride)
+            assert (big[:, :shift] == 7).all() and (big[:, shift + n:] == 7).all(), (name, stride)
+
+
 @pytest.mark.parametrize("batch,rows", [(1, 40), (2, 240), (3, 100), (5, 33), (9, 20), (40, 7)])
 def test_gemm_qkv_rope_routed_by_batch(batch, rows):
     """One routing table per batch entry: the same bits in every buffer as one launch per entry, whichever tables a tile or
