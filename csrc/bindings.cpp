@@ -1171,6 +1171,7 @@ void check_grads(at::TensorList grads, const Tensor& sq) {
 void grad_sq_list(at::TensorList grads, double scale, Tensor sq) {
   c10::cuda::CUDAGuard guard(sq.device());
   check_grads(grads, sq);
+  Tensor sums = at::empty({cosmos::OPT_SUMS}, sq.options());
   for (size_t i = 0; i < grads.size(); i += cosmos::OPT_MAX) {
     cosmos::OptTensor t[cosmos::OPT_MAX] = {};
     const int n = (int)std::min<size_t>(cosmos::OPT_MAX, grads.size() - i);
@@ -1178,7 +1179,7 @@ void grad_sq_list(at::TensorList grads, double scale, Tensor sq) {
       t[j].grad = grads[i + j].data_ptr();
       t[j].n = grads[i + j].numel();
     }
-    cosmos::grad_sq_list(t, n, (float)scale, sq.data_ptr<double>(), cur_stream());
+    cosmos::grad_sq_list(t, n, (float)scale, sums.data_ptr<double>(), sq.data_ptr<double>(), cur_stream());
   }
 }
 

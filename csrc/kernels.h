@@ -317,8 +317,10 @@ void rs_adamw(const long long* grads_dev, int world, long long shard_off, long l
 void reduce_scatter_pull(const long long* grads_dev, const void* mc, int world, long long shard_off, long long n,
                          float* out, bool accumulate, float scale, float* sq_out, cudaStream_t s);
 // Optimizer steps over lists of up to OPT_MAX tensors (csrc/optim.cu): bf16 gradients, fp32 weights and moments, bf16
-// parameters, all contiguous and of one length per entry. `sq`: device sum of squares of the scaled gradients.
+// parameters, all contiguous and of one length per entry. `sq`: device sum of squares of the scaled gradients, the same bits
+// for the same gradients; `sums`: scratch of OPT_SUMS values.
 constexpr int OPT_MAX = 64;
+constexpr int OPT_SUMS = 148 * 8;
 struct OptTensor {
   const void* grad;
   float *master, *m, *v;
@@ -326,7 +328,7 @@ struct OptTensor {
   long long n;
   int vec;   // set by the launcher: 16-byte accesses are possible
 };
-void grad_sq_list(const OptTensor* t, int n, float scale, double* sq, cudaStream_t s);
+void grad_sq_list(const OptTensor* t, int n, float scale, double* sums, double* sq, cudaStream_t s);
 void adamw_list(const OptTensor* t, int n, float scale, const double* sq, float max_norm, float lr, float b1, float b2, float eps,
                 float wd, int step, cudaStream_t s);
 // AdamW on a local fp32 gradient shard (fp32 master + moments, bf16 parameter shard rewritten).

@@ -37,11 +37,23 @@ __device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
   f[4] = bf16lo(u.z); f[5] = bf16hi(u.z); f[6] = bf16lo(u.w); f[7] = bf16hi(u.w);
 }
 
-// sq += scale^2 * sum of squares of all gradients. A thread's few hundred squares are added in fp32, the threads' sums in
-// fp64, so the result does not depend on the order in which blocks finish beyond the last bits of a double.
-__global__ void __launch_bounds__(OPT_THREADS)
-grad_sq_kernel(const __grid_constant__ OptList l, float scale, double* sq) {
+// Sum over the block in a fixed order; valid in thread 0.
+__device__ __forceinline__ double block_sum(double sum) {
   __shared__ double red[OPT_THREADS / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < OPT_THREADS / 32; ++w) sum += red[w];
+  }
+  return sum;
+}
+
+// sums[block] = sum of squares of the block's chunks: a thread's few hundred squares in fp32, the threads' sums in fp64.
+__global__ void __launch_bounds__(OPT_THREADS)
+grad_sq_kernel(const __grid_constant__ OptList l, double* sums) {
   double sum = 0.0;
   for (long long ch = blockIdx.x; ch < l.first_chunk[l.n]; ch += gridDim.x) {
     const int k = opt_find(l, ch);
@@ -69,15 +81,19 @@ grad_sq_kernel(const __grid_constant__ OptList l, float scale, double* sq) {
     }
     sum += (double)s;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < OPT_THREADS / 32; ++w) sum += red[w];
-    atomicAdd(sq, sum * (double)scale * (double)scale);
-  }
+  sum = block_sum(sum);
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+}
+
+// sq += scale^2 * the blocks' sums, in a fixed order: the ranks of a data-parallel step add up the squares of replicated gradients
+// each by itself, and their clip factors, and with them the replicated weights, stay the same bits. (Blocks that added to
+// sq by themselves gave 11 results in 40 runs.) One block, about 3 us behind a norm of 170.
+__global__ void __launch_bounds__(OPT_THREADS)
+add_sums_kernel(const double* sums, int n, float scale, double* sq) {
+  double sum = 0.0;
+  for (int i = threadIdx.x; i < n; i += OPT_THREADS) sum += sums[i];
+  sum = block_sum(sum);
+  if (threadIdx.x == 0) *sq += sum * (double)scale * (double)scale;
 }
 
 struct AdamWStep {
@@ -161,11 +177,13 @@ static long long fill_list(const cosmos::OptTensor* t, int n, OptList& l) {
 
 namespace cosmos {
 
-void grad_sq_list(const OptTensor* t, int n, float scale, double* sq, cudaStream_t s) {
+void grad_sq_list(const OptTensor* t, int n, float scale, double* sums, double* sq, cudaStream_t s) {
   cb::OptList l;
   const long long chunks = cb::fill_list(t, n, l);
   if (chunks == 0) return;
-  cb::grad_sq_kernel<<<(int)std::min<long long>(chunks, 148 * 8), cb::OPT_THREADS, 0, s>>>(l, scale, sq);
+  const int blocks = (int)std::min<long long>(chunks, OPT_SUMS);
+  cb::grad_sq_kernel<<<blocks, cb::OPT_THREADS, 0, s>>>(l, sums);
+  cb::add_sums_kernel<<<1, cb::OPT_THREADS, 0, s>>>(sums, blocks, scale, sq);
 }
 
 void adamw_list(const OptTensor* t, int n, float scale, const double* sq, float max_norm, float lr, float b1, float b2, float eps,

@@ -938,6 +938,25 @@ def test_optimizer_list_kernels_match_the_definition(sizes, shift):
             assert torch.equal(p[i], w[i].bfloat16())
 
 
+@pytest.mark.parametrize("sizes", [(8192 * 1500,), (8192 * 700 + 5, 3, 8192 * 900), (8192 * 20,) * 70])
+def test_gradient_norm_is_the_same_bits_every_time(sizes):
+    """Chunks of very different size, so that an fp64 sum shows its order: the ranks of a data-parallel step take this sum each by
+    itself and must arrive at the same clip factor."""
+    g = torch.Generator(device=DEV).manual_seed(len(sizes))
+    grads = []
+    for n in sizes:
+        t = torch.randn(n, device=DEV, generator=g)
+        grads.append((t * torch.exp2(-torch.arange(n, device=DEV).div(8192, rounding_mode="floor").mul(7).remainder(20).float())).bfloat16())
+    seen = set()
+    for _ in range(40):
+        sq = torch.full((1,), 1e-3, device=DEV, dtype=torch.float64)
+        torch.ops.cosmos_b200.grad_sq_list(grads, 0.5, sq)
+        seen.add(sq.item())
+    assert len(seen) == 1
+    want = 1e-3 + 0.25 * sum(t.double().square().sum().item() for t in grads)
+    assert abs(seen.pop() - want) <= 1e-6 * want     # fp32 sums of at most a few hundred squares a thread
+
+
 def _volume(x):
     """[C, T, H, W] -> zero-bordered channels-last volume behind two zero context frames."""
     c, t, h, w = x.shape
