@@ -1202,7 +1202,7 @@ void adamw_list(at::TensorList grads, at::TensorList masters, at::TensorList ms,
       TORCH_CHECK(p.is_contiguous() && p.numel() == g.numel() && p.device() == g.device(), "adamw_list: parameter size mismatch");
       t[j] = {g.data_ptr(), w.data_ptr<float>(), m.data_ptr<float>(), v.data_ptr<float>(), p.data_ptr(), g.numel(), 0};
     }
-    cosmos::adamw_list(t, n, (float)scale, sq.data_ptr<double>(), (float)max_norm, (float)lr, (float)b1, (float)b2, (float)eps,
+    cosmos::adamw_list(t, n, (float)scale, sq.data_ptr<double>(), (float)max_norm, (float)lr, b1, b2, (float)eps,
                        (float)wd, (int)step, cur_stream());
   }
 }

@@ -329,7 +329,7 @@ struct OptTensor {
   int vec;   // set by the launcher: 16-byte accesses are possible
 };
 void grad_sq_list(const OptTensor* t, int n, float scale, double* sums, double* sq, cudaStream_t s);
-void adamw_list(const OptTensor* t, int n, float scale, const double* sq, float max_norm, float lr, float b1, float b2, float eps,
+void adamw_list(const OptTensor* t, int n, float scale, const double* sq, float max_norm, float lr, double b1, double b2, float eps,
                 float wd, int step, cudaStream_t s);
 // AdamW on a local fp32 gradient shard (fp32 master + moments, bf16 parameter shard rewritten).
 void adamw_shard(const float* grad, long long n, float* master, float* m, float* v, void* param_shard,

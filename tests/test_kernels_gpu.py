@@ -938,6 +938,25 @@ def test_optimizer_list_kernels_match_the_definition(sizes, shift):
             assert torch.equal(p[i], w[i].bfloat16())
 
 
+@pytest.mark.parametrize("b1,b2", [(0.9, 0.999), (0.9, 0.95), (0.99, 0.9999)])
+@pytest.mark.parametrize("step", [1, 2, 1000])
+def test_optimizer_list_kernel_keeps_the_factors(b1, b2, step):
+    """First and second moments against fp64: 1 - beta and the bias corrections carry no more than their rounding to fp32. A moment
+    is a sum of two products (at most five roundings, 3.6e-7, where the terms have one sign); the update has about eight more."""
+    k = torch.ops.cosmos_b200
+    g = torch.Generator(device=DEV).manual_seed(step)
+    n, lr, eps = 8192 + 100, 1e-2, 1e-8
+    gr = torch.rand(n, device=DEV, generator=g).bfloat16() + 0.5
+    m, v = (torch.rand(n, device=DEV, generator=g) * 1e-3 for _ in range(2))
+    w, p = torch.zeros(n, device=DEV), torch.zeros(n, device=DEV, dtype=torch.bfloat16)
+    gd = gr.double()
+    mr, vr = b1 * m.double() + (1 - b1) * gd, b2 * v.double() + (1 - b2) * gd * gd
+    wr = -lr * (mr / (1 - b1 ** step)) / ((vr / (1 - b2 ** step)).sqrt() + eps)
+    k.adamw_list([gr], [w], [m], [v], [p], 1.0, torch.zeros(1, device=DEV, dtype=torch.float64), -1.0, lr, b1, b2, eps, 0.0, step)
+    for got, want, bound in ((m, mr, 3.6e-7), (v, vr, 3.6e-7), (w, wr, 1e-6)):
+        assert ((got.double() - want).abs() <= bound * want.abs()).all()
+
+
 @pytest.mark.parametrize("sizes", [(8192 * 1500,), (8192 * 700 + 5, 3, 8192 * 900), (8192 * 20,) * 70])
 def test_gradient_norm_is_the_same_bits_every_time(sizes):
     """Chunks of very different size, so that an fp64 sum shows its order: the ranks of a data-parallel step take this sum each by
