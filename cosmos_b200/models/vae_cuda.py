@@ -12,6 +12,7 @@ from __future__ import annotations
 from typing import Dict, List, Optional, Tuple
 
 import torch
+import torch.nn.functional as F
 
 from .vae import CausalVideoVAE, ResBlock
 
@@ -202,7 +203,8 @@ class CLEncoder(_CLConvs):
       (2j, 2i).
     * The 1x1x1 skip projections of the widening blocks are further columns of the block's second convolution: its sum runs
       over the 27 taps of its own input and then over the channels of the block's input.
-    * The first layer's 9 spatial taps x 3 colours are packed into the 64 channels of an operand row.
+    * The first layer's 9 spatial taps x 3 colours are packed into the 64 channels of an operand row. A tokenizer of another
+      number of input channels (up to 64) has them zero-extended to 64 and takes all 27 taps.
 
     Frames are encoded in temporal chunks (the first frame alone, then `chunk_frames` at a time); each
     convolution's two context frames are carried over, so the result equals one pass over the clip.
@@ -210,12 +212,16 @@ class CLEncoder(_CLConvs):
 
     def __init__(self, vae: CausalVideoVAE):
         super().__init__(vae, vae.enc_norm.eps)
-        w = vae.enc_in.weight.data   # [C, 3, 3, 3, 3]
-        assert vae.enc_in.k == (3, 3, 3) and w.shape[1] == 3 and w.shape[0] % 64 == 0, "channel widths must be multiples of 64"
-        p = torch.zeros(w.shape[0], 3, 64, dtype=torch.bfloat16, device=self.device)
-        p[:, :, :27] = w.permute(0, 2, 3, 4, 1).reshape(w.shape[0], 3, 27).to(torch.bfloat16)
-        self.w["in"] = p.reshape(w.shape[0], 192)
-        self.b["in"] = vae.enc_in.bias.data.float().contiguous()
+        w = vae.enc_in.weight.data   # [C, in_channels, 3, 3, 3]
+        self.in_channels = w.shape[1]
+        if self.in_channels == 3:
+            assert vae.enc_in.k == (3, 3, 3) and w.shape[0] % 64 == 0, "channel widths must be multiples of 64"
+            p = torch.zeros(w.shape[0], 3, 64, dtype=torch.bfloat16, device=self.device)
+            p[:, :, :27] = w.permute(0, 2, 3, 4, 1).reshape(w.shape[0], 3, 27).to(torch.bfloat16)
+            self.w["in"] = p.reshape(w.shape[0], 192)
+            self.b["in"] = vae.enc_in.bias.data.float().contiguous()
+        else:
+            self._add_conv("in", vae.enc_in, 64)
         self.downs: List[bool] = []
         self.skips: Dict[str, bool] = {}
 
@@ -243,14 +249,23 @@ class CLEncoder(_CLConvs):
 
     @torch.no_grad()
     def encode_chunk(self, frames: torch.Tensor, cache: Dict, t0: int) -> torch.Tensor:
-        """frames [3, n, H, W] in [-1, 1] (global index of the first one: t0) -> moments [2C, n', H/8, W/8] fp32."""
-        _, n, h, w = frames.shape
-        if frames.dtype not in (torch.float32, torch.bfloat16):
-            frames = frames.float()
-        if frames.stride(3) != 1 or frames.stride(2) != w or (n > 1 and frames.stride(1) != h * w):
-            frames = frames.contiguous()
-        vol = self._empty(n + TPAD, h + 2, w + 2, 64)
-        torch.ops.cosmos_b200.conv_pack_rgb(frames, vol)
+        """frames [C, n, H, W] in [-1, 1], on any device and of any dtype (global index of the first one: t0) -> moments
+        [2C, n', H/8, W/8] fp32. Channels that the tokenizer does not have are ignored, missing ones are zero."""
+        c, n, h, w = frames.shape
+        assert c <= 64
+        if self.in_channels == 3:
+            frames = frames.to(self.device)
+            if c != 3:
+                frames = F.pad(frames[:3], (0, 0, 0, 0, 0, 0, 0, max(0, 3 - c)))
+            if frames.dtype not in (torch.float32, torch.bfloat16):
+                frames = frames.to(torch.bfloat16)
+            if frames.stride(3) != 1 or frames.stride(2) != w or (n > 1 and frames.stride(1) != h * w):
+                frames = frames.contiguous()
+            vol = self._empty(n + TPAD, h + 2, w + 2, 64)
+            torch.ops.cosmos_b200.conv_pack_rgb(frames, vol)
+        else:
+            vol = torch.zeros(n + TPAD, h + 2, w + 2, 64, dtype=torch.bfloat16, device=self.device)
+            vol[TPAD:, 1:-1, 1:-1, :c] = frames.permute(1, 2, 3, 0).to(torch.bfloat16)
         x, y = self._conv(cache, "in", vol, norm=self.g["b0.n1"])
         last = len(self.downs) - 1
         for i, temporal in enumerate(self.downs):

@@ -866,6 +866,41 @@ def test_vae_channels_last_encoder_matches_pytorch():
     assert (other - got).abs().max().item() <= 0.02 * want.abs().max().item()   # chunking does not change the result
 
 
+def test_vae_encoder_takes_frames_as_they_come():
+    """Frames on the host, in fp64, cut out of a larger clip, of fewer or more channels than the tokenizer has (missing ones are
+    zero, further ones ignored): the bits of the plain call."""
+    from cosmos_b200.models.vae import CausalVideoVAE
+    from cosmos_b200.models.vae_cuda import CLEncoder
+    torch.manual_seed(22)
+    enc = CLEncoder(CausalVideoVAE(16, (64, 64, 128, 128)).to(device=DEV, dtype=torch.bfloat16).eval())
+    video = (torch.rand(1, 3, 9, 32, 40, device=DEV) * 2 - 1).bfloat16().float()
+    want = enc.encode(video)
+    big = torch.zeros(1, 5, 9, 40, 48, device=DEV)
+    big[:, :3, :, 4:36, 4:44], big[:, 3:] = video, math.nan
+    for what, v in {"host": video.cpu(), "host bf16": video.bfloat16().cpu(), "fp64": video.double(), "fp16": video.half(),
+                    "cut": big[:, :3, :, 4:36, 4:44], "five channels": big[:, :, :, 4:36, 4:44]}.items():
+        tol = 0 if what != "fp16" else 2 ** -8 * want.abs().max().item()    # bf16 values below 2^-14 are subnormal in fp16
+        assert (enc.encode(v) - want).abs().max() <= tol, what
+    grey = torch.zeros_like(video)
+    grey[:, :1] = video[:, :1]
+    assert torch.equal(enc.encode(video[:, :1]), enc.encode(grey))
+
+
+@pytest.mark.parametrize("channels", [1, 4])
+def test_vae_encoder_of_other_input_channels(channels):
+    """A tokenizer of 1 or 4 input channels against the fp32 modules; the bounds of three channels."""
+    from cosmos_b200.models.vae import CausalVideoVAE
+    from cosmos_b200.models.vae_cuda import CLEncoder
+    torch.manual_seed(23)
+    vae = CausalVideoVAE(16, (64, 128, 128, 128), in_channels=channels).to(DEV).float().eval()
+    video = torch.rand(1, channels, 9, 32, 40, device=DEV) * 2 - 1
+    with torch.no_grad():
+        want = vae.encode(video)
+    got = CLEncoder(vae).encode(video.cpu() if channels == 1 else video)
+    err = (got - want).abs()
+    assert got.shape == want.shape and err.mean() < 0.03 * want.abs().mean() and err.max() < 0.25 * want.abs().max()
+
+
 @pytest.mark.parametrize("n,off", [(4096, 0), (1003, 0), (2048, 3), (777, 8)])
 def test_adamw_kernels_match_the_fp32_definition(n, off):
     """`rs_adamw` (gradients read from bf16 buffers, here one local source) and `adamw_shard` (fp32 reduced
