@@ -14,6 +14,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 import torch.nn.functional as F
 
+from .. import ops
 from .vae import CausalVideoVAE, ResBlock
 
 TPAD = 2  # context frames in front of every volume (temporal kernel 3, stride 1)
@@ -43,7 +44,7 @@ class _CLConvs:
 
     def __init__(self, vae: CausalVideoVAE, eps: float):
         self.device = next(vae.parameters()).device
-        assert self.device.type == "cuda", "the channels-last tokenizer runs on CUDA"
+        assert self.device.type == "cuda" and ops.load_extension(), "the channels-last tokenizer runs on CUDA, on the kernel library"
         self.latent_channels = vae.latent_channels
         self.eps = eps
         self.w: Dict[str, torch.Tensor] = {}

@@ -886,6 +886,16 @@ def test_vae_encoder_takes_frames_as_they_come():
     assert torch.equal(enc.encode(video[:, :1]), enc.encode(grey))
 
 
+def test_vae_encoder_is_enough_to_load_the_kernels():
+    """A program that builds the encoder and calls nothing else before it."""
+    import subprocess
+    import sys
+    code = ("import torch; from cosmos_b200.models.vae import CausalVideoVAE; from cosmos_b200.models.vae_cuda import CLEncoder; "
+            "v = CausalVideoVAE(16, (64, 64, 64, 64)).cuda().bfloat16(); print(CLEncoder(v).encode(torch.zeros(1, 3, 1, 16, 16)).shape)")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "[1, 16, 1, 2, 2]" in r.stdout, r.stderr[-800:]
+
+
 @pytest.mark.parametrize("channels", [1, 4])
 def test_vae_encoder_of_other_input_channels(channels):
     """A tokenizer of 1 or 4 input channels against the fp32 modules; the bounds of three channels."""
