@@ -855,7 +855,8 @@ void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT
   cosmos::conv3d_fused(a, cur_stream());
 }
 
-// One convolution without fusions: out and resid [F, Hp, Wp, Cout]; frames from `tpad` on are written.
+// One convolution without fusions: out and resid [F, Hp, Wp, Cout]; the interior of the frames from `tpad` on is written, the border
+// is left untouched.
 void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& resid, Tensor out, int64_t tpad) {
   check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w"); check_bf16_cuda(out, "out");
   c10::cuda::CUDAGuard guard(x.device());
@@ -864,8 +865,9 @@ void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& r
   TORCH_CHECK(out.size(0) == F && out.size(1) == Hp && out.size(2) == Wp, "out must have the padded shape of x");
   TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == Cout && w.size(1) == 27 * C, "w must be [Cout, 27 * C]");
   TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
-  TORCH_CHECK(tpad >= 0, "tpad must not be negative");
+  tpad = std::max<int64_t>(tpad, 0);
   cosmos::ConvArgs a;
+  a.keep_border = 1;
   a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
   a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout;
   a.tpad = (int)tpad; a.f_out = (int)std::max<int64_t>(0, F - tpad);

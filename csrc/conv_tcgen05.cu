@@ -68,6 +68,7 @@ struct ConvParams {
   float eps;
   uint8_t* rgb;
   int mode;              // CONV_OUT_*
+  int keep_border;       // CONV_OUT_SAME: the border's cells are not written
   int tpad;              // context frames in front of every output volume
   int f_out;             // frames computed
   int up_t, up_first;    // CONV_OUT_UP: temporal doubling, first chunk (its first frame is not doubled)
@@ -400,7 +401,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
             for (int k = 0; k < 8; ++k) pk[k] = 0u;
           }
-          if (p.out && row_ok) {
+          if (p.out && (inside || (row_ok && !p.keep_border))) {
             bf16* o = p.out + dst.row * ld + n_base + c;
             if (p.mode != CONV_OUT_UP) {
               cv_store16(o, pk);
@@ -596,6 +597,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   if ((a.skip && (strided || a.mode == CONV_OUT_UP)) || (a.resid && (strided || rgb)))
     throw std::runtime_error("conv: no residual or skip input in this form");
   if (a.out_norm && (a.mode == CONV_OUT_S2D || a.mode == CONV_OUT_UP)) throw std::runtime_error("conv: no norm in this form");
+  if (a.keep_border && (a.mode != CONV_OUT_SAME || a.out_norm || rgb)) throw std::runtime_error("conv: this form writes its border");
   if (a.f_out < 1) return;
   cb::ConvParams p{};
   p.cblocks = a.c / 64;
@@ -610,6 +612,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   p.eps = a.eps;
   p.rgb = reinterpret_cast<uint8_t*>(a.rgb);
   p.mode = a.mode;
+  p.keep_border = a.keep_border;
   p.tpad = a.tpad;
   p.f_out = a.f_out;
   p.up_t = a.up_temporal;

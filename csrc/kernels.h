@@ -219,6 +219,7 @@ struct ConvArgs {
   float eps = 1e-6f;
   void* rgb = nullptr;          // uint8 [f_out, hp - 2, wp - 2, 3]; n_out = 9: rows of w = the 3 channels' weights in 3 bf16 terms
   int mode = CONV_OUT_SAME;
+  int keep_border = 0;          // CONV_OUT_SAME without the norm: cells of the border keep what they hold (else zero)
   int frames_in = 0, hp = 0, wp = 0, c = 0, skip_c = 0, n_out = 0, f_out = 0, tpad = 2;
   int taps_t_only = 0;
   int up_temporal = 0, up_first = 0;

@@ -364,6 +364,25 @@ def test_conv3d_implicit_gemm_matches_conv3d(cin, cout):
     assert out[:2].abs().max() == 0 and out[:, 0].abs().max() == 0 and out[:, :, -1].abs().max() == 0
 
 
+@pytest.mark.parametrize("cin,cout,tpad", [(64, 64, 2), (128, 320, 2), (64, 256, 1), (64, 32, 0)])
+def test_conv3d_cl_writes_the_interior_only(cin, cout, tpad):
+    """Border cells and the frames before `tpad` keep what they hold; the interior has the bits of the form that zeroes its border."""
+    torch.manual_seed(24)
+    k = torch.ops.cosmos_b200
+    vol = torch.zeros(6, 14, 22, cin, device=DEV, dtype=torch.bfloat16)
+    vol[:, 1:-1, 1:-1] = _rand(6, 12, 20, cin)
+    wp, b = _rand(cout, 27 * cin, scale=1 / math.sqrt(27 * cin)), _rand(cout)
+    out = torch.full((6, 14, 22, cout), 7.0, device=DEV, dtype=torch.bfloat16)
+    k.conv3d_cl(vol, wp, b, None, out, tpad)
+    full = torch.empty_like(out)
+    k.conv3d_fused(vol, wp, b, None, None, full, None, None, 1e-6, 0, 0, 0)
+    lo = max(tpad, 2)
+    assert torch.equal(out[lo:, 1:-1, 1:-1], full[lo:, 1:-1, 1:-1])
+    assert (out[tpad:, 1:-1, 1:-1] != 7).any(-1).all()
+    out[tpad:, 1:-1, 1:-1] = 7.0
+    assert (out == 7).all()
+
+
 def test_vae_channels_last_decoder_matches_pytorch():
     from cosmos_b200.models.vae import CausalVideoVAE
     from cosmos_b200.models.vae_cuda import CLDecoder
