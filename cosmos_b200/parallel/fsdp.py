@@ -111,10 +111,12 @@ class ShardedUnit:
             self._prefetched = None
             torch.cuda.current_stream().wait_event(ev)
             return full
-        if self.ws == 1:
-            return self.shard.detach()   # the shard is the whole tensor; nothing writes it before the optimizer step
+        if self.ws == 1 and self.owner is not None and self.owner.recomputed:
+            return self.shard.detach()   # the shard is the whole tensor, and no graph keeps it beyond an update
         full = torch.empty(self.n, dtype=self.dtype, device=self.device)
-        if self.fused:
+        if self.ws == 1:
+            full.copy_(self.shard.data)
+        elif self.fused:
             self._pull(full)
         else:
             dist.all_gather_into_tensor(full, self.shard.data.contiguous(), group=self.group)
@@ -162,6 +164,10 @@ class FSDP:
         self.rep_v = [torch.zeros_like(m) for m in self.rep_master]
         self.lr, self.betas, self.eps, self.wd, self.max_grad_norm = lr, betas, eps, weight_decay, max_grad_norm
         self.step_count = 0
+        # Whether every layer's forward pass is recomputed in backward (checkpointed blocks): then a graph keeps no gathered
+        # parameters, and the only rank of a shard group hands out its shard in place of a copy. A graph that keeps them, such as
+        # one whose backward pass runs after an update, needs the values of its forward pass.
+        self.recomputed = False
 
     # ------------------------------------------------------------------ forward hook
     def layer_params(self, tower: str, i: int) -> Dict[str, torch.Tensor]:

@@ -82,6 +82,7 @@ class Trainer:
         rep_group = mesh.group("dp_replicate") if rep > 1 and dist.is_initialized() else None
         self.fsdp = FSDP(model, group, ranks, towers, tc.fused, tc.lr, weight_decay=tc.weight_decay,
                          max_grad_norm=tc.max_grad_norm, replicate_group=rep_group, replicate_size=rep)
+        self.fsdp.recomputed = tc.checkpoint_blocks
         self.ctx = LOCAL_ATTN
         if mesh.size("cp") > 1:
             from .parallel.ulysses import UlyssesAttn

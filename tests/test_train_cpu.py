@@ -138,3 +138,21 @@ def test_gradient_accumulation_equals_the_larger_batch_and_the_schedule_sets_the
     assert tc.lr_at(1) == 0.5 and tc.lr_at(4) == 2.0 and abs(tc.lr_at(8) - 2.0 * (0.25 + 0.75 * 0.5)) < 1e-12
     assert abs(tc.lr_at(12) - 0.5) < 1e-12 and abs(tc.lr_at(40) - 0.5) < 1e-12
     assert TrainConfig(lr=3.0).lr_at(7) == 3.0
+
+
+def test_gathered_parameters_keep_the_values_of_their_forward_pass():
+    """Without checkpointed blocks a graph holds the parameters that a layer gathered; an update must not change them under it."""
+    from cosmos_b200.config import ParallelConfig
+    from cosmos_b200.models.mot import MoTModel
+    from cosmos_b200.parallel.mesh import Mesh
+    from cosmos_b200.train import TrainConfig, Trainer
+    model = MoTModel(_cfg(), pad_to=128)
+    model.init_weights(seed=3)
+    tr = Trainer(model, Mesh(ParallelConfig(), 1, 0), TrainConfig(lr=1e-2, fused=False, checkpoint_blocks=False))
+    held = tr.fsdp.layer_params("dm", 0)
+    before = {k: v.detach().clone() for k, v in held.items()}
+    lat, ids, t, eps = _data(1)
+    tr.train_step(lat, ids, t=t, eps=eps)
+    assert not torch.equal(tr.fsdp.layer_params("dm", 0)["wqkv"], before["wqkv"])
+    for k, v in held.items():
+        assert torch.equal(v, before[k]), k
