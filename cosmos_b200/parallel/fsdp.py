@@ -262,7 +262,7 @@ class FSDP:
                 p.grad.div_(ws)
             self._avg_over_replicas(p.grad)
         inv_ws = 1.0 / ws
-        sq = torch.zeros(1, dtype=torch.float64, device=next(iter(self.parameters())).device)
+        sq = torch.zeros(1, dtype=torch.float64, device=next(self.model.parameters()).device)
         local = self._local_kernel() and self.rep == 1
         rep_kernel = self._rep_kernel()
         reduced: Dict[Tuple[str, int], torch.Tensor] = {}

@@ -156,3 +156,11 @@ def test_gathered_parameters_keep_the_values_of_their_forward_pass():
     assert not torch.equal(tr.fsdp.layer_params("dm", 0)["wqkv"], before["wqkv"])
     for k, v in held.items():
         assert torch.equal(v, before[k]), k
+
+
+def test_fsdp_step_without_trainable_parameters():
+    from cosmos_b200.models.mot import MoTModel
+    from cosmos_b200.parallel.fsdp import FSDP
+    model = MoTModel(_cfg(), pad_to=128)
+    model.requires_grad_(False)
+    assert FSDP(model, None, [0], towers=(), fused=False).step() == 0.0
