@@ -203,6 +203,8 @@ class WorkspaceAttn(AttnContext):
             vb[:, :n_pre].copy_(prefix[1])
         gq = q_norm if cfg.qk_norm else None
         gk = k_norm if cfg.qk_norm else None
+        if cos is not None and cos.shape[0] > s:   # tables for more positions: every entry takes the first rows
+            cos, sin = cos[:s], sin[:s]
         # all batch entries in one launch, each through its own routing table (guided steps: two branches; at 240 tokens a
         # branch, where 24 pairs of CTAs have a tile each, the two launches took 79 us and one takes 42)
         ops.gemm_qkv_rope(h.reshape(b * s, -1), w, None, cos, sin, gq, gk, cfg.n_heads, cfg.n_kv_heads, cfg.rms_eps,

@@ -323,6 +323,9 @@ Tensor gemm_qkv_rope(const Tensor& A_, const Tensor& W, const OptT& bias, const 
                 "cos/sin tables must be contiguous fp32 [rows, 64]");
     g.cos_tab = cos_t->data_ptr<float>(); g.sin_tab = sin_t->data_ptr<float>();
     g.rope_rows = (int)(cos_t->numel() / 64);
+    // row m of A takes row m % rope_rows of the tables, so an entry's rows get their own positions only if these sizes match
+    TORCH_CHECK(!g.route_rows || M == 0 || (g.rope_rows > 0 && g.route_rows % g.rope_rows == 0),
+                "cos/sin tables must have route_rows rows (or a divisor of them)");
   }
   if (gamma_q.has_value() && gamma_q->defined()) { check_bf16_cuda(*gamma_q, "gamma_q"); g.gamma_q = gamma_q->data_ptr(); }
   if (gamma_k.has_value() && gamma_k->defined()) { check_bf16_cuda(*gamma_k, "gamma_k"); g.gamma_k = gamma_k->data_ptr(); }

@@ -1311,6 +1311,31 @@ def test_gemm_qkv_rope_routed_by_batch(batch, rows):
     _close(outs[1][0][-1].reshape(rows, -1), want[:, :hq * 128], 3e-2, 2e-2, "routed by batch")
 
 
+@pytest.mark.parametrize("batch", [1, 2, 3])
+def test_workspace_qkv_with_longer_rotary_tables(batch):
+    """Tables for more positions than there are tokens: every batch entry takes the first rows. The operator refuses tables that
+    would give the second entry other positions."""
+    from cosmos_b200.config import get_model_config
+    from cosmos_b200.models.mot import WorkspaceAttn
+    torch.manual_seed(47)
+    cfg = get_model_config("tiny128")
+    rows, heads = 40, cfg.n_heads + 2 * cfg.n_kv_heads
+    h, w = _rand(batch, rows, cfg.d_model), _rand(heads * 128, cfg.d_model, scale=1 / math.sqrt(cfg.d_model))
+    ang = torch.rand(64, 64, device=DEV) * 6.28
+    cos, sin, gamma = ang.cos(), ang.sin(), torch.ones(128, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad():
+        long = [t.clone() for t in WorkspaceAttn().qkv_project(h, w, cos, sin, gamma, gamma, cfg)]
+        for b in range(batch):
+            for got, want in zip(long, WorkspaceAttn().qkv_project(h[b:b + 1], w, cos[:rows], sin[:rows], gamma, gamma, cfg)):
+                assert torch.equal(got[b:b + 1], want)
+        buf = torch.empty(rows, heads * 128, device=DEV, dtype=torch.bfloat16)
+        ptr = torch.full((batch, heads), buf.data_ptr(), device=DEV, dtype=torch.int64)
+        ld = torch.full_like(ptr, heads * 128)
+        with pytest.raises(RuntimeError, match="route_rows rows"):
+            ops.gemm_qkv_rope(h.view(batch * rows, -1), w, None, cos, sin, gamma, gamma, cfg.n_heads, cfg.n_kv_heads, 1e-6, ptr, ld,
+                              route_rows=rows)
+
+
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 100, 128])
 @pytest.mark.parametrize("n,k", [(272, 72), (1024, 4096), (40000, 512)])
 def test_gemm_of_a_partly_filled_row_tile(m, n, k):
