@@ -566,7 +566,8 @@ void conv_launch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, int smem
     pairs = std::min(n, sms / 2);
   }
   const int total = p.n_seg * p.tiles_per_seg * p.n_tiles;
-  cfg.gridDim = dim3(2 * std::min(pairs, total));
+  const int limit = gemm_grid_limit(), at_once = limit > 0 ? std::min(pairs, std::max(1, limit / 2)) : pairs;
+  cfg.gridDim = dim3(2 * std::min(at_once, total));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], p);

@@ -1325,6 +1325,7 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
 }
 
 void gemm_set_grid_limit(int max_ctas) { g_grid_limit = max_ctas > 0 ? max_ctas : 0; }
+int gemm_grid_limit() { return g_grid_limit; }
 void gemm_set_cta_pair(bool on) { g_pair = on ? 1 : 0; }
 void gemm_set_debug(int bits) { g_debug = bits; }
 

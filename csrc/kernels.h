@@ -81,8 +81,9 @@ struct GemmArgs {
 };
 // Split count that fills the machine for a skinny problem (1 = do not split).
 int gemm_pick_k_splits(int M, int N, int K, int epi);
-// Debug knob for race hunting: at most `max_ctas` persistent CTAs per GEMM launch (0 = one per SM).
+// Debug knob for race hunting: at most `max_ctas` persistent CTAs per launch of a GEMM or a convolution (0 = one per SM).
 void gemm_set_grid_limit(int max_ctas);
+int gemm_grid_limit();
 // A/B switch: problems taller than one 128-row tile run on CTA pairs (256-row tiles, tcgen05 cta_group::2)
 // when on (the default; COSMOS_GEMM_CTA_PAIR=0 starts with it off).
 void gemm_set_cta_pair(bool on);

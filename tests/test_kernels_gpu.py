@@ -1067,7 +1067,7 @@ def _volume(x):
 @pytest.mark.parametrize("cin,cout", [(64, 64), (64, 128), (128, 128), (256, 256), (320, 96), (128, 320)])
 def test_conv3d_fused_forms(cin, cout, t, h, w):
     """Every layout a convolution writes, with residual, skip projection and norm, against fp64 convolutions of the same
-    bf16 inputs: volumes smaller than a tile and with a remainder, channels in several blocks and output tiles. Bound:
+    bf16 inputs (a CTA pair has one tile here; the schedules are the next test's): volumes smaller than a tile and with a remainder, channels in several blocks and output tiles. Bound:
     one bf16 rounding of the result (2^-9 relative), twice with the norm."""
     import torch.nn.functional as F
     k = torch.ops.cosmos_b200
@@ -1138,6 +1138,43 @@ def test_conv3d_fused_forms(cin, cout, t, h, w):
         if fused:
             check(dn[2:, 1:-1, 1:-1], norm(want), "stride 2, norm", 2 ** -6)
             border(dn[2:])
+
+
+@pytest.mark.parametrize("cin,cout", [(64, 64), (128, 128), (256, 256), (320, 96), (128, 320)])
+def test_conv3d_results_do_not_depend_on_the_schedule(cin, cout):
+    """4608 rows are 9 tiles of 512 (up to 128 output channels) or 18 of 256: one and three CTA pairs walk three to eighteen tiles
+    each, through both accumulators, ring phases carried from tile to tile and both buffers of the norm's row sums. The same
+    bits as with a pair for every tile, in every form."""
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(cin + cout)
+    t, h, w = 2, 34, 62
+    fused = cout in (64, 128, 256)
+    vol, resid, skip = _volume(_rand(cin, t, h, w)), _volume(_rand(cout, t, h, w)), _volume(_rand(64, t, h, w))
+    wp = _rand(cout, 27 * cin, scale=1 / math.sqrt(27 * cin))
+    ws = torch.cat([wp, _rand(cout, 64, scale=0.125)], 1).contiguous()
+    b, g = torch.randn(cout, device=DEV), _rand(cout) if fused else None
+    xs = torch.zeros(12, 4, h // 2 + 1, w // 2 + 1, cin, device=DEV, dtype=torch.bfloat16)    # 10 frames kept: 10 segments
+    xs[2:] = _rand(10, 4, h // 2 + 1, w // 2 + 1, cin)
+    x64, terms = _volume(_rand(64, t, h, w)), _rand(9, 27 * 64, scale=0.02)
+
+    def run():
+        new = lambda *s: torch.full((*s, cout), 7.0, device=DEV, dtype=torch.bfloat16)  # noqa: E731
+        outs = [new(t + 2, h + 2, w + 2), new(t + 2, h + 2, w + 2), new(t + 2, 4, h // 2 + 1, w // 2 + 1),
+                new(2 * t + 2, 2 * h + 2, 2 * w + 2), new(12, h // 2 + 2, w // 2 + 2), new(12, h // 2 + 2, w // 2 + 2)]
+        k.conv3d_fused(vol, wp, b, resid, None, outs[0], outs[1] if fused else None, g, 1e-6, 0, 0, 0)
+        k.conv3d_fused(vol, ws, b, None, skip, outs[2], None, None, 1e-6, 1, 0, 0)
+        k.conv3d_fused(vol, wp, b, resid, None, outs[3], None, None, 1e-6, 2, 1, 0)
+        k.conv3d_fused(xs, wp, b, None, None, outs[4], outs[5] if fused else None, g, 1e-6, 3, 0, 1)
+        return outs + [k.conv3d_rgb(x64, terms, b[:3].contiguous())]
+
+    want = run()
+    try:
+        for limit in (2, 6):
+            k.gemm_set_grid_limit(limit)
+            for i, (got, ref_) in enumerate(zip(run(), want)):
+                assert torch.equal(got, ref_), (limit, i)
+    finally:
+        k.gemm_set_grid_limit(0)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
