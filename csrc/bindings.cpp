@@ -1048,6 +1048,13 @@ Tensor gemm_decode_qkv_post(const Tensor& h, const Tensor& w, int64_t n_q_heads,
 
 bool bounds_check_enabled() { return cosmos::bounds_check_enabled(); }
 void gemm_set_grid_limit(int64_t max_ctas) { cosmos::gemm_set_grid_limit((int)max_ctas); }
+void gemm_set_tile(int64_t ctas, int64_t col_tiles) { cosmos::gemm_set_tile((int)ctas, (int)col_tiles); }
+// (CTAs a tile, column tiles at once) of a launch without split-K; host-side, needs no device.
+std::tuple<int64_t, int64_t> gemm_pick_tile(int64_t M, int64_t N, int64_t K, int64_t epi) {
+  int ctas, cols;
+  cosmos::gemm_pick_tile((int)M, (int)N, (int)K, (int)epi, ctas, cols);
+  return {ctas, cols};
+}
 // A/B switches for timing and tests: CTA-pair GEMM tiles on/off, attention forward variant bits.
 void gemm_set_cta_pair(bool on) { cosmos::gemm_set_cta_pair(on); }
 // Decode-step sampling: the 64 best penalised logits of this rank's vocabulary shard per sequence ...
@@ -1385,6 +1392,8 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("bounds_check_enabled", &bounds_check_enabled);
   m.def("gemm_set_grid_limit", &gemm_set_grid_limit);
   m.def("gemm_set_cta_pair", &gemm_set_cta_pair);
+  m.def("gemm_set_tile", &gemm_set_tile);
+  m.def("gemm_pick_tile", &gemm_pick_tile);
   m.def("gemm_set_debug", &gemm_set_debug);
   m.def("gemm_pick_k_splits", &gemm_pick_k_splits);
   m.def("set_pdl", &set_pdl);

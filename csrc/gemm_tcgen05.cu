@@ -1156,6 +1156,7 @@ static int sm_count() {
 // Whether problems with more than one 128-row tile run on CTA pairs (COSMOS_GEMM_CTA_PAIR=0 keeps
 // every launch on single CTAs, for A/B timing).
 static int g_debug = 0;
+static int g_tile_ctas = 0, g_tile_cols = 0;   // gemm_set_tile
 static int g_pair = -1;
 static bool pair_enabled() {
   if (g_pair < 0) {
@@ -1326,6 +1327,12 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
 
 void gemm_set_grid_limit(int max_ctas) { g_grid_limit = max_ctas > 0 ? max_ctas : 0; }
 int gemm_grid_limit() { return g_grid_limit; }
+void gemm_set_tile(int ctas, int col_tiles) {
+  if (!(ctas == 0 && col_tiles == 0) && !(ctas == 1 && col_tiles == 1) && !(ctas == 2 && (col_tiles == 1 || col_tiles == 2)))
+    throw std::runtime_error("gemm_set_tile: (1, 1), (2, 1), (2, 2) or (0, 0)");
+  g_tile_ctas = ctas;
+  g_tile_cols = col_tiles;
+}
 void gemm_set_cta_pair(bool on) { g_pair = on ? 1 : 0; }
 void gemm_set_debug(int bits) { g_debug = bits; }
 
@@ -1375,6 +1382,13 @@ int gemm_pick_k_splits(int M, int N, int K, int epi) {
 // 4096 x 12288 residual M 14080 1143 -> 924, M 3600 352 -> 272; 4096 x 4096 residual M 3600 124 -> 103; 6144 x 4096 with
 // norm and rotary embedding M 14080 577 -> 550, but M 1920 101 -> 118.
 static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) {
+  nc = nw = 1;
+  if (!pair_enabled() || (args[0].M <= cb::BM && (n < 2 || args[1].M <= cb::BM))) return;
+  if (g_tile_ctas) {
+    nc = g_tile_ctas;
+    nw = wide_epi(args[0].epi) ? g_tile_cols : 1;
+    return;
+  }
   const int ctas = limit > 0 && limit < sm_count() ? limit : sm_count();
   const int epi = args[0].epi, k_blocks = (args[0].K + cb::BK - 1) / cb::BK;
   auto cost = [&](int c, int w, int kb_bytes) {
@@ -1393,6 +1407,12 @@ static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) 
   if (wide_epi(epi) && cost(2, 2, 48) <= (single ? cost(1, 1, 48) - 1 : cost(2, 1, 32))) nc = nw = 2;
 }
 
+void gemm_pick_tile(int M, int N, int K, int epi, int& ctas, int& col_tiles) {
+  GemmArgs a;
+  a.M = M; a.N = N; a.K = K; a.epi = epi;
+  pick_tile(&a, 1, g_grid_limit, ctas, col_tiles);
+}
+
 // One launch for one or two problems that share the epilogue kind.
 void gemm_bf16_grouped(const GemmArgs* args, int n, cudaStream_t stream) {
   if (n < 1 || n > 2) throw std::runtime_error("gemm_bf16_grouped: 1 or 2 problems per launch");
@@ -1404,8 +1424,7 @@ void gemm_bf16_grouped(const GemmArgs* args, int n, cudaStream_t stream) {
   int limit = args[0].max_ctas > 0 ? args[0].max_ctas : 0;
   if (g_grid_limit > 0 && (limit == 0 || limit > g_grid_limit)) limit = g_grid_limit;
   int nc = args[0].tile_map ? args[0].tile_m / cb::BM : 1, nw = 1;
-  if (!args[0].tile_map && pair_enabled() && (args[0].M > cb::BM || (two && args[1].M > cb::BM)))
-    pick_tile(args, two ? 2 : 1, limit, nc, nw);
+  if (!args[0].tile_map) pick_tile(args, two ? 2 : 1, limit, nc, nw);
   if (nc != 1 && nc != 2) throw std::runtime_error("gemm_bf16_grouped: tile rows must be 128 or 256");
   cb::GemmGroup g{};
   CUtensorMap maps[4];

@@ -84,6 +84,11 @@ int gemm_pick_k_splits(int M, int N, int K, int epi);
 // Debug knob for race hunting: at most `max_ctas` persistent CTAs per launch of a GEMM or a convolution (0 = one per SM).
 void gemm_set_grid_limit(int max_ctas);
 int gemm_grid_limit();
+// Debug knob: the tile of problems taller than 128 rows, as CTAs a tile and 256-column tiles a CTA pair computes at once:
+// (1, 1), (2, 1) or (2, 2), where the epilogue has it; (0, 0): the launcher's choice. Results must not depend on it.
+void gemm_set_tile(int ctas, int col_tiles);
+// The tile that a launch of this problem without split-K takes.
+void gemm_pick_tile(int M, int N, int K, int epi, int& ctas, int& col_tiles);
 // A/B switch: problems taller than one 128-row tile run on CTA pairs (256-row tiles, tcgen05 cta_group::2)
 // when on (the default; COSMOS_GEMM_CTA_PAIR=0 starts with it off).
 void gemm_set_cta_pair(bool on);

@@ -10,6 +10,7 @@ from cosmos_b200.ops import reference as ref
 pytestmark = pytest.mark.gpu
 
 DEV = "cuda"
+GELU = 7     # EPI_GELU of the kernels
 
 
 def _rand(*shape, scale=1.0, dtype=torch.bfloat16):
@@ -1219,11 +1220,11 @@ def test_vae_decode_to_host_is_the_decode(t, chunk):
 
 
 @pytest.mark.parametrize("m,n,k", [(129, 512, 64), (300, 768, 136), (513, 1032, 320), (700, 1536, 1088), (1024, 2048, 192),
-                                    (257, 1024, 2048)])
+                                    (257, 1024, 2048), (700, 3328, 1088)])
 def test_gemm_wide_tiles(m, n, k):
-    """256x512 tiles (a launch of one or two CTA pairs takes them at these sizes) against the fp32 definition, for each
-    epilogue and operand order; ragged rows, columns, k-blocks and an odd number of 256-column tiles. A tile's products are
-    summed in the same order whichever pair computes it, so both launches give the same bits."""
+    """Every tile shape (128x256 on single CTAs, 256x256 and 256x512 on pairs) on one and on two pairs, against the fp32
+    definition, for each epilogue and operand order and for two problems in one launch; ragged rows, columns, k-blocks and an odd
+    number of 256-column tiles. A tile's products are summed in the same order whoever computes it, so all give the same bits."""
     torch.manual_seed(41)
     kern = torch.ops.cosmos_b200
     a, w, r = _rand(m, k), _rand(n, k, scale=1 / math.sqrt(k)), _rand(m, n)
@@ -1241,7 +1242,20 @@ def test_gemm_wide_tiles(m, n, k):
     want = {"plain": a.float() @ w.float().t() + bias.float(),
             "resid": ref.gemm(a.float(), w.float(), None, ops.EPI_GATED_RESID, r.float(), gate.float(), rpb),
             "b_mn": a.float() @ w.float().t()}
+    m2 = m // 2 + 1
+    a2, w2, r2 = _rand(m2, k), _rand(n, k, scale=1 / math.sqrt(k)), _rand(m2, n)
+    two = lambda epi, *rs: torch.cat(ops.gemm_grouped2(a, w, a2, w2, epi, *rs))  # noqa: E731
+    ab, wb = (a.float(), a2.float()), (w.float(), w2.float())
+    calls["gelu"] = lambda: ops.gemm(a, w, bias, GELU)
+    want["gelu"] = torch.nn.functional.gelu(want["plain"])
+    calls["two plain"] = lambda: two(ops.EPI_PLAIN)
+    want["two plain"] = torch.cat([x @ y.t() for x, y in zip(ab, wb)])
+    calls["two resid"] = lambda: two(ops.EPI_GATED_RESID, r, r2, None, gate, m, (m2 + 1) // 2)
+    want["two resid"] = torch.cat([ref.gemm(a.float(), w.float(), None, ops.EPI_GATED_RESID, r.float(), None, m),
+                                   ref.gemm(a2.float(), w2.float(), None, ops.EPI_GATED_RESID, r2.float(), gate.float(), (m2 + 1) // 2)])
     if n % 16 == 0:
+        calls["two swiglu"] = lambda: two(ops.EPI_SWIGLU)
+        want["two swiglu"] = torch.cat([ref.gemm(x, y, epi=ops.EPI_SWIGLU) for x, y in zip(ab, wb)])
         calls["swiglu"] = lambda: ops.gemm(a, w, epi=ops.EPI_SWIGLU)
         want["swiglu"] = ref.gemm(a.float(), w.float(), epi=ops.EPI_SWIGLU)
     if n % 128 == 0:
@@ -1254,16 +1268,26 @@ def test_gemm_wide_tiles(m, n, k):
         at = a.t().contiguous()
         calls["a_mn"] = lambda: kern.gemm_ex(at, wt, True, True, None)
         want["a_mn"] = want["b_mn"]
+    epi = {"swiglu": ops.EPI_SWIGLU, "two swiglu": ops.EPI_SWIGLU, "resid": ops.EPI_GATED_RESID, "two resid": ops.EPI_GATED_RESID,
+           "gelu": GELU, "qkv": ops.EPI_QKV_ROPE, "qkv plain": ops.EPI_QKV_ROPE}
     try:
         for name, call in calls.items():
-            got = {}
-            for limit in (2, 4):
-                kern.gemm_set_grid_limit(limit)
-                got[limit] = call().clone()
-            _close(got[2], want[name], 3e-2, 2e-2, f"{name} {m}x{n}x{k}")
-            assert torch.equal(got[2], got[4]), name
+            first = None
+            if name in ("plain", "resid", "gelu", "swiglu") and kern.gemm_pick_k_splits(m, n, k, epi.get(name, ops.EPI_PLAIN)) > 1:
+                continue     # split-K launches have tiles of their own
+            for tile in ((2, 2), (2, 1), (1, 1)):
+                kern.gemm_set_tile(*tile)
+                for limit in (2, 4):
+                    kern.gemm_set_grid_limit(limit)
+                    assert kern.gemm_pick_tile(m, n, k, epi.get(name, ops.EPI_PLAIN)) == tile
+                    got = call().clone()
+                    if first is None:
+                        first = got
+                        _close(got, want[name], 3e-2, 2e-2, f"{name} {m}x{n}x{k}")
+                    assert torch.equal(got, first), (name, tile, limit)
     finally:
         kern.gemm_set_grid_limit(0)
+        kern.gemm_set_tile(0, 0)
 
 
 def test_gemm_swiglu_keeps_the_limits_of_silu():
@@ -1307,7 +1331,7 @@ def test_gemm_epilogues_take_views_that_start_anywhere(m, n, shift):
 
     flat = torch.empty(2 * n + 8, device=DEV, dtype=torch.bfloat16)[shift:shift + 2 * n].view(2, n).copy_(gate)
     for name, call in {"plain": lambda r, g, **o: ops.gemm(a, w, **o),
-                       "gelu": lambda r, g, **o: ops.gemm(a, w, epi=7, **o),     # EPI_GELU of the kernels
+                       "gelu": lambda r, g, **o: ops.gemm(a, w, epi=GELU, **o),
                        "resid": lambda r, g, **o: ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, g, rpb, **o),
                        "swiglu": lambda r, g, **o: ops.gemm(a, w2, epi=ops.EPI_SWIGLU, **o)}.items():
         want = call(r, gate)
@@ -1319,11 +1343,13 @@ def test_gemm_epilogues_take_views_that_start_anywhere(m, n, shift):
 
 
 @pytest.mark.parametrize("batch,rows", [(1, 40), (2, 240), (3, 100), (5, 33), (9, 20), (40, 7)])
-def test_gemm_qkv_rope_routed_by_batch(batch, rows):
+@pytest.mark.parametrize("hq,tile,limit", [(4, (0, 0), 0), (6, (2, 2), 0), (6, (2, 2), 2), (4, (2, 2), 4), (6, (2, 1), 2), (4, (1, 1), 2)])
+def test_gemm_qkv_rope_routed_by_batch(batch, rows, hq, tile, limit):
     """One routing table per batch entry: the same bits in every buffer as one launch per entry, whichever tables a tile or
-    a warp's 32 rows cross; rows that belong to nobody stay untouched."""
+    a warp's 32 rows cross, for every tile shape (6 query heads make an odd number of 256-column tiles) and schedule; rows that
+    belong to nobody stay untouched."""
     torch.manual_seed(43)
-    k, hq, hk, pre = 256, 4, 2, 3
+    k, hk, pre = 256, 2, 3
     a = _rand(batch, rows, k)
     w = _rand((hq + 2 * hk) * 128, k, scale=1 / math.sqrt(k))
     ang = torch.rand(rows, 64, device=DEV) * 6.28
@@ -1337,7 +1363,13 @@ def test_gemm_qkv_rope_routed_by_batch(batch, rows):
                             for b in range(batch)], device=DEV)
         ld = torch.tensor([[hq * 128] * hq + [hk * 128] * 2 * hk] * batch, device=DEV)
         if merged:
-            ops.gemm_qkv_rope(a.view(batch * rows, k), w, None, cos, sin, gamma, gamma, hq, hk, 1e-6, ptr, ld, route_rows=rows)
+            try:
+                torch.ops.cosmos_b200.gemm_set_tile(*tile)
+                torch.ops.cosmos_b200.gemm_set_grid_limit(limit)
+                ops.gemm_qkv_rope(a.view(batch * rows, k), w, None, cos, sin, gamma, gamma, hq, hk, 1e-6, ptr, ld, route_rows=rows)
+            finally:
+                torch.ops.cosmos_b200.gemm_set_tile(0, 0)
+                torch.ops.cosmos_b200.gemm_set_grid_limit(0)
         else:
             for b in range(batch):
                 ops.gemm_qkv_rope(a[b], w, None, cos, sin, gamma, gamma, hq, hk, 1e-6, ptr[b].contiguous(), ld[b].contiguous())
