@@ -11,14 +11,15 @@
 //     columns, double-buffered against the epilogue;
 //   * activations and weights have rings of their own, so that a weight tile holds its slot for one product and an
 //     activation tile for three.
-// Per 64 channels and tap a CTA of the pair stages 5.7 + 8 KB in place of 32 KB at 128 output channels.
+// Per 64 channels, tap and 128 rows a CTA of the pair stages 5.6 KB of activations and 4 of weights at 128 output channels, where
+// a tile for each tap would take 16 and 8.
 //
 // A strided convolution reads its input split into the four parities of (row, column) ("s2d": [frames, 4, (H + 2) / 2,
 // (W + 2) / 2, C]), which the layer before it writes; each tap is then again a row offset, taps of equal column parity share
 // a tile, and only the kept positions and frames are computed.
 //
 // The epilogue adds bias and residual, writes zeros on the border, and can write: the volume, the s2d form, the nearest
-// x2 / x4 / x8 upsampling that the next convolution reads, and / or silu(rmsnorm(.)) over the channels (a thread holds a
+// upsampling by two in space, and in time, that the next convolution reads, and / or silu(rmsnorm(.)) over the channels (a thread holds a
 // whole row); or, for the 3 output channels of the decoder, uint8 pixels.
 //
 // Measured (480p, chunks of 8 frames at full resolution): 128 -> 128 channels with skip projection 1.95 ms = 1.47 PFLOP/s,

@@ -1376,7 +1376,8 @@ int gemm_pick_k_splits(int M, int N, int K, int epi) {
 // Tile of a problem taller than 128 rows: 128x256 on single CTAs (only for SwiGLU, whose pairs of 256x256 are slower), 256x256
 // or 256x512 on CTA pairs. All three are bound by the bytes that a CTA stages per k-block (48, 32 and 48 KB), so the cost
 // of a launch is its rounds of the persistent CTAs times those bytes; ties go to the larger tile where that does not pad more
-// rows. The norm and rotary epilogue holds an accumulator for about 3 us, which 256x512 tiles hide only in part: counted
+// rows. (An approximation where there are few rounds: a round of 256x512 over 4096 columns of K took 48.9 us at 480 rows of the
+// 24576-wide SwiGLU, one of 128x256 took 33.5 at 333 rows, and both count 48.) The norm and rotary epilogue holds an accumulator for about 3 us, which 256x512 tiles hide only in part: counted
 // like 10 k-blocks.
 // Measured, 256x256 (SwiGLU: 128x256) -> 256x512, us: N x K = 24576 x 4096 SwiGLU M 14080 2291 -> 1821, M 1920 319 -> 290;
 // 4096 x 12288 residual M 14080 1143 -> 924, M 3600 352 -> 272; 4096 x 4096 residual M 3600 124 -> 103; 6144 x 4096 with
@@ -1459,7 +1460,9 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   cb::GemmGroup g{};
   CUtensorMap maps[4];
   // more than one 128-row tile (a serving batch of 256): CTA pairs, so that each CTA stages half of the weight tile
-  // (the skinny GEMMs of such a batch are bound by operand delivery into shared memory, not by HBM)
+  // (the skinny GEMMs of such a batch are bound by operand delivery into shared memory, not by HBM). The split count was
+  // chosen for single CTAs, so pairs can need a second, mostly empty round where those had one: 257 - 384 rows of a 4096-wide
+  // projection are 96 pair items on 74 pairs, 44.8 us at 333 rows where 480 rows (64 items) take 35.2.
   const int nc = a.tile_map ? a.tile_m / cb::BM : (pair_enabled() && a.epi != EPI_SWIGLU && a.M > cb::BM) ? 2 : 1;
   if (nc != 1 && nc != 2) throw std::runtime_error("gemm_bf16: tile rows must be 128 or 256");
   fill_problem(a, g.p[0], maps[0], maps[1], nc);

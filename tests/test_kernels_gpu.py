@@ -866,8 +866,8 @@ def test_gemm_decode_qkv_post_reduces_the_split_k_partials_in_the_glue_kernel(b,
 
 
 def test_vae_channels_last_encoder_matches_pytorch():
-    """Implicit-GEMM encoder (strided convolutions as stride-1 + even positions, 1x1 skips as GEMMs, chunked in time)
-    against the fp32 PyTorch modules in one pass."""
+    """Channels-last encoder (strided convolutions over parity planes, 1x1 skips as columns of the block's second convolution, chunked
+    in time) against the fp32 PyTorch modules in one pass."""
     from cosmos_b200.models.vae import CausalVideoVAE
     from cosmos_b200.models.vae_cuda import CLEncoder
     torch.manual_seed(21)
