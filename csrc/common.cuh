@@ -437,7 +437,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 __device__ __forceinline__ float gelu_erf(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 // silu(g) = g / (1 + exp(-g)) of 16 values, in the bits that the division gives. A division has a branch, so that 16 of them run
-// one after another: SwiGLU of 240 x 24576 x 4096 takes 74 us with them and 55 without. The quotient here is g times an approximate
+// one after another: SwiGLU of 240 x 24576 x 4096 takes 74 us with them and 56 without. The quotient here is g times an approximate
 // reciprocal, refined twice by its residual g - q den (exact in a fused multiply-add; each step of this iterative refinement
 // multiplies the error by that of the reciprocal, about 2^-23). Residuals that could underflow or overflow are left to the
 // division. Compared with it for every one of the 2^32 gates (silu_selftest): no bit differs; after one step two results do.
