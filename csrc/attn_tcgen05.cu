@@ -65,38 +65,6 @@ struct AttnParams {
   int debug;  // timing experiments only: bit 0 skips the QK MMAs, bit 1 the PV MMAs, bit 2 the exponentials
 };
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Packed / three-input fp32 instructions of sm_100: they halve the instruction count of the softmax
-// inner loop, which (not the tensor or MUFU pipe) is what bounds this kernel.
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // Two exponentials at once on the FMA pipe with packed fp32 instructions, for scores already turned into
 // x = s * scale_log2 - m with x >= -126 (the caller clamps the raw score, one FMNMX each):
 // round-to-nearest split x = n + f with f in [-0.5, 0.5] by the magic-number add (the integer n sits in the low

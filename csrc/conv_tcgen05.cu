@@ -41,7 +41,8 @@ constexpr int CV_MAX_GROUPS = 18;
 constexpr int CV_CHUNK = 4;                    // channel blocks of 64 whose tiles are staged together
 constexpr int CV_SMEM_MAX = 227 * 1024;
 constexpr int CV_BARS = 512;                   // bytes for barriers, tensor-memory slot and abort flag
-constexpr int CV_SUMS = 8192;                  // row sums of the norm: [2 tiles][2 row tiles][2 column halves][128 rows][2] floats
+constexpr int CV_SUMS = 4096;                  // row sums of the norm: [2 tiles][2 row tiles][2 column halves][128 rows] floats
+constexpr int CV_GAMMA = 1024;                 // the norm's weights as fp32
 
 // Taps that read one staged tile: row offset of the tile, and per tap its shift inside the tile and its index in the weights.
 struct ConvGroup {
@@ -87,6 +88,36 @@ struct ConvCfg {
 __device__ __forceinline__ void cv_store16(bf16* dst, const uint32_t (&pk)[8]) {
   reinterpret_cast<uint4*>(dst)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   reinterpret_cast<uint4*>(dst)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+}
+
+// silu(z) = z / (1 + exp(-z)) of 16 values given as their negatives, rounded to bf16. The quotient is z times an approximate
+// reciprocal, refined once by its residual (of all 2^32 fp32 values, two then differ from the division's, in their last bit);
+// negatives of value and reciprocal let every step be a packed instruction. Beyond 80, where the exponential leaves its range,
+// and for infinities the division itself.
+__device__ __forceinline__ void cv_silu16(const uint64_t (&zn)[8], uint32_t (&out)[8]) {
+  const uint64_t log2e = pack2(1.4426950408889634f, 1.4426950408889634f), one = pack2(1.f, 1.f);
+  float top = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float2 z = unpack2(zn[k]);
+    top = fmaxf(top, fmaxf(fabsf(z.x), fabsf(z.y)));
+    const float2 t = unpack2(mul2(zn[k], log2e));
+    const uint64_t den = add2(pack2(ex2(t.x), ex2(t.y)), one);
+    const float2 d = unpack2(den);
+    float r0, r1;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d.y));
+    const uint64_t rn = pack2(r0, r1), q = mul2(zn[k], rn);
+    const float2 y = unpack2(fma2(fma2(q, den, zn[k]), rn, q));
+    out[k] = pack_bf16(y.x, y.y);
+  }
+  if (top >= 80.f) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float2 z = unpack2(zn[k]);
+      out[k] = pack_bf16(-z.x / (1.f + __expf(z.x)), -z.y / (1.f + __expf(z.y)));
+    }
+  }
 }
 
 // Meeting of the two warps that share the rows of a quadrant; true when both say so.
@@ -160,7 +191,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint8_t* gen = smem_raw + (tmem_slot - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 8);
-  float2* row_sums = reinterpret_cast<float2*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
+  float* row_sums = reinterpret_cast<float*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
+  float* gamma = row_sums + CV_SUMS / 4;
 
   const uint32_t rank = cluster_ctarank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -175,6 +207,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     fence_barrier_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
+  }
+  if constexpr (NC > 0) {
+    for (int c = threadIdx.x; c < NC; c += Cfg::THREADS) gamma[c] = __bfloat162float(p.gamma[c]);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
@@ -360,14 +395,11 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         __syncwarp();
         const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
-        // Squares are added per 8 channels and these sums in the order of a warp's butterfly: groups in bit-reversed order,
-        // summed like a binary counter.
-        float lvl[3][2], sum[2] = {0.f, 0.f};
+        uint64_t sq[2] = {0, 0};                         // sums of squares, two pairs
         const int groups = (NC > 0 ? NC : n_end) >> 5;   // of this warp
 #pragma unroll 1
         for (int i = 0; i < groups; ++i) {
-          const int ri = NC == 256 ? ((i & 1) << 2 | (i & 2) | i >> 2) : NC == 128 ? ((i & 1) << 1 | i >> 1) : i;
-          const int c = 32 * ri + 16 * half;
+          const int c = 32 * i + 16 * half;
           uint32_t v[16], pk[8];
           tmem_ld16(ta + c, v);
           uint4 ru[2];
@@ -377,15 +409,16 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           tmem_wait_ld();
           if (inside) {
-            float a[16];
+            uint64_t a[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = __uint_as_float(v[k]);
+            for (int k = 0; k < 8; ++k) a[k] = pack2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
             if (p.bias) {
               const float4* b4 = reinterpret_cast<const float4*>(p.bias + n_base + c);
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const float4 b = b4[k];
-                a[4 * k] += b.x; a[4 * k + 1] += b.y; a[4 * k + 2] += b.z; a[4 * k + 3] += b.w;
+                a[2 * k] = add2(a[2 * k], pack2(b.x, b.y));
+                a[2 * k + 1] = add2(a[2 * k + 1], pack2(b.z, b.w));
               }
             }
             if (res) {
@@ -393,11 +426,15 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               for (int k = 0; k < 2; ++k) {
                 const uint32_t w[4] = {ru[k].x, ru[k].y, ru[k].z, ru[k].w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) { a[k * 8 + 2 * e] += bf16lo(w[e]); a[k * 8 + 2 * e + 1] += bf16hi(w[e]); }
+                for (int e = 0; e < 4; ++e) a[4 * k + e] = add2(a[4 * k + e], pack2(bf16lo(w[e]), bf16hi(w[e])));
               }
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) pk[k] = pack_bf16(a[2 * k], a[2 * k + 1]);
+            for (int k = 0; k < 8; ++k) {
+              float lo, hi;
+              unpack2(a[k], lo, hi);
+              pk[k] = pack_bf16(lo, hi);
+            }
           } else {
 #pragma unroll
             for (int k = 0; k < 8; ++k) pk[k] = 0u;
@@ -414,26 +451,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           if constexpr (NC > 0) {
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              float s = 0.f;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float lo = bf16lo(pk[4 * k + e]), hi = bf16hi(pk[4 * k + e]);
-                s += lo * lo;
-                s += hi * hi;
-              }
-              if (i & 1) {
-                s = lvl[0][k] + s;
-                if (i & 2) {
-                  s = lvl[1][k] + s;
-                  if (i & 4) s = lvl[2][k] + s; else lvl[2][k] = s;
-                } else {
-                  lvl[1][k] = s;
-                }
-              } else {
-                lvl[0][k] = s;
-              }
-              sum[k] = s;
+            for (int k = 0; k < 8; ++k) {
+              const uint64_t x = pack2(bf16lo(pk[k]), bf16hi(pk[k]));
+              sq[k & 1] = fma2(x, x, sq[k & 1]);
             }
             __syncwarp();
             tmem_st8(ta + c, pk);   // the rounded values wait in place of their accumulators
@@ -441,33 +461,31 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           __syncwarp();
         }
         if constexpr (NC > 0) {
-          // the other half's sums (two buffers: a warp is at most one meeting ahead of its partner)
-          float2* mine = row_sums + ((buf * 2 + r) * 2 + half) * 128 + quad * 32 + lane;
-          *mine = make_float2(sum[0], sum[1]);
+          // the other half's sum (two buffers: a warp is at most one meeting ahead of its partner)
+          const float2 s2 = unpack2(add2(sq[0], sq[1]));
+          const float sum = s2.x + s2.y;
+          row_sums[((buf * 2 + r) * 2 + half) * 128 + quad * 32 + lane] = sum;
           tmem_wait_st();
           cv_pair_and(pair_id, true);
-          const float2 other = row_sums[((buf * 2 + r) * 2 + (half ^ 1)) * 128 + quad * 32 + lane];
-          const float s0 = half ? other.x + sum[0] : sum[0] + other.x, s1 = half ? other.y + sum[1] : sum[1] + other.y;
-          const float rinv = rsqrtf((s0 + s1) / (float)NC + p.eps);
+          const float other = row_sums[((buf * 2 + r) * 2 + (half ^ 1)) * 128 + quad * 32 + lane];
+          const float rneg = -rsqrtf((sum + other) / (float)NC + p.eps);
+          const uint64_t rneg2 = pack2(rneg, rneg);
           bf16* o = p.out_norm + dst.row * ld;
 #pragma unroll 1
           for (int c = 16 * half; c < NC; c += 32) {
             uint32_t pk[8], on[8];
+            uint64_t zn[8];
             tmem_ld8(ta + c, pk);
-            uint4 gu[2];
-            gu[0] = reinterpret_cast<const uint4*>(p.gamma + c)[0];
-            gu[1] = reinterpret_cast<const uint4*>(p.gamma + c)[1];
+            const float4* g4 = reinterpret_cast<const float4*>(gamma + c);
+            float4 g[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) g[k] = g4[k];
             tmem_wait_ld();
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const uint32_t gw[4] = {gu[k].x, gu[k].y, gu[k].z, gu[k].w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const uint32_t u = pk[4 * k + e];
-                const float lo = bf16lo(u) * rinv * bf16lo(gw[e]), hi = bf16hi(u) * rinv * bf16hi(gw[e]);
-                on[4 * k + e] = pack_bf16(lo / (1.f + __expf(-lo)), hi / (1.f + __expf(-hi)));   // zero on the border
-              }
-            }
+            for (int k = 0; k < 8; ++k)
+              zn[k] = mul2(mul2(pack2(bf16lo(pk[k]), bf16hi(pk[k])), rneg2),
+                           k & 1 ? pack2(g[k >> 1].z, g[k >> 1].w) : pack2(g[k >> 1].x, g[k >> 1].y));
+            cv_silu16(zn, on);   // zero on the border
             if (row_ok) cv_store16(o + c, on);
             __syncwarp();
           }
@@ -663,7 +681,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   const int R = p.mma_n <= 128 ? 2 : 1;
   p.tiles_per_seg = (p.seg_rows + 256 * R - 1) / (256 * R);
   const int a_slot = (128 * R + 8) * 128, b_slot = p.mma_n * 64;
-  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_BARS - cb::CV_SUMS;
+  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_BARS - cb::CV_SUMS - cb::CV_GAMMA;
   const int chunk = std::min(cb::CV_CHUNK, std::max(p.cblocks, p.skip_cblocks));
   // activations: one group's tiles and as many of the next one as fit beside the weight tiles: eight of those, or six where
   // four channel blocks meet 256 output channels
