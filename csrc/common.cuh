@@ -369,6 +369,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar)
                : "memory");
 }
+// The same without an order for this thread's global stores, for which the cluster-scope release waits: enough to hand back tensor
+// memory, whose accesses a tcgen05.wait and tcgen05.fence::before_thread_sync have completed.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 // TMA loads of a CTA pair: the data lands in this CTA's shared memory, the bytes are counted on
 // the mbarrier at `cluster_bar`, which may live in the other CTA of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m,

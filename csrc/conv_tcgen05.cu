@@ -41,8 +41,9 @@ constexpr int CV_MAX_GROUPS = 18;
 constexpr int CV_CHUNK = 4;                    // channel blocks of 64 whose tiles are staged together
 constexpr int CV_SMEM_MAX = 227 * 1024;
 constexpr int CV_BARS = 512;                   // bytes for barriers, tensor-memory slot and abort flag
-constexpr int CV_SUMS = 4096;                  // row sums of the norm: [2 tiles][2 row tiles][2 column halves][128 rows] floats
-constexpr int CV_GAMMA = 1024;                 // the norm's weights as fp32
+constexpr int CV_SUMS = 8192;                  // row sums of the norm: [2 tiles][2 row tiles][2 column halves][128 rows][2] floats
+constexpr int CV_GAMMA = 1024;                 // the norm's weights as fp32; behind them the bias (up to 256 channels)
+constexpr int CV_TAIL = CV_BARS + CV_SUMS + 2 * CV_GAMMA;
 
 // Taps that read one staged tile: row offset of the tile, and per tap its shift inside the tile and its index in the weights.
 struct ConvGroup {
@@ -73,6 +74,9 @@ struct ConvParams {
   int keep_border;       // CONV_OUT_SAME: the border's cells are not written
   int tpad;              // context frames in front of every output volume
   int f_out;             // frames computed
+  int seg_frames;        // conv_time_kernel: output frames of a time segment (n_seg of them)
+  int kt_taps;           // taps of a frame in the weights: 9, or 1 (taps in time only)
+  int nt;                // conv_time_kernel: accumulator columns of a frame, 16, 32 or 64
   int up_t, up_first;    // CONV_OUT_UP: temporal doubling, first chunk (its first frame is not doubled)
   int* status;
 };
@@ -82,12 +86,20 @@ struct ConvCfg {
   static constexpr int A_ROWS = 128 * R + 8;
   static constexpr int A_SLOT = A_ROWS * 128;
   static constexpr int ACC_COLS = 256 / R;     // tensor-memory columns of one accumulator
-  static constexpr int THREADS = 64 + 256 * R; // producer, MMA issuer, eight epilogue warps per row tile
+  static constexpr int THREADS = 96 + 256 * R; // producer, MMA issuer, eight epilogue warps per row tile, second producer
 };
 
-__device__ __forceinline__ void cv_store16(bf16* dst, const uint32_t (&pk)[8]) {
-  reinterpret_cast<uint4*>(dst)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-  reinterpret_cast<uint4*>(dst)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+// The 16 columns of a row are 32 bytes, one sector, held by one thread. Stored by it as two vectors they reach L2 as half sectors,
+// two requests for each, and L2 reads the sector from memory to complete it: the first layer of the encoder (64 channels, two outputs)
+// read 1.23 GB where its input has 0.41. So neighbouring lanes swap halves, and a store instruction writes whole sectors of every
+// other row: first those of the even lanes' rows (`even`), then those of the odd lanes' (`odd`), lane parity = half of the sector.
+__device__ __forceinline__ void cv_swap_halves(const uint32_t (&pk)[8], int lane, uint4& even, uint4& odd) {
+  const bool o = lane & 1;
+  uint32_t r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r[k] = __shfl_xor_sync(0xffffffffu, o ? pk[k] : pk[4 + k], 1);
+  even = o ? make_uint4(r[0], r[1], r[2], r[3]) : make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  odd = o ? make_uint4(pk[4], pk[5], pk[6], pk[7]) : make_uint4(r[0], r[1], r[2], r[3]);
 }
 
 // silu(z) = z / (1 + exp(-z)) of 16 values given as their negatives, rounded to bf16. The quotient is z times an approximate
@@ -120,19 +132,9 @@ __device__ __forceinline__ void cv_silu16(const uint64_t (&zn)[8], uint32_t (&ou
   }
 }
 
-// Meeting of the two warps that share the rows of a quadrant; true when both say so.
-__device__ __forceinline__ bool cv_pair_and(int id, bool ok) {
-  int r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.s32 q, %1, 0;\n\t"
-      "barrier.cta.red.and.pred p, %2, 64, q;\n\t"
-      "selp.s32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)
-      : "r"(ok ? 1 : 0), "r"(id)
-      : "memory");
-  return r != 0;
-}
+// Meeting of the two warps that share the rows of a quadrant. Both come to every one of them: a warp whose wait for an accumulator
+// gave up goes on without storing (the later waits give up at once).
+__device__ __forceinline__ void cv_meet(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
 // Where a row of the result goes: `n_t` x `n_y` x `n_x` rows starting at `row` (one row except for the upsampled form).
 struct ConvDest {
@@ -166,8 +168,214 @@ __device__ __forceinline__ ConvDest conv_dest(const ConvParams& p, int f, int y,
   return d;
 }
 
-// R row tiles per CTA; NC = channels of the fused norm (64, 128, 256) or 0; RGB: pixels.
-template <int R, int NC, bool RGB>
+// One accumulator's row per thread, at tensor-memory address `ta` (the quadrant's lanes): row (y, x) of the plane, `rem` in it, of
+// frame `f`; output channels from `n_base` on. The two warps of a quadrant take every other group of 16 columns (`half`) and
+// meet at named barrier `pair_id`; sums: where this row's sum of squares goes, [2 halves][128]. ZERO: the accumulator is left
+// zero for the next frame's products.
+// `release` hands the accumulator back and is called once the last of it is read.
+template <int NC, bool RGB, bool ZERO, int U, typename Release>
+__device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int f, int rem, int y, int x, bool row_ok, int n_base,
+                                          int half, int pair_id, float2* sums, const float* gamma, const float* bias, Release release) {
+  const bool down = p.mode == CONV_OUT_DOWN;
+  const bool inside = row_ok && (down ? (y < p.hp - 1 && x < p.wp - 1) : (y >= 1 && y <= p.hp - 2 && x >= 1 && x <= p.wp - 2));
+  const uint32_t zero16[16] = {};
+  if constexpr (RGB) {
+    uint32_t v[16];
+    tmem_ld16(ta, v);
+    tmem_wait_ld();
+    if constexpr (ZERO) {
+      if (half == 0) tmem_st16(ta, zero16);
+      tmem_wait_st();
+    }
+    release();
+    if (inside && half == 0) {
+      uint8_t* o = p.rgb + (((long long)f * (p.hp - 2) + y - 1) * (p.wp - 2) + x - 1) * 3;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        // columns 3 .. 8: the low parts of fp32 weights, exact in three bf16 terms
+        const float a = ((__uint_as_float(v[6 + c]) + __uint_as_float(v[3 + c])) + __uint_as_float(v[c])) + bias[c];
+        o[c] = (uint8_t)__float2int_rn((fminf(fmaxf(a, -1.f), 1.f) + 1.f) * 127.5f);
+      }
+    }
+  } else {
+    const ConvDest dst = conv_dest(p, f, y, x);
+    const int n_end = min(256, p.n_out - n_base);
+    const long long ld = p.n_out;
+    if (down && row_ok && half == 0 && (x == 0 || y == 0)) {
+      // border cells that no position of the plane maps to: left column, top row
+      for (int k = 0; k < 3; ++k) {
+        if ((k == 0 && x != 0) || (k == 1 && y != 0) || (k == 2 && (x != 0 || y != 0))) continue;
+        const long long cell = dst.row - (k == 1 ? 0 : 1) - (k == 0 ? 0 : p.wp + 1);
+        for (int c = 0; c < n_end; c += 8) {
+          if (p.out) *reinterpret_cast<uint4*>(p.out + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+          if (p.out_norm) *reinterpret_cast<uint4*>(p.out_norm + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+        }
+      }
+    }
+    __syncwarp();
+    // the rows that this lane stores: its pair's even and odd one (bits of `to`: copies in time, y and x; result and norm stored)
+    const int lane = threadIdx.x & 31;
+    const int info = dst.n_t | dst.n_y << 2 | dst.n_x << 4 | (row_ok && (inside || !p.keep_border) ? 64 : 0) | (row_ok ? 128 : 0);
+    const long long row0 = __shfl_sync(0xffffffffu, dst.row, lane & ~1), row1 = __shfl_sync(0xffffffffu, dst.row, lane | 1);
+    const int to0 = __shfl_sync(0xffffffffu, info, lane & ~1), to1 = __shfl_sync(0xffffffffu, info, lane | 1);
+    auto store = [&](bf16* o, const uint4& v, int to) {
+      if (p.mode != CONV_OUT_UP) {
+        *reinterpret_cast<uint4*>(o) = v;
+      } else {
+        for (int tt = 0; tt < (to & 3); ++tt)
+          for (int yy = 0; yy < (to >> 2 & 3); ++yy)
+            for (int xx = 0; xx < (to >> 4 & 3); ++xx) *reinterpret_cast<uint4*>(o + (tt * dst.st + yy * dst.sy + xx) * ld) = v;
+      }
+    };
+    const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
+    static_assert(U == 2 || (U == 1 && NC != 64), "columns at a time");
+    constexpr bool KEEP = NC == 64;   // the rounded values stay in registers until the row's norm is known; else in tensor memory
+    // Squares are added per 8 channels (two such chains side by side) and these sums in the order of a warp's butterfly: groups
+    // in bit-reversed order, summed like a binary counter.
+    uint64_t lvl[3] = {0, 0, 0}, sum = 0;
+    uint32_t pk[U][8];
+    const int groups = (NC > 0 ? NC : n_end) >> 5;   // of 16 columns, of this warp; U at a time
+#pragma unroll 1
+    for (int i = 0; i < groups; i += U) {
+      int c[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = i + u;
+        c[u] = 32 * (NC == 256 ? ((j & 1) << 2 | (j & 2) | j >> 2) : NC == 128 ? ((j & 1) << 1 | j >> 1) : j) + 16 * half;
+      }
+      const bool two = U == 2 && (NC > 0 || i + 1 < groups);
+      uint32_t v[U][16];
+      uint4 ru[U][2];
+      tmem_ld16(ta + c[0], v[0]);
+      if (two) tmem_ld16(ta + c[U - 1], v[U - 1]);
+      if (res && inside) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (u == 0 || two) {
+            ru[u][0] = reinterpret_cast<const uint4*>(res + c[u])[0];
+            ru[u][1] = reinterpret_cast<const uint4*>(res + c[u])[1];
+          }
+      }
+      tmem_wait_ld();
+      if constexpr (ZERO) {
+        tmem_st16(ta + c[0], zero16);
+        if (two) tmem_st16(ta + c[U - 1], zero16);
+      }
+      if ((NC == 0 || KEEP) && i + U >= groups) {
+        if constexpr (ZERO) tmem_wait_st();
+        release();
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (u == 1 && !two) break;
+        uint64_t a[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a[k] = pack2(__uint_as_float(v[u][2 * k]), __uint_as_float(v[u][2 * k + 1]));
+        if (bias) {
+          const float4* b4 = reinterpret_cast<const float4*>(bias + n_base + c[u]);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 b = b4[k];
+            a[2 * k] = add2(a[2 * k], pack2(b.x, b.y));
+            a[2 * k + 1] = add2(a[2 * k + 1], pack2(b.z, b.w));
+          }
+        }
+        if (res) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const uint32_t w[4] = {ru[u][k].x, ru[u][k].y, ru[u][k].z, ru[u][k].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[4 * k + e] = add2(a[4 * k + e], pack2(bf16lo(w[e]), bf16hi(w[e])));
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float2 y2 = unpack2(a[k]);
+          pk[u][k] = inside ? pack_bf16(y2.x, y2.y) : 0u;
+        }
+        if (p.out) {
+          uint4 v0, v1;
+          cv_swap_halves(pk[u], lane, v0, v1);
+          bf16* o = p.out + n_base + c[u] + 8 * (lane & 1);
+          if (to0 & 64) store(o + row0 * ld, v0, to0);
+          if (to1 & 64) store(o + row1 * ld, v1, to1);
+          __syncwarp();
+        }
+      }
+      if constexpr (NC > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          uint64_t q = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint64_t lo = pack2(bf16lo(pk[u][k]), bf16lo(pk[u][4 + k])), hi = pack2(bf16hi(pk[u][k]), bf16hi(pk[u][4 + k]));
+            q = fma2(lo, lo, q);
+            q = fma2(hi, hi, q);
+          }
+          const int j = i + u;
+          if (j & 1) {
+            q = add2(lvl[0], q);
+            if (j & 2) {
+              q = add2(lvl[1], q);
+              if (j & 4) q = add2(lvl[2], q); else lvl[2] = q;
+            } else {
+              lvl[1] = q;
+            }
+          } else {
+            lvl[0] = q;
+          }
+          sum = q;
+        }
+        if constexpr (!KEEP) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) tmem_st8(ta + c[u], pk[u]);   // in place of their accumulators
+        }
+      }
+    }
+    if constexpr (NC > 0) {
+      // the other half's sums (two buffers: a warp is at most one meeting ahead of its partner)
+      const float2 own = unpack2(sum);
+      sums[half * 128] = own;
+      if constexpr (!KEEP) tmem_wait_st();
+      cv_meet(pair_id);
+      const float2 other = sums[(half ^ 1) * 128];
+      const float s0 = own.x + other.x, s1 = own.y + other.y;
+      const float rneg = -rsqrtf((s0 + s1) / (float)NC + p.eps);
+      const uint64_t rneg2 = pack2(rneg, rneg);
+      bf16 *o0 = p.out_norm + row0 * ld + 8 * (lane & 1), *o1 = p.out_norm + row1 * ld + 8 * (lane & 1);
+#pragma unroll 1
+      for (int c = 16 * half; c < NC; c += 32 * U) {
+        if constexpr (!KEEP) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) tmem_ld8(ta + c + 32 * u, pk[u]);
+          tmem_wait_ld();
+          if (c + 32 * U >= NC) release();
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          uint32_t on[8];
+          uint64_t zn[8];
+          const float4* g4 = reinterpret_cast<const float4*>(gamma + c + 32 * u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 g = g4[k];
+            zn[2 * k] = mul2(mul2(pack2(bf16lo(pk[u][2 * k]), bf16hi(pk[u][2 * k])), rneg2), pack2(g.x, g.y));
+            zn[2 * k + 1] = mul2(mul2(pack2(bf16lo(pk[u][2 * k + 1]), bf16hi(pk[u][2 * k + 1])), rneg2), pack2(g.z, g.w));
+          }
+          cv_silu16(zn, on);   // zero on the border
+          uint4 v0, v1;
+          cv_swap_halves(on, lane, v0, v1);
+          if (to0 & 128) *reinterpret_cast<uint4*>(o0 + c + 32 * u) = v0;
+          if (to1 & 128) *reinterpret_cast<uint4*>(o1 + c + 32 * u) = v1;
+          __syncwarp();
+        }
+      }
+    }
+  }
+}
+
+// R row tiles per CTA; NC = channels of the fused norm (64, 128, 256) or 0.
+template <int R, int NC>
 __global__ void __launch_bounds__(ConvCfg<R>::THREADS, 1)
 conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
             const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmX2,
@@ -191,8 +399,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint8_t* gen = smem_raw + (tmem_slot - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 8);
-  float* row_sums = reinterpret_cast<float*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
-  float* gamma = row_sums + CV_SUMS / 4;
+  float2* row_sums = reinterpret_cast<float2*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
+  float* gamma = reinterpret_cast<float*>(row_sums) + CV_SUMS / 4;
 
   const uint32_t rank = cluster_ctarank();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -211,6 +419,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if constexpr (NC > 0) {
     for (int c = threadIdx.x; c < NC; c += Cfg::THREADS) gamma[c] = __bfloat162float(p.gamma[c]);
   }
+  if (p.n_tiles == 1)
+    for (int c = threadIdx.x; c < p.n_out; c += Cfg::THREADS) gamma[CV_GAMMA / 4 + c] = p.bias ? p.bias[c] : 0.f;
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
@@ -223,12 +433,13 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   if (warp == 0) {
     if (lane == 0) {
-      // ---------------- TMA producer: both rings, in the order in which the products consume them
-      int ia = 0, ib = 0;
-      uint32_t pha = 0, phb = 0;   // phase parities of the rings
+      // ---------------- TMA producer of the activations, in the order in which the products consume them (the last warp brings
+      // the weights: a thread's instructions for both take longer than a tap's products of 64 columns)
+      int ia = 0;
+      uint32_t pha = 0;
       bool ok = true;
       for (int t = first_tile; t < total && ok; t += tile_step) {
-        const int nt = t % p.n_tiles, mt = t / p.n_tiles;
+        const int mt = t / p.n_tiles;
         const int seg = mt / p.tiles_per_seg, tile = mt - seg * p.tiles_per_seg;
         const int local = tile * TILE_M + int(rank) * (128 * R);
         for (int ph = 0; ph < 2 && ok; ++ph) {
@@ -240,27 +451,50 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             const int nc = min(CV_CHUNK, cblocks - c0);
             const int n_groups = ph ? 1 : p.n_groups;
             for (int g = 0; g < n_groups && ok; ++g) {
-              const int n_taps = ph ? 1 : p.g[g].n_taps;
               const int y = row + (ph ? 0 : p.g[g].off);
-              for (int i = 0; i < n_taps && ok; ++i) {
-                const int kcol = ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64;
-                for (int c = 0; c < nc; ++c) {
-                  if (i == 0) {
-                    if (!mbar_wait(empty_a(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
-                    if (rank == 0) mbar_arrive_expect_tx(full_a(ia), 2 * Cfg::A_SLOT);
-                    const uint32_t fb = mapa(full_a(ia), 0);
-                    const uint32_t dst = smem_base + ia * Cfg::A_SLOT;
-                    tma_load_2d_pair(dst, m0, fb, (c0 + c) * 64, y);
+              for (int c = 0; c < nc; ++c) {
+                if (!mbar_wait(empty_a(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+                if (rank == 0) mbar_arrive_expect_tx(full_a(ia), 2 * Cfg::A_SLOT);
+                const uint32_t fb = mapa(full_a(ia), 0);
+                const uint32_t dst = smem_base + ia * Cfg::A_SLOT;
+                tma_load_2d_pair(dst, m0, fb, (c0 + c) * 64, y);
 #pragma unroll
-                    for (int r = 1; r < R; ++r)
-                      tma_load_2d_pair(dst + (CV_HALO_ROWS + (r - 1) * 128) * 128, m1, fb, (c0 + c) * 64,
-                                       y + CV_HALO_ROWS + (r - 1) * 128);
-                    if (++ia == NA) { ia = 0; pha ^= 1; }
-                  }
+                for (int r = 1; r < R; ++r)
+                  tma_load_2d_pair(dst + (CV_HALO_ROWS + (r - 1) * 128) * 128, m1, fb, (c0 + c) * 64,
+                                   y + CV_HALO_ROWS + (r - 1) * 128);
+                if (++ia == NA) { ia = 0; pha ^= 1; }
+              }
+            }
+          }
+        }
+      }
+      if (!ok) {
+        // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      }
+    }
+  } else if (warp == Cfg::THREADS / 32 - 1) {
+    if (lane == 0) {
+      // ---------------- TMA producer of the weights
+      int ib = 0;
+      uint32_t phb = 0;
+      bool ok = true;
+      for (int t = first_tile; t < total && ok; t += tile_step) {
+        const int y = (t % p.n_tiles) * 256 + int(rank) * (p.mma_n >> 1);
+        for (int ph = 0; ph < 2 && ok; ++ph) {
+          const int cblocks = ph ? p.skip_cblocks : p.cblocks;
+          for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
+            const int nc = min(CV_CHUNK, cblocks - c0);
+            const int n_groups = ph ? 1 : p.n_groups;
+            for (int g = 0; g < n_groups && ok; ++g) {
+              const int n_taps = ph ? 1 : p.g[g].n_taps;
+              for (int i = 0; i < n_taps && ok; ++i) {
+                const int x = (ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64) + c0 * 64;
+                for (int c = 0; c < nc; ++c) {
                   if (!mbar_wait(empty_b(ib), phb ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
                   if (rank == 0) mbar_arrive_expect_tx(full_b(ib), 2 * b_slot);
-                  tma_load_2d_pair(b_base + ib * b_slot, &tmB, mapa(full_b(ib), 0), kcol + (c0 + c) * 64,
-                                   nt * 256 + int(rank) * (p.mma_n >> 1));
+                  tma_load_2d_pair(b_base + ib * b_slot, &tmB, mapa(full_b(ib), 0), x + c * 64, y);
                   if (++ib == NB) { ib = 0; phb ^= 1; }
                 }
               }
@@ -269,7 +503,6 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
       }
       if (!ok) {
-        // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000ll) {}
       }
@@ -348,7 +581,9 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // all, which are exact so that the result is the separate norm kernel's), hence the number of warps.
     const int quad = warp & 3, half = ((warp - 2) >> 2) & 1, r = (warp - 2) >> 3;
     const int pair_id = 1 + r * 4 + quad;
+    const float* bias = p.n_tiles == 1 ? gamma + CV_GAMMA / 4 : p.bias;
     int tcount = 0;
+    bool alive = true;
     for (int t = first_tile; t < total; t += tile_step, ++tcount) {
       const int buf = tcount & 1;
       const int nt = t % p.n_tiles, mt = t / p.n_tiles;
@@ -358,144 +593,275 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const bool row_ok = q < p.seg_rows;
       const int f0 = q / p.plane, rem = q - f0 * p.plane;
       const int f = f0 + seg, y = rem / p.pw, x = rem - y * p.pw;   // several segments: one frame each
-      const bool down = p.mode == CONV_OUT_DOWN;
-      const bool inside = row_ok && (down ? (y < p.hp - 1 && x < p.wp - 1) : (y >= 1 && y <= p.hp - 2 && x >= 1 && x <= p.wp - 2));
-      bool go = mbar_wait(tfull(buf), (tcount >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EPI);
-      // warps that meet below leave together: a wait that one of them gave up is given up by both
-      go = NC > 0 ? cv_pair_and(pair_id, go) : __all_sync(0xffffffffu, go);
-      if (!go) break;
+      alive = mbar_wait(tfull(buf), (tcount >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EPI) && alive;
+      __syncwarp();
       tc_fence_after();
-      if constexpr (RGB) {
-        uint32_t v[16];
-        tmem_ld16(ta, v);
-        tmem_wait_ld();
-        if (inside && half == 0) {
-          uint8_t* o = p.rgb + (((long long)f * (p.hp - 2) + y - 1) * (p.wp - 2) + x - 1) * 3;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            // columns 3 .. 8: the low parts of fp32 weights, exact in three bf16 terms
-            const float a = ((__uint_as_float(v[6 + c]) + __uint_as_float(v[3 + c])) + __uint_as_float(v[c])) + p.bias[c];
-            o[c] = (uint8_t)__float2int_rn((fminf(fmaxf(a, -1.f), 1.f) + 1.f) * 127.5f);
-          }
-        }
-      } else {
-        const ConvDest dst = conv_dest(p, f, y, x);
-        const int n_base = nt * 256, n_end = min(256, p.n_out - n_base);
-        const long long ld = p.n_out;
-        if (down && row_ok && half == 0 && (x == 0 || y == 0)) {
-          // border cells that no position of the plane maps to: left column, top row
-          for (int k = 0; k < 3; ++k) {
-            if ((k == 0 && x != 0) || (k == 1 && y != 0) || (k == 2 && (x != 0 || y != 0))) continue;
-            const long long cell = dst.row - (k == 1 ? 0 : 1) - (k == 0 ? 0 : p.wp + 1);
-            for (int c = 0; c < n_end; c += 8) {
-              if (p.out) *reinterpret_cast<uint4*>(p.out + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
-              if (p.out_norm) *reinterpret_cast<uint4*>(p.out_norm + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+      conv_emit<NC, false, false, R == 1 || NC == 64 ? 2 : 1>(p, ta, f, rem, y, x, row_ok && alive, nt * 256, half, pair_id,
+                                  row_sums + (buf * 2 + r) * 256 + quad * 32 + lane, gamma, bias, [&] {
+                                    tc_fence_before();
+                                    __syncwarp();
+                                    if (lane == 0) {
+                                      if (rank != 0) mbar_arrive_peer(mapa(tempty(buf), 0));
+                                      else mbar_arrive(tempty(buf));
+                                    }
+                                  });
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+// Convolutions with at most 64 output channels: a CTA pair walks its 512 positions through time, and one product of up to
+// 3 x 64 columns adds an input frame's tap to the three output frames that the frame belongs to (temporal taps side by side along
+// N). With 64 columns a product is bound by the reads of its A operand from shared memory (32 clocks for 32 of MMA, and a
+// fresh A three times), and a frame's activations crossed L2 -> shared memory for each temporal tap; here every activation tile
+// crosses 3 times and not 9, and its reads are shared by 192 columns (96 clocks).
+// A ring of four accumulators per row tile: three frames being summed, one being drained. The epilogue leaves a drained
+// accumulator zero, so that every product accumulates. Where the ring wraps, the frames' columns are not contiguous and a
+// tap takes two products.
+// 480p, 8 frames, us, before -> after: CONVT_FIGURES
+constexpr int CT_SLOTS = 4;
+constexpr int CT_THREADS = ConvCfg<2>::THREADS;
+__host__ __device__ constexpr int ct_stage(int nt) { return ConvCfg<2>::A_SLOT + 9 * nt * 64; }
+template <int NC, bool RGB>
+__global__ void __launch_bounds__(CT_THREADS, 1)
+conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
+                 const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ConvParams p) {
+  using Cfg = ConvCfg<2>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int NS = p.na;
+  const int piece = p.nt * 64;        // half of a frame's columns: (nt / 2 rows) x 128 bytes
+  const int stage = ct_stage(p.nt);   // activations, and a CTA's half of the weights of three taps for three frames
+  const uint32_t bar_base = smem_base + NS * stage;
+  auto full = [&](int s) { return bar_base + 8u * s; };
+  auto empty = [&](int s) { return bar_base + 8u * (NS + s); };
+  const uint32_t t_base = bar_base + 16u * NS;
+  auto tfull = [&](int b) { return t_base + 8u * b; };
+  auto tempty = [&](int b) { return t_base + 8u * (CT_SLOTS + b); };
+  const uint32_t tmem_slot = t_base + 16u * CT_SLOTS;
+  uint8_t* gen = smem_raw + (tmem_slot - smem_u32(smem_raw));
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 8);
+  float2* row_sums = reinterpret_cast<float2*>(smem_raw + (bar_base + CV_BARS - smem_u32(smem_raw)));
+  float* gamma = reinterpret_cast<float*>(row_sums) + CV_SUMS / 4;
+
+  const uint32_t rank = cluster_ctarank();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int total = p.n_seg * p.tiles_per_seg;
+  const int n_taps = p.g[0].n_taps;   // of every group: the three columns of a filter row, or one
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NS; ++s) { mbar_init(full(s), 2); mbar_init(empty(s), 1); }   // two producers
+    for (int b = 0; b < CT_SLOTS; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 32); }
+    *abort_flag = 0;
+    fence_barrier_init();
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  if constexpr (NC > 0) {
+    for (int c = threadIdx.x; c < NC; c += CT_THREADS) gamma[c] = __bfloat162float(p.gamma[c]);
+  }
+  for (int c = threadIdx.x; c < min(p.n_out, 64); c += CT_THREADS) gamma[CV_GAMMA / 4 + c] = p.bias && (!RGB || c < 3) ? p.bias[c] : 0.f;
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot_ptr;
+
+  // Output frames lo .. lo + n - 1 take part in the products of input frame `i` (frame i - 2 + k with tap k of time);
+  // n1 of them up to the end of the ring. `base`: frames that this pair has begun in earlier tiles.
+  struct Step { int lo, n, n1, slot; };
+  auto step_of = [&](int i, int j0, int j1, int base) {
+    Step st;
+    st.lo = max(j0, i - 2);
+    st.n = min(j1 - 1, i) - st.lo + 1;
+    st.slot = (base + st.lo - j0) & (CT_SLOTS - 1);
+    st.n1 = min(st.n, CT_SLOTS - st.slot);
+    return st;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---------------- TMA producer of the activations (the last warp brings the weights: one thread's instructions for both took
+      // about 850 clocks a tap, more than its products)
+      int ia = 0;
+      uint32_t pha = 0;
+      bool ok = true;
+      for (int t = first_tile; t < total && ok; t += tile_step) {
+        const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
+        const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
+        int row = p.a_row0 + (j0 - 2) * p.plane + tile * 512 + int(rank) * 256;
+        for (int i = j0; i < j1 + 2 && ok; ++i, row += p.plane) {
+          for (int g = 0; g < p.n_groups && ok; ++g) {
+            const int y = row + p.g[0].off + g * p.pw;
+            for (int c = 0; c < p.cblocks; ++c) {
+              if (!mbar_wait(empty(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+              if (rank == 0) mbar_arrive_expect_tx(full(ia), 2 * Cfg::A_SLOT);
+              const uint32_t fa = mapa(full(ia), 0);
+              const uint32_t dst = smem_base + ia * stage;
+              tma_load_2d_pair(dst, &tmA, fa, c * 64, y);
+              tma_load_2d_pair(dst + CV_HALO_ROWS * 128, &tmA2, fa, c * 64, y + CV_HALO_ROWS);
+              if (++ia == NS) { ia = 0; pha ^= 1; }
             }
-          }
-        }
-        __syncwarp();
-        const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
-        uint64_t sq[2] = {0, 0};                         // sums of squares, two pairs
-        const int groups = (NC > 0 ? NC : n_end) >> 5;   // of this warp
-#pragma unroll 1
-        for (int i = 0; i < groups; ++i) {
-          const int c = 32 * i + 16 * half;
-          uint32_t v[16], pk[8];
-          tmem_ld16(ta + c, v);
-          uint4 ru[2];
-          if (res && inside) {
-            ru[0] = reinterpret_cast<const uint4*>(res + c)[0];
-            ru[1] = reinterpret_cast<const uint4*>(res + c)[1];
-          }
-          tmem_wait_ld();
-          if (inside) {
-            uint64_t a[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) a[k] = pack2(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-            if (p.bias) {
-              const float4* b4 = reinterpret_cast<const float4*>(p.bias + n_base + c);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float4 b = b4[k];
-                a[2 * k] = add2(a[2 * k], pack2(b.x, b.y));
-                a[2 * k + 1] = add2(a[2 * k + 1], pack2(b.z, b.w));
-              }
-            }
-            if (res) {
-#pragma unroll
-              for (int k = 0; k < 2; ++k) {
-                const uint32_t w[4] = {ru[k].x, ru[k].y, ru[k].z, ru[k].w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) a[4 * k + e] = add2(a[4 * k + e], pack2(bf16lo(w[e]), bf16hi(w[e])));
-              }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float lo, hi;
-              unpack2(a[k], lo, hi);
-              pk[k] = pack_bf16(lo, hi);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) pk[k] = 0u;
-          }
-          if (p.out && (inside || (row_ok && !p.keep_border))) {
-            bf16* o = p.out + dst.row * ld + n_base + c;
-            if (p.mode != CONV_OUT_UP) {
-              cv_store16(o, pk);
-            } else {
-              for (int tt = 0; tt < dst.n_t; ++tt)
-                for (int yy = 0; yy < dst.n_y; ++yy)
-                  for (int xx = 0; xx < dst.n_x; ++xx) cv_store16(o + (tt * dst.st + yy * dst.sy + xx) * ld, pk);
-            }
-          }
-          if constexpr (NC > 0) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const uint64_t x = pack2(bf16lo(pk[k]), bf16hi(pk[k]));
-              sq[k & 1] = fma2(x, x, sq[k & 1]);
-            }
-            __syncwarp();
-            tmem_st8(ta + c, pk);   // the rounded values wait in place of their accumulators
-          }
-          __syncwarp();
-        }
-        if constexpr (NC > 0) {
-          // the other half's sum (two buffers: a warp is at most one meeting ahead of its partner)
-          const float2 s2 = unpack2(add2(sq[0], sq[1]));
-          const float sum = s2.x + s2.y;
-          row_sums[((buf * 2 + r) * 2 + half) * 128 + quad * 32 + lane] = sum;
-          tmem_wait_st();
-          cv_pair_and(pair_id, true);
-          const float other = row_sums[((buf * 2 + r) * 2 + (half ^ 1)) * 128 + quad * 32 + lane];
-          const float rneg = -rsqrtf((sum + other) / (float)NC + p.eps);
-          const uint64_t rneg2 = pack2(rneg, rneg);
-          bf16* o = p.out_norm + dst.row * ld;
-#pragma unroll 1
-          for (int c = 16 * half; c < NC; c += 32) {
-            uint32_t pk[8], on[8];
-            uint64_t zn[8];
-            tmem_ld8(ta + c, pk);
-            const float4* g4 = reinterpret_cast<const float4*>(gamma + c);
-            float4 g[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) g[k] = g4[k];
-            tmem_wait_ld();
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              zn[k] = mul2(mul2(pack2(bf16lo(pk[k]), bf16hi(pk[k])), rneg2),
-                           k & 1 ? pack2(g[k >> 1].z, g[k >> 1].w) : pack2(g[k >> 1].x, g[k >> 1].y));
-            cv_silu16(zn, on);   // zero on the border
-            if (row_ok) cv_store16(o + c, on);
-            __syncwarp();
           }
         }
       }
+      if (!ok) {
+        // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      }
+    }
+  } else if (warp == CT_THREADS / 32 - 1) {
+    if (lane == 0) {
+      // ---------------- TMA producer of the weights
+      int ib = 0, base = 0;
+      uint32_t phb = 0;
+      bool ok = true;
+      const int c_in = p.cblocks * 64;
+      for (int t = first_tile; t < total && ok; t += tile_step) {
+        const int seg = t / p.tiles_per_seg;
+        const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
+        for (int i = j0; i < j1 + 2 && ok; ++i) {
+          const Step st = step_of(i, j0, j1, base);
+          // a product of n frames has 2 n pieces along N, of which the even CTA holds the first n
+          int x[3], y[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int first = k < st.n1 ? 0 : st.n1, len = k < st.n1 ? st.n1 : st.n - st.n1;
+            const int q = (k - first) + int(rank) * len;           // piece of this product
+            const int kt = i - (st.lo + first + (q >> 1));         // tap of time of the piece's frame: i = frame + kt
+            x[k] = kt * p.kt_taps * c_in;
+            y[k] = (q & 1) * (p.nt >> 1);
+          }
+          for (int g = 0; g < p.n_groups && ok; ++g) {
+            for (int c = 0; c < p.cblocks && ok; ++c) {
+              if (!mbar_wait(empty(ib), phb ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+              if (rank == 0) mbar_arrive_expect_tx(full(ib), 2 * n_taps * st.n * piece);
+              const uint32_t fb = mapa(full(ib), 0);
+              uint32_t to = smem_base + ib * stage + Cfg::A_SLOT;
+              int col = g * n_taps * c_in + c * 64;
+              for (int w = 0; w < n_taps; ++w, col += c_in, to += 3 * piece) {
+                tma_load_2d_pair(to, &tmB, fb, x[0] + col, y[0]);
+                if (st.n > 1) tma_load_2d_pair(to + piece, &tmB, fb, x[1] + col, y[1]);
+                if (st.n > 2) tma_load_2d_pair(to + 2 * piece, &tmB, fb, x[2] + col, y[2]);
+              }
+              if (++ib == NS) { ib = 0; phb ^= 1; }
+            }
+          }
+        }
+        base += j1 - j0;
+      }
+      if (!ok) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      // ---------------- MMA issuer (the whole warp walks the loop, one elected lane issues)
+      int ia = 0, base = 0;
+      uint32_t pha = 0;
+      bool ok = true;
+      for (int t = first_tile; t < total && ok; t += tile_step) {
+        const int seg = t / p.tiles_per_seg;
+        const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
+        for (int i = j0; i < j1 + 2 && ok; ++i) {
+          const Step st = step_of(i, j0, j1, base);
+          if (i < j1) {   // a new frame: its accumulator is drained and zero
+            const int n = base + i - j0;
+            if (!__all_sync(0xffffffffu, mbar_wait(tempty(n & (CT_SLOTS - 1)), (n / CT_SLOTS) & 1, abort_flag, p.status, ST_TIMEOUT_MMA))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+          }
+          const int n2 = st.n - st.n1;
+          const uint32_t idesc1 = make_idesc_bf16(256, st.n1 * p.nt, 0, 0), idesc2 = make_idesc_bf16(256, n2 * p.nt, 0, 0);
+          for (int g = 0; g < p.n_groups && ok; ++g) {
+            for (int c = 0; c < p.cblocks && ok; ++c) {
+              if (!__all_sync(0xffffffffu, mbar_wait(full(ia), pha, abort_flag, p.status, ST_TIMEOUT_MMA))) { ok = false; break; }
+              tc_fence_after();
+              if (elect_one()) {
+                const uint32_t sa = smem_base + ia * stage;
+                uint64_t a = make_smem_desc_sw128(sa, 16, 1024), b1 = make_smem_desc_sw128(sa + Cfg::A_SLOT, 16, 1024);
+                for (int w = 0; w < n_taps; ++w) {   // a tap further: a row of the activations, three pieces of the weights
+#pragma unroll
+                  for (int r = 0; r < 2; ++r) {
+                    const uint32_t d = tmem_base + r * CT_SLOTS * p.nt;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) mma_ss_pair(d + st.slot * p.nt, a + r * 1024 + 2 * k, b1 + 2 * k, idesc1, 1u);
+                    if (n2 > 0) {
+                      const uint64_t b2 = b1 + (st.n1 * piece >> 4);
+#pragma unroll
+                      for (int k = 0; k < 4; ++k) mma_ss_pair(d, a + r * 1024 + 2 * k, b2 + 2 * k, idesc2, 1u);
+                    }
+                  }
+                  a += 8;
+                  b1 += 3 * piece >> 4;
+                }
+                tc_commit_both(empty(ia));
+              }
+              __syncwarp();
+              if (++ia == NS) { ia = 0; pha ^= 1; }
+            }
+          }
+          if (ok && i - 2 >= j0) {
+            if (elect_one()) tc_commit_both(tfull((base + i - 2 - j0) & (CT_SLOTS - 1)));
+            __syncwarp();
+          }
+        }
+        base += j1 - j0;
+      }
+    }
+  } else {
+    // ---------------- epilogue (as in conv_kernel)
+    const int quad = warp & 3, half = ((warp - 2) >> 2) & 1, r = (warp - 2) >> 3;
+    const int pair_id = 1 + r * 4 + quad;
+    const uint32_t mine = tmem_base + (uint32_t(quad * 32) << 16) + r * CT_SLOTS * p.nt;
+    auto hand_back = [&](int slot) {
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if (rank != 0) mbar_arrive_cluster(mapa(tempty(buf), 0));
-        else mbar_arrive(tempty(buf));
+        if (rank != 0) mbar_arrive_peer(mapa(tempty(slot), 0));
+        else mbar_arrive(tempty(slot));
+      }
+    };
+    {
+      const uint32_t zero16[16] = {};
+      for (int c = 16 * half; c < CT_SLOTS * p.nt; c += 32) tmem_st16(mine + c, zero16);
+      tmem_wait_st();
+      for (int slot = 0; slot < CT_SLOTS; ++slot) hand_back(slot);
+    }
+    int n = 0;
+    bool alive = true;
+    for (int t = first_tile; t < total; t += tile_step) {
+      const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
+      const int rem = tile * 512 + int(rank) * 256 + r * 128 + quad * 32 + lane;
+      const bool row_ok = rem < p.plane;
+      const int y = rem / p.pw, x = rem - y * p.pw;
+      const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
+      for (int j = j0; j < j1; ++j, ++n) {
+        const int slot = n & (CT_SLOTS - 1);
+        alive = mbar_wait(tfull(slot), (n / CT_SLOTS) & 1, abort_flag, p.status, ST_TIMEOUT_EPI) && alive;
+        __syncwarp();
+        tc_fence_after();
+        conv_emit<NC, RGB, true, 2>(p, mine + slot * p.nt, j, rem, y, x, row_ok && alive, 0, half, pair_id,
+                                 row_sums + ((n & 1) * 2 + r) * 256 + quad * 32 + lane, gamma, gamma + CV_GAMMA / 4,
+                                 [&] { hand_back(slot); });
       }
     }
   }
@@ -560,48 +926,99 @@ CUtensorMap rows_map(const void* base, long long rows, int c, int box_rows) {
   return cbh::make_tmap_bf16(base, 2, dims, str, box, true);
 }
 
-template <int R, int NC, bool RGB>
-void conv_launch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, int smem, cudaStream_t s) {
-  auto kern = cb::conv_kernel<R, NC, RGB>;
-  static int pairs = 0;   // of this kernel, at its largest shared-memory size
-  cudaLaunchConfig_t cfg{};
-  cfg.blockDim = dim3(cb::ConvCfg<R>::THREADS);
-  cfg.dynamicSmemBytes = cb::CV_SMEM_MAX;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  if (pairs == 0) {
-    int dev = 0, sms = 148, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cb::CV_SMEM_MAX);
-    cfg.gridDim = dim3(sms & ~1);
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = sms / 2;
-    }
-    pairs = std::min(n, sms / 2);
+// CTA pairs of `kern` that the GPU holds at once, with one CTA an SM; the kernel's shared-memory limit is raised on the way.
+template <typename K>
+int conv_pairs(K kern, cudaLaunchConfig_t cfg) {
+  int dev = 0, sms = 148, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cb::CV_SMEM_MAX);
+  cfg.gridDim = dim3(sms & ~1);
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = sms / 2;
   }
-  const int total = p.n_seg * p.tiles_per_seg * p.n_tiles;
-  const int limit = gemm_grid_limit(), at_once = limit > 0 ? std::min(pairs, std::max(1, limit / 2)) : pairs;
-  cfg.gridDim = dim3(2 * std::min(at_once, total));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], p);
+  return std::min(n, sms / 2);
+}
+
+struct ConvLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  ConvLaunch(int threads, cudaStream_t s) {
+    cfg.blockDim = dim3(threads);
+    // always the whole shared memory: a second CTA on the SM would wait for tensor memory that the first one holds
+    cfg.dynamicSmemBytes = cb::CV_SMEM_MAX;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cfg.stream = s;
+  }
+  ConvLaunch(const ConvLaunch&) = delete;
+};
+
+int pairs_allowed(int pairs) {
+  const int limit = gemm_grid_limit();
+  return limit > 0 ? std::min(pairs, std::max(1, limit / 2)) : pairs;
+}
+
+void conv_check(cudaError_t e) {
   if (e != cudaSuccess) throw std::runtime_error(std::string("conv: launch failed: ") + cudaGetErrorString(e));
 }
 
+template <int R, int NC>
+void conv_launch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, cudaStream_t s) {
+  auto kern = cb::conv_kernel<R, NC>;
+  static int pairs = 0;   // of this kernel
+  ConvLaunch l(cb::ConvCfg<R>::THREADS, s);
+  if (pairs == 0) pairs = conv_pairs(kern, l.cfg);
+  l.cfg.gridDim = dim3(2 * std::min(pairs_allowed(pairs), p.n_seg * p.tiles_per_seg * p.n_tiles));
+  conv_check(cudaLaunchKernelEx(&l.cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], p));
+}
+
+// The chunk's frames are cut into time segments where whole columns of frames would leave pairs idle: each cut costs two input
+// frames more. Clocks of a segment: products (40 is what the reads of A take), or the epilogue's about 4000 a frame.
+void pick_segments(cb::ConvParams& p, int pairs) {
+  long long best = 0;
+  for (int n_seg = 1; n_seg <= p.f_out; ++n_seg) {
+    const int frames = (p.f_out + n_seg - 1) / n_seg;
+    if (n_seg > 1 && frames == p.seg_frames) continue;
+    long long mma = 0;
+    for (int i = 0; i < frames + 2; ++i) {
+      const int act = std::min(frames - 1, i) - std::max(0, i - 2) + 1;
+      mma += std::max(40, act * p.nt / 2) * 8ll * p.n_groups * p.g[0].n_taps * p.cblocks;
+    }
+    const int segs = (p.f_out + frames - 1) / frames;
+    const long long rounds = ((long long)segs * p.tiles_per_seg + pairs - 1) / pairs;
+    const long long cost = rounds * std::max(mma, frames * 4000ll);
+    if (n_seg == 1 || cost < best) {
+      best = cost;
+      p.n_seg = segs;
+      p.seg_frames = frames;
+    }
+  }
+}
+
+template <int NC, bool RGB>
+void conv_time_launch(const CUtensorMap& a, const CUtensorMap& a2, const CUtensorMap& b, cb::ConvParams p, cudaStream_t s) {
+  auto kern = cb::conv_time_kernel<NC, RGB>;
+  static int pairs = 0;
+  ConvLaunch l(cb::CT_THREADS, s);
+  if (pairs == 0) pairs = conv_pairs(kern, l.cfg);
+  const int at_once = pairs_allowed(pairs);
+  pick_segments(p, at_once);
+  l.cfg.gridDim = dim3(2 * std::min(at_once, p.n_seg * p.tiles_per_seg));
+  conv_check(cudaLaunchKernelEx(&l.cfg, kern, a, a2, b, p));
+}
+
 template <int R>
-void conv_dispatch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, int smem, cudaStream_t s) {
-  if (p.rgb) return conv_launch<2, 0, true>(maps, p, smem, s);
-  if (!p.out_norm) return conv_launch<R, 0, false>(maps, p, smem, s);
+void conv_dispatch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, cudaStream_t s) {
+  if (!p.out_norm) return conv_launch<R, 0>(maps, p, s);
   if constexpr (R == 2) {
-    if (p.n_out == 64) return conv_launch<2, 64, false>(maps, p, smem, s);
-    if (p.n_out == 128) return conv_launch<2, 128, false>(maps, p, smem, s);
+    if (p.n_out == 64) return conv_launch<2, 64>(maps, p, s);
+    if (p.n_out == 128) return conv_launch<2, 128>(maps, p, s);
   } else {
-    if (p.n_out == 256) return conv_launch<1, 256, false>(maps, p, smem, s);
+    if (p.n_out == 256) return conv_launch<1, 256>(maps, p, s);
   }
   throw std::runtime_error("conv: the fused norm takes 64, 128 or 256 channels");
 }
@@ -677,11 +1094,27 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
     p.skip_kcol = 27 * a.c;
     p.skip_row0 = p.a_row0;
   }
+  const int k_cols = (a.taps_t_only ? 3 : 27) * a.c + a.skip_c;
+  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_TAIL;
+  if (!strided && !a.skip && a.n_out <= 64) {
+    // one group per filter row, for all taps of time (strided convolutions and skip inputs would take columns of their own)
+    p.nt = rgb ? 16 : a.n_out;
+    p.kt_taps = a.taps_t_only ? 1 : 9;
+    p.n_groups = a.taps_t_only ? 1 : 3;
+    for (int kh = 0; kh < p.n_groups; ++kh) p.g[kh] = {a.taps_t_only ? 0 : (kh - 1) * a.wp - 1, a.taps_t_only ? 1 : 3, {0, 1, 2}, {0, 0, 0}};
+    p.tiles_per_seg = (plane + 511) / 512;
+    p.na = stage_max / cb::ct_stage(p.nt);   // 3, 4 or 5 stages
+    const CUtensorMap m0 = rows_map(a.x, rows, a.c, cb::CV_HALO_ROWS), m1 = rows_map(a.x, rows, a.c, 128);
+    const CUtensorMap mb = rows_map(a.w, a.n_out, k_cols, p.nt / 2);
+    if (rgb) return conv_time_launch<0, true>(m0, m1, mb, p, s);
+    if (!a.out_norm) return conv_time_launch<0, false>(m0, m1, mb, p, s);
+    if (a.n_out == 64) return conv_time_launch<64, false>(m0, m1, mb, p, s);
+    throw std::runtime_error("conv: the fused norm takes 64, 128 or 256 channels");
+  }
   // two row tiles share a weight tile where tensor memory holds two double-buffered accumulators
   const int R = p.mma_n <= 128 ? 2 : 1;
   p.tiles_per_seg = (p.seg_rows + 256 * R - 1) / (256 * R);
   const int a_slot = (128 * R + 8) * 128, b_slot = p.mma_n * 64;
-  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_BARS - cb::CV_SUMS - cb::CV_GAMMA;
   const int chunk = std::min(cb::CV_CHUNK, std::max(p.cblocks, p.skip_cblocks));
   // activations: one group's tiles and as many of the next one as fit beside the weight tiles: eight of those, or six where
   // four channel blocks meet 256 output channels
@@ -689,17 +1122,14 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   if ((stage_max - p.nb * b_slot) / a_slot < chunk + 2) p.nb = 6;
   p.na = std::min(2 * chunk + (chunk == 1 ? 1 : 0), (stage_max - p.nb * b_slot) / a_slot);
   if (p.na < chunk + 1) throw std::runtime_error("conv: no room for the operand rings");
-  // always the whole shared memory: a second CTA on the SM would wait for tensor memory that the first one holds
-  const int smem = cb::CV_SMEM_MAX;
-  const int k_cols = (a.taps_t_only ? 3 : 27) * a.c + a.skip_c;
   CUtensorMap maps[5];
   maps[0] = rows_map(a.x, rows, a.c, cb::CV_HALO_ROWS);
   maps[1] = rows_map(a.x, rows, a.c, 128);
   maps[2] = a.skip ? rows_map(a.skip, rows, a.skip_c, cb::CV_HALO_ROWS) : maps[0];
   maps[3] = a.skip ? rows_map(a.skip, rows, a.skip_c, 128) : maps[1];
   maps[4] = rows_map(a.w, a.n_out, k_cols, p.mma_n / 2);
-  if (R == 2) conv_dispatch<2>(maps, p, smem, s);
-  else conv_dispatch<1>(maps, p, smem, s);
+  if (R == 2) conv_dispatch<2>(maps, p, s);
+  else conv_dispatch<1>(maps, p, s);
 }
 
 void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, int n, int h, int w, cudaStream_t s) {

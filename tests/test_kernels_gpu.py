@@ -1178,6 +1178,43 @@ def test_conv3d_results_do_not_depend_on_the_schedule(cin, cout):
         k.gemm_set_grid_limit(0)
 
 
+@pytest.mark.parametrize("t", [1, 2, 4, 5, 9])
+@pytest.mark.parametrize("cin,cout,h,w", [(64, 64, 34, 62), (128, 64, 6, 10), (192, 32, 20, 38)])
+def test_conv3d_narrow_outputs_over_time(t, cin, cout, h, w):
+    """At most 64 output channels: a CTA pair walks positions through time with three frames' sums in a ring of four accumulators. Frame
+    counts around the ring's length, one to five tiles of 512 positions, and one and three pairs as well as one for every tile
+    and time segment, so that the ring wraps at every place and is carried from tile to tile. Against fp64 (one bf16 rounding of the
+    result), and the same bits whatever the schedule."""
+    import torch.nn.functional as F
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(t + cin)
+    x, wt, b = _rand(cin, t, h, w), _rand(cout, cin, 3, 3, 3, scale=1 / math.sqrt(27 * cin)), torch.randn(cout, device=DEV)
+    vol = _volume(x)
+    vol[:2] = _rand(2, h + 2, w + 2, cin)
+    vol[:2, 0], vol[:2, -1], vol[:2, :, 0], vol[:2, :, -1] = 0, 0, 0, 0
+    full = vol.permute(3, 0, 1, 2)[None].double()
+    want = F.conv3d(full, wt.double(), b.double())[0].permute(1, 2, 3, 0)
+    wp = wt.permute(0, 2, 3, 4, 1).reshape(cout, 27 * cin).contiguous()
+    x64, terms, rb = vol[..., :64].contiguous(), _rand(9, 27 * 64, scale=0.02), torch.randn(3, device=DEV) * 0.1
+    wo = terms.double().view(3, 3, 3, 3, 3, 64).sum(0).permute(0, 4, 1, 2, 3)
+    pix = (((F.conv3d(full[:, :64], wo, rb.double())[0]).clamp(-1, 1) + 1) * 127.5).permute(1, 2, 3, 0)
+
+    def run():
+        out = torch.full((t + 2, h + 2, w + 2, cout), 7.0, device=DEV, dtype=torch.bfloat16)
+        k.conv3d_fused(vol, wp, b, None, None, out, None, None, 1e-6, 0, 0, 0)
+        return out, k.conv3d_rgb(x64, terms, rb)
+
+    first = run()
+    assert (first[0][2:, 1:-1, 1:-1].double() - want).abs().max() <= 2 ** -8 * max(1.0, want.abs().max().item())
+    assert (first[1].double() - pix).abs().max() <= 0.5 + 1e-3     # rounding, and fp32 sums of 1728 products
+    try:
+        for limit in (2, 6):
+            k.gemm_set_grid_limit(limit)
+            assert all(torch.equal(u, v) for u, v in zip(run(), first)), limit
+    finally:
+        k.gemm_set_grid_limit(0)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 10, 22)])
 def test_conv3d_of_colours(dtype, t, h, w):
