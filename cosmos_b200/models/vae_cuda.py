@@ -3,7 +3,8 @@
 (csrc/conv_tcgen05.cu). A convolution's epilogue also does what follows it: the residual, the channel RMS-norm + SiLU, the
 nearest upsampling, the layout that a strided convolution reads, or the conversion to pixels, so that a layer is one launch.
 Clips run in temporal chunks; the causal context of every convolution (the last two frames of its input) is carried from
-chunk to chunk, so the result equals one pass over the clip.
+chunk to chunk, so the result equals one pass over the clip. These two frames are a tensor of their own (`Volume.tail`), which the
+next chunk's convolution reads where it is.
 
 Built from a `CausalVideoVAE` (same weights); requires channel widths that are multiples of 64.
 """
@@ -17,7 +18,7 @@ import torch.nn.functional as F
 from .. import ops
 from .vae import CausalVideoVAE, ResBlock
 
-TPAD = 2  # context frames in front of every volume (temporal kernel 3, stride 1)
+TAIL = 2  # frames that a convolution needs of the chunk before (temporal kernel 3, stride 1)
 SAME, S2D, UP, DOWN = 0, 1, 2, 3   # layouts that a convolution can write (csrc/kernels.h, ConvOut)
 NORM_WIDTHS = (64, 128, 256)       # channels that the fused norm takes: a thread of the epilogue holds a whole row
 
@@ -37,6 +38,26 @@ def _bf16_terms(w: torch.Tensor, n: int = 3) -> torch.Tensor:
         out.append(rest.to(torch.bfloat16))
         rest = rest - out[-1].float()
     return torch.cat(out).contiguous()
+
+
+class Volume:
+    """Padded channels-last frames of one chunk: all but the last two in `body`, those in `tail` (a single frame is the tail's
+    second). A tail outlives its chunk as the next one's context without keeping the body."""
+
+    def __init__(self, frames: int, frame_shape, device, zero: bool = False):
+        new = torch.zeros if zero else torch.empty
+        self.frames = frames
+        self.body = new(max(0, frames - TAIL), *frame_shape, dtype=torch.bfloat16, device=device)
+        self.tail = new(TAIL, *frame_shape, dtype=torch.bfloat16, device=device)
+
+    @property
+    def parts(self) -> List[torch.Tensor]:
+        return [self.body, self.tail]
+
+    def pieces(self) -> List[Tuple[int, int, torch.Tensor]]:
+        """(first frame, end, the tensor that holds them) of both parts."""
+        n = self.body.shape[0]
+        return [p for p in ((0, n, self.body), (n, self.frames, self.tail[n + TAIL - self.frames:])) if p[1] > p[0]]
 
 
 class _CLConvs:
@@ -65,45 +86,39 @@ class _CLConvs:
         self._add_conv(name + ".c2", blk.c2)
 
     # ------------------------------------------------------------------ launches
-    def _ctx(self, cache: Dict, key: str, vol: torch.Tensor) -> None:
-        """Fills the context frames of `vol` from the previous chunk and remembers this chunk's tail. In a volume of few frames
-        the tail stays a view (nothing writes a volume again once the next chunk has begun, and it is let go when that one takes
-        its place); of a longer one it is copied, so that a tail holds at most three times its own memory. 720p, GiB above
-        the weights and ms for 33 frames, all views / this rule / all copies: decode 8.97 / 5.65 / 5.26 and 62.3 / 63.3 / 64.1,
-        encode 13.3 / 10.4 / 9.8 and 97.3 / 99.0 / 100.6."""
-        if key in cache:
-            vol[:TPAD].copy_(cache[key])
-        else:
-            vol[:TPAD].zero_()
-        tail = vol[-TPAD:]
-        cache[key] = tail if vol.shape[0] <= 3 * TPAD else tail.clone()
+    def _ctx(self, cache: Dict, key: str, vol: Volume) -> Optional[torch.Tensor]:
+        """The context frames of `vol` (None: the clip starts here); its own tail takes their place for the next chunk."""
+        ctx = cache.get(key)
+        if vol.frames == 1:
+            vol.tail[0].copy_(ctx[1]) if ctx is not None else vol.tail[0].zero_()
+        cache[key] = vol.tail
+        return ctx
 
-    def _empty(self, *shape) -> torch.Tensor:
-        return torch.empty(*shape, dtype=torch.bfloat16, device=self.device)
+    def _volume(self, frames: int, *frame_shape, zero: bool = False) -> Volume:
+        return Volume(frames, frame_shape, self.device, zero)
 
-    def _conv(self, cache: Dict, name: str, x: torch.Tensor, resid=None, skip=None, norm: Optional[torch.Tensor] = None,
-              raw: bool = True, mode: int = SAME, a: int = 0, b: int = 0, frames: Optional[int] = None
-              ) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
-        """One convolution of `x` (context frames filled in here). Returns (result, silu(rmsnorm(result) * norm)); `raw`
-        False: the first is not wanted. `mode`, `a`, `b`: the layout written (`ops.conv3d_fused`); `frames`: its frame count."""
-        self._ctx(cache, name, x)
+    def _conv(self, cache: Dict, name: str, x: Volume, resid: Optional[Volume] = None, skip: Optional[Volume] = None,
+              norm: Optional[torch.Tensor] = None, raw: bool = True, mode: int = SAME, a: int = 0, b: int = 0,
+              frames: Optional[int] = None) -> Tuple[Optional[Volume], Optional[Volume]]:
+        """One convolution of `x`. Returns (result, silu(rmsnorm(result) * norm)); `raw` False: the first is not wanted. `mode`,
+        `a`, `b`: the layout written (`ops.conv3d_chunk`); `frames`: its frame count, where it differs from x's."""
+        ctx = self._ctx(cache, name, x)
         w = self.w[name]
         cout = w.shape[0]
-        if mode == DOWN:
-            shape = (frames + TPAD, x.shape[2] + 1, x.shape[3] + 1, cout)
-        elif mode == S2D:
-            shape = (x.shape[0], 4, x.shape[1] // 2, x.shape[2] // 2, cout)
-        elif mode == UP:
-            shape = (frames + TPAD, 2 * x.shape[1] - 2, 2 * x.shape[2] - 2, cout)
-        else:
-            shape = (*x.shape[:3], cout)
+        hp, wp = x.tail.shape[-3:-1]
+        shape = {DOWN: (hp + 1, wp + 1, cout), S2D: (4, hp // 2, wp // 2, cout), UP: (2 * hp - 2, 2 * wp - 2, cout),
+                 SAME: (hp, wp, cout)}[mode]
         fused = norm is not None and cout in NORM_WIDTHS
-        out = self._empty(*shape) if raw or not fused else None
-        out_norm = self._empty(*shape) if fused else None
-        torch.ops.cosmos_b200.conv3d_fused(x, w, self.b[name], resid, skip, out, out_norm, norm if fused else None, self.eps,
-                                           mode, a, b)
+        n = frames or x.frames
+        out = self._volume(n, *shape) if raw or not fused else None
+        out_norm = self._volume(n, *shape) if fused else None
+        parts = lambda v: [] if v is None else v.parts  # noqa: E731
+        torch.ops.cosmos_b200.conv3d_chunk(x.parts, ctx, w, self.b[name], parts(resid), parts(skip), parts(out), parts(out_norm),
+                                           norm if fused else None, self.eps, mode, x.frames, a, b)
         if norm is not None and not fused:
-            out_norm = torch.ops.cosmos_b200.rmsnorm_silu(out, norm, self.eps)
+            out_norm = self._volume(n, *shape)
+            for (_, _, src), (_, _, dst) in zip(out.pieces(), out_norm.pieces()):
+                dst.copy_(torch.ops.cosmos_b200.rmsnorm_silu(src, norm, self.eps))
         return out, out_norm
 
 
@@ -129,8 +144,9 @@ class CLDecoder(_CLConvs):
     def decode_chunk(self, z: torch.Tensor, cache: Dict, first: bool) -> torch.Tensor:
         """z [C, tc, h, w] -> uint8 frames [T, 8h, 8w, 3]."""
         c, tc, h, w = z.shape
-        vol = torch.zeros(tc + TPAD, h + 2, w + 2, 64, dtype=torch.bfloat16, device=self.device)
-        vol[TPAD:, 1:-1, 1:-1, :c] = z.permute(1, 2, 3, 0).to(torch.bfloat16)
+        vol = self._volume(tc, h + 2, w + 2, 64, zero=True)
+        for s, e, part in vol.pieces():
+            part[:, 1:-1, 1:-1, :c] = z[:, s:e].permute(1, 2, 3, 0)
         x, n = self._conv(cache, "in", vol, norm=self.g["mid.n1"])
         _, n = self._conv(cache, "mid.c1", n, norm=self.g["mid.n2"], raw=False)
         x, n = self._conv(cache, "mid.c2", n, resid=x, norm=self.g["b0.n1"])
@@ -141,8 +157,7 @@ class CLDecoder(_CLConvs):
                 tc = 2 * tc - 1 if first else 2 * tc
             x, _ = self._conv(cache, f"b{i}.c2", n, resid=x, mode=UP, a=int(temporal), b=int(first), frames=tc)
             x, n = self._conv(cache, f"u{i}", x, norm=self.g["out" if i == last else f"b{i + 1}.n1"], raw=i < last)
-        self._ctx(cache, "out", n)
-        return torch.ops.cosmos_b200.conv3d_rgb(n, self.w_out, self.b_out)
+        return torch.ops.cosmos_b200.conv3d_rgb_chunk(n.parts, self._ctx(cache, "out", n), self.w_out, self.b_out, n.frames)
 
     @torch.no_grad()
     def decode(self, z: torch.Tensor, chunk_latents: int = 2) -> torch.Tensor:
@@ -266,11 +281,13 @@ class CLEncoder(_CLConvs):
                 frames = frames.to(torch.bfloat16)
             if frames.stride(3) != 1 or frames.stride(2) != w or (n > 1 and frames.stride(1) != h * w):
                 frames = frames.contiguous()
-            vol = self._empty(n + TPAD, h + 2, w + 2, 64)
-            torch.ops.cosmos_b200.conv_pack_rgb(frames, vol)
+            vol = self._volume(n, h + 2, w + 2, 64)
+            for s, e, part in vol.pieces():
+                torch.ops.cosmos_b200.conv_pack_frames(frames[:, s:e], part)
         else:
-            vol = torch.zeros(n + TPAD, h + 2, w + 2, 64, dtype=torch.bfloat16, device=self.device)
-            vol[TPAD:, 1:-1, 1:-1, :c] = frames.permute(1, 2, 3, 0).to(torch.bfloat16)
+            vol = self._volume(n, h + 2, w + 2, 64, zero=True)
+            for s, e, part in vol.pieces():
+                part[:, 1:-1, 1:-1, :c] = frames[:, s:e].permute(1, 2, 3, 0)
         x, y = self._conv(cache, "in", vol, norm=self.g["b0.n1"])
         last = len(self.downs) - 1
         for i, temporal in enumerate(self.downs):
@@ -287,7 +304,7 @@ class CLEncoder(_CLConvs):
             n = kept
         _, y = self._res(cache, "mid", x, y, norm=self.g["out"], raw=False)
         y, _ = self._conv(cache, "out", y)
-        return y[TPAD:, 1:-1, 1:-1].permute(3, 0, 1, 2).float()
+        return torch.cat([part[:, 1:-1, 1:-1].permute(3, 0, 1, 2) for _, _, part in y.pieces()], dim=1).float()
 
     @torch.no_grad()
     def encode(self, video: torch.Tensor, chunk_frames: int = 8) -> torch.Tensor:

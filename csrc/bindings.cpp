@@ -790,10 +790,115 @@ void conv_bias(cosmos::ConvArgs& a, const OptT& bias, Tensor& keep) {
   a.bias = keep.data_ptr<float>();
 }
 
-// x: padded channels-last volume [F, Hp, Wp, C] (C % 64 == 0; F includes two context frames), mode 3: its s2d form [F, 4,
-// Hp / 2, Wp / 2, C]; w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only); `out` / `out_norm`: outputs (at least
-// one) in the mode's layout, written from their third frame on, border included. (a, b): mode 2 temporal doubling and first
-// chunk, mode 3 first kept frame and frame step.
+// A volume of a chunk as the kernel takes it: one tensor of all frames, or {all but the last two, the last two} (a volume of one
+// frame: {none, two frames of which the second is it}). Frames [per, ...]; checks the sizes and returns the number of frames.
+int64_t conv_volume(at::TensorList v, const char* name, at::IntArrayRef frame, int64_t want, const void*& body, const void*& tail) {
+  TORCH_CHECK(v.size() == 1 || v.size() == 2, name, " must be one tensor or two");
+  for (const Tensor& t : v) {
+    check_bf16_cuda(t, name);
+    TORCH_CHECK(t.is_contiguous() && t.dim() == (int64_t)frame.size() + 1 && t.sizes().slice(1) == frame, name,
+                " has the wrong size for this mode");
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, name, " must start on a 16-byte boundary");
+    TORCH_CHECK(t.device() == v[0].device(), name, " must be on one device");
+  }
+  int64_t n = v[0].size(0);
+  body = n > 0 ? v[0].data_ptr() : nullptr;
+  tail = nullptr;
+  if (v.size() == 2) {
+    TORCH_CHECK(v[1].size(0) == 2, name, ": the second tensor holds two frames");
+    tail = v[1].data_ptr();
+    if (n == 0) n = want == 1 ? 1 : 2;
+    else n += 2;
+  }
+  TORCH_CHECK(n >= 1 && (want < 0 || n == want), name, " has the wrong number of frames");
+  return n;
+}
+
+// What both entry points share: `a` has its volumes, f = frames of x, frame sizes and channels.
+void conv_run(cosmos::ConvArgs& a, const Tensor& x, const Tensor& w, const OptT& bias, const OptT& gamma, double eps) {
+  Tensor bias_keep;
+  conv_bias(a, bias, bias_keep);
+  TORCH_CHECK(w.dim() == 2 && w.is_contiguous(), "w must be a contiguous matrix");
+  a.w = w.data_ptr();
+  const bool down = a.mode == cosmos::CONV_OUT_DOWN, skip = a.skip || a.skip_tail;
+  a.taps_t_only = w.size(1) == 3 * a.c && !skip && !down;
+  TORCH_CHECK(a.taps_t_only || w.size(1) == 27 * a.c + a.skip_c, "w must be [Cout, 27 * C (+ skip channels)] or [Cout, 3 * C]");
+  if (a.out_norm || a.out_norm_tail) {
+    TORCH_CHECK(gamma.has_value() && gamma->defined(), "the fused norm needs gamma");
+    check_bf16_cuda(*gamma, "gamma");
+    TORCH_CHECK(gamma->is_contiguous() && gamma->numel() == a.n_out && reinterpret_cast<uintptr_t>(gamma->data_ptr()) % 16 == 0, "gamma: one value per channel, 16-byte aligned");
+    a.gamma = gamma->data_ptr();
+  }
+  a.eps = (float)eps;
+  a.status = status_tensor(x.get_device()).data_ptr<int>();
+  cosmos::conv3d_fused(a, cur_stream());
+}
+
+// Frame shape and number of frames that mode (a.mode, ma, mb) writes; sets the mode's fields.
+std::vector<int64_t> conv_mode(cosmos::ConvArgs& a, int64_t ma, int64_t mb, int64_t& f_dst) {
+  const int64_t f = a.frames, Hp = a.hp, Wp = a.wp, n = a.n_out;
+  a.f_out = (int)f;
+  f_dst = f;
+  if (a.mode == cosmos::CONV_OUT_SAME) return {Hp, Wp, n};
+  if (a.mode == cosmos::CONV_OUT_S2D) return {4, Hp / 2, Wp / 2, n};
+  if (a.mode == cosmos::CONV_OUT_UP) {
+    a.up_temporal = ma != 0;
+    a.up_first = mb != 0;
+    f_dst = ma ? 2 * f - (mb ? 1 : 0) : f;
+    return {2 * (Hp - 2) + 2, 2 * (Wp - 2) + 2, n};
+  }
+  TORCH_CHECK(ma >= 0 && mb >= 1, "conv3d: bad kept frames");
+  a.t_first = (int)ma;
+  a.t_step = (int)mb;
+  f_dst = a.f_out = ma < f ? (int)((f - ma + mb - 1) / mb) : 0;
+  return {Hp / 2 + 1, Wp / 2 + 1, n};
+}
+
+// One convolution of a chunk. x: channels-last volume of padded frames [Hp, Wp, C] (C % 64 == 0), mode 3: of s2d frames [4, Hp / 2,
+// Wp / 2, C]; volumes (x, resid, skip and both outputs) as conv_volume takes them, empty lists for those that are absent; ctx: the
+// two frames before x, or none, which stands for zeros; w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only). Outputs (at
+// least one) are written border included. (ma, mb): mode 2 temporal doubling and first chunk, mode 3 first kept frame and frame step.
+void conv3d_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const OptT& bias, at::TensorList resid, at::TensorList skip,
+                  at::TensorList out, at::TensorList out_norm, const OptT& gamma, double eps, int64_t mode, int64_t frames, int64_t ma,
+                  int64_t mb) {
+  check_bf16_cuda(w, "w");
+  TORCH_CHECK(x.size() == 1 || x.size() == 2, "x must be one tensor or two");
+  c10::cuda::CUDAGuard guard(w.device());
+  TORCH_CHECK(mode >= 0 && mode <= 3, "conv3d_chunk: unknown mode");
+  const bool down = mode == cosmos::CONV_OUT_DOWN;
+  const Tensor& x0 = x[x.size() - 1];
+  TORCH_CHECK(x0.dim() == (down ? 5 : 4) && (!down || x0.size(1) == 4) && x0.device() == w.device(), "x must be a volume on w's device");
+  cosmos::ConvArgs a;
+  const std::vector<int64_t> frame = x0.sizes().slice(1).vec();
+  a.frames = (int)conv_volume(x, "x", frame, frames, a.x, a.x_tail);
+  const int64_t Hp = frame[down ? 1 : 0] * (down ? 2 : 1), Wp = frame[down ? 2 : 1] * (down ? 2 : 1);
+  a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)frame.back(); a.n_out = (int)w.size(0); a.mode = (int)mode;
+  TORCH_CHECK((int64_t)(a.frames + 2) * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; use shorter temporal chunks");
+  if (ctx.has_value() && ctx->defined()) {
+    const void* none = nullptr;
+    TORCH_CHECK(conv_volume({*ctx}, "ctx", frame, 2, a.ctx, none) == 2 && ctx->device() == w.device());
+    a.ctx_frames = 2;
+  }
+  if (!skip.empty()) {
+    TORCH_CHECK(!down, "no skip input in this form");
+    a.skip_c = (int)skip[0].size(-1);
+    conv_volume(skip, "skip", {Hp, Wp, a.skip_c}, a.frames, a.skip, a.skip_tail);
+  }
+  int64_t f_dst = 0;
+  const std::vector<int64_t> dst = conv_mode(a, ma, mb, f_dst);
+  TORCH_CHECK(f_dst >= 1, "conv3d_chunk: no frame is kept");
+  if (!resid.empty()) conv_volume(resid, "resid", {Hp, Wp, a.n_out}, a.frames, a.resid, a.resid_tail);
+  const void *o = nullptr, *ot = nullptr;
+  if (!out.empty()) conv_volume(out, "out", dst, f_dst, o, ot);
+  a.out = const_cast<void*>(o); a.out_tail = const_cast<void*>(ot);
+  o = ot = nullptr;
+  if (!out_norm.empty()) conv_volume(out_norm, "out_norm", dst, f_dst, o, ot);
+  a.out_norm = const_cast<void*>(o); a.out_norm_tail = const_cast<void*>(ot);
+  conv_run(a, x0, w, bias, gamma, eps);
+}
+
+// The same on volumes [F, ...] whose first two frames are the context: x, resid, skip and the outputs, which are written from their
+// third frame on.
 void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& resid, const OptT& skip, const OptT& out,
                   const OptT& out_norm, const OptT& gamma, double eps, int64_t mode, int64_t ma, int64_t mb) {
   check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
@@ -806,56 +911,33 @@ void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT
   const int64_t C = x.size(-1), Cout = w.size(0);
   TORCH_CHECK(F > 2, "x needs two context frames and at least one more");
   TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; use shorter temporal chunks");
-  a.x = x.data_ptr(); a.w = w.data_ptr();
-  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout; a.mode = (int)mode;
-  a.f_out = (int)F - 2;
-  Tensor bias_keep;
-  conv_bias(a, bias, bias_keep);
+  a.frames = (int)F - 2; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout; a.mode = (int)mode;
+  auto behind = [](const Tensor& t) { return static_cast<char*>(t.data_ptr()) + 2 * t.stride(0) * t.element_size(); };
+  a.ctx = x.data_ptr();
+  a.x = behind(x);
   if (skip.has_value() && skip->defined()) {
     check_bf16_cuda(*skip, "skip");
     TORCH_CHECK(!down && skip->is_contiguous() && skip->dim() == 4 && skip->size(0) == F && skip->size(1) == Hp && skip->size(2) == Wp,
                 "skip must be a volume of x's size");
-    a.skip = skip->data_ptr(); a.skip_c = (int)skip->size(3);
+    a.skip = behind(*skip); a.skip_c = (int)skip->size(3);
   }
-  TORCH_CHECK(w.dim() == 2 && w.is_contiguous(), "w must be a contiguous matrix");
-  a.taps_t_only = w.size(1) == 3 * C && !a.skip && !down;
-  TORCH_CHECK(a.taps_t_only || w.size(1) == 27 * C + a.skip_c, "w must be [Cout, 27 * C (+ skip channels)] or [Cout, 3 * C]");
-  std::vector<int64_t> shape;
-  if (mode == cosmos::CONV_OUT_SAME) {
-    shape = {F, Hp, Wp, Cout};
-  } else if (mode == cosmos::CONV_OUT_S2D) {
-    shape = {F, 4, Hp / 2, Wp / 2, Cout};
-  } else if (mode == cosmos::CONV_OUT_UP) {
-    a.up_temporal = ma != 0; a.up_first = mb != 0;
-    shape = {2 + (ma ? 2 * (F - 2) - (mb ? 1 : 0) : F - 2), 2 * (Hp - 2) + 2, 2 * (Wp - 2) + 2, Cout};
-  } else {
-    TORCH_CHECK(ma >= 0 && mb >= 1, "conv3d_fused: bad kept frames");
-    a.t_first = (int)ma; a.t_step = (int)mb;
-    a.f_out = ma < F - 2 ? (int)((F - 2 - ma + mb - 1) / mb) : 0;
-    shape = {2 + a.f_out, Hp / 2 + 1, Wp / 2 + 1, Cout};
-  }
+  int64_t f_dst = 0;
+  std::vector<int64_t> shape = conv_mode(a, ma, mb, f_dst);
+  shape.insert(shape.begin(), f_dst + 2);
   if (resid.has_value() && resid->defined()) {
     check_bf16_cuda(*resid, "resid");
     TORCH_CHECK(resid->is_contiguous() && resid->sizes() == at::IntArrayRef({F, Hp, Wp, Cout}), "resid must have x's padded size");
-    a.resid = resid->data_ptr();
+    a.resid = behind(*resid);
   }
   auto output = [&](const OptT& t, const char* name) -> void* {
     if (!t.has_value() || !t->defined()) return nullptr;
     check_bf16_cuda(*t, name);
     TORCH_CHECK(t->is_contiguous() && t->sizes() == at::IntArrayRef(shape), name, " has the wrong size for this mode");
-    return t->data_ptr();
+    return behind(*t);
   };
   a.out = output(out, "out");
   a.out_norm = output(out_norm, "out_norm");
-  if (a.out_norm) {
-    TORCH_CHECK(gamma.has_value() && gamma->defined(), "the fused norm needs gamma");
-    check_bf16_cuda(*gamma, "gamma");
-    TORCH_CHECK(gamma->is_contiguous() && gamma->numel() == Cout && reinterpret_cast<uintptr_t>(gamma->data_ptr()) % 16 == 0, "gamma: one value per channel, 16-byte aligned");
-    a.gamma = gamma->data_ptr();
-  }
-  a.eps = (float)eps;
-  a.status = status_tensor(x.get_device()).data_ptr<int>();
-  cosmos::conv3d_fused(a, cur_stream());
+  conv_run(a, x, w, bias, gamma, eps);
 }
 
 // One convolution without fusions: out and resid [F, Hp, Wp, Cout]; the interior of the frames from `tpad` on is written, the border
@@ -869,52 +951,88 @@ void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& r
   TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == Cout && w.size(1) == 27 * C, "w must be [Cout, 27 * C]");
   TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
   tpad = std::max<int64_t>(tpad, 0);
+  if (tpad >= F) return;
   cosmos::ConvArgs a;
   a.keep_border = 1;
-  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
-  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout;
-  a.tpad = (int)tpad; a.f_out = (int)std::max<int64_t>(0, F - tpad);
+  const int64_t frame = Hp * Wp * x.element_size();
+  a.ctx_frames = (int)std::min<int64_t>(tpad, 2);
+  a.ctx = a.ctx_frames ? static_cast<char*>(x.data_ptr()) + (tpad - a.ctx_frames) * frame * C : nullptr;
+  a.x = static_cast<char*>(x.data_ptr()) + tpad * frame * C;
+  a.w = w.data_ptr();
+  a.out = static_cast<char*>(out.data_ptr()) + tpad * frame * Cout;
+  a.frames = a.f_out = (int)(F - tpad); a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout;
   Tensor bias_keep;
   conv_bias(a, bias, bias_keep);
   if (resid.has_value() && resid->defined()) {
     check_bf16_cuda(*resid, "resid");
     TORCH_CHECK(resid->is_contiguous() && resid->sizes() == out.sizes());
-    a.resid = resid->data_ptr();
+    a.resid = static_cast<char*>(resid->data_ptr()) + tpad * frame * Cout;
   }
   a.status = status_tensor(x.get_device()).data_ptr<int>();
   cosmos::conv3d_fused(a, cur_stream());
 }
 
-// Last layer of the decoder with the conversion to pixels. x: [F, Hp, Wp, C]; w [9, 27 C]: row c + 3 i = term i of channel
-// c's weights; bias [3] fp32 -> uint8 [F - 2, Hp - 2, Wp - 2, 3] = round((clamp(y, -1, 1) + 1) 127.5)
-Tensor conv3d_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
-  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
-  c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(0) > 2 && x.size(1) > 2 && x.size(2) > 2, "x must be a padded volume");
-  const int64_t F = x.size(0), Hp = x.size(1), Wp = x.size(2), C = x.size(3);
+// Last layer of the decoder with the conversion to pixels. x: frames [Hp, Wp, C]; w [9, 27 C]: row c + 3 i = term i of channel
+// c's weights; bias [3] fp32 -> uint8 [frames, Hp - 2, Wp - 2, 3] = round((clamp(y, -1, 1) + 1) 127.5)
+Tensor conv_rgb(cosmos::ConvArgs& a, const Tensor& x, const Tensor& w, const Tensor& bias) {
+  const int64_t Hp = x.size(1), Wp = x.size(2), C = x.size(3);
   TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == 9 && w.size(1) == 27 * C, "w must be [9, 27 * C]");
   TORCH_CHECK(bias.is_cuda() && bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.numel() == 3);
-  TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
-  Tensor out = at::empty({F - 2, Hp - 2, Wp - 2, 3}, x.options().dtype(at::kByte));
-  cosmos::ConvArgs a;
-  a.x = x.data_ptr(); a.w = w.data_ptr(); a.bias = bias.data_ptr<float>(); a.rgb = out.data_ptr();
-  a.frames_in = (int)F; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = 9; a.f_out = (int)F - 2;
+  TORCH_CHECK((a.frames + 2) * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; decode in temporal chunks");
+  Tensor out = at::empty({a.frames, Hp - 2, Wp - 2, 3}, x.options().dtype(at::kByte));
+  a.w = w.data_ptr(); a.bias = bias.data_ptr<float>(); a.rgb = out.data_ptr();
+  a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = 9; a.f_out = a.frames;
   a.status = status_tensor(x.get_device()).data_ptr<int>();
   cosmos::conv3d_fused(a, cur_stream());
   return out;
 }
 
-// frames [3, n, h, w] (fp32 or bf16; channel stride free, the rest dense) -> dst [2 + n, h + 2, w + 2, 64] from frame 2 on
-void conv_pack_rgb(const Tensor& frames, Tensor dst) {
+// x: [F, Hp, Wp, C], its first two frames the context
+Tensor conv3d_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
+  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(0) > 2 && x.size(1) > 2 && x.size(2) > 2, "x must be a padded volume");
+  cosmos::ConvArgs a;
+  a.ctx = x.data_ptr();
+  a.x = static_cast<char*>(x.data_ptr()) + 2 * x.stride(0) * x.element_size();
+  a.frames = (int)x.size(0) - 2;
+  return conv_rgb(a, x, w, bias);
+}
+
+// x and ctx as conv3d_chunk takes them
+Tensor conv3d_rgb_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const Tensor& bias, int64_t frames) {
+  check_bf16_cuda(w, "w");
+  TORCH_CHECK(x.size() == 1 || x.size() == 2, "x must be one tensor or two");
+  c10::cuda::CUDAGuard guard(w.device());
+  const Tensor& x0 = x[x.size() - 1];
+  TORCH_CHECK(x0.dim() == 4 && x0.size(1) > 2 && x0.size(2) > 2 && x0.device() == w.device(), "x must be a padded volume on w's device");
+  cosmos::ConvArgs a;
+  const std::vector<int64_t> frame = x0.sizes().slice(1).vec();
+  a.frames = (int)conv_volume(x, "x", frame, frames, a.x, a.x_tail);
+  if (ctx.has_value() && ctx->defined()) {
+    const void* none = nullptr;
+    TORCH_CHECK(conv_volume({*ctx}, "ctx", frame, 2, a.ctx, none) == 2 && ctx->device() == w.device());
+  }
+  return conv_rgb(a, x0, w, bias);
+}
+
+// frames [3, n, h, w] (fp32 or bf16; channel stride free, the rest dense) -> dst [n, h + 2, w + 2, 64]
+void conv_pack_frames(const Tensor& frames, Tensor dst) {
   check_bf16_cuda(dst, "dst");
   c10::cuda::CUDAGuard guard(dst.device());
   TORCH_CHECK(frames.is_cuda() && (frames.scalar_type() == at::kFloat || frames.scalar_type() == at::kBFloat16) &&
               frames.dim() == 4 && frames.size(0) == 3, "frames must be [3, n, h, w], fp32 or bf16");
   const int64_t n = frames.size(1), h = frames.size(2), w = frames.size(3);
-  TORCH_CHECK(frames.stride(3) == 1 && frames.stride(2) == w && (n == 1 || frames.stride(1) == h * w), "frames must be dense within a channel");
-  TORCH_CHECK(dst.is_contiguous() && dst.sizes() == at::IntArrayRef({n + 2, h + 2, w + 2, 64}), "dst must be [2 + n, h + 2, w + 2, 64]");
+  TORCH_CHECK(frames.stride(3) == 1 && frames.stride(2) == w && (n <= 1 || frames.stride(1) == h * w), "frames must be dense within a channel");
+  TORCH_CHECK(dst.is_contiguous() && dst.sizes() == at::IntArrayRef({n, h + 2, w + 2, 64}), "dst must be [n, h + 2, w + 2, 64]");
   cosmos::conv_pack_rgb(frames.data_ptr(), frames.scalar_type() == at::kFloat, frames.stride(0), dst.data_ptr(), (int)n, (int)h,
                         (int)w, cur_stream());
+}
+
+// The same into dst [2 + n, h + 2, w + 2, 64] from frame 2 on
+void conv_pack_rgb(const Tensor& frames, Tensor dst) {
+  TORCH_CHECK(dst.dim() == 4 && dst.size(0) >= 2, "dst must be [2 + n, h + 2, w + 2, 64]");
+  conv_pack_frames(frames, dst.slice(0, 2));
 }
 
 Tensor rmsnorm_silu(const Tensor& x, const Tensor& gamma, double eps) {
@@ -1381,6 +1499,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("conv3d_fused", &conv3d_fused);
   m.def("conv3d_rgb", &conv3d_rgb);
   m.def("conv_pack_rgb", &conv_pack_rgb);
+  m.def("conv3d_chunk", &conv3d_chunk);
+  m.def("conv3d_rgb_chunk", &conv3d_rgb_chunk);
+  m.def("conv_pack_frames", &conv_pack_frames);
   m.def("paged_decode", &paged_decode);
   m.def("paged_decode_pick_splits", &paged_decode_pick_splits);
   m.def("comm_barrier", &comm_barrier);

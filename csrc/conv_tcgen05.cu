@@ -1,7 +1,9 @@
 // K13: causal 3x3x3 convolutions of the video tokenizer as an implicit GEMM on tcgen05, on channels-last bf16 volumes
-// [frames, H + 2, W + 2, C] with a zero border and two context frames in front.
+// [frames, H + 2, W + 2, C] with a zero border. The two frames before the first one are a tensor of their own (absent: zero, and
+// their products are left out), and so may be a volume's last two frames, which are the next chunk's: what a chunk hands on is
+// neither copied nor holds the whole volume.
 //
-// A CTA pair (cta_group::2) computes R x 256 rows (positions of the flattened volume) by up to 256 output channels. What
+// A CTA pair (cta_group::2) computes R x 256 rows (positions of a frame) by up to 256 output channels. What
 // bounds such a kernel is the delivery of the operands from L2 into shared memory (about 45 B per clock and SM): a plain
 // implicit GEMM fetches a fresh 128-row tile of activations for each of the 27 taps. Here
 //   * the three taps of one row of the filter read one staged tile of 128 R + 8 rows at row offsets 0, 1 and 2: the matrix
@@ -23,9 +25,9 @@
 // whole row); or, for the 3 output channels of the decoder, uint8 pixels.
 //
 // Measured (480p, chunks of 8 frames at full resolution): 128 -> 128 channels with skip projection 1.95 ms = 1.47 PFLOP/s,
-// 256 -> 256 at half resolution 1.74 ms = 1.62, 128 -> 64 upsampled 1.57 ms = 0.90 (at 64 columns the reads of A from shared
-// memory bound the product). The one-tile-per-tap form with its separate passes took 48 ms a chunk of the encoder's
-// convolutions and norms where this takes 9.5.
+// 256 -> 256 at half resolution 1.9 ms = 1.5, 256 -> 128 0.93 ms = 1.52, 64 -> 128 with norm 1.2 ms = 1.2: at these rates the GPU runs at
+// its power limit (1.45 GHz, tensor pipe busy 83 % of the clocks). The one-tile-per-tap form with its separate passes took 48 ms a
+// chunk of the encoder's convolutions and norms where this takes 8.7.
 // Order of the sum: filter taps, then channel blocks of 64 (of up to 256 channels at a time). Waits are bounded as
 // everywhere (common.cuh).
 #include <algorithm>
@@ -36,7 +38,9 @@
 namespace cb {
 using namespace cosmos;   // ConvOut
 
-constexpr int CV_HALO_ROWS = 136;              // rows of the first box of a tile: 128 and the 2 rows that shifted taps need
+// Rows of a tile: those of its row tiles and the 2 that shifted taps need, in boxes of whole swizzle atoms (8 rows).
+__host__ __device__ constexpr int cv_box_rows(int r) { return r == 2 ? 88 : 136; }
+__host__ __device__ constexpr int cv_boxes(int r) { return r == 2 ? 3 : 1; }
 constexpr int CV_MAX_GROUPS = 18;
 constexpr int CV_CHUNK = 4;                    // channel blocks of 64 whose tiles are staged together
 constexpr int CV_SMEM_MAX = 227 * 1024;
@@ -47,9 +51,18 @@ constexpr int CV_TAIL = CV_BARS + CV_SUMS + 2 * CV_GAMMA;
 
 // Taps that read one staged tile: row offset of the tile, and per tap its shift inside the tile and its index in the weights.
 struct ConvGroup {
-  int off;
+  int kt;                // tap of time: input frame = output frame (kept frame's place) + kt - 2
+  int off;               // rows, inside the input frame
   int n_taps;
   short shift[3], tap[3];
+};
+
+// Frames 0 .. split - 1 in one tensor, the others in a second.
+template <typename P>
+struct Split {
+  P body, tail;          // `tail`: where frame 0 of the second tensor's frames would be
+  int split;
+  __device__ __forceinline__ P at(int frame) const { return frame < split ? body : tail; }
 };
 
 struct ConvParams {
@@ -60,19 +73,22 @@ struct ConvParams {
   int na, nb;            // ring slots
   // rows: n_seg segments (frames of a strided convolution, else one) of seg_rows rows
   int n_seg, seg_rows, tiles_per_seg;
-  int a_row0, a_seg_stride, skip_row0;
+  int frame_rows;        // rows of an input frame
+  int ctx_shift;         // context tensor: place of its first frame before the volume's first, 2 or 1; 0: absent
+  int v_first, v_step;   // segment s begins at input frame v_first + s v_step (counted from the first context frame)
+  int x_split, skip_split;
   int pw, plane;         // width and size of the plane that a segment's rows walk through
   int hp, wp;            // padded size of that plane (strided: kept rows + 1, kept columns + 1)
   const float* bias;
-  const bf16* resid;     // layout of the volume
-  bf16* out;             // raw result or null
-  bf16* out_norm;        // silu(rmsnorm(result)) or null
+  Split<const bf16*> resid;   // layout of the volume; null body and tail: none
+  Split<bf16*> out;           // raw result
+  Split<bf16*> out_norm;      // silu(rmsnorm(result))
+  int has_resid, has_out, has_norm;
   const bf16* gamma;
   float eps;
   uint8_t* rgb;
   int mode;              // CONV_OUT_*
   int keep_border;       // CONV_OUT_SAME: the border's cells are not written
-  int tpad;              // context frames in front of every output volume
   int f_out;             // frames computed
   int seg_frames;        // conv_time_kernel: output frames of a time segment (n_seg of them)
   int kt_taps;           // taps of a frame in the weights: 9, or 1 (taps in time only)
@@ -83,7 +99,7 @@ struct ConvParams {
 
 template <int R>
 struct ConvCfg {
-  static constexpr int A_ROWS = 128 * R + 8;
+  static constexpr int BOX = cv_box_rows(R), BOXES = cv_boxes(R), A_ROWS = BOX * BOXES;
   static constexpr int A_SLOT = A_ROWS * 128;
   static constexpr int ACC_COLS = 256 / R;     // tensor-memory columns of one accumulator
   static constexpr int THREADS = 96 + 256 * R; // producer, MMA issuer, eight epilogue warps per row tile, second producer
@@ -136,21 +152,34 @@ __device__ __forceinline__ void cv_silu16(const uint64_t (&zn)[8], uint32_t (&ou
 // gave up goes on without storing (the later waits give up at once).
 __device__ __forceinline__ void cv_meet(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
+// Input frame v, counted from the first context frame: the tensor that holds it and its first row there.
+struct ConvSource {
+  const CUtensorMap* map;
+  int row;
+};
+__device__ __forceinline__ ConvSource conv_source(const ConvParams& p, int v, const CUtensorMap* ctx, const CUtensorMap* body,
+                                                  const CUtensorMap* tail) {
+  if (v < 2) return {ctx, (v + p.ctx_shift - 2) * p.frame_rows};
+  if (v - 2 < p.x_split) return {body, (v - 2) * p.frame_rows};
+  return {tail, (v - 2 - p.x_split) * p.frame_rows};
+}
+
 // Where a row of the result goes: `n_t` x `n_y` x `n_x` rows starting at `row` (one row except for the upsampled form).
 struct ConvDest {
   long long row, st, sy;
+  int frame;             // the first of the frames
   int n_t, n_y, n_x;
 };
 
 __device__ __forceinline__ ConvDest conv_dest(const ConvParams& p, int f, int y, int x) {
-  ConvDest d{0, 0, 0, 1, 1, 1};
+  ConvDest d{0, 0, 0, f, 1, 1, 1};
   if (p.mode == CONV_OUT_SAME) {
-    d.row = (long long)(f + p.tpad) * p.plane + y * p.pw + x;
+    d.row = (long long)f * p.plane + y * p.pw + x;
   } else if (p.mode == CONV_OUT_S2D) {
     const int q = (p.hp >> 1) * (p.wp >> 1);
-    d.row = ((long long)(f + p.tpad) * 4 + (y & 1) * 2 + (x & 1)) * q + (y >> 1) * (p.wp >> 1) + (x >> 1);
+    d.row = ((long long)f * 4 + (y & 1) * 2 + (x & 1)) * q + (y >> 1) * (p.wp >> 1) + (x >> 1);
   } else if (p.mode == CONV_OUT_DOWN) {
-    d.row = ((long long)(f + p.tpad) * (p.hp + 1) + y + 1) * (p.wp + 1) + x + 1;
+    d.row = ((long long)f * (p.hp + 1) + y + 1) * (p.wp + 1) + x + 1;
   } else {  // CONV_OUT_UP: interior position (y, x) -> rows 2y - 1, 2y and columns 2x - 1, 2x; the border stays one wide
     const int hd = 2 * (p.hp - 2) + 2, wd = 2 * (p.wp - 2) + 2;
     const int y0 = y == 0 ? 0 : 2 * y - 1, x0 = x == 0 ? 0 : 2 * x - 1;
@@ -163,7 +192,8 @@ __device__ __forceinline__ ConvDest conv_dest(const ConvParams& p, int f, int y,
     d.n_x = (x == 0 || x == p.wp - 1) ? 1 : 2;
     d.sy = wd;
     d.st = (long long)hd * wd;
-    d.row = (t0 + p.tpad) * d.st + (long long)y0 * wd + x0;
+    d.frame = t0;
+    d.row = t0 * d.st + (long long)y0 * wd + x0;   // both frames of a doubled one are in one tensor: the last two share a pair
   }
   return d;
 }
@@ -207,15 +237,17 @@ __device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int 
         if ((k == 0 && x != 0) || (k == 1 && y != 0) || (k == 2 && (x != 0 || y != 0))) continue;
         const long long cell = dst.row - (k == 1 ? 0 : 1) - (k == 0 ? 0 : p.wp + 1);
         for (int c = 0; c < n_end; c += 8) {
-          if (p.out) *reinterpret_cast<uint4*>(p.out + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
-          if (p.out_norm) *reinterpret_cast<uint4*>(p.out_norm + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+          if (p.has_out) *reinterpret_cast<uint4*>(p.out.at(f) + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
+          if (p.has_norm) *reinterpret_cast<uint4*>(p.out_norm.at(f) + cell * ld + n_base + c) = make_uint4(0, 0, 0, 0);
         }
       }
     }
     __syncwarp();
-    // the rows that this lane stores: its pair's even and odd one (bits of `to`: copies in time, y and x; result and norm stored)
+    // the rows that this lane stores: its pair's even and odd one (bits of `to`: copies in time, y and x; result
+    // stored, norm stored, frame in the second tensor)
     const int lane = threadIdx.x & 31;
-    const int info = dst.n_t | dst.n_y << 2 | dst.n_x << 4 | (row_ok && (inside || !p.keep_border) ? 64 : 0) | (row_ok ? 128 : 0);
+    const int info = dst.n_t | dst.n_y << 2 | dst.n_x << 4 | (row_ok && (inside || !p.keep_border) ? 64 : 0) | (row_ok ? 128 : 0) |
+                     (dst.frame < p.out.split ? 0 : 256);
     const long long row0 = __shfl_sync(0xffffffffu, dst.row, lane & ~1), row1 = __shfl_sync(0xffffffffu, dst.row, lane | 1);
     const int to0 = __shfl_sync(0xffffffffu, info, lane & ~1), to1 = __shfl_sync(0xffffffffu, info, lane | 1);
     auto store = [&](bf16* o, const uint4& v, int to) {
@@ -227,7 +259,7 @@ __device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int 
             for (int xx = 0; xx < (to >> 4 & 3); ++xx) *reinterpret_cast<uint4*>(o + (tt * dst.st + yy * dst.sy + xx) * ld) = v;
       }
     };
-    const bf16* res = p.resid ? p.resid + ((long long)(f + p.tpad) * p.plane + rem) * ld + n_base : nullptr;
+    const bf16* res = p.has_resid ? p.resid.at(f) + ((long long)f * p.plane + rem) * ld + n_base : nullptr;
     static_assert(U == 2 || (U == 1 && NC != 64), "columns at a time");
     constexpr bool KEEP = NC == 64;   // the rounded values stay in registers until the row's norm is known; else in tensor memory
     // Squares are added per 8 channels (two such chains side by side) and these sums in the order of a warp's butterfly: groups
@@ -293,12 +325,12 @@ __device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int 
           const float2 y2 = unpack2(a[k]);
           pk[u][k] = inside ? pack_bf16(y2.x, y2.y) : 0u;
         }
-        if (p.out) {
+        if (p.has_out) {
           uint4 v0, v1;
           cv_swap_halves(pk[u], lane, v0, v1);
-          bf16* o = p.out + n_base + c[u] + 8 * (lane & 1);
-          if (to0 & 64) store(o + row0 * ld, v0, to0);
-          if (to1 & 64) store(o + row1 * ld, v1, to1);
+          const int col = n_base + c[u] + 8 * (lane & 1);
+          if (to0 & 64) store((to0 & 256 ? p.out.tail : p.out.body) + row0 * ld + col, v0, to0);
+          if (to1 & 64) store((to1 & 256 ? p.out.tail : p.out.body) + row1 * ld + col, v1, to1);
           __syncwarp();
         }
       }
@@ -342,7 +374,8 @@ __device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int 
       const float s0 = own.x + other.x, s1 = own.y + other.y;
       const float rneg = -rsqrtf((s0 + s1) / (float)NC + p.eps);
       const uint64_t rneg2 = pack2(rneg, rneg);
-      bf16 *o0 = p.out_norm + row0 * ld + 8 * (lane & 1), *o1 = p.out_norm + row1 * ld + 8 * (lane & 1);
+      bf16* const o0 = (to0 & 256 ? p.out_norm.tail : p.out_norm.body) + row0 * ld + 8 * (lane & 1);
+      bf16* const o1 = (to1 & 256 ? p.out_norm.tail : p.out_norm.body) + row1 * ld + 8 * (lane & 1);
 #pragma unroll 1
       for (int c = 16 * half; c < NC; c += 32 * U) {
         if constexpr (!KEEP) {
@@ -377,9 +410,10 @@ __device__ __forceinline__ void conv_emit(const ConvParams& p, uint32_t ta, int 
 // R row tiles per CTA; NC = channels of the fused norm (64, 128, 256) or 0.
 template <int R, int NC>
 __global__ void __launch_bounds__(ConvCfg<R>::THREADS, 1)
-conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
-            const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmX2,
-            const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ConvParams p) {
+conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ CUtensorMap tmBody,
+            const __grid_constant__ CUtensorMap tmTail, const __grid_constant__ CUtensorMap tmSkip,
+            const __grid_constant__ CUtensorMap tmSkipTail, const __grid_constant__ CUtensorMap tmB,
+            const __grid_constant__ ConvParams p) {
   using Cfg = ConvCfg<R>;
   constexpr int TILE_M = 256 * R;
   extern __shared__ uint8_t smem_raw[];
@@ -413,7 +447,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     for (int b = 0; b < 2; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 16 * R); }
     *abort_flag = 0;
     fence_barrier_init();
-    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmBody);
     prefetch_tmap(&tmB);
   }
   if constexpr (NC > 0) {
@@ -441,27 +475,31 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       for (int t = first_tile; t < total && ok; t += tile_step) {
         const int mt = t / p.n_tiles;
         const int seg = mt / p.tiles_per_seg, tile = mt - seg * p.tiles_per_seg;
-        const int local = tile * TILE_M + int(rank) * (128 * R);
+        const int local = tile * TILE_M + int(rank) * (128 * R), v0 = p.v_first + seg * p.v_step;
         for (int ph = 0; ph < 2 && ok; ++ph) {
           const int cblocks = ph ? p.skip_cblocks : p.cblocks;
-          const int row = (ph ? p.skip_row0 : p.a_row0 + seg * p.a_seg_stride) + local;
-          const CUtensorMap* m0 = ph ? &tmX : &tmA;
-          const CUtensorMap* m1 = ph ? &tmX2 : &tmA2;
           for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
             const int nc = min(CV_CHUNK, cblocks - c0);
             const int n_groups = ph ? 1 : p.n_groups;
             for (int g = 0; g < n_groups && ok; ++g) {
-              const int y = row + (ph ? 0 : p.g[g].off);
+              ConvSource src;
+              if (ph) {
+                src = seg < p.skip_split ? ConvSource{&tmSkip, seg * p.frame_rows} : ConvSource{&tmSkipTail, (seg - p.skip_split) * p.frame_rows};
+              } else {
+                const int v = v0 + p.g[g].kt;
+                if (v < 2 && !p.ctx_shift) continue;
+                src = conv_source(p, v, &tmCtx, &tmBody, &tmTail);
+                src.row += p.g[g].off;
+              }
+              const int y = src.row + local;
               for (int c = 0; c < nc; ++c) {
                 if (!mbar_wait(empty_a(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
                 if (rank == 0) mbar_arrive_expect_tx(full_a(ia), 2 * Cfg::A_SLOT);
                 const uint32_t fb = mapa(full_a(ia), 0);
                 const uint32_t dst = smem_base + ia * Cfg::A_SLOT;
-                tma_load_2d_pair(dst, m0, fb, (c0 + c) * 64, y);
 #pragma unroll
-                for (int r = 1; r < R; ++r)
-                  tma_load_2d_pair(dst + (CV_HALO_ROWS + (r - 1) * 128) * 128, m1, fb, (c0 + c) * 64,
-                                   y + CV_HALO_ROWS + (r - 1) * 128);
+                for (int r = 0; r < Cfg::BOXES; ++r)
+                  tma_load_2d_pair(dst + r * Cfg::BOX * 128, src.map, fb, (c0 + c) * 64, y + r * Cfg::BOX);
                 if (++ia == NA) { ia = 0; pha ^= 1; }
               }
             }
@@ -482,12 +520,14 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       bool ok = true;
       for (int t = first_tile; t < total && ok; t += tile_step) {
         const int y = (t % p.n_tiles) * 256 + int(rank) * (p.mma_n >> 1);
+        const int v0 = p.v_first + t / p.n_tiles / p.tiles_per_seg * p.v_step;
         for (int ph = 0; ph < 2 && ok; ++ph) {
           const int cblocks = ph ? p.skip_cblocks : p.cblocks;
           for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
             const int nc = min(CV_CHUNK, cblocks - c0);
             const int n_groups = ph ? 1 : p.n_groups;
             for (int g = 0; g < n_groups && ok; ++g) {
+              if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
               const int n_taps = ph ? 1 : p.g[g].n_taps;
               for (int i = 0; i < n_taps && ok; ++i) {
                 const int x = (ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64) + c0 * 64;
@@ -519,6 +559,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (!__all_sync(0xffffffffu, mbar_wait(tempty(buf), ((tcount >> 1) & 1) ^ 1, abort_flag, p.status, ST_TIMEOUT_MMA))) break;
         tc_fence_after();
         const uint32_t d = tmem_base + buf * 256;
+        const int v0 = p.v_first + t / p.n_tiles / p.tiles_per_seg * p.v_step;
         uint32_t acc = 0;
         for (int ph = 0; ph < 2 && ok; ++ph) {
           const int cblocks = ph ? p.skip_cblocks : p.cblocks;
@@ -526,6 +567,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             const int nc = min(CV_CHUNK, cblocks - c0);
             const int n_groups = ph ? 1 : p.n_groups;
             for (int g = 0; g < n_groups && ok; ++g) {
+              if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
               const int n_taps = ph ? 1 : p.g[g].n_taps;
               int ia = ia0;
               uint32_t pha = pha0;
@@ -591,12 +633,11 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const int q = tile * TILE_M + int(rank) * (128 * R) + r * 128 + quad * 32 + lane;
       const uint32_t ta = tmem_base + (uint32_t(quad * 32) << 16) + buf * 256 + r * Cfg::ACC_COLS;
       const bool row_ok = q < p.seg_rows;
-      const int f0 = q / p.plane, rem = q - f0 * p.plane;
-      const int f = f0 + seg, y = rem / p.pw, x = rem - y * p.pw;   // several segments: one frame each
+      const int y = q / p.pw, x = q - y * p.pw;
       alive = mbar_wait(tfull(buf), (tcount >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_EPI) && alive;
       __syncwarp();
       tc_fence_after();
-      conv_emit<NC, false, false, R == 1 || NC == 64 ? 2 : 1>(p, ta, f, rem, y, x, row_ok && alive, nt * 256, half, pair_id,
+      conv_emit<NC, false, false, R == 1 || NC == 64 ? 2 : 1>(p, ta, seg, q, y, x, row_ok && alive, nt * 256, half, pair_id,
                                   row_sums + (buf * 2 + r) * 256 + quad * 32 + lane, gamma, bias, [&] {
                                     tc_fence_before();
                                     __syncwarp();
@@ -626,14 +667,18 @@ conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 // A ring of four accumulators per row tile: three frames being summed, one being drained. The epilogue leaves a drained
 // accumulator zero, so that every product accumulates. Where the ring wraps, the frames' columns are not contiguous and a
 // tap takes two products.
-// 480p, 8 frames, us, before -> after: CONVT_FIGURES
+// 480p, 8 frames, us, against the flattened walk of conv_kernel on one box: 128 -> 64 channels 1648 -> 908 (1.55 PFLOP/s), pixels
+// 1000 -> 300, first layer (epilogue-bound) 555 -> 397. One thread's instructions for both operands and a barrier for every tap took
+// 850 clocks a tap, whatever the products (pixels 455 us with the same walk); hence two producer threads and one stage for the three
+// taps of a filter row (249 us).
 constexpr int CT_SLOTS = 4;
 constexpr int CT_THREADS = ConvCfg<2>::THREADS;
 __host__ __device__ constexpr int ct_stage(int nt) { return ConvCfg<2>::A_SLOT + 9 * nt * 64; }
 template <int NC, bool RGB>
 __global__ void __launch_bounds__(CT_THREADS, 1)
-conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
-                 const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ConvParams p) {
+conv_time_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ CUtensorMap tmBody,
+                 const __grid_constant__ CUtensorMap tmTail, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ ConvParams p) {
   using Cfg = ConvCfg<2>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -664,7 +709,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int b = 0; b < CT_SLOTS; ++b) { mbar_init(tfull(b), 1); mbar_init(tempty(b), 32); }
     *abort_flag = 0;
     fence_barrier_init();
-    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmBody);
     prefetch_tmap(&tmB);
   }
   if constexpr (NC > 0) {
@@ -681,7 +726,8 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
-  // Output frames lo .. lo + n - 1 take part in the products of input frame `i` (frame i - 2 + k with tap k of time);
+  // Output frames lo .. lo + n - 1 take part in the products of input frame `i`, counted from the first context frame (output frame
+  // i - k by tap k of time);
   // n1 of them up to the end of the ring. `base`: frames that this pair has begun in earlier tiles.
   struct Step { int lo, n, n1, slot; };
   auto step_of = [&](int i, int j0, int j1, int base) {
@@ -703,17 +749,19 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int t = first_tile; t < total && ok; t += tile_step) {
         const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
         const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
-        int row = p.a_row0 + (j0 - 2) * p.plane + tile * 512 + int(rank) * 256;
-        for (int i = j0; i < j1 + 2 && ok; ++i, row += p.plane) {
+        const int local = tile * 512 + int(rank) * 256;
+        for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
+          const ConvSource src = conv_source(p, i, &tmCtx, &tmBody, &tmTail);
           for (int g = 0; g < p.n_groups && ok; ++g) {
-            const int y = row + p.g[0].off + g * p.pw;
+            const int y = src.row + local + p.g[0].off + g * p.pw;
             for (int c = 0; c < p.cblocks; ++c) {
               if (!mbar_wait(empty(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
               if (rank == 0) mbar_arrive_expect_tx(full(ia), 2 * Cfg::A_SLOT);
               const uint32_t fa = mapa(full(ia), 0);
               const uint32_t dst = smem_base + ia * stage;
-              tma_load_2d_pair(dst, &tmA, fa, c * 64, y);
-              tma_load_2d_pair(dst + CV_HALO_ROWS * 128, &tmA2, fa, c * 64, y + CV_HALO_ROWS);
+#pragma unroll
+              for (int r = 0; r < Cfg::BOXES; ++r)
+                tma_load_2d_pair(dst + r * Cfg::BOX * 128, src.map, fa, c * 64, y + r * Cfg::BOX);
               if (++ia == NS) { ia = 0; pha ^= 1; }
             }
           }
@@ -735,7 +783,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int t = first_tile; t < total && ok; t += tile_step) {
         const int seg = t / p.tiles_per_seg;
         const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
-        for (int i = j0; i < j1 + 2 && ok; ++i) {
+        for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
           const Step st = step_of(i, j0, j1, base);
           // a product of n frames has 2 n pieces along N, of which the even CTA holds the first n
           int x[3], y[3];
@@ -791,7 +839,8 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           const int n2 = st.n - st.n1;
           const uint32_t idesc1 = make_idesc_bf16(256, st.n1 * p.nt, 0, 0), idesc2 = make_idesc_bf16(256, n2 * p.nt, 0, 0);
-          for (int g = 0; g < p.n_groups && ok; ++g) {
+          const int n_groups = i < 2 && !p.ctx_shift ? 0 : p.n_groups;   // no frame there: zeros
+          for (int g = 0; g < n_groups && ok; ++g) {
             for (int c = 0; c < p.cblocks && ok; ++c) {
               if (!__all_sync(0xffffffffu, mbar_wait(full(ia), pha, abort_flag, p.status, ST_TIMEOUT_MMA))) { ok = false; break; }
               tc_fence_after();
@@ -881,7 +930,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // channels and three taps in time are left. Bound by its writes (128 B a position).
 template <typename T>
 __global__ void __launch_bounds__(256)
-conv_pack_rgb_kernel(const T* __restrict__ src, long long c_stride, uint4* __restrict__ dst, int n, int h, int w, int tpad) {
+conv_pack_rgb_kernel(const T* __restrict__ src, long long c_stride, uint4* __restrict__ dst, int n, int h, int w) {
   const long long total = (long long)n * (h + 2) * (w + 2);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(i % (w + 2));
@@ -902,7 +951,7 @@ conv_pack_rgb_kernel(const T* __restrict__ src, long long c_stride, uint4* __res
               v[(kh * 3 + kw) * 3 + c] = (float)src[c * c_stride + ((long long)f * h + yy) * w + xx];
         }
     }
-    uint4* o = dst + (i + (long long)tpad * (h + 2) * (w + 2)) * 8;
+    uint4* o = dst + i * 8;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       o[k] = make_uint4(pack_bf16(v[8 * k], v[8 * k + 1]), pack_bf16(v[8 * k + 2], v[8 * k + 3]),
@@ -967,13 +1016,13 @@ void conv_check(cudaError_t e) {
 }
 
 template <int R, int NC>
-void conv_launch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, cudaStream_t s) {
+void conv_launch(const CUtensorMap (&maps)[6], const cb::ConvParams& p, cudaStream_t s) {
   auto kern = cb::conv_kernel<R, NC>;
   static int pairs = 0;   // of this kernel
   ConvLaunch l(cb::ConvCfg<R>::THREADS, s);
   if (pairs == 0) pairs = conv_pairs(kern, l.cfg);
   l.cfg.gridDim = dim3(2 * std::min(pairs_allowed(pairs), p.n_seg * p.tiles_per_seg * p.n_tiles));
-  conv_check(cudaLaunchKernelEx(&l.cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], p));
+  conv_check(cudaLaunchKernelEx(&l.cfg, kern, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p));
 }
 
 // The chunk's frames are cut into time segments where whole columns of frames would leave pairs idle: each cut costs two input
@@ -1000,7 +1049,7 @@ void pick_segments(cb::ConvParams& p, int pairs) {
 }
 
 template <int NC, bool RGB>
-void conv_time_launch(const CUtensorMap& a, const CUtensorMap& a2, const CUtensorMap& b, cb::ConvParams p, cudaStream_t s) {
+void conv_time_launch(const CUtensorMap (&maps)[6], cb::ConvParams p, cudaStream_t s) {
   auto kern = cb::conv_time_kernel<NC, RGB>;
   static int pairs = 0;
   ConvLaunch l(cb::CT_THREADS, s);
@@ -1008,12 +1057,12 @@ void conv_time_launch(const CUtensorMap& a, const CUtensorMap& a2, const CUtenso
   const int at_once = pairs_allowed(pairs);
   pick_segments(p, at_once);
   l.cfg.gridDim = dim3(2 * std::min(at_once, p.n_seg * p.tiles_per_seg));
-  conv_check(cudaLaunchKernelEx(&l.cfg, kern, a, a2, b, p));
+  conv_check(cudaLaunchKernelEx(&l.cfg, kern, maps[0], maps[1], maps[2], maps[5], p));
 }
 
 template <int R>
-void conv_dispatch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, cudaStream_t s) {
-  if (!p.out_norm) return conv_launch<R, 0>(maps, p, s);
+void conv_dispatch(const CUtensorMap (&maps)[6], const cb::ConvParams& p, cudaStream_t s) {
+  if (!p.has_norm) return conv_launch<R, 0>(maps, p, s);
   if constexpr (R == 2) {
     if (p.n_out == 64) return conv_launch<2, 64>(maps, p, s);
     if (p.n_out == 128) return conv_launch<2, 128>(maps, p, s);
@@ -1025,16 +1074,32 @@ void conv_dispatch(const CUtensorMap (&maps)[5], const cb::ConvParams& p, cudaSt
 
 }  // namespace
 
+namespace {
+
+// A volume of `frames` frames of `elems` elements: all of them at `body`, or the last two (one of one, then the second) at `tail`.
+template <typename P>
+cb::Split<P> split_of(const void* body, const void* tail, int frames, long long elems) {
+  cb::Split<P> r;
+  r.split = tail ? frames - 2 : frames;
+  r.body = reinterpret_cast<P>(reinterpret_cast<uintptr_t>(body));
+  r.tail = reinterpret_cast<P>(reinterpret_cast<uintptr_t>(tail) - (uintptr_t)(2 * elems * r.split));
+  return r;
+}
+
+}  // namespace
+
 void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   const bool strided = a.mode == CONV_OUT_DOWN, rgb = a.rgb != nullptr;
+  const bool has_out = a.out || a.out_tail, has_norm = a.out_norm || a.out_norm_tail, has_skip = a.skip || a.skip_tail;
+  const bool has_resid = a.resid || a.resid_tail;
   if (a.c <= 0 || a.c % 64 || a.skip_c % 64 || a.hp < 3 || a.wp < 3 || (!rgb && (a.n_out <= 0 || a.n_out % 32)))
     throw std::runtime_error("conv: needs input channels % 64 == 0, output channels % 32 == 0 and a padded volume");
   if ((strided || a.mode == CONV_OUT_S2D) && (a.hp % 2 || a.wp % 2)) throw std::runtime_error("conv: stride 2 needs even padded sizes");
-  if (rgb ? a.n_out != 9 : (!a.out && !a.out_norm)) throw std::runtime_error("conv: nothing to write");
-  if ((a.skip && (strided || a.mode == CONV_OUT_UP)) || (a.resid && (strided || rgb)))
+  if (rgb ? a.n_out != 9 : (!has_out && !has_norm)) throw std::runtime_error("conv: nothing to write");
+  if ((has_skip && (strided || a.mode == CONV_OUT_UP)) || (has_resid && (strided || rgb)))
     throw std::runtime_error("conv: no residual or skip input in this form");
-  if (a.out_norm && (a.mode == CONV_OUT_S2D || a.mode == CONV_OUT_UP)) throw std::runtime_error("conv: no norm in this form");
-  if (a.keep_border && (a.mode != CONV_OUT_SAME || a.out_norm || rgb)) throw std::runtime_error("conv: this form writes its border");
+  if (has_norm && (a.mode == CONV_OUT_S2D || a.mode == CONV_OUT_UP)) throw std::runtime_error("conv: no norm in this form");
+  if (a.keep_border && (a.mode != CONV_OUT_SAME || has_norm || rgb)) throw std::runtime_error("conv: this form writes its border");
   if (a.f_out < 1) return;
   cb::ConvParams p{};
   p.cblocks = a.c / 64;
@@ -1042,79 +1107,107 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   p.n_tiles = (a.n_out + 255) / 256;
   p.mma_n = p.n_tiles > 1 ? 256 : (a.n_out + 15) / 16 * 16;
   p.bias = a.bias;
-  p.resid = reinterpret_cast<const bf16*>(a.resid);
-  p.out = reinterpret_cast<bf16*>(a.out);
-  p.out_norm = reinterpret_cast<bf16*>(a.out_norm);
+  const long long plane = (long long)a.hp * a.wp, sub = (long long)(a.hp / 2) * (a.wp / 2);
+  if ((a.frames + 1) * plane > 0x7fffffffll) throw std::runtime_error("conv: volume too large for 32-bit row indices; use shorter chunks");
+  int f_dst = a.f_out;
+  long long dst_rows = plane;
+  if (a.mode == CONV_OUT_UP) {
+    f_dst = a.up_temporal ? 2 * a.f_out - (a.up_first ? 1 : 0) : a.f_out;
+    dst_rows = (2ll * (a.hp - 2) + 2) * (2ll * (a.wp - 2) + 2);
+  } else if (strided) {
+    dst_rows = (a.hp / 2 + 1ll) * (a.wp / 2 + 1ll);
+  }
+  p.has_out = has_out;
+  p.has_norm = has_norm;
+  p.has_resid = has_resid;
+  p.resid = split_of<const bf16*>(a.resid, a.resid_tail, a.frames, plane * a.n_out);
+  p.out = split_of<bf16*>(a.out, a.out_tail, f_dst, dst_rows * a.n_out);
+  p.out_norm = split_of<bf16*>(a.out_norm, a.out_norm_tail, f_dst, dst_rows * a.n_out);
+  // one frame index decides for both outputs
+  if (has_out && has_norm && p.out.split != p.out_norm.split) throw std::runtime_error("conv: outputs split in different ways");
+  if (!has_out) p.out.split = p.out_norm.split;
   p.gamma = reinterpret_cast<const bf16*>(a.gamma);
   p.eps = a.eps;
   p.rgb = reinterpret_cast<uint8_t*>(a.rgb);
   p.mode = a.mode;
   p.keep_border = a.keep_border;
-  p.tpad = a.tpad;
   p.f_out = a.f_out;
   p.up_t = a.up_temporal;
   p.up_first = a.up_first;
   p.status = a.status;
-  const int plane = a.hp * a.wp, sub = (a.hp / 2) * (a.wp / 2);
-  const long long rows = (long long)a.frames_in * plane;
-  if (rows + plane > 0x7fffffffll) throw std::runtime_error("conv: volume too large for 32-bit row indices; use shorter chunks");
+  p.frame_rows = (int)plane;
+  p.ctx_shift = a.ctx ? a.ctx_frames : 0;
+  p.x_split = a.x_tail ? a.frames - 2 : a.frames;
+  p.skip_split = a.skip_tail ? a.frames - 2 : a.frames;
+  p.n_seg = a.f_out;
+  p.v_step = 1;
+  const int k_cols = (a.taps_t_only ? 3 : 27) * a.c + a.skip_c;
+  // two row tiles share a weight tile where tensor memory holds two double-buffered accumulators
+  const int R = p.mma_n <= 128 ? 2 : 1, box = cb::cv_box_rows(R);
+  CUtensorMap maps[6];
+  // a volume whose frames are all in one of its tensors has that one's map twice
+  auto volume = [&](CUtensorMap& body, CUtensorMap& tail, const void* x, const void* t, int c) {
+    const int n = t ? a.frames - 2 : a.frames;
+    if (t) tail = rows_map(t, 2 * plane, c, box);
+    body = n > 0 ? rows_map(x, n * plane, c, box) : tail;
+    if (!t) tail = body;
+  };
+  volume(maps[1], maps[2], a.x, a.x_tail, a.c);
+  maps[0] = a.ctx ? rows_map(a.ctx, a.ctx_frames * plane, a.c, box) : maps[1];
+  if (has_skip) volume(maps[3], maps[4], a.skip, a.skip_tail, a.skip_c);
+  else maps[3] = maps[4] = maps[1];
+  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_TAIL;
   if (!strided) {
-    p.n_seg = 1;
-    p.seg_rows = a.f_out * plane;
-    p.a_row0 = a.tpad * plane;
-    p.plane = plane;
+    p.seg_rows = (int)plane;
+    p.plane = (int)plane;
     p.pw = a.wp; p.hp = a.hp; p.wp = a.wp;
-    if (a.taps_t_only) {
-      for (int kt = 0; kt < 3; ++kt) p.g[p.n_groups++] = {(kt - 2) * plane, 1, {0, 0, 0}, {(short)kt, 0, 0}};
-    } else {
-      for (int kt = 0; kt < 3; ++kt)
-        for (int kh = 0; kh < 3; ++kh) {
-          const short t0 = (short)((kt * 3 + kh) * 3);
-          p.g[p.n_groups++] = {(kt - 2) * plane + (kh - 1) * a.wp - 1, 3, {0, 1, 2}, {t0, (short)(t0 + 1), (short)(t0 + 2)}};
-        }
-    }
   } else {
     // segment = kept frame; the kept position (j, i) of a frame sits at padded (2 j + kh, 2 i + kw) for tap (kh, kw)
-    p.n_seg = a.f_out;
-    p.seg_rows = sub;
-    p.a_row0 = a.t_first * 4 * sub;
-    p.a_seg_stride = a.t_step * 4 * sub;
-    p.plane = sub;
+    p.v_first = a.t_first;
+    p.v_step = a.t_step;
+    p.seg_rows = (int)sub;
+    p.plane = (int)sub;
     p.pw = a.wp / 2; p.hp = a.hp / 2; p.wp = a.wp / 2;
-    for (int kt = 0; kt < 3; ++kt)
-      for (int kh = 0; kh < 3; ++kh) {
-        const int base = (kt * 4 + (kh & 1) * 2) * sub + (kh >> 1) * (a.wp / 2);
-        const short t0 = (short)((kt * 3 + kh) * 3);
-        p.g[p.n_groups++] = {base, 2, {0, 1, 0}, {t0, (short)(t0 + 2), 0}};
-        p.g[p.n_groups++] = {base + sub, 1, {0, 0, 0}, {(short)(t0 + 1), 0, 0}};
-      }
   }
-  if (a.skip) {
-    p.skip_cblocks = a.skip_c / 64;
-    p.skip_kcol = 27 * a.c;
-    p.skip_row0 = p.a_row0;
-  }
-  const int k_cols = (a.taps_t_only ? 3 : 27) * a.c + a.skip_c;
-  const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_TAIL;
-  if (!strided && !a.skip && a.n_out <= 64) {
+  if (!strided && !has_skip && a.n_out <= 64) {
     // one group per filter row, for all taps of time (strided convolutions and skip inputs would take columns of their own)
     p.nt = rgb ? 16 : a.n_out;
     p.kt_taps = a.taps_t_only ? 1 : 9;
     p.n_groups = a.taps_t_only ? 1 : 3;
-    for (int kh = 0; kh < p.n_groups; ++kh) p.g[kh] = {a.taps_t_only ? 0 : (kh - 1) * a.wp - 1, a.taps_t_only ? 1 : 3, {0, 1, 2}, {0, 0, 0}};
-    p.tiles_per_seg = (plane + 511) / 512;
+    p.g[0] = {0, a.taps_t_only ? 0 : -a.wp - 1, a.taps_t_only ? 1 : 3, {0, 1, 2}, {0, 0, 0}};
+    p.tiles_per_seg = (int)((plane + 511) / 512);
     p.na = stage_max / cb::ct_stage(p.nt);   // 3, 4 or 5 stages
-    const CUtensorMap m0 = rows_map(a.x, rows, a.c, cb::CV_HALO_ROWS), m1 = rows_map(a.x, rows, a.c, 128);
-    const CUtensorMap mb = rows_map(a.w, a.n_out, k_cols, p.nt / 2);
-    if (rgb) return conv_time_launch<0, true>(m0, m1, mb, p, s);
-    if (!a.out_norm) return conv_time_launch<0, false>(m0, m1, mb, p, s);
-    if (a.n_out == 64) return conv_time_launch<64, false>(m0, m1, mb, p, s);
+    maps[5] = rows_map(a.w, a.n_out, k_cols, p.nt / 2);
+    if (rgb) return conv_time_launch<0, true>(maps, p, s);
+    if (!has_norm) return conv_time_launch<0, false>(maps, p, s);
+    if (a.n_out == 64) return conv_time_launch<64, false>(maps, p, s);
     throw std::runtime_error("conv: the fused norm takes 64, 128 or 256 channels");
   }
-  // two row tiles share a weight tile where tensor memory holds two double-buffered accumulators
-  const int R = p.mma_n <= 128 ? 2 : 1;
+  if (!strided) {
+    if (a.taps_t_only) {
+      for (int kt = 0; kt < 3; ++kt) p.g[p.n_groups++] = {kt, 0, 1, {0, 0, 0}, {(short)kt, 0, 0}};
+    } else {
+      for (int kt = 0; kt < 3; ++kt)
+        for (int kh = 0; kh < 3; ++kh) {
+          const short t0 = (short)((kt * 3 + kh) * 3);
+          p.g[p.n_groups++] = {kt, (kh - 1) * a.wp - 1, 3, {0, 1, 2}, {t0, (short)(t0 + 1), (short)(t0 + 2)}};
+        }
+    }
+  } else {
+    for (int kt = 0; kt < 3; ++kt)
+      for (int kh = 0; kh < 3; ++kh) {
+        const int base = (int)((kh & 1) * 2 * sub + (kh >> 1) * (a.wp / 2));
+        const short t0 = (short)((kt * 3 + kh) * 3);
+        p.g[p.n_groups++] = {kt, base, 2, {0, 1, 0}, {t0, (short)(t0 + 2), 0}};
+        p.g[p.n_groups++] = {kt, base + (int)sub, 1, {0, 0, 0}, {(short)(t0 + 1), 0, 0}};
+      }
+  }
+  if (has_skip) {
+    p.skip_cblocks = a.skip_c / 64;
+    p.skip_kcol = 27 * a.c;
+  }
   p.tiles_per_seg = (p.seg_rows + 256 * R - 1) / (256 * R);
-  const int a_slot = (128 * R + 8) * 128, b_slot = p.mma_n * 64;
+  const int a_slot = box * cb::cv_boxes(R) * 128, b_slot = p.mma_n * 64;
   const int chunk = std::min(cb::CV_CHUNK, std::max(p.cblocks, p.skip_cblocks));
   // activations: one group's tiles and as many of the next one as fit beside the weight tiles: eight of those, or six where
   // four channel blocks meet 256 output channels
@@ -1122,12 +1215,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   if ((stage_max - p.nb * b_slot) / a_slot < chunk + 2) p.nb = 6;
   p.na = std::min(2 * chunk + (chunk == 1 ? 1 : 0), (stage_max - p.nb * b_slot) / a_slot);
   if (p.na < chunk + 1) throw std::runtime_error("conv: no room for the operand rings");
-  CUtensorMap maps[5];
-  maps[0] = rows_map(a.x, rows, a.c, cb::CV_HALO_ROWS);
-  maps[1] = rows_map(a.x, rows, a.c, 128);
-  maps[2] = a.skip ? rows_map(a.skip, rows, a.skip_c, cb::CV_HALO_ROWS) : maps[0];
-  maps[3] = a.skip ? rows_map(a.skip, rows, a.skip_c, 128) : maps[1];
-  maps[4] = rows_map(a.w, a.n_out, k_cols, p.mma_n / 2);
+  maps[5] = rows_map(a.w, a.n_out, k_cols, p.mma_n / 2);
   if (R == 2) conv_dispatch<2>(maps, p, s);
   else conv_dispatch<1>(maps, p, s);
 }
@@ -1137,9 +1225,9 @@ void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, i
   if (total == 0) return;
   const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 16);
   if (is_f32)
-    cb::conv_pack_rgb_kernel<float><<<blocks, 256, 0, s>>>((const float*)src, c_stride, (uint4*)dst, n, h, w, 2);
+    cb::conv_pack_rgb_kernel<float><<<blocks, 256, 0, s>>>((const float*)src, c_stride, (uint4*)dst, n, h, w);
   else
-    cb::conv_pack_rgb_kernel<bf16><<<blocks, 256, 0, s>>>((const bf16*)src, c_stride, (uint4*)dst, n, h, w, 2);
+    cb::conv_pack_rgb_kernel<bf16><<<blocks, 256, 0, s>>>((const bf16*)src, c_stride, (uint4*)dst, n, h, w);
 }
 
 }  // namespace cosmos

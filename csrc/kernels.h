@@ -208,32 +208,40 @@ void rmsnorm_silu(const void* x, const void* gamma, void* y, long long rows, int
 
 // ---- causal 3x3x3 convolutions of the tokenizer on padded channels-last volumes (conv_tcgen05.cu) ----
 enum ConvOut : int {
-  CONV_OUT_SAME = 0,   // [tpad + f_out, hp, wp, n_out]
-  CONV_OUT_S2D = 1,    // [tpad + f_out, 4, hp / 2, wp / 2, n_out]: a plane per parity of (row, column) of the padded volume
-  CONV_OUT_UP = 2,     // nearest x2 in space (and in time): [tpad + frames, 2 (hp - 2) + 2, 2 (wp - 2) + 2, n_out]
-  CONV_OUT_DOWN = 3,   // stride 2: x in s2d form; kept frames t_first + i t_step; [tpad + f_out, hp / 2 + 1, wp / 2 + 1, n_out]
+  CONV_OUT_SAME = 0,   // [f_out, hp, wp, n_out]
+  CONV_OUT_S2D = 1,    // [f_out, 4, hp / 2, wp / 2, n_out]: a plane per parity of (row, column) of the padded volume
+  CONV_OUT_UP = 2,     // nearest x2 in space (and in time): [frames, 2 (hp - 2) + 2, 2 (wp - 2) + 2, n_out]
+  CONV_OUT_DOWN = 3,   // stride 2: x in s2d form; kept frames t_first + i t_step; [f_out, hp / 2 + 1, wp / 2 + 1, n_out]
 };
+// A volume is one tensor, or two: its last two frames are then the `_tail` (a volume of one frame: the second of the tail's two).
 struct ConvArgs {
-  const void* x = nullptr;      // [frames_in, hp, wp, c] (CONV_OUT_DOWN: [frames_in, 4, hp / 2, wp / 2, c])
+  const void* x = nullptr;      // [frames, hp, wp, c] (CONV_OUT_DOWN: [frames, 4, hp / 2, wp / 2, c])
+  const void* x_tail = nullptr;
+  const void* ctx = nullptr;    // the ctx_frames (1 or 2) frames before x; those that are missing are zero
+  int ctx_frames = 2;
   const void* w = nullptr;      // [n_out, 27 c (+ skip_c)], tap-major; taps_t_only: [n_out, 3 c]
   const float* bias = nullptr;  // [n_out]; pixels: [3]
   const void* resid = nullptr;  // added; layout of a CONV_OUT_SAME output
-  const void* skip = nullptr;   // second input [frames_in, hp, wp, skip_c] of a 1x1x1 projection in the weights' last columns
+  const void* resid_tail = nullptr;
+  const void* skip = nullptr;   // second input [frames, hp, wp, skip_c] of a 1x1x1 projection in the weights' last columns
+  const void* skip_tail = nullptr;
   void* out = nullptr;          // bf16 result (may be null)
+  void* out_tail = nullptr;
   void* out_norm = nullptr;     // silu(rmsnorm(bf16 result) * gamma) over 64, 128 or 256 channels, layout of out
+  void* out_norm_tail = nullptr;
   const void* gamma = nullptr;
   float eps = 1e-6f;
   void* rgb = nullptr;          // uint8 [f_out, hp - 2, wp - 2, 3]; n_out = 9: rows of w = the 3 channels' weights in 3 bf16 terms
   int mode = CONV_OUT_SAME;
   int keep_border = 0;          // CONV_OUT_SAME without the norm: cells of the border keep what they hold (else zero)
-  int frames_in = 0, hp = 0, wp = 0, c = 0, skip_c = 0, n_out = 0, f_out = 0, tpad = 2;
+  int frames = 0, hp = 0, wp = 0, c = 0, skip_c = 0, n_out = 0, f_out = 0;
   int taps_t_only = 0;
   int up_temporal = 0, up_first = 0;
   int t_first = 0, t_step = 1;
   int* status = nullptr;
 };
 void conv3d_fused(const ConvArgs& a, cudaStream_t s);
-// src [3, n, h, w] planes (fp32 or bf16) -> dst [2 + n, h + 2, w + 2, 64]: the 9 spatial taps x 3 channels as 27 channels
+// src [3, n, h, w] planes (fp32 or bf16) -> dst [n, h + 2, w + 2, 64]: the 9 spatial taps x 3 channels as 27 channels
 void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, int n, int h, int w, cudaStream_t s);
 
 // ---- paged-KV decode attention (paged_decode.cu) ----

@@ -1215,6 +1215,64 @@ def test_conv3d_narrow_outputs_over_time(t, cin, cout, h, w):
         k.gemm_set_grid_limit(0)
 
 
+@pytest.mark.parametrize("t", [1, 2, 3, 4, 7])
+@pytest.mark.parametrize("cin,cout", [(64, 64), (64, 128), (128, 256), (64, 32)])
+def test_conv3d_chunk_is_conv3d_fused(t, cin, cout):
+    """Volumes in two tensors (all frames but the last two, those) and the context in a third, or absent, against one volume with the
+    context in front: the same bits in every form. 1 to 7 frames: nothing, nothing, one frame and more in the first tensor; the
+    shape has tiles that cross from frame to frame in memory and a remainder."""
+    from cosmos_b200.models.vae_cuda import Volume
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(t + cin + cout)
+    h, w = 14, 38
+    fused = cout in (64, 128, 256)
+    wp, sw = _rand(cout, 27 * cin, scale=1 / math.sqrt(27 * cin)), _rand(cout, 64, scale=0.125)
+    ws, b, g = torch.cat([wp, sw], 1).contiguous(), torch.randn(cout, device=DEV), _rand(cout) if fused else None
+
+    def full(c, s2d, ctx):
+        shape = (t + 2, 4, h // 2 + 1, w // 2 + 1, c) if s2d else (t + 2, h + 2, w + 2, c)
+        v = _rand(*shape)
+        if not ctx:
+            v[:2] = 0
+        return v
+
+    def split(v):
+        vol = Volume(v.shape[0] - 2, v.shape[1:], DEV)
+        for lo, hi, part in vol.pieces():
+            part.copy_(v[2 + lo:2 + hi])
+        return vol
+
+    def new(frames, *shape):
+        vol = Volume(frames, (*shape, cout), DEV)
+        vol.body.fill_(7.0)
+        vol.tail.fill_(7.0)
+        return vol
+
+    def same(vol, ref_):
+        return all(torch.equal(part, ref_[2 + lo:2 + hi]) for lo, hi, part in vol.pieces())
+
+    for ctx in (True, False):
+        x, xs, r, sk = full(cin, False, ctx), full(cin, True, ctx), full(cout, False, True), full(64, False, True)
+        forms = [(x, wp, r, None, 0, 0, 0, t, (h + 2, w + 2), fused), (x, ws, None, sk, 1, 0, 0, t, (4, h // 2 + 1, w // 2 + 1), False),
+                 (x, wp, r, None, 2, 0, 0, t, (2 * h + 2, 2 * w + 2), False), (x, wp, r, None, 2, 1, 0, 2 * t, (2 * h + 2, 2 * w + 2), False),
+                 (x, wp, r, None, 2, 1, 1, 2 * t - 1, (2 * h + 2, 2 * w + 2), False), (xs, wp, None, None, 3, 0, 1, t, (h // 2 + 2, w // 2 + 2), fused),
+                 (xs, wp, None, None, 3, 0, 2, (t + 1) // 2, (h // 2 + 2, w // 2 + 2), fused)]
+        if t > 1:
+            forms.append((xs, wp, None, None, 3, 1, 2, t // 2, (h // 2 + 2, w // 2 + 2), fused))
+        for v, wt, res, skip, mode, ma, mb, n, shape, norm in forms:
+            want = [torch.full((n + 2, *shape, cout), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+            k.conv3d_fused(v, wt, b, res, skip, want[0], want[1] if norm else None, g, 1e-6, mode, ma, mb)
+            got = [new(n, *shape), new(n, *shape)]
+            k.conv3d_chunk(split(v).parts, v[:2].contiguous() if ctx else None, wt, b, split(res).parts if res is not None else [],
+                           split(skip).parts if skip is not None else [], got[0].parts, got[1].parts if norm else [], g, 1e-6, mode, t, ma, mb)
+            assert same(got[0], want[0]) and (not norm or same(got[1], want[1])), (ctx, mode, ma, mb)
+            if n == 1:
+                assert (got[0].tail[0] == 7.0).all()      # the frame before the only one is not this chunk's
+        if cin == 64:
+            terms, rb = _rand(9, 27 * 64, scale=0.02), torch.randn(3, device=DEV)
+            assert torch.equal(k.conv3d_rgb_chunk(split(x).parts, x[:2].contiguous() if ctx else None, terms, rb, t), k.conv3d_rgb(x, terms, rb))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 10, 22)])
 def test_conv3d_of_colours(dtype, t, h, w):
