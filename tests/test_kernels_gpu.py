@@ -457,6 +457,24 @@ def test_attention_autograd_on_own_kernels(b, sq, skv, hq, hkv, mask, n_ar, mate
     _close(v.grad, vf.grad, 3e-2, 3e-2, "dV")
 
 
+@pytest.mark.parametrize("sq,skv", [(1, 1), (128, 129), (129, 512), (385, 128), (256, 897), (1025, 641)])
+def test_attention_backward_rings(sq, skv):
+    """One to nine tiles through rings of two and three slots, with full and ragged last tiles. bf16 P and dS as in the
+    case above, whose bounds hold for fewer terms too."""
+    from cosmos_b200.ops import autograd as own
+    torch.manual_seed(29)
+    t = [_rand(2, s, h, 128) for s, h in ((sq, 4), (skv, 2), (skv, 2))]
+    g = _rand(2, sq, 4, 128)
+    a = [x.clone().requires_grad_(True) for x in t]
+    own.attention(*a, None, ops.MASK_FULL, 0).backward(g)
+    torch.cuda.synchronize()
+    ops.check_status()
+    f = [x.float().requires_grad_(True) for x in t]
+    ref.attention(*f, None, ops.MASK_FULL, 0)[0].backward(g.float())
+    for x, y, n in zip(a, f, ("dQ", "dK", "dV")):
+        _close(x.grad, y.grad, 3e-2, 3e-2, n)
+
+
 def _grads_close(own_in, ref_in, names, atol=4e-2, rtol=4e-2):
     for a, b, n in zip(own_in, ref_in, names):
         assert a.grad is not None, f"no gradient for {n}"
