@@ -82,7 +82,7 @@ class AttentionFn(torch.autograd.Function):
         group = hq // hkv
         do = do.contiguous()
         if not _MATERIALIZED:
-            delta = (do.float() * o.float()).sum(-1).permute(0, 2, 1).contiguous()  # [B, Hq, Sq]
+            delta = _k().attn_bwd_delta(do, o)  # [B, Hq, Sq]
             dq, dk, dv = _k().attn_bwd(q, k, v, do, lse, delta, scale, mask, n_ar)
             return dq, dk, dv, None, None, None
         dq = torch.empty_like(q)

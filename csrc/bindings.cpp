@@ -481,6 +481,22 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q, const Tensor& k, co
   return {dq, dk, dv};
 }
 
+// delta = rowsum(dO * O) in fp32: [B, S, H, 128] bf16 (any layout of `dO` and `O`) -> [B, H, S]
+Tensor attn_bwd_delta(const Tensor& dout, const Tensor& o) {
+  check_bf16_cuda(dout, "do"); check_bf16_cuda(o, "o");
+  c10::cuda::CUDAGuard guard(o.device());
+  TORCH_CHECK(o.dim() == 4 && o.size(3) == 128 && dout.sizes() == o.sizes(), "do/o must be [B, S, H, 128]");
+  auto rows = [](const Tensor& t) {   // contiguous, and a view may start at any element
+    const Tensor c = t.contiguous();
+    return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+  };
+  const Tensor d = rows(dout), oc = rows(o);
+  Tensor delta = at::empty({o.size(0), o.size(2), o.size(1)}, o.options().dtype(at::kFloat));
+  cosmos::attn_bwd_delta(d.data_ptr(), oc.data_ptr(), delta.data_ptr<float>(), (int)o.size(0), (int)o.size(1), (int)o.size(2),
+                         cur_stream());
+  return delta;
+}
+
 std::tuple<Tensor, Tensor> rmsnorm(const Tensor& x, const OptT& gamma, double eps, const OptT& residual) {
   check_bf16_cuda(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
@@ -1480,6 +1496,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_bwd_scores", &attn_bwd_scores);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_bwd_delta", &attn_bwd_delta);
   m.def("attn_fwd_sources", &attn_fwd_sources);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("gated_residual_bwd", &gated_residual_bwd);

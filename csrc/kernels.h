@@ -175,6 +175,8 @@ struct AttnBwdArgs {
   int* status = nullptr;
 };
 void flash_attn_bwd(const AttnBwdArgs& a, cudaStream_t stream);
+// delta = rowsum(dO * O): O, dO [B, Sq, Hq, 128] contiguous bf16 -> [B, Hq, Sq] fp32 (elementwise_bwd.cu)
+void attn_bwd_delta(const void* dO, const void* O, float* delta, int B, int Sq, int Hq, cudaStream_t stream);
 
 // ---- bandwidth kernels (elementwise.cu) ----
 void rmsnorm(const void* x, const void* gamma, void* y, long long rows, int d, float eps,

@@ -475,6 +475,20 @@ def test_attention_backward_rings(sq, skv):
         _close(x.grad, y.grad, 3e-2, 3e-2, n)
 
 
+@pytest.mark.parametrize("b,s,h", [(1, 1, 1), (2, 33, 3), (1, 130, 32)])
+def test_attention_backward_delta(b, s, h):
+    o, do = _rand(b, s, h, 128), _rand(b, h, s, 128).transpose(1, 2)
+    flat = torch.empty(o.numel() + 1, dtype=o.dtype, device=o.device)
+    odd = flat[1:].view_as(o).copy_(o)   # starts at an odd element
+    want = (do.double() * o.double()).sum(-1).permute(0, 2, 1)
+    bound = 128 * 2 ** -24 * (do.double() * o.double()).abs().sum(-1).permute(0, 2, 1)   # exact products, 128 sums in fp32
+    same = (do.contiguous().float() * o.float()).sum(-1).permute(0, 2, 1)
+    for x in (o, odd):
+        got = torch.ops.cosmos_b200.attn_bwd_delta(do, x)
+        assert ((got.double() - want).abs() <= bound).all()
+        assert b * s * h < 16 or torch.equal(got, same)
+
+
 def _grads_close(own_in, ref_in, names, atol=4e-2, rtol=4e-2):
     for a, b, n in zip(own_in, ref_in, names):
         assert a.grad is not None, f"no gradient for {n}"
