@@ -149,7 +149,7 @@ class AttnContext:
         q, k, v = qkv_project_local(h, w, cos, sin, q_norm, k_norm, cfg)
         if prefix is not None:
             # a prefix that is a view of the projection's output (strided rows) would take both tensors of the concatenation to
-            # its element-wise path: 139 us for 14336 rows of 1024, against 20 with the prefix copied first
+            # its element-wise path: 139 us for 14336 rows of 1024, against 12 with the prefix copied first
             k = torch.cat([prefix[0].contiguous(), k], dim=1)
             v = torch.cat([prefix[1].contiguous(), v], dim=1)
         return q, k, v
