@@ -38,11 +38,10 @@ constexpr int A_BYTES = BM * BK * 2;      // 16 KB
 // NC = 2: a CTA pair per 256x256 tile (tcgen05 cta_group::2, M = 256): each CTA stages its own 128 rows
 // of A and its own 128 of the tile's 256 B rows, so a stage is 32 KB per CTA and the B operand crosses
 // shared memory once per pair instead of once per CTA; 6 stages.
-// NW = 2 (pairs only): a pair computes 256 x 512, two neighbouring 256-column tiles of one A tile. What bounds a tall
-// GEMM is the delivery of operands from L2 into shared memory, about 45 B per clock and SM: a 256x256 tile stages 32 KB per
-// CTA and 512 clocks of MMA (64 B per clock), a 256x512 tile 48 KB per 1024 clocks (48 B per clock). The two accumulators
-// fill tensor memory, so they are not double-buffered: the first and last k-blocks of a tile are issued accumulator by
-// accumulator, so that one is drained while the other is computed. 4 stages.
+// NW = 2 (pairs only): a pair computes 256 x 512, two neighbouring 256-column tiles of one A tile, with 48 KB of operands per CTA
+// and 1024 clocks of products where a 256x256 tile has 32 KB and 512. The two accumulators fill tensor memory, so they are not
+// double-buffered: the first and last k-blocks of a tile are issued accumulator by accumulator, so that one is drained while the
+// other is computed. 4 stages.
 constexpr int EPI_WARPS = 8;   // two per quadrant of accumulator rows, each with half of the columns
 constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr int gamma_smem(int epi) { return epi == EPI_QKV_ROPE ? 1024 : 0; }  // both norms' weights as fp32, behind the barriers
@@ -661,105 +660,105 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // dependent; the successor may begin its own set-up now. Every thread but the producer waits here for the
   // previous kernel's results; the producer first starts the weight tiles of its first stages (below).
   pdl_launch_dependents();
-  const bool is_producer = warp == 0 && lane == 0;
-  if (!is_producer) pdl_wait();
+  if (warp != 0) pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer
-      int it = 0;
-      bool ok = true;
-      pdl_wait();
-      for (int t = first_tile; t < total_tiles && ok; t += tile_step) {
-        const int second = t >= tiles0;
-        const GemmParams& p = g.p[second];
-        const CUtensorMap* mA = second ? &tmA1 : &tmA;
-        const CUtensorMap* mB = second ? &tmB1 : &tmB;
-        const int k_blocks = (p.K + BK - 1) / BK;
-        const int tl = second ? t - tiles0 : t;
-        const int ks = tl % p.k_splits;
-        const int kb0 = ks * k_blocks / p.k_splits, kb1 = (ks + 1) * k_blocks / p.k_splits;
-        int tm, tn;
-        tile_coords(tl / p.k_splits, second ? p.m_tiles : m_tiles0, p.n_tiles, tm, tn);
-        const TileRows tr = tile_rows<TILE_M>(p, tm);
-        const int m0 = (p.debug & 1) ? 0 : tr.m0 + int(cta_rank) * BM;
-        const int n0 = (p.debug & 1) ? 0 : tr.b_row + ((EPI == EPI_SWIGLU) ? tn * NW * 128 : tn * NW * BN);
-        if (p.debug & 2) continue;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          const uint32_t sa = smem_base + s * STAGE_BYTES;
-          if (it < prefetched) {
-            // stage already armed and its B half in flight: only the A half is left
-            if (p.a_mn) {
-              tma_load_2d(sa, mA, full_bar(s), m0, kb * BK);
-              tma_load_2d(sa + A_BYTES / 2, mA, full_bar(s), m0 + 64, kb * BK);
-            } else {
-              tma_load_2d(sa, mA, full_bar(s), kb * BK, m0);
-            }
-            continue;
-          }
-          if (!mbar_wait(empty_bar(s), ph ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) {
-            ok = false;
-            break;
+    // ---------------- TMA producer. The whole warp walks the loop, so that barrier phases, addresses and coordinates are
+    // warp-uniform values, and one elected lane issues the copies. With one lane alone in the loop, every operand of a copy went
+    // through a vector register, and that thread's instructions, not the copies, bounded the delivery of operands to 41 B per
+    // clock and SM: 880 x 4096 x 12288 95 us (with the products but no copies 68), now 76; 1920 x 6144 x 4096 with norm and
+    // rotary embedding 105 -> 84.
+    pdl_wait();
+    prefetched = __shfl_sync(0xffffffffu, prefetched, 0);
+    const bool issuer = elect_one();
+    const uint32_t full0 = NC == 2 ? mapa(full_bar(0), 0) : full_bar(0);  // the pair's bytes are counted on the leader's barriers
+    int it = 0, s = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int t = first_tile; t < total_tiles && ok; t += tile_step) {
+      const int second = t >= tiles0;
+      const GemmParams& p = g.p[second];
+      const CUtensorMap* mA = second ? &tmA1 : &tmA;
+      const CUtensorMap* mB = second ? &tmB1 : &tmB;
+      const int k_blocks = (p.K + BK - 1) / BK;
+      const int tl = second ? t - tiles0 : t;
+      const int ks = tl % p.k_splits;
+      const int kb0 = ks * k_blocks / p.k_splits, kb1 = (ks + 1) * k_blocks / p.k_splits;
+      int tm, tn;
+      tile_coords(tl / p.k_splits, second ? p.m_tiles : m_tiles0, p.n_tiles, tm, tn);
+      const TileRows tr = tile_rows<TILE_M>(p, tm);
+      const int m0 = (p.debug & 1) ? 0 : tr.m0 + int(cta_rank) * BM;
+      const int n0 = ((p.debug & 1) ? 0 : tr.b_row + ((EPI == EPI_SWIGLU) ? tn * NW * 128 : tn * NW * BN)) + int(cta_rank) * p.b_row1;
+      if (p.debug & 2) continue;
+      const bool a_mn = p.a_mn, b_mn = p.b_mn;
+      const int b_row1 = p.b_row1;
+      const uint32_t bytes = NC == 2 ? 2 * STAGE_BYTES : B_BYTES + p.a_rows * BK * 2;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const uint32_t sa = smem_base + s * STAGE_BYTES, fb = full0 + 8u * s;
+        // a prefetched stage is armed already and its B half in flight: only the A half is left
+        const bool fresh = it >= prefetched;
+        if (fresh && !__all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph, abort_flag, p.status, ST_TIMEOUT_TMA))) {
+          ok = false;
+          break;
+        }
+        if (issuer) {
+          const int k0 = kb * BK;
+          if (fresh && (NC == 1 || cta_rank == 0)) mbar_arrive_expect_tx(full_bar(s), bytes);
+          auto load = [&](uint32_t dst, const CUtensorMap* m, int x, int y) {
+            if constexpr (NC == 2) tma_load_2d_pair(dst, m, fb, x, y);
+            else tma_load_2d(dst, m, fb, x, y);
+          };
+          if (a_mn) {
+            load(sa, mA, m0, k0);
+            load(sa + A_BYTES / 2, mA, m0 + 64, k0);
+          } else {
+            load(sa, mA, k0, m0);
           }
           if constexpr (NC == 2) {
-            // both CTAs' bytes are counted on the leader's barrier, which expects the pair's total
-            const uint32_t fb = mapa(full_bar(s), 0);
-            if (cta_rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * STAGE_BYTES);
-            if (p.a_mn) {
-              tma_load_2d_pair(sa, mA, fb, m0, kb * BK);
-              tma_load_2d_pair(sa + A_BYTES / 2, mA, fb, m0 + 64, kb * BK);
-            } else {
-              tma_load_2d_pair(sa, mA, fb, kb * BK, m0);
-            }
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
               // this CTA's 128 B rows (N columns) of each column tile
-              const int nb = n0 + w * (EPI == EPI_SWIGLU ? 128 : BN) + int(cta_rank) * p.b_row1;
+              const int nb = n0 + w * (EPI == EPI_SWIGLU ? 128 : BN);
               const uint32_t sb = sa + A_BYTES + w * TN;
-              if (p.b_mn) {
-                tma_load_2d_pair(sb, mB, fb, nb, kb * BK);
-                tma_load_2d_pair(sb + TN / 2, mB, fb, nb + 64, kb * BK);
+              if (b_mn) {
+                load(sb, mB, nb, k0);
+                load(sb + TN / 2, mB, nb + 64, k0);
               } else {
-                tma_load_2d_pair(sb, mB, fb, kb * BK, nb);
+                load(sb, mB, k0, nb);
               }
             }
-            continue;
-          }
-          mbar_arrive_expect_tx(full_bar(s), B_BYTES + p.a_rows * BK * 2);
-          if (p.a_mn) {
-            tma_load_2d(sa, mA, full_bar(s), m0, kb * BK);
-            tma_load_2d(sa + A_BYTES / 2, mA, full_bar(s), m0 + 64, kb * BK);
-          } else {
-            tma_load_2d(sa, mA, full_bar(s), kb * BK, m0);
-          }
-          if (p.b_mn) {
+          } else if (fresh) {
+            if (b_mn) {
 #pragma unroll
-            for (int h = 0; h < 4; ++h)
-              tma_load_2d(sa + A_BYTES + h * (B_BYTES / 4), mB, full_bar(s),
-                          n0 + (h & 1) * 64 + (h >> 1) * p.b_row1, kb * BK);
-          } else {
-            tma_load_2d(sa + A_BYTES, mB, full_bar(s), kb * BK, n0);
-            tma_load_2d(sa + A_BYTES + B_BYTES / 2, mB, full_bar(s), kb * BK, n0 + p.b_row1);
+              for (int h = 0; h < 4; ++h) load(sa + A_BYTES + h * (B_BYTES / 4), mB, n0 + (h & 1) * 64 + (h >> 1) * b_row1, k0);
+            } else {
+              load(sa + A_BYTES, mB, k0, n0);
+              load(sa + A_BYTES + B_BYTES / 2, mB, k0, n0 + b_row1);
+            }
           }
         }
-      }
-      if (!ok) {
-        // Drain our own copies in flight (bounded) before the CTA leaves.
-        if (NC == 2 && cta_rank != 0) {
-          // this CTA's copies are counted on the leader's barrier, which only the leader can wait
-          // on: give them a fixed time (far beyond a copy's latency) to land instead
-          const long long t0 = clock64();
-          while (clock64() - t0 < 2000000ll) {}
-        } else {
-          volatile int no_abort = 0;
-          const int first = it > STAGES ? it - STAGES : 0;
-          for (int j = first; j < it; ++j)
-            mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, &no_abort, nullptr, 0);
+        __syncwarp();
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1;
         }
       }
     }
+    if (!ok && issuer) {
+      // Drain our own copies in flight (bounded) before the CTA leaves.
+      if (NC == 2 && cta_rank != 0) {
+        // this CTA's copies are counted on the leader's barrier, which only the leader can wait
+        // on: give them a fixed time (far beyond a copy's latency) to land instead
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000ll) {}
+      } else {
+        volatile int no_abort = 0;
+        const int first = it > STAGES ? it - STAGES : 0;
+        for (int j = first; j < it; ++j)
+          mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, &no_abort, nullptr, 0);
+      }
+    }
+    __syncwarp();
   } else if (warp == 1) {
     if (cta_rank == 0) {
       // ---------------- MMA issuer. The whole warp walks the loop, so barrier phases, descriptors and
@@ -1373,15 +1372,15 @@ int gemm_pick_k_splits(int M, int N, int K, int epi) {
   return best;
 }
 
-// Tile of a problem taller than 128 rows: 128x256 on single CTAs (only for SwiGLU, whose pairs of 256x256 are slower), 256x256
-// or 256x512 on CTA pairs. All three are bound by the bytes that a CTA stages per k-block (48, 32 and 48 KB), so the cost
-// of a launch is its rounds of the persistent CTAs times those bytes; ties go to the larger tile where that does not pad more
-// rows. (An approximation where there are few rounds: a round of 256x512 over 4096 columns of K took 48.9 us at 480 rows of the
-// 24576-wide SwiGLU, one of 128x256 took 33.5 at 333 rows, and both count 48.) The norm and rotary epilogue holds an accumulator for about 3 us, which 256x512 tiles hide only in part: counted
-// like 10 k-blocks.
-// Measured, 256x256 (SwiGLU: 128x256) -> 256x512, us: N x K = 24576 x 4096 SwiGLU M 14080 2291 -> 1821, M 1920 319 -> 290;
-// 4096 x 12288 residual M 14080 1143 -> 924, M 3600 352 -> 272; 4096 x 4096 residual M 3600 124 -> 103; 6144 x 4096 with
-// norm and rotary embedding M 14080 577 -> 550, but M 1920 101 -> 118.
+// Tile of a problem taller than 128 rows: 128x256 on single CTAs (only for SwiGLU), 256x256 or 256x512 on CTA pairs. Cost of a
+// launch: its rounds of the persistent CTAs times the time of a tile, in k-blocks of 256x256 (0.35 us: bound by the products). A
+// 256x512 tile has twice the products, 4 % faster (48 KB of operands for each 1024 clocks of products instead of 64 KB), but its
+// accumulators are not double-buffered: its drain costs about 14 k-blocks, 10 more with norm and rotary embedding, against 2 of the
+// last tile alone. A 128x256 tile is bound by its 48 KB of operands a k-block: 1.4. So wide tiles pay where K is long or where
+// they make one round of two, and single CTAs where they fill two rounds that pairs fill to 2.6.
+// Measured back to back, 256x256 and 256x512, us: N x K = 24576 x 4096 SwiGLU M 14080 2009 / 2117, M 1920 311 / 343; 4096 x 12288
+// M 14080 1076 / 1058, M 8448 (transposed weights) 679 / 649, M 2560 231 / 269; 4096 x 4096 M 3600 109 / 116; 6144 x 4096
+// with norm and rotary embedding M 14080 565 / 669, M 1920 91 / 126. SwiGLU M 333 on single CTAs 76, on pairs 82, M 480 100 / 82.
 static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) {
   nc = nw = 1;
   if (!pair_enabled() || (args[0].M <= cb::BM && (n < 2 || args[1].M <= cb::BM))) return;
@@ -1392,7 +1391,7 @@ static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) 
   }
   const int ctas = limit > 0 && limit < sm_count() ? limit : sm_count();
   const int epi = args[0].epi, k_blocks = (args[0].K + cb::BK - 1) / cb::BK;
-  auto cost = [&](int c, int w, int kb_bytes) {
+  auto cost = [&](int c, int w, double per_kb, double per_tile) {
     long long tiles = 0;
     for (int i = 0; i < n; ++i) {
       const int cols = epi == EPI_SWIGLU ? args[i].N / 2 : args[i].N;
@@ -1400,12 +1399,19 @@ static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) 
       tiles += (long long)((args[i].M + cb::BM * c - 1) / (cb::BM * c)) * ((cols + tile_n - 1) / tile_n);
     }
     const int at_once = ctas / c > 0 ? ctas / c : 1;
-    return (tiles + at_once - 1) / at_once * kb_bytes * (k_blocks + (w == 2 && epi == EPI_QKV_ROPE ? 10 : 0));
+    return (tiles + at_once - 1) / at_once * (k_blocks * per_kb + per_tile);
   };
-  const bool single = epi == EPI_SWIGLU;
-  nc = single ? 1 : 2;
+  nc = 2;
   nw = 1;
-  if (wide_epi(epi) && cost(2, 2, 48) <= (single ? cost(1, 1, 48) - 1 : cost(2, 1, 32))) nc = nw = 2;
+  double best = cost(2, 1, 1.0, 2.0);
+  if (wide_epi(epi)) {
+    const double wide = cost(2, 2, 1.92, epi == EPI_QKV_ROPE ? 24.0 : 14.0);
+    if (wide < best) {
+      nw = 2;
+      best = wide;
+    }
+  }
+  if (epi == EPI_SWIGLU && cost(1, 1, 1.4, 2.0) < best) nc = nw = 1;
 }
 
 void gemm_pick_tile(int M, int N, int K, int epi, int& ctas, int& col_tiles) {
