@@ -466,87 +466,93 @@ conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ C
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer of the activations, in the order in which the products consume them (the last warp brings
-      // the weights: a thread's instructions for both take longer than a tap's products of 64 columns)
-      int ia = 0;
-      uint32_t pha = 0;
-      bool ok = true;
-      for (int t = first_tile; t < total && ok; t += tile_step) {
-        const int mt = t / p.n_tiles;
-        const int seg = mt / p.tiles_per_seg, tile = mt - seg * p.tiles_per_seg;
-        const int local = tile * TILE_M + int(rank) * (128 * R), v0 = p.v_first + seg * p.v_step;
-        for (int ph = 0; ph < 2 && ok; ++ph) {
-          const int cblocks = ph ? p.skip_cblocks : p.cblocks;
-          for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
-            const int nc = min(CV_CHUNK, cblocks - c0);
-            const int n_groups = ph ? 1 : p.n_groups;
-            for (int g = 0; g < n_groups && ok; ++g) {
-              ConvSource src;
-              if (ph) {
-                src = seg < p.skip_split ? ConvSource{&tmSkip, seg * p.frame_rows} : ConvSource{&tmSkipTail, (seg - p.skip_split) * p.frame_rows};
-              } else {
-                const int v = v0 + p.g[g].kt;
-                if (v < 2 && !p.ctx_shift) continue;
-                src = conv_source(p, v, &tmCtx, &tmBody, &tmTail);
-                src.row += p.g[g].off;
-              }
-              const int y = src.row + local;
-              for (int c = 0; c < nc; ++c) {
-                if (!mbar_wait(empty_a(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+    // ---------------- TMA producer of the activations, in the order in which the products consume them (the last warp brings
+    // the weights: a thread's instructions for both take longer than a tap's products of 64 columns)
+    const bool issuer = elect_one();
+    int ia = 0;
+    uint32_t pha = 0;
+    bool ok = true;
+    for (int t = first_tile; t < total && ok; t += tile_step) {
+      const int mt = t / p.n_tiles;
+      const int seg = mt / p.tiles_per_seg, tile = mt - seg * p.tiles_per_seg;
+      const int local = tile * TILE_M + int(rank) * (128 * R), v0 = p.v_first + seg * p.v_step;
+      for (int ph = 0; ph < 2 && ok; ++ph) {
+        const int cblocks = ph ? p.skip_cblocks : p.cblocks;
+        for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
+          const int nc = min(CV_CHUNK, cblocks - c0);
+          const int n_groups = ph ? 1 : p.n_groups;
+          for (int g = 0; g < n_groups && ok; ++g) {
+            ConvSource src;
+            if (ph) {
+              src = seg < p.skip_split ? ConvSource{&tmSkip, seg * p.frame_rows} : ConvSource{&tmSkipTail, (seg - p.skip_split) * p.frame_rows};
+            } else {
+              const int v = v0 + p.g[g].kt;
+              if (v < 2 && !p.ctx_shift) continue;
+              src = conv_source(p, v, &tmCtx, &tmBody, &tmTail);
+              src.row += p.g[g].off;
+            }
+            const int y = src.row + local;
+            for (int c = 0; c < nc; ++c) {
+              if (!__all_sync(0xffffffffu, mbar_wait(empty_a(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA))) { ok = false; break; }
+              if (issuer) {
                 if (rank == 0) mbar_arrive_expect_tx(full_a(ia), 2 * Cfg::A_SLOT);
                 const uint32_t fb = mapa(full_a(ia), 0);
                 const uint32_t dst = smem_base + ia * Cfg::A_SLOT;
 #pragma unroll
                 for (int r = 0; r < Cfg::BOXES; ++r)
                   tma_load_2d_pair(dst + r * Cfg::BOX * 128, src.map, fb, (c0 + c) * 64, y + r * Cfg::BOX);
-                if (++ia == NA) { ia = 0; pha ^= 1; }
               }
+              __syncwarp();
+              if (++ia == NA) { ia = 0; pha ^= 1; }
             }
           }
         }
       }
-      if (!ok) {
-        // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000ll) {}
-      }
     }
+    if (!ok && issuer) {
+      // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) {}
+    }
+    __syncwarp();
   } else if (warp == Cfg::THREADS / 32 - 1) {
-    if (lane == 0) {
-      // ---------------- TMA producer of the weights
-      int ib = 0;
-      uint32_t phb = 0;
-      bool ok = true;
-      for (int t = first_tile; t < total && ok; t += tile_step) {
-        const int y = (t % p.n_tiles) * 256 + int(rank) * (p.mma_n >> 1);
-        const int v0 = p.v_first + t / p.n_tiles / p.tiles_per_seg * p.v_step;
-        for (int ph = 0; ph < 2 && ok; ++ph) {
-          const int cblocks = ph ? p.skip_cblocks : p.cblocks;
-          for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
-            const int nc = min(CV_CHUNK, cblocks - c0);
-            const int n_groups = ph ? 1 : p.n_groups;
-            for (int g = 0; g < n_groups && ok; ++g) {
-              if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
-              const int n_taps = ph ? 1 : p.g[g].n_taps;
-              for (int i = 0; i < n_taps && ok; ++i) {
-                const int x = (ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64) + c0 * 64;
-                for (int c = 0; c < nc; ++c) {
-                  if (!mbar_wait(empty_b(ib), phb ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+    // ---------------- TMA producer of the weights
+    const bool issuer = elect_one();
+    int ib = 0;
+    uint32_t phb = 0;
+    bool ok = true;
+    for (int t = first_tile; t < total && ok; t += tile_step) {
+      const int y = (t % p.n_tiles) * 256 + int(rank) * (p.mma_n >> 1);
+      const int v0 = p.v_first + t / p.n_tiles / p.tiles_per_seg * p.v_step;
+      for (int ph = 0; ph < 2 && ok; ++ph) {
+        const int cblocks = ph ? p.skip_cblocks : p.cblocks;
+        for (int c0 = 0; c0 < cblocks && ok; c0 += CV_CHUNK) {
+          const int nc = min(CV_CHUNK, cblocks - c0);
+          const int n_groups = ph ? 1 : p.n_groups;
+          for (int g = 0; g < n_groups && ok; ++g) {
+            if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
+            const int n_taps = ph ? 1 : p.g[g].n_taps;
+            for (int i = 0; i < n_taps && ok; ++i) {
+              const int x = (ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64) + c0 * 64;
+              for (int c = 0; c < nc; ++c) {
+                if (!__all_sync(0xffffffffu, mbar_wait(empty_b(ib), phb ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA))) { ok = false; break; }
+                if (issuer) {
                   if (rank == 0) mbar_arrive_expect_tx(full_b(ib), 2 * b_slot);
                   tma_load_2d_pair(b_base + ib * b_slot, &tmB, mapa(full_b(ib), 0), x + c * 64, y);
-                  if (++ib == NB) { ib = 0; phb ^= 1; }
                 }
+                __syncwarp();
+                if (++ib == NB) { ib = 0; phb ^= 1; }
               }
             }
           }
         }
       }
-      if (!ok) {
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000ll) {}
-      }
     }
+    if (!ok && issuer) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) {}
+    }
+    __syncwarp();
   } else if (warp == 1) {
     if (rank == 0) {
       // ---------------- MMA issuer (the whole warp walks the loop, one elected lane issues)
@@ -740,39 +746,42 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constan
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer of the activations (the last warp brings the weights: one thread's instructions for both took
-      // about 850 clocks a tap, more than its products)
-      int ia = 0;
-      uint32_t pha = 0;
-      bool ok = true;
-      for (int t = first_tile; t < total && ok; t += tile_step) {
-        const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
-        const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
-        const int local = tile * 512 + int(rank) * 256;
-        for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
-          const ConvSource src = conv_source(p, i, &tmCtx, &tmBody, &tmTail);
-          for (int g = 0; g < p.n_groups && ok; ++g) {
-            const int y = src.row + local + p.g[0].off + g * p.pw;
-            for (int c = 0; c < p.cblocks; ++c) {
-              if (!mbar_wait(empty(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA)) { ok = false; break; }
+    // ---------------- TMA producer of the activations (the last warp brings the weights: one thread's instructions for both took
+    // about 850 clocks a tap, more than its products)
+    const bool issuer = elect_one();
+    int ia = 0;
+    uint32_t pha = 0;
+    bool ok = true;
+    for (int t = first_tile; t < total && ok; t += tile_step) {
+      const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
+      const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
+      const int local = tile * 512 + int(rank) * 256;
+      for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
+        const ConvSource src = conv_source(p, i, &tmCtx, &tmBody, &tmTail);
+        for (int g = 0; g < p.n_groups && ok; ++g) {
+          const int y = src.row + local + p.g[0].off + g * p.pw;
+          for (int c = 0; c < p.cblocks; ++c) {
+            if (!__all_sync(0xffffffffu, mbar_wait(empty(ia), pha ^ 1, abort_flag, p.status, ST_TIMEOUT_TMA))) { ok = false; break; }
+            if (issuer) {
               if (rank == 0) mbar_arrive_expect_tx(full(ia), 2 * Cfg::A_SLOT);
               const uint32_t fa = mapa(full(ia), 0);
               const uint32_t dst = smem_base + ia * stage;
 #pragma unroll
               for (int r = 0; r < Cfg::BOXES; ++r)
                 tma_load_2d_pair(dst + r * Cfg::BOX * 128, src.map, fa, c * 64, y + r * Cfg::BOX);
-              if (++ia == NS) { ia = 0; pha ^= 1; }
             }
+            __syncwarp();
+            if (++ia == NS) { ia = 0; pha ^= 1; }
           }
         }
       }
-      if (!ok) {
-        // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000ll) {}
-      }
     }
+    if (!ok && issuer) {
+      // copies in flight are counted on the leader's barriers: give them a fixed time, far beyond a copy's latency
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) {}
+    }
+    __syncwarp();
   } else if (warp == CT_THREADS / 32 - 1) {
     if (lane == 0) {
       // ---------------- TMA producer of the weights
