@@ -200,6 +200,8 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if constexpr (NC == 2) cluster_sync_all();  // the peer's barriers are initialised before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  pdl_launch_dependents();   // the next kernel may set itself up
+  pdl_wait();                // and this one did while the kernel before it finished
 
   // Register re-partitioning: the CTA owns 384 x 168 registers; 128 x 56 + 256 x 224 uses
   // exactly that many. A split that needs more would block in setmaxnreg.inc forever.
@@ -593,10 +595,12 @@ static void launch_attn(int nc, dim3 grid, const CUtensorMap& tq, const cb::KVMa
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(cb::ATT_THREADS, 1, 1);
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch.cuh
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
   if (nc == 2) {
     static bool configured = false;
     if (!configured) {

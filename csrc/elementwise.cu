@@ -3,6 +3,7 @@
 // One warp per row, 16-byte vector accesses, fp32 math, bf16 storage.
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace cb {
 
@@ -97,6 +98,8 @@ rmsnorm_row_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma, b
                    const bf16* __restrict__ shift, const bf16* __restrict__ scale, int rows_per_batch,
                    long long mod_stride) {
   __shared__ float red[8];
+  pdl_launch_dependents();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * d);
@@ -408,11 +411,11 @@ static void launch_norm(const void* x, const void* gamma, void* y, long long row
     int threads = ((nvec + 3) / 4 + 31) / 32 * 32;
     if (threads > 256) {
       if (nvec > 256 * 8) throw std::runtime_error("rmsnorm: feature size above 16384 is not supported");
-      cb::rmsnorm_row_kernel<8, MODE><<<(unsigned)rows, 256, 0, s>>>(
+      launch_early(cb::rmsnorm_row_kernel<8, MODE>, dim3((unsigned)rows), dim3(256), 0, s,
           (const bf16*)x, (const bf16*)gamma, (bf16*)y, d, eps, (const bf16*)rin, (bf16*)rout,
           (const bf16*)shift, (const bf16*)scale, rows_per_batch, mod_stride);
     } else {
-      cb::rmsnorm_row_kernel<4, MODE><<<(unsigned)rows, threads, 0, s>>>(
+      launch_early(cb::rmsnorm_row_kernel<4, MODE>, dim3((unsigned)rows), dim3(threads), 0, s,
           (const bf16*)x, (const bf16*)gamma, (bf16*)y, d, eps, (const bf16*)rin, (bf16*)rout,
           (const bf16*)shift, (const bf16*)scale, rows_per_batch, mod_stride);
     }

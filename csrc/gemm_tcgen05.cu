@@ -96,6 +96,7 @@ struct GemmParams {
   // grouped by a tile map (see the file comment): {group, first row, rows, unused} per m-tile; tile rows = TILE_M
   const int4* tile_map;
   const int* n_tiles_m;  // number of m-tiles of this launch (device)
+  int early_b;           // B may be read before the kernels ahead of this one have finished
   int debug;             // timing experiments (wrong results): 1 = every tile loads operand tile (0, 0); 2 = no loads at all
 };
 
@@ -623,9 +624,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       prefetch_tmap(&tmB1);
     }
     // Weight prefetch (single-CTA tiles, B in its [N, K] layout): the B halves of the first tile's first stages are
-    // requested here, while warp 1 still allocates tensor memory and before the dependency wait of a programmatic
-    // launch; their A halves follow in the producer loop. A stage's full barrier completes when both have landed.
-    if (NC == 1 && first_tile < total_tiles && first_tile < tiles0 && !g.p[0].b_mn &&
+    // requested here, while warp 1 still allocates tensor memory and before the dependency wait, where B is known to be a weight
+    // that no kernel before this one writes (early_b); their A halves follow in the producer loop. A stage's full barrier
+    // completes when both have landed.
+    if (NC == 1 && g.p[0].early_b && first_tile < total_tiles && first_tile < tiles0 && !g.p[0].b_mn &&
         !g.p[0].debug && !g.p[0].tile_map) {
       const GemmParams& p = g.p[0];
       const int k_blocks = (p.K + BK - 1) / BK;
@@ -656,9 +658,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if constexpr (NC == 2) cluster_sync_all();  // the peer's barriers are initialised before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  // The set-up above overlapped the previous kernel's tail when this one was launched as its programmatic
-  // dependent; the successor may begin its own set-up now. Every thread but the producer waits here for the
-  // previous kernel's results; the producer first starts the weight tiles of its first stages (below).
+  // The set-up above overlapped the previous kernel's tail (every launch but a grouped one is its programmatic dependent); the
+  // successor may begin its own set-up now. Everybody waits for the previous kernel's results.
   pdl_launch_dependents();
   if (warp != 0) pdl_wait();
 
@@ -1216,7 +1217,7 @@ static void launch(const CUtensorMap* maps, const cb::GemmGroup& g, int units, i
   at[0].val.clusterDim.x = NC; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = (NC == 1 && pdl_on() && !g.p[0].tile_map) ? 2 : 1;
+  cfg.attrs = at; cfg.numAttrs = g.p[0].tile_map ? 1 : 2;
   cudaLaunchKernelEx(&cfg, cb::gemm_bf16_kernel<EPI, NC, NW>, maps[0], maps[1], maps[2], maps[3], g);
 }
 
@@ -1313,6 +1314,7 @@ static void fill_problem(const GemmArgs& a, cb::GemmParams& p, CUtensorMap& ta, 
   p.status = a.status;
   p.k_splits = 1;
   p.partial = nullptr;
+  p.early_b = pdl_on() ? 1 : 0;
   p.debug = g_debug;
   p.tile_map = reinterpret_cast<const int4*>(a.tile_map);
   p.n_tiles_m = a.n_tiles_m;
@@ -1499,7 +1501,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (a.norm_out) {
     if (a.epi != EPI_PLAIN || a.N > 8192 || a.N % 4 != 0 || a.ldc % 4 != 0 || (a.R && a.ldr % 4 != 0))
       throw std::runtime_error("gemm_bf16: the fused reduce + RMS-norm pass needs a plain epilogue and N <= 8192");
-    launch_pdl(cb::splitk_reduce_rmsnorm_kernel, dim3(a.M), dim3(cb::RN_THREADS), 0, stream,
+    launch_early(cb::splitk_reduce_rmsnorm_kernel, dim3(a.M), dim3(cb::RN_THREADS), 0, stream,
         a.partial, ks, a.M, a.N, reinterpret_cast<const bf16*>(a.R), a.ldr, reinterpret_cast<const bf16*>(a.norm_gamma),
         a.norm_eps, reinterpret_cast<bf16*>(a.C), reinterpret_cast<bf16*>(a.norm_out), a.ldc);
     return;
@@ -1507,7 +1509,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   const int n_out = a.epi == EPI_SWIGLU ? a.N / 2 : a.N;
   const long long vecs = (long long)a.M * (n_out / 4);
   const int blocks = (int)std::min<long long>((vecs + 255) / 256, 148 * 8);
-  launch_pdl(cb::splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream,
+  launch_early(cb::splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream,
       a.partial, ks, a.M, a.N, a.epi, reinterpret_cast<bf16*>(a.C), a.ldc,
       reinterpret_cast<const bf16*>(a.bias), reinterpret_cast<const bf16*>(a.R), a.ldr,
       reinterpret_cast<const bf16*>(a.gate), a.rows_per_batch > 0 ? a.rows_per_batch : (a.M > 0 ? a.M : 1));

@@ -24,11 +24,10 @@ enum AttnMask : int {
 
 namespace cosmos {
 
-// Programmatic dependent launch for the decode-step kernels (GEMM, split-K reductions, QKV post-processing, paged
-// attention and its merge, all-reduce + norm): while on, those kernels are launched so that their set-up and their
-// weight prefetch overlap the tail of the kernel before them. Only kernels whose early part reads nothing that
-// another kernel of the stream writes honour it; the caller turns it on around a decode step (where the GEMMs'
-// B operands are weights) and off afterwards. The switch is process-wide: launches from other host threads see it.
+// Programmatic dependent launch. GEMMs, split-K reductions, row norms and attention over contiguous keys are always launched so
+// that their set-up overlaps the tail of the kernel before them. While this is on, the other kernels of a decode step (QKV
+// post-processing, paged attention and its merge, all-reduce + norm) are too, and GEMMs on single CTAs read their first weight
+// tiles ahead; the caller turns it on around a decode step (where the GEMMs' B operands are weights) and off afterwards. The switch is process-wide: launches from other host threads see it.
 void set_pdl(bool on);
 bool pdl_on();
 
