@@ -1376,12 +1376,13 @@ int gemm_pick_k_splits(int M, int N, int K, int epi) {
 
 // Tile of a problem taller than 128 rows: 128x256 on single CTAs (only for SwiGLU), 256x256 or 256x512 on CTA pairs. Cost of a
 // launch: its rounds of the persistent CTAs times the time of a tile, in k-blocks of 256x256 (0.35 us: bound by the products). A
-// 256x512 tile has twice the products, 4 % faster (48 KB of operands for each 1024 clocks of products instead of 64 KB), but its
-// accumulators are not double-buffered: its drain costs about 14 k-blocks, 10 more with norm and rotary embedding, against 2 of the
-// last tile alone. A 128x256 tile is bound by its 48 KB of operands a k-block: 1.4. So wide tiles pay where K is long or where
-// they make one round of two, and single CTAs where they fill two rounds that pairs fill to 2.6.
+// 256x512 tile has twice the products, which take 1.85 times as long (48 KB of operands for 1024 clocks of products instead of
+// 64 KB, and less power), but its accumulators are not double-buffered: its drain costs about 20 k-blocks, 10 more with norm and
+// rotary embedding, against 2. A 128x256 tile is bound by its 48 KB of operands a k-block: 1.4. A last round that is not full
+// costs about half of what it leaves idle (under the power cap the others clock higher). So wide tiles pay where K is long, and
+// single CTAs where they fill two rounds that pairs fill to 2.6.
 // Measured back to back, 256x256 and 256x512, us: N x K = 24576 x 4096 SwiGLU M 14080 2009 / 2117, M 1920 311 / 343; 4096 x 12288
-// M 14080 1076 / 1058, M 8448 (transposed weights) 679 / 649, M 2560 231 / 269; 4096 x 4096 M 3600 109 / 116; 6144 x 4096
+// M 57600 4841 / 4656, M 14080 1076 / 1058, M 8448 (transposed weights) 679 / 649, M 2560 231 / 269; 4096 x 4096 M 3600 109 / 116; 6144 x 4096
 // with norm and rotary embedding M 14080 565 / 669, M 1920 91 / 126. SwiGLU M 333 on single CTAs 76, on pairs 82, M 480 100 / 82.
 static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) {
   nc = nw = 1;
@@ -1401,13 +1402,14 @@ static void pick_tile(const GemmArgs* args, int n, int limit, int& nc, int& nw) 
       tiles += (long long)((args[i].M + cb::BM * c - 1) / (cb::BM * c)) * ((cols + tile_n - 1) / tile_n);
     }
     const int at_once = ctas / c > 0 ? ctas / c : 1;
-    return (tiles + at_once - 1) / at_once * (k_blocks * per_kb + per_tile);
+    const long long rounds = (tiles + at_once - 1) / at_once;
+    return 0.5 * (rounds + double(tiles) / at_once) * (k_blocks * per_kb + per_tile);
   };
   nc = 2;
   nw = 1;
   double best = cost(2, 1, 1.0, 2.0);
   if (wide_epi(epi)) {
-    const double wide = cost(2, 2, 1.92, epi == EPI_QKV_ROPE ? 24.0 : 14.0);
+    const double wide = cost(2, 2, 1.85, epi == EPI_QKV_ROPE ? 30.0 : 20.0);
     if (wide < best) {
       nw = 2;
       best = wide;
@@ -1467,11 +1469,16 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (!a.partial || a.N % 8 != 0) throw std::runtime_error("gemm_bf16: split-K needs a partial buffer and N % 8 == 0");
   cb::GemmGroup g{};
   CUtensorMap maps[4];
-  // more than one 128-row tile (a serving batch of 256): CTA pairs, so that each CTA stages half of the weight tile
-  // (the skinny GEMMs of such a batch are bound by operand delivery into shared memory, not by HBM). The split count was
-  // chosen for single CTAs, so pairs can need a second, mostly empty round where those had one: 257 - 384 rows of a 4096-wide
-  // projection are 96 pair items on 74 pairs, 44.8 us at 333 rows where 480 rows (64 items) take 35.2.
-  const int nc = a.tile_map ? a.tile_m / cb::BM : (pair_enabled() && a.epi != EPI_SWIGLU && a.M > cb::BM) ? 2 : 1;
+  // More than one 128-row tile (a serving batch of 256): CTA pairs, so that each CTA stages half of the weight tile. The split
+  // count was chosen for single CTAs, so pairs can need a second, mostly empty round where those have one: 257 - 384 rows of a
+  // 4096-wide projection are 96 items on 74 pairs, or 144 on 148 CTAs whose k-block takes 1.4 times as long (see pick_tile).
+  // 333 x 4096 x 4096 with the reduction 36 us on pairs, 30 on single CTAs; 333 x 4096 x 12288 67 and 54.
+  auto rounds = [&](int c) {
+    const long long items = (long long)((a.M + cb::BM * c - 1) / (cb::BM * c)) * ((a.N + cb::BN - 1) / cb::BN) * a.k_splits;
+    return (items + sm_count() / c - 1) / (sm_count() / c);
+  };
+  const bool pairs = pair_enabled() && a.epi != EPI_SWIGLU && a.M > cb::BM && rounds(2) * 1.0 <= rounds(1) * 1.4;
+  const int nc = a.tile_map ? a.tile_m / cb::BM : pairs ? 2 : 1;
   if (nc != 1 && nc != 2) throw std::runtime_error("gemm_bf16: tile rows must be 128 or 256");
   fill_problem(a, g.p[0], maps[0], maps[1], nc);
   const int k_blocks = (a.K + cb::BK - 1) / cb::BK;

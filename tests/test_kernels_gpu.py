@@ -1417,6 +1417,24 @@ def test_gemm_wide_tiles(m, n, k):
         kern.gemm_set_tile(0, 0)
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 4096, 512), (256, 768, 1024), (257, 4096, 768), (333, 4096, 1088), (384, 4096, 512), (385, 3072, 1024)])
+def test_gemm_split_on_pairs_and_single_ctas(m, n, k):
+    """Split-K launches of two to four row tiles, on the side that the number of rounds takes (pairs at 256 and 385 rows, single CTAs
+    at 257 to 384) and on the other: the same sums."""
+    kern = torch.ops.cosmos_b200
+    assert kern.gemm_pick_k_splits(m, n, k, ops.EPI_GATED_RESID) > 1
+    a, w, r = _rand(m, k), _rand(n, k) * 0.05, _rand(m, n)
+    got = ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, None, m)
+    _close(got, r.float() + a.float() @ w.float().t(), 3e-2, 2e-2, f"{m}x{n}x{k}")
+    kern.gemm_set_cta_pair(False)
+    try:
+        assert torch.equal(got, ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, None, m))
+    finally:
+        kern.gemm_set_cta_pair(True)
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
 def test_gemm_swiglu_keeps_the_limits_of_silu():
     """Gates beyond the range in which the quotient of silu is refined: large of both signs, tiny, zero, infinite. Two spacings of
     subnormal bf16 (9.2e-41) absolutely, far below every value that is checked."""
