@@ -201,8 +201,11 @@ class WorkspaceAttn(AttnContext):
         n_pre = 0 if prefix is None else prefix[0].shape[1]
         qb, kb, vb, routes = self._buffers(b, s, n_pre, cfg, h)
         if prefix is not None:
-            kb[:, :n_pre].copy_(prefix[0])
-            vb[:, :n_pre].copy_(prefix[1])
+            if all(t.device == kb.device and t.dtype == kb.dtype and t.dim() == 4 for t in prefix):
+                torch.ops.cosmos_b200.copy_prefix(prefix[0], prefix[1], kb, vb)
+            else:
+                kb[:, :n_pre].copy_(prefix[0])
+                vb[:, :n_pre].copy_(prefix[1])
         gq = q_norm if cfg.qk_norm else None
         gk = k_norm if cfg.qk_norm else None
         if cos is not None and cos.shape[0] > s:   # tables for more positions: every entry takes the first rows
@@ -244,6 +247,13 @@ def dm_modulation(t_mod: torch.Tensor, mod_table: torch.Tensor) -> List[torch.Te
     -> six [B, d] tensors: shift1, scale1, gate1, shift2, scale2, gate2."""
     b = t_mod.shape[0]
     d = mod_table.shape[-1]
+    if t_mod.dtype == mod_table.dtype and d % 8 == 0 and t_mod.dim() == 2 and mod_table.dim() == 2:
+        # one kernel forward and one backward, with the roundings of the expressions below
+        if ops._use_cuda(t_mod, mod_table):
+            return list(torch.ops.cosmos_b200.dm_modulation(t_mod, mod_table).unbind(0))
+        if ops._train_cuda(t_mod, mod_table):
+            from ..ops import autograd as own
+            return list(own.dm_modulation(t_mod, mod_table))
     if t_mod.dtype == mod_table.dtype and not torch.is_grad_enabled():
         # one sum and (b > 1) one copy in place of three casts, the sum and six copies; an addition of two bf16 tensors is
         # rounded once, as the fp32 sum's cast is

@@ -192,6 +192,19 @@ class QKVPostFn(torch.autograd.Function):
         return d_qkv, None, None, None, dgq, dgk, None
 
 
+class ModulationFn(torch.autograd.Function):
+    """t_mod [B, 6d] + table [6, d] -> six [B, d] tensors."""
+
+    @staticmethod
+    def forward(ctx, t_mod, table):
+        ctx.like, ctx.shape = table.new_empty(0), (t_mod.shape[0], table.shape[1])
+        return _k().dm_modulation(t_mod, table).unbind(0)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        return _k().dm_modulation_bwd(list(grads), ctx.like, *ctx.shape)
+
+
 class SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up):
@@ -223,6 +236,10 @@ class GatedResidualFn(torch.autograd.Function):
         df, part = _k().gated_residual_bwd(dy.contiguous(), f, gate, ctx.rpb)
         dgate = _sum_to(part.sum(1), gate) if ctx.needs_input_grad[2] else None
         return dy, df, dgate, None
+
+
+def dm_modulation(t_mod, table):
+    return ModulationFn.apply(t_mod, table)
 
 
 def adaln_rmsnorm(x, gamma, shift, scale, rows_per_batch: int, eps: float = 1e-6):

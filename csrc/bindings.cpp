@@ -481,16 +481,75 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q, const Tensor& k, co
   return {dq, dk, dv};
 }
 
+Tensor aligned_rows(const Tensor& t) {   // contiguous, and 16-byte aligned: a view may start at any element
+  const Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+
+// The six modulation rows of a layer: t_mod [B, 6d] + table [6, d] -> [6, B, d]
+Tensor dm_modulation(const Tensor& t_mod, const Tensor& table) {
+  check_bf16_cuda(t_mod, "t_mod"); check_bf16_cuda(table, "table");
+  c10::cuda::CUDAGuard guard(t_mod.device());
+  TORCH_CHECK(t_mod.dim() == 2 && table.dim() == 2 && table.size(0) == 6 && t_mod.size(1) == 6 * table.size(1), "t_mod [B, 6d] and table [6, d] expected");
+  const Tensor tm = aligned_rows(t_mod), tb = aligned_rows(table);
+  Tensor out = at::empty({6, t_mod.size(0), table.size(1)}, t_mod.options());
+  cosmos::dm_modulation(tm.data_ptr(), tb.data_ptr(), out.data_ptr(), (int)t_mod.size(0), (int)table.size(1), cur_stream());
+  return out;
+}
+
+// Gradients of the six rows ([B, d], or none) -> those of t_mod [B, 6d] and of the table [6, d]
+std::tuple<Tensor, Tensor> dm_modulation_bwd(const c10::List<c10::optional<Tensor>>& grads, const Tensor& like, int64_t B, int64_t d) {
+  check_bf16_cuda(like, "like");
+  c10::cuda::CUDAGuard guard(like.device());
+  TORCH_CHECK(grads.size() == 6, "six gradients expected");
+  Tensor keep[6];
+  const void* g[6] = {};
+  for (int i = 0; i < 6; ++i) {
+    const c10::optional<Tensor> t = grads.get(i);
+    if (!t.has_value() || !t->defined()) continue;
+    check_bf16_cuda(*t, "grad");
+    TORCH_CHECK(t->numel() == B * d, "a gradient per row expected");
+    keep[i] = aligned_rows(*t);
+    g[i] = keep[i].data_ptr();
+  }
+  Tensor dt = at::empty({B, 6 * d}, like.options()), dtable = at::empty({6, d}, like.options());
+  cosmos::dm_modulation_bwd(g, dt.data_ptr(), dtable.data_ptr(), (int)B, (int)d, cur_stream());
+  return {dt, dtable};
+}
+
+// Keys and values of a prefix [B or 1, n, H, 128] -> the first n rows of two buffers [B, rows, H, 128]
+void copy_prefix(const Tensor& k, const Tensor& v, const Tensor& kb, const Tensor& vb) {
+  check_bf16_cuda(k, "k"); check_bf16_cuda(v, "v"); check_bf16_cuda(kb, "kb"); check_bf16_cuda(vb, "vb");
+  c10::cuda::CUDAGuard guard(kb.device());
+  TORCH_CHECK(kb.dim() == 4 && kb.is_contiguous() && vb.is_contiguous() && kb.sizes() == vb.sizes() && kb.size(3) == 128, "buffers must be contiguous [B, rows, H, 128]");
+  cosmos::PrefixArgs a{};
+  a.B = (int)kb.size(0); a.H = (int)kb.size(2); a.n = (int)k.size(1);
+  a.dst_b = kb.stride(0);
+  const Tensor *src[2] = {&k, &v}, *dst[2] = {&kb, &vb};
+  bool fits = true;
+  for (int i = 0; i < 2; ++i) {
+    const Tensor& t = *src[i];
+    TORCH_CHECK(t.dim() == 4 && (t.size(0) == a.B || t.size(0) == 1) && t.size(1) == a.n && a.n <= kb.size(1) && t.size(2) == a.H && t.size(3) == 128,
+                "a prefix of [B, n, H, 128] expected");
+    a.src[i] = t.data_ptr(); a.dst[i] = dst[i]->data_ptr();
+    a.sb[i] = t.size(0) == 1 ? 0 : t.stride(0); a.ss[i] = t.stride(1); a.sh[i] = t.stride(2);
+    fits = fits && t.stride(3) == 1 && (a.sb[i] | a.ss[i] | a.sh[i]) % 8 == 0 &&
+           (reinterpret_cast<uintptr_t>(a.src[i]) | reinterpret_cast<uintptr_t>(a.dst[i])) % 16 == 0;
+  }
+  if (a.n == 0) return;
+  if (fits) {
+    cosmos::copy_prefix(a, cur_stream());
+    return;
+  }
+  for (int i = 0; i < 2; ++i) dst[i]->narrow(1, 0, a.n).copy_(*src[i]);   // rows that 16-byte accesses cannot take
+}
+
 // delta = rowsum(dO * O) in fp32: [B, S, H, 128] bf16 (any layout of `dO` and `O`) -> [B, H, S]
 Tensor attn_bwd_delta(const Tensor& dout, const Tensor& o) {
   check_bf16_cuda(dout, "do"); check_bf16_cuda(o, "o");
   c10::cuda::CUDAGuard guard(o.device());
   TORCH_CHECK(o.dim() == 4 && o.size(3) == 128 && dout.sizes() == o.sizes(), "do/o must be [B, S, H, 128]");
-  auto rows = [](const Tensor& t) {   // contiguous, and a view may start at any element
-    const Tensor c = t.contiguous();
-    return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
-  };
-  const Tensor d = rows(dout), oc = rows(o);
+  const Tensor d = aligned_rows(dout), oc = aligned_rows(o);
   Tensor delta = at::empty({o.size(0), o.size(2), o.size(1)}, o.options().dtype(at::kFloat));
   cosmos::attn_bwd_delta(d.data_ptr(), oc.data_ptr(), delta.data_ptr<float>(), (int)o.size(0), (int)o.size(1), (int)o.size(2),
                          cur_stream());
@@ -1497,6 +1556,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_bwd_delta", &attn_bwd_delta);
+  m.def("dm_modulation", &dm_modulation);
+  m.def("dm_modulation_bwd", &dm_modulation_bwd);
+  m.def("copy_prefix", &copy_prefix);
   m.def("attn_fwd_sources", &attn_fwd_sources);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("gated_residual_bwd", &gated_residual_bwd);

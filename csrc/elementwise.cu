@@ -387,6 +387,72 @@ __global__ void l2_flush_kernel(uint4* buf, size_t n) {
     buf[i] = make_uint4(0, 0, 0, 0);
 }
 
+// ---------------------------------------------------------------------- a layer's modulation, and its prefix of keys and values
+// Small tensors (100 KB), so launches count: the sum and a transposing copy of torch took 7.4 us and a gap, the two copies of a
+// prefix 7 and another; each of these takes about 2, behind the end of the kernel before it.
+__device__ __forceinline__ uint4 add_bf16x8(uint4 a, uint4 b) {
+  float x[8], y[8];
+  unpack8(a, x);
+  unpack8(b, y);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] += y[e];   // one rounding, as the sum of two bf16 tensors
+  return pack8(x);
+}
+
+__global__ void __launch_bounds__(128)
+dm_modulation_kernel(const uint4* __restrict__ t_mod, const uint4* __restrict__ table, uint4* __restrict__ out, int nvec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int v = blockIdx.x * 128 + threadIdx.x, i = blockIdx.y, b = blockIdx.z;
+  if (v < nvec)
+    out[((long long)i * gridDim.z + b) * nvec + v] = add_bf16x8(t_mod[((long long)b * 6 + i) * nvec + v], table[(long long)i * nvec + v]);
+}
+
+struct ModGrads {
+  const uint4* g[6];
+};
+// The gradient of the table is the fp32 sum over the batch, four partial sums in turn (the order of a reduction over a leading
+// dimension, which it was).
+__global__ void __launch_bounds__(128)
+dm_modulation_bwd_kernel(const ModGrads m, uint4* __restrict__ dt, uint4* __restrict__ dtable, int B, int nvec) {
+  const int v = blockIdx.x * 128 + threadIdx.x, i = blockIdx.y;
+  if (v >= nvec) return;
+  const uint4* g = i == 0 ? m.g[0] : i == 1 ? m.g[1] : i == 2 ? m.g[2] : i == 3 ? m.g[3] : i == 4 ? m.g[4] : m.g[5];
+  float acc[4][8] = {};
+  for (int b0 = 0; b0 < B; b0 += 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int b = b0 + j;
+      if (b >= B) break;
+      const uint4 u = g ? g[(long long)b * nvec + v] : make_uint4(0, 0, 0, 0);
+      dt[((long long)b * 6 + i) * nvec + v] = u;
+      float f[8];
+      unpack8(u, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[j][e] += f[e];
+    }
+  }
+  float o[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) o[e] = ((acc[0][e] + acc[1][e]) + acc[2][e]) + acc[3][e];
+  dtable[(long long)i * nvec + v] = pack8(o);
+}
+
+__global__ void __launch_bounds__(256) copy_prefix_kernel(const cosmos::PrefixArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)a.B * a.n * a.H * 16) return;
+  const int k = blockIdx.y, c = int(i & 15) * 8;
+  const long long row = i >> 4;
+  const int h = int(row % a.H);
+  const long long r = row / a.H, s = r % a.n, b = r / a.n;
+  const bf16* src = (k ? (const bf16*)a.src[1] + b * a.sb[1] + s * a.ss[1] + h * a.sh[1]
+                       : (const bf16*)a.src[0] + b * a.sb[0] + s * a.ss[0] + h * a.sh[0]) + c;
+  bf16* dst = (k ? (bf16*)a.dst[1] : (bf16*)a.dst[0]) + b * a.dst_b + (s * a.H + h) * 128 + c;
+  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+}
+
 }  // namespace cb
 
 namespace cosmos {
@@ -430,6 +496,31 @@ static void launch_norm(const void* x, const void* gamma, void* y, long long row
   if (d <= 256) COSMOS_NORM(1);   // one warp per row; rows of 1024 elements and more took the row kernel above
   else COSMOS_NORM(4);
 #undef COSMOS_NORM
+}
+
+static void check_d8_mod(int d) {
+  if (d <= 0 || d % 8 != 0) throw std::runtime_error("dm_modulation: the feature size must be a multiple of 8");
+}
+
+void dm_modulation(const void* t_mod, const void* table, void* out, int B, int d, cudaStream_t s) {
+  check_d8_mod(d);
+  if (B <= 0) return;
+  launch_early(cb::dm_modulation_kernel, dim3((unsigned)((d / 8 + 127) / 128), 6, (unsigned)B), dim3(128), 0, s, (const uint4*)t_mod,
+               (const uint4*)table, (uint4*)out, d / 8);
+}
+
+void dm_modulation_bwd(const void* const* g, void* dt, void* dtable, int B, int d, cudaStream_t s) {
+  check_d8_mod(d);
+  if (B <= 0) return;
+  cb::ModGrads m;
+  for (int i = 0; i < 6; ++i) m.g[i] = (const uint4*)g[i];
+  cb::dm_modulation_bwd_kernel<<<dim3((unsigned)((d / 8 + 127) / 128), 6), 128, 0, s>>>(m, (uint4*)dt, (uint4*)dtable, B, d / 8);
+}
+
+void copy_prefix(const PrefixArgs& a, cudaStream_t s) {
+  const long long vecs = (long long)a.B * a.n * a.H * 16;
+  if (vecs <= 0) return;
+  launch_early(cb::copy_prefix_kernel, dim3((unsigned)((vecs + 255) / 256), 2), dim3(256), 0, s, a);
 }
 
 void rmsnorm(const void* x, const void* gamma, void* y, long long rows, int d, float eps,

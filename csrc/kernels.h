@@ -174,6 +174,19 @@ struct AttnBwdArgs {
   int* status = nullptr;
 };
 void flash_attn_bwd(const AttnBwdArgs& a, cudaStream_t stream);
+// out[i][b] = t_mod[b][i] + table[i] for the six modulation rows of a layer: t_mod [B, 6, d], table [6, d] -> [6, B, d], bf16, d % 8 == 0
+void dm_modulation(const void* t_mod, const void* table, void* out, int B, int d, cudaStream_t s);
+// Its gradients: g[i] [B, d] or null -> dt [B, 6, d], dtable [6, d]
+void dm_modulation_bwd(const void* const* g, void* dt, void* dtable, int B, int d, cudaStream_t s);
+// Rows of two prefixes [B, n, H, 128] (element strides, unit inner stride) to the front of two buffers [B, rows, H, 128].
+struct PrefixArgs {
+  const void* src[2];
+  void* dst[2];
+  long long sb[2], ss[2], sh[2];   // source strides; sb 0: one prefix for every batch entry
+  int B, n, H;
+  long long dst_b;                 // elements between the batch entries of a buffer
+};
+void copy_prefix(const PrefixArgs& a, cudaStream_t s);
 // delta = rowsum(dO * O): O, dO [B, Sq, Hq, 128] contiguous bf16 -> [B, Hq, Sq] fp32 (elementwise_bwd.cu)
 void attn_bwd_delta(const void* dO, const void* O, float* delta, int B, int Sq, int Hq, cudaStream_t stream);
 

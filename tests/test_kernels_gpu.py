@@ -489,6 +489,48 @@ def test_attention_backward_delta(b, s, h):
         assert b * s * h < 16 or torch.equal(got, same)
 
 
+@pytest.mark.parametrize("b,d,unused", [(1, 4096, ()), (2, 1032, (1,)), (7, 8, (0, 5))])
+def test_dm_modulation(b, d, unused):
+    """The bits of the expressions that it stands for: a sum rounded once, gradients that are copies, and a sum over the batch in
+    fp32 that is rounded once (its order is the reduction's up to four entries; beyond, two spacings of bf16)."""
+    from cosmos_b200.models.mot import dm_modulation
+    t, tab = _rand(b, 6 * d), _rand(6, d)
+    want = [(t.view(b, 6, d).float() + tab.float()[None]).to(t.dtype)[:, i] for i in range(6)]
+    odd = torch.empty(tab.numel() + 1, dtype=tab.dtype, device=tab.device)[1:].view_as(tab).copy_(tab)
+    for table in (tab, odd):
+        assert all(torch.equal(x, y) for x, y in zip(dm_modulation(t, table), want))
+    t1, tab1 = t.clone().requires_grad_(True), tab.clone().requires_grad_(True)
+    t2, tab2 = t.clone().requires_grad_(True), tab.clone().requires_grad_(True)
+    g = [_rand(b, d) for _ in range(6)]
+    use = [i for i in range(6) if i not in unused]
+    got = dm_modulation(t1, tab1)
+    torch.autograd.backward([got[i] for i in use], [g[i] for i in use])
+    m = (t2.view(b, 6, d).float() + tab2.float()[None]).to(t.dtype)
+    torch.autograd.backward([m[:, i] for i in use], [g[i] for i in use])
+    assert torch.equal(t1.grad, t2.grad)
+    if b <= 4:
+        assert torch.equal(tab1.grad, tab2.grad)
+    assert ((tab1.grad - tab2.grad).abs() <= 2 ** -7 * tab2.grad.abs()).all()
+
+
+@pytest.mark.parametrize("b,one,n,rows,h", [(1, False, 1, 3, 2), (2, True, 77, 317, 8), (3, False, 5, 5, 1), (2, False, 0, 4, 2)])
+@pytest.mark.parametrize("form", ["contiguous", "view of a projection", "odd start"])
+def test_copy_prefix(b, one, n, rows, h, form):
+    bp = 1 if one else b
+    if form == "view of a projection":
+        qkv = _rand(bp, n, 3 * h, 128)
+        k, v = qkv[:, :, h:2 * h], qkv[:, :, 2 * h:]
+    elif form == "odd start":
+        k, v = (_rand(bp * n * h * 128 + 1)[1:].view(bp, n, h, 128) for _ in range(2))
+    else:
+        k, v = _rand(bp, n, h, 128), _rand(bp, n, h, 128)
+    kb, vb = _rand(b, rows, h, 128), _rand(b, rows, h, 128)
+    wk, wv = kb.clone(), vb.clone()
+    wk[:, :n], wv[:, :n] = k, v
+    torch.ops.cosmos_b200.copy_prefix(k, v, kb, vb)
+    assert torch.equal(kb, wk) and torch.equal(vb, wv)
+
+
 def _grads_close(own_in, ref_in, names, atol=4e-2, rtol=4e-2):
     for a, b, n in zip(own_in, ref_in, names):
         assert a.grad is not None, f"no gradient for {n}"
