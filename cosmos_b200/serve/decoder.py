@@ -57,6 +57,9 @@ class StepDecoder:
         if self.sampling is not None:
             self._sample(logits)                     # global ids across the vocab shards, into self.next_tokens
             return
+        if self.tp == 1 and logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and ops.get_backend() != "library":
+            torch.ops.cosmos_b200.greedy_pick(logits, 0, self.cfg.vocab_size - 1, self.next_tokens)
+            return
         val, idx = logits.float().max(dim=-1)
         idx = idx + self.rank * self.v_loc
         if self.tp > 1:
@@ -247,27 +250,16 @@ class TPDecoder(StepDecoder):
     def _step_impl(self) -> None:
         """Consumes self.tokens / self.lens (device), writes self.next_tokens and advances lens."""
         b = self.tokens.shape[0]
-        pos = self.lens.long()                       # cache position of the new token = current length
-        # rotary position: the same for text; prompts with vision grids advance slower than one per token
-        # (3-D ids), so the serving engine keeps a per-slot offset
-        rpos = pos if self.pos_delta is None else pos + self.pos_delta
-        ang = rpos.float()[:, None] * self.inv_freq[None]
-        cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
-        slots = PagedKVCache.slots(self.table, pos[:, None], self.page_size)[:, 0].contiguous()
-        # attention sees the token being written; idle slots of a serving batch do not advance
-        if self.step_inc is None:
-            self.lens.add_(1)
+        # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
+        if self.embed.is_cuda and self.embed.dtype == torch.bfloat16 and ops.get_backend() != "library" and self.cfg.d_model % 8 == 0:
+            x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
+                                                                    self.page_size, self.tokens, self.embed)
         else:
-            self.lens.add_(self.step_inc)
-        x = self.embed[self.tokens]
+            x, cos, sin, slots = self._begin_step()
         # Programmatic dependent launch for the layer kernels: each one's set-up, and the GEMMs' first weight tiles,
-        # may overlap the tail of the kernel before it. Measured per step: 5.80 -> 5.45 ms at TP 4 and 8.96 -> 8.77 ms
-        # at TP 2, but 12.45 -> 12.6 ms on one GPU at batch 32 and 5.30 -> 5.50 ms at batch 1 (a GEMM CTA needs most
-        # of an SM's shared memory, so the next GEMM cannot become resident before the current one leaves, and the
-        # programmatic edges cost about 0.5 us per launch in the replayed graph). Hence on from TP 4, where the step
-        # is latency-bound; COSMOS_DECODE_PDL=0 / 1 overrides.
-        pdl = self.device.type == "cuda" and ops.get_backend() != "library" and \
-            os.environ.get("COSMOS_DECODE_PDL", "1" if self.tp >= 4 else "0") == "1"
+        # may overlap the tail of the kernel before it. Batch 1 over 1500 tokens, eight layers: 1080 -> 1050 us; batch 32 over 8448:
+        # 2475 -> 2465. COSMOS_DECODE_PDL=0 turns it off.
+        pdl = self.device.type == "cuda" and ops.get_backend() != "library" and os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
         if pdl:
             torch.ops.cosmos_b200.set_pdl(True)
         try:
@@ -276,6 +268,21 @@ class TPDecoder(StepDecoder):
             if pdl:
                 torch.ops.cosmos_b200.set_pdl(False)
         self._finish_step(logits, b)
+
+    def _begin_step(self):
+        """The embeddings, rotary tables and cache slots of the step's tokens, and the lengths moved on."""
+        pos = self.lens.long()                       # cache position of the new token = current length
+        # rotary position: the same for text; prompts with vision grids advance slower than one per token
+        # (3-D ids), so the serving engine keeps a per-slot offset
+        rpos = pos if self.pos_delta is None else pos + self.pos_delta
+        ang = rpos.float()[:, None] * self.inv_freq[None]
+        cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+        slots = PagedKVCache.slots(self.table, pos[:, None], self.page_size)[:, 0].contiguous()
+        if self.step_inc is None:
+            self.lens.add_(1)
+        else:
+            self.lens.add_(self.step_inc)
+        return self.embed[self.tokens], cos, sin, slots
 
     def _forward_layers(self, x, cos, sin, slots) -> torch.Tensor:
         if self.tp == 1:

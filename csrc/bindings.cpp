@@ -486,6 +486,59 @@ Tensor aligned_rows(const Tensor& t) {   // contiguous, and 16-byte aligned: a v
   return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
 }
 
+// cos, sin [S, half] of pos [3, S] (see rope.py)
+std::tuple<Tensor, Tensor> make_rope_tables(const Tensor& pos, int64_t head_dim, double theta, int64_t sh, int64_t sw) {
+  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.dim() == 2 && pos.size(0) == 3 && head_dim % 2 == 0 && head_dim <= 512,
+              "rope_tables: int64 positions [3, S] on the GPU");
+  c10::cuda::CUDAGuard guard(pos.device());
+  const Tensor p = pos.contiguous();
+  const int64_t S = p.size(1), half = head_dim / 2;
+  Tensor c = at::empty({S, half}, p.options().dtype(at::kFloat)), sn = at::empty_like(c);
+  cosmos::rope_tables((const long long*)p.data_ptr<int64_t>(), (int)S, (int)half, theta, (int)head_dim, (int)(3 * sh), (int)(3 * sw),
+                      c.data_ptr<float>(), sn.data_ptr<float>(), cur_stream());
+  return {c, sn};
+}
+
+// What a decode step needs before its layers: (x [B, d], cos, sin [B, half], slots [B]); advances `lens`.
+std::tuple<Tensor, Tensor, Tensor, Tensor> decode_begin(const Tensor& lens, const OptT& inc, const OptT& pos_delta, const Tensor& inv_freq,
+                                                        const Tensor& table, int64_t page_size, const Tensor& tokens, const Tensor& embed) {
+  check_bf16_cuda(embed, "embed");
+  c10::cuda::CUDAGuard guard(embed.device());
+  const int64_t B = lens.numel(), d = embed.size(1), half = inv_freq.numel();
+  const auto on = [&](const Tensor& t, at::ScalarType type, int64_t n, const char* name) {
+    TORCH_CHECK(t.is_cuda() && t.device() == embed.device() && t.scalar_type() == type && t.is_contiguous() && t.numel() == n, "decode_begin: bad ", name);
+  };
+  on(lens, at::kInt, B, "lens"); on(inv_freq, at::kFloat, half, "inv_freq"); on(tokens, at::kLong, B, "tokens");
+  TORCH_CHECK(table.is_cuda() && table.scalar_type() == at::kInt && table.dim() == 2 && table.size(0) == B && table.stride(1) == 1 && table.size(1) > 0 &&
+                  page_size > 0, "decode_begin: bad table");
+  TORCH_CHECK(embed.dim() == 2 && embed.stride(1) == 1 && embed.stride(0) % 8 == 0 && d % 8 == 0 && embed.size(0) > 0 &&
+                  reinterpret_cast<uintptr_t>(embed.data_ptr()) % 16 == 0, "decode_begin: rows of embed must be whole 16-byte vectors");
+  cosmos::DecodeBeginArgs a{};
+  if (inc.has_value() && inc->defined()) { on(*inc, at::kInt, B, "inc"); a.inc = inc->data_ptr<int>(); }
+  if (pos_delta.has_value() && pos_delta->defined()) { on(*pos_delta, at::kLong, B, "pos_delta"); a.pos_delta = (const long long*)pos_delta->data_ptr<int64_t>(); }
+  Tensor c = at::empty({B, half}, inv_freq.options()), sn = at::empty_like(c);
+  Tensor slots = at::empty({B}, tokens.options()), x = at::empty({B, d}, embed.options());
+  a.lens = lens.data_ptr<int>(); a.inv_freq = inv_freq.data_ptr<float>(); a.table = table.data_ptr<int>();
+  a.tokens = (const long long*)tokens.data_ptr<int64_t>(); a.embed = embed.data_ptr();
+  a.cos_t = c.data_ptr<float>(); a.sin_t = sn.data_ptr<float>(); a.slots = (long long*)slots.data_ptr<int64_t>(); a.x = x.data_ptr();
+  a.status = status_tensor(embed.get_device()).data_ptr<int>();
+  a.table_stride = table.stride(0); a.embed_stride = embed.stride(0);
+  a.B = (int)B; a.half = (int)half; a.pages = (int)table.size(1); a.page_size = (int)page_size; a.d = (int)d; a.vocab = (int)embed.size(0);
+  cosmos::decode_begin(a, cur_stream());
+  return {x, c, sn, slots};
+}
+
+// next[b] = min(first + index of the largest logit of row b, limit)
+void greedy_pick(const Tensor& logits, int64_t first, int64_t limit, const Tensor& next) {
+  check_bf16_cuda(logits, "logits");
+  c10::cuda::CUDAGuard guard(logits.device());
+  TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.size(1) > 0 && logits.size(1) < (1ll << 31), "greedy_pick: logits [B, V] with unit inner stride");
+  TORCH_CHECK(next.is_cuda() && next.device() == logits.device() && next.scalar_type() == at::kLong && next.is_contiguous() && next.numel() == logits.size(0),
+              "greedy_pick: next must be int64 [B]");
+  cosmos::greedy_pick(logits.data_ptr(), logits.stride(0), (int)logits.size(0), (int)logits.size(1), first, limit,
+                      (long long*)next.data_ptr<int64_t>(), cur_stream());
+}
+
 // The six modulation rows of a layer: t_mod [B, 6d] + table [6, d] -> [6, B, d]
 Tensor dm_modulation(const Tensor& t_mod, const Tensor& table) {
   check_bf16_cuda(t_mod, "t_mod"); check_bf16_cuda(table, "table");
@@ -1557,6 +1610,9 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_bwd_delta", &attn_bwd_delta);
   m.def("dm_modulation", &dm_modulation);
+  m.def("rope_tables", &make_rope_tables);
+  m.def("decode_begin", &decode_begin);
+  m.def("greedy_pick", &greedy_pick);
   m.def("dm_modulation_bwd", &dm_modulation_bwd);
   m.def("copy_prefix", &copy_prefix);
   m.def("attn_fwd_sources", &attn_fwd_sources);

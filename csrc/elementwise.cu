@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(256) copy_prefix_kernel(const cosmos::PrefixAr
 
 namespace cosmos {
 
-static bool g_pdl = false;
+static thread_local bool g_pdl = false;   // a GEMM of another thread may have a B that a kernel before it writes
 void set_pdl(bool on) { g_pdl = on; }
 bool pdl_on() { return g_pdl; }
 

@@ -27,8 +27,8 @@ namespace cosmos {
 // Programmatic dependent launch. GEMMs, split-K reductions, row norms and attention over contiguous keys are always launched so
 // that their set-up overlaps the tail of the kernel before them. While this is on, the other kernels of a decode step (QKV
 // post-processing, paged attention and its merge, all-reduce + norm) are too, and GEMMs on single CTAs read their first weight
-// tiles ahead; the caller turns it on around a decode step (where the GEMMs' B operands are weights) and off afterwards. The switch is process-wide: launches from other host threads see it.
-void set_pdl(bool on);
+// tiles ahead; the caller turns it on around a decode step (where the GEMMs' B operands are weights) and off afterwards.
+void set_pdl(bool on);   // for the calling thread
 bool pdl_on();
 
 struct GemmArgs {
@@ -174,6 +174,27 @@ struct AttnBwdArgs {
   int* status = nullptr;
 };
 void flash_attn_bwd(const AttnBwdArgs& a, cudaStream_t stream);
+// ---- both ends of a step (step_edges.cu) ----
+// cos, sin [S, half] fp32 of positions pos [3, S] with interleaved axes; h3, w3: three times the section of H and W
+void rope_tables(const long long* pos, int S, int half, double theta, int head_dim, int h3, int w3, float* cos_t, float* sin_t, cudaStream_t s);
+struct DecodeBeginArgs {
+  int* lens;                    // [B], advanced by inc (or 1)
+  const int* inc;               // [B] or null
+  const long long* pos_delta;   // [B] or null: rotary position minus cache position
+  const float* inv_freq;        // [half]
+  const int* table;             // [B, pages], row stride table_stride
+  const long long* tokens;      // [B]
+  const void* embed;            // [vocab, d] bf16, row stride embed_stride
+  float *cos_t, *sin_t;         // [B, half]
+  long long* slots;             // [B]
+  void* x;                      // [B, d] bf16
+  int* status;
+  long long table_stride, embed_stride;
+  int B, half, pages, page_size, d, vocab;
+};
+void decode_begin(const DecodeBeginArgs& a, cudaStream_t s);
+// next[b] = min(first + smallest index of the largest of logits[b][0 .. V), limit); bf16, row stride ld
+void greedy_pick(const void* logits, long long ld, int B, int V, long long first, long long limit, long long* next, cudaStream_t s);
 // out[i][b] = t_mod[b][i] + table[i] for the six modulation rows of a layer: t_mod [B, 6, d], table [6, d] -> [6, B, d], bf16, d % 8 == 0
 void dm_modulation(const void* t_mod, const void* table, void* out, int B, int d, cudaStream_t s);
 // Its gradients: g[i] [B, d] or null -> dt [B, 6, d], dtable [6, d]

@@ -531,6 +531,51 @@ def test_copy_prefix(b, one, n, rows, h, form):
     assert torch.equal(kb, wk) and torch.equal(vb, wv)
 
 
+@pytest.mark.parametrize("n,theta,section", [(1, 5.0e5, (24, 20, 20)), (333, 1.0e4, (24, 20, 20)), (2001, 5.0e6, (10, 11, 11))])
+def test_rope_tables(n, theta, section):
+    """The bits of the expressions in fp64, for positions up to a million and in any layout."""
+    from cosmos_b200.models import rope
+    pos = torch.randint(0, 10 ** 6, (n, 3), generator=torch.Generator().manual_seed(n)).t()   # [3, n], rows strided
+    want = rope.rope_tables(pos, 2 * sum(section), theta, section)
+    for p in (pos.cuda(), pos.cuda().contiguous()):
+        got = rope.rope_tables(p, 2 * sum(section), theta, section)
+        for x, y in zip(got, want):   # the CPU's own library: half a spacing of fp32 at most
+            assert (x.cpu() - y).abs().max() <= 2 ** -24
+
+
+@pytest.mark.parametrize("b,d,page,delta,inc", [(1, 64, 16, False, False), (3, 4096, 32, True, True), (70, 1032, 16, True, False)])
+def test_decode_begin(b, d, page, delta, inc):
+    from types import SimpleNamespace
+    from cosmos_b200.serve.decoder import TPDecoder
+    g = torch.Generator(device="cuda").manual_seed(b)
+    ids = lambda hi, *s: torch.randint(0, hi, s, generator=g, device="cuda")  # noqa: E731
+    dec = SimpleNamespace(lens=ids(20 * page, b).int(), tokens=ids(1000, b), table=ids(5000, b, 20).int(), page_size=page, embed=_rand(1000, d),
+                          inv_freq=torch.rand(64, generator=g, device="cuda"), pos_delta=-ids(7, b) if delta else None,
+                          step_inc=ids(2, b).int() if inc else None)
+    lens = dec.lens.clone()
+    got = torch.ops.cosmos_b200.decode_begin(lens, dec.step_inc, dec.pos_delta, dec.inv_freq, dec.table, page, dec.tokens, dec.embed)
+    want = TPDecoder._begin_step(dec)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[3], want[3]) and torch.equal(lens, dec.lens)
+    for x, y in zip(got[1:3], want[1:3]):
+        assert (x - y).abs().max() <= 2 ** -22   # two spacings of the functions' results
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("b,v,stride", [(1, 151936, 151936), (33, 1000, 1000), (2, 7, 7), (3, 4097, 5001), (1, 1, 1)])
+def test_greedy_pick(b, v, stride):
+    x = _rand(b, stride)[:, :v]
+    x[0, v // 2:] = x[0].max() + 1          # ties: the smallest index
+    if b > 2:
+        x[1] = -float("inf")
+        x[2, v - 1] = float("nan")          # counts as the largest
+    nxt = torch.full((b,), -1, device="cuda")
+    torch.ops.cosmos_b200.greedy_pick(x, 0, v - 1, nxt)
+    assert torch.equal(nxt, x.float().max(dim=-1)[1])
+    torch.ops.cosmos_b200.greedy_pick(x, 3, 5, nxt)
+    assert torch.equal(nxt, (x.float().max(dim=-1)[1] + 3).clamp(max=5))
+
+
 def _grads_close(own_in, ref_in, names, atol=4e-2, rtol=4e-2):
     for a, b, n in zip(own_in, ref_in, names):
         assert a.grad is not None, f"no gradient for {n}"
