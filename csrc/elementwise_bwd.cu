@@ -66,10 +66,12 @@ attn_bwd_delta_kernel(const uint4* __restrict__ dout, const uint4* __restrict__ 
 // ---------------------------------------------------------------------- RMSNorm / AdaLN rows
 // y = n * w + shift,  n = x * rinv,  rinv = rsqrt(mean(x^2) + eps),  w = gamma * (1 + scale)
 // dx = rinv * (dy * w) - x * rinv^3 * mean(dy * w * x);  rinv is saved for the column sums.
-// One CTA (256 threads) per row, grid-strided; a thread holds up to MAXJ 8-element vectors.
+// One CTA (256 threads) per row, grid-strided; a thread holds up to MAXJ 8-element vectors. The next row is requested before this
+// one's sums meet, which its loads would otherwise wait for, and rows of up to 4096 elements take the form with half the
+// registers: 14080 x 4096 120 -> 75 us.
 constexpr int NB_THREADS = 256;
-constexpr int NB_MAXJ = 4;  // d <= 8192
 
+template <int NB_MAXJ>   // 2: d <= 4096; 4: d <= 8192
 __global__ void __launch_bounds__(NB_THREADS)
 rmsnorm_bwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ gamma,
                         const bf16* __restrict__ scale, long long rows, int d, int rows_per_batch,
@@ -85,10 +87,20 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
     for (int e = 0; e < 8; ++e) gv[j][e] = 1.f;
     if (gamma && vi < nvec) bw_unpack8(reinterpret_cast<const uint4*>(gamma)[vi], gv[j]);
   }
+  uint4 xn[NB_MAXJ], gn[NB_MAXJ];
+  auto request = [&](long long row) {
+#pragma unroll
+    for (int j = 0; j < NB_MAXJ; ++j) {
+      const int vi = tid + j * NB_THREADS;
+      if (row < rows && vi < nvec) {
+        xn[j] = reinterpret_cast<const uint4*>(x + row * d)[vi];
+        gn[j] = reinterpret_cast<const uint4*>(dy + row * d)[vi];
+      }
+    }
+  };
+  request(blockIdx.x);
   int it = 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x, ++it) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * d);
-    const uint4* gr = reinterpret_cast<const uint4*>(dy + row * d);
     const uint4* sr = scale ? reinterpret_cast<const uint4*>(scale + (row / rows_per_batch) * mod_stride) : nullptr;
     float xv[NB_MAXJ][8], gw[NB_MAXJ][8];
     float a = 0.f, c = 0.f;
@@ -96,8 +108,8 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
     for (int j = 0; j < NB_MAXJ; ++j) {
       const int vi = tid + j * NB_THREADS;
       if (vi < nvec) {
-        bw_unpack8(xr[vi], xv[j]);
-        bw_unpack8(gr[vi], gw[j]);
+        bw_unpack8(xn[j], xv[j]);
+        bw_unpack8(gn[j], gw[j]);
         float sc[8];
         if (sr) bw_unpack8(sr[vi], sc);
 #pragma unroll
@@ -109,6 +121,7 @@ rmsnorm_bwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
         }
       }
     }
+    request(row + gridDim.x);
     a = bw_warp_sum(a);
     c = bw_warp_sum(c);
     const int buf = it & 1;  // two buffers: the next row's writes cannot overtake this row's reads
@@ -249,119 +262,170 @@ swiglu_bwd_kernel(const bf16* __restrict__ gate_up, const bf16* __restrict__ dy,
 // ---------------------------------------------------------------------- q/k norm + rotary, q/k/v split
 // Forward: qkv [rows, Hq + 2 Hkv, 128] -> q [rows, Hq, 128], k, v [rows, Hkv, 128]; q and k heads get
 // RMS-norm (gamma_q / gamma_k, may be null) and the rotary rotation (cos/sin [rope_rows, 64], row
-// r uses table row r % rope_rows; may be null). One warp per (row, head); a lane holds elements
-// [2l, 2l+1] of both 64-channel halves.
+// r uses table row r % rope_rows; may be null). One warp per four heads of a row, grid-strided; a lane holds elements
+// [2l, 2l+1] of both 64-channel halves. Bound by memory once four heads' loads are in flight together and the tables and norm
+// weights are read for all of them: 14080 rows of 48 heads, us: forward 153 -> 95, backward 326 -> 165 (one head a warp,
+// and the norm weights' gradient by atomics in shared memory, whose order differed from run to run).
+constexpr int QP_HEADS = 4;
+
+struct QkvLane {   // a lane's part of one head: two neighbours in either half
+  uint32_t lo, hi;
+  __device__ __forceinline__ void load(const bf16* p, int lane) {
+    lo = reinterpret_cast<const uint32_t*>(p)[lane];
+    hi = reinterpret_cast<const uint32_t*>(p + 64)[lane];
+  }
+  __device__ __forceinline__ void store(bf16* p, int lane) const {
+    reinterpret_cast<uint32_t*>(p)[lane] = lo;
+    reinterpret_cast<uint32_t*>(p + 64)[lane] = hi;
+  }
+};
+__device__ __forceinline__ void qkv_gamma(const bf16* gamma, int lane, float (&g)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) g[e] = gamma ? __bfloat162float(gamma[(e >> 1) * 64 + 2 * lane + (e & 1)]) : 1.f;
+}
+// head h of a row in the split tensors
+__device__ __forceinline__ long long qkv_part(long long row, int h, int Hq, int Hkv, int& which) {
+  which = h < Hq ? 0 : h < Hq + Hkv ? 1 : 2;
+  return which == 0 ? (row * Hq + h) * 128 : (row * Hkv + (h - Hq) % Hkv) * 128;
+}
+
 __global__ void __launch_bounds__(256)
 qkv_post_fwd_kernel(const bf16* __restrict__ qkv, long long rows, int Hq, int Hkv, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rope_rows, const bf16* __restrict__ gamma_q,
                     const bf16* __restrict__ gamma_k, float eps, bf16* __restrict__ q, bf16* __restrict__ k,
                     bf16* __restrict__ v) {
   const int lane = threadIdx.x & 31;
-  const int heads = Hq + 2 * Hkv;
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= rows * heads) return;
-  const long long row = w / heads;
-  const int h = (int)(w % heads);
-  const bf16* p = qkv + w * 128;
-  const uint32_t lo = reinterpret_cast<const uint32_t*>(p)[lane];
-  const uint32_t hi = reinterpret_cast<const uint32_t*>(p + 64)[lane];
-  bf16* dst;
-  if (h < Hq) dst = q + (row * Hq + h) * 128;
-  else if (h < Hq + Hkv) dst = k + (row * Hkv + (h - Hq)) * 128;
-  else dst = v + (row * Hkv + (h - Hq - Hkv)) * 128;
-  uint32_t out_lo = lo, out_hi = hi;
-  if (h < Hq + Hkv) {
-    const bf16* gamma = h < Hq ? gamma_q : gamma_k;
-    float a0 = bf16lo(lo), a1 = bf16hi(lo), b0 = bf16lo(hi), b1 = bf16hi(hi);
-    if (gamma) {
-      const float ss = bw_warp_sum(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1);
-      const float rinv = rsqrtf(ss * (1.f / 128.f) + eps);
-      a0 *= rinv * __bfloat162float(gamma[2 * lane]);
-      a1 *= rinv * __bfloat162float(gamma[2 * lane + 1]);
-      b0 *= rinv * __bfloat162float(gamma[64 + 2 * lane]);
-      b1 *= rinv * __bfloat162float(gamma[64 + 2 * lane + 1]);
-    }
+  const int heads = Hq + 2 * Hkv, groups = (heads + QP_HEADS - 1) / QP_HEADS;
+  float gq[4], gk[4];
+  qkv_gamma(gamma_q, lane, gq);
+  qkv_gamma(gamma_k, lane, gk);
+  const long long total = rows * groups;
+  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total;
+       w += (long long)gridDim.x * (blockDim.x >> 5)) {
+    const long long row = w / groups;
+    const int h0 = (int)(w % groups) * QP_HEADS;
+    QkvLane in[QP_HEADS];
+#pragma unroll
+    for (int j = 0; j < QP_HEADS; ++j)
+      if (h0 + j < heads) in[j].load(qkv + (row * heads + h0 + j) * 128, lane);
+    float2 c = make_float2(1.f, 1.f), s = make_float2(0.f, 0.f);
     if (cos_t) {
       const long long tr = (row % rope_rows) * 64;
-      const float2 c = reinterpret_cast<const float2*>(cos_t + tr)[lane];
-      const float2 s = reinterpret_cast<const float2*>(sin_t + tr)[lane];
-      const float r0 = a0 * c.x - b0 * s.x, r1 = a1 * c.y - b1 * s.y;
-      const float q0 = b0 * c.x + a0 * s.x, q1 = b1 * c.y + a1 * s.y;
-      a0 = r0; a1 = r1; b0 = q0; b1 = q1;
+      c = reinterpret_cast<const float2*>(cos_t + tr)[lane];
+      s = reinterpret_cast<const float2*>(sin_t + tr)[lane];
     }
-    out_lo = pack_bf16(a0, a1);
-    out_hi = pack_bf16(b0, b1);
+#pragma unroll
+    for (int j = 0; j < QP_HEADS; ++j) {
+      const int h = h0 + j;
+      if (h >= heads) break;
+      int which;
+      const long long at = qkv_part(row, h, Hq, Hkv, which);
+      QkvLane out = in[j];
+      if (which < 2) {
+        float a0 = bf16lo(out.lo), a1 = bf16hi(out.lo), b0 = bf16lo(out.hi), b1 = bf16hi(out.hi);
+        if (which == 0 ? gamma_q != nullptr : gamma_k != nullptr) {
+          const float ss = bw_warp_sum(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1);
+          const float rinv = rsqrtf(ss * (1.f / 128.f) + eps);
+          a0 *= rinv * (which == 0 ? gq[0] : gk[0]);
+          a1 *= rinv * (which == 0 ? gq[1] : gk[1]);
+          b0 *= rinv * (which == 0 ? gq[2] : gk[2]);
+          b1 *= rinv * (which == 0 ? gq[3] : gk[3]);
+        }
+        if (cos_t) {
+          // the contractions are spelled out: the training step keeps its bits
+          const float r0 = fmaf(a0, c.x, -__fmul_rn(b0, s.x)), r1 = fmaf(a1, c.y, -__fmul_rn(b1, s.y));
+          const float q0 = fmaf(b0, c.x, __fmul_rn(a0, s.x)), q1 = fmaf(b1, c.y, __fmul_rn(a1, s.y));
+          a0 = r0; a1 = r1; b0 = q0; b1 = q1;
+        }
+        out.lo = pack_bf16(a0, a1);
+        out.hi = pack_bf16(b0, b1);
+      }
+      out.store((which == 0 ? q : which == 1 ? k : v) + at, lane);
+    }
   }
-  reinterpret_cast<uint32_t*>(dst)[lane] = out_lo;
-  reinterpret_cast<uint32_t*>(dst + 64)[lane] = out_hi;
 }
 
-// Backward of the above: d_qkv from (dq, dk, dv) and the raw qkv; per-CTA partial sums of d gamma_q /
-// d gamma_k in part[block][2][128].
+// Backward of the above: d_qkv from (dq, dk, dv) and the raw qkv; per-CTA partial sums of d gamma_q / d gamma_k in
+// part[block][2][128], a lane's own in registers, then the warps' in their order.
 __global__ void __launch_bounds__(256)
 qkv_post_bwd_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ dq, const bf16* __restrict__ dk,
                     const bf16* __restrict__ dv, long long rows, int Hq, int Hkv, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rope_rows, const bf16* __restrict__ gamma_q,
                     const bf16* __restrict__ gamma_k, float eps, bf16* __restrict__ d_qkv,
                     float* __restrict__ part) {
-  __shared__ float acc[2][128];
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 256) acc[threadIdx.x >> 7][threadIdx.x & 127] = 0.f;
-  __syncthreads();
-  const int heads = Hq + 2 * Hkv;
-  const long long total = rows * heads;
-  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total;
-       w += (long long)gridDim.x * (blockDim.x >> 5)) {
-    const long long row = w / heads;
-    const int h = (int)(w % heads);
-    const bf16* src;
-    if (h < Hq) src = dq + (row * Hq + h) * 128;
-    else if (h < Hq + Hkv) src = dk + (row * Hkv + (h - Hq)) * 128;
-    else src = dv + (row * Hkv + (h - Hq - Hkv)) * 128;
-    const uint32_t glo = reinterpret_cast<const uint32_t*>(src)[lane];
-    const uint32_t ghi = reinterpret_cast<const uint32_t*>(src + 64)[lane];
-    uint32_t out_lo = glo, out_hi = ghi;
-    if (h < Hq + Hkv) {
-      const int which = h < Hq ? 0 : 1;
-      const bf16* gamma = which == 0 ? gamma_q : gamma_k;
-      float ga0 = bf16lo(glo), ga1 = bf16hi(glo), gb0 = bf16lo(ghi), gb1 = bf16hi(ghi);
-      if (cos_t) {  // transpose of the rotation
-        const long long tr = (row % rope_rows) * 64;
-        const float2 c = reinterpret_cast<const float2*>(cos_t + tr)[lane];
-        const float2 s = reinterpret_cast<const float2*>(sin_t + tr)[lane];
-        const float t0 = ga0 * c.x + gb0 * s.x, t1 = ga1 * c.y + gb1 * s.y;
-        const float u0 = gb0 * c.x - ga0 * s.x, u1 = gb1 * c.y - ga1 * s.y;
-        ga0 = t0; ga1 = t1; gb0 = u0; gb1 = u1;
-      }
-      if (gamma) {
-        const bf16* p = qkv + w * 128;
-        const uint32_t lo = reinterpret_cast<const uint32_t*>(p)[lane];
-        const uint32_t hi = reinterpret_cast<const uint32_t*>(p + 64)[lane];
-        const float x0 = bf16lo(lo), x1 = bf16hi(lo), x2 = bf16lo(hi), x3 = bf16hi(hi);
-        const float ss = bw_warp_sum(x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3);
-        const float rinv = rsqrtf(ss * (1.f / 128.f) + eps);
-        const float n0 = x0 * rinv, n1 = x1 * rinv, n2 = x2 * rinv, n3 = x3 * rinv;
-        atomicAdd(&acc[which][2 * lane], ga0 * n0);
-        atomicAdd(&acc[which][2 * lane + 1], ga1 * n1);
-        atomicAdd(&acc[which][64 + 2 * lane], gb0 * n2);
-        atomicAdd(&acc[which][64 + 2 * lane + 1], gb1 * n3);
-        const float w0 = ga0 * __bfloat162float(gamma[2 * lane]), w1 = ga1 * __bfloat162float(gamma[2 * lane + 1]);
-        const float w2 = gb0 * __bfloat162float(gamma[64 + 2 * lane]);
-        const float w3 = gb1 * __bfloat162float(gamma[64 + 2 * lane + 1]);
-        const float m = bw_warp_sum(w0 * n0 + w1 * n1 + w2 * n2 + w3 * n3) * (1.f / 128.f);
-        ga0 = rinv * (w0 - n0 * m); ga1 = rinv * (w1 - n1 * m);
-        gb0 = rinv * (w2 - n2 * m); gb1 = rinv * (w3 - n3 * m);
-      }
-      out_lo = pack_bf16(ga0, ga1);
-      out_hi = pack_bf16(gb0, gb1);
+  __shared__ float acc[8][2][128];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int heads = Hq + 2 * Hkv, groups = (heads + QP_HEADS - 1) / QP_HEADS;
+  float gq[4], gk[4], sq[4] = {}, sk[4] = {};
+  qkv_gamma(gamma_q, lane, gq);
+  qkv_gamma(gamma_k, lane, gk);
+  const long long total = rows * groups;
+  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + warp; w < total; w += (long long)gridDim.x * (blockDim.x >> 5)) {
+    const long long row = w / groups;
+    const int h0 = (int)(w % groups) * QP_HEADS;
+    QkvLane grad[QP_HEADS], in[QP_HEADS];
+#pragma unroll
+    for (int j = 0; j < QP_HEADS; ++j) {
+      if (h0 + j >= heads) continue;
+      int which;
+      const long long at = qkv_part(row, h0 + j, Hq, Hkv, which);
+      grad[j].load((which == 0 ? dq : which == 1 ? dk : dv) + at, lane);
+      if (which == 0 ? gamma_q != nullptr : which == 1 && gamma_k != nullptr) in[j].load(qkv + (row * heads + h0 + j) * 128, lane);
     }
-    bf16* dst = d_qkv + w * 128;
-    reinterpret_cast<uint32_t*>(dst)[lane] = out_lo;
-    reinterpret_cast<uint32_t*>(dst + 64)[lane] = out_hi;
+    float2 c = make_float2(1.f, 1.f), s = make_float2(0.f, 0.f);
+    if (cos_t) {
+      const long long tr = (row % rope_rows) * 64;
+      c = reinterpret_cast<const float2*>(cos_t + tr)[lane];
+      s = reinterpret_cast<const float2*>(sin_t + tr)[lane];
+    }
+#pragma unroll
+    for (int j = 0; j < QP_HEADS; ++j) {
+      const int h = h0 + j;
+      if (h >= heads) break;
+      const int which = h < Hq ? 0 : h < Hq + Hkv ? 1 : 2;
+      QkvLane out = grad[j];
+      if (which < 2) {
+        float ga0 = bf16lo(out.lo), ga1 = bf16hi(out.lo), gb0 = bf16lo(out.hi), gb1 = bf16hi(out.hi);
+        if (cos_t) {  // transpose of the rotation
+          const float t0 = ga0 * c.x + gb0 * s.x, t1 = ga1 * c.y + gb1 * s.y;
+          const float u0 = gb0 * c.x - ga0 * s.x, u1 = gb1 * c.y - ga1 * s.y;
+          ga0 = t0; ga1 = t1; gb0 = u0; gb1 = u1;
+        }
+        if (which == 0 ? gamma_q != nullptr : gamma_k != nullptr) {
+          const float x0 = bf16lo(in[j].lo), x1 = bf16hi(in[j].lo), x2 = bf16lo(in[j].hi), x3 = bf16hi(in[j].hi);
+          const float ss = bw_warp_sum(x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3);
+          const float rinv = rsqrtf(ss * (1.f / 128.f) + eps);
+          const float n0 = x0 * rinv, n1 = x1 * rinv, n2 = x2 * rinv, n3 = x3 * rinv;
+          const float d0 = ga0 * n0, d1 = ga1 * n1, d2 = gb0 * n2, d3 = gb1 * n3;
+          if (which == 0) {
+            sq[0] += d0; sq[1] += d1; sq[2] += d2; sq[3] += d3;
+          } else {
+            sk[0] += d0; sk[1] += d1; sk[2] += d2; sk[3] += d3;
+          }
+          const float w0 = ga0 * (which == 0 ? gq[0] : gk[0]), w1 = ga1 * (which == 0 ? gq[1] : gk[1]);
+          const float w2 = gb0 * (which == 0 ? gq[2] : gk[2]);
+          const float w3 = gb1 * (which == 0 ? gq[3] : gk[3]);
+          const float m = bw_warp_sum(w0 * n0 + w1 * n1 + w2 * n2 + w3 * n3) * (1.f / 128.f);
+          ga0 = rinv * (w0 - n0 * m); ga1 = rinv * (w1 - n1 * m);
+          gb0 = rinv * (w2 - n2 * m); gb1 = rinv * (w3 - n3 * m);
+        }
+        out.lo = pack_bf16(ga0, ga1);
+        out.hi = pack_bf16(gb0, gb1);
+      }
+      out.store(d_qkv + (row * heads + h) * 128, lane);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    acc[warp][0][(e >> 1) * 64 + 2 * lane + (e & 1)] = sq[e];
+    acc[warp][1][(e >> 1) * 64 + 2 * lane + (e & 1)] = sk[e];
   }
   __syncthreads();
-  if (part && threadIdx.x < 256)
-    part[(long long)blockIdx.x * 256 + threadIdx.x] = acc[threadIdx.x >> 7][threadIdx.x & 127];
+  if (part) {
+    float t = 0.f;
+    for (int i = 0; i < 8; ++i) t += acc[i][threadIdx.x >> 7][threadIdx.x & 127];
+    part[(long long)blockIdx.x * 256 + threadIdx.x] = t;
+  }
 }
 
 }  // namespace cb
@@ -376,11 +440,12 @@ void rmsnorm_bwd(const void* x, const void* dy, const void* gamma, const void* s
                  int rows_per_batch, long long mod_stride, float eps, void* dx, float* rinv, float* part,
                  cudaStream_t s) {
   check_d8(d, "rmsnorm_bwd");
-  if (d > 8 * cb::NB_THREADS * cb::NB_MAXJ) throw std::runtime_error("rmsnorm_bwd: row length above 8192 is not supported");
+  if (d > 8 * cb::NB_THREADS * 4) throw std::runtime_error("rmsnorm_bwd: row length above 8192 is not supported");
   if (rows <= 0) return;
   if (rows_per_batch <= 0 || rows % rows_per_batch != 0) throw std::runtime_error("rmsnorm_bwd: rows must be a multiple of rows_per_batch");
   const int grid = (int)std::min<long long>(rows, 148 * 8);
-  cb::rmsnorm_bwd_rows_kernel<<<grid, cb::NB_THREADS, 0, s>>>((const bf16*)x, (const bf16*)dy, (const bf16*)gamma,
+  const auto rows_kernel = d <= 8 * cb::NB_THREADS * 2 ? cb::rmsnorm_bwd_rows_kernel<2> : cb::rmsnorm_bwd_rows_kernel<4>;
+  rows_kernel<<<grid, cb::NB_THREADS, 0, s>>>((const bf16*)x, (const bf16*)dy, (const bf16*)gamma,
                                                              (const bf16*)scale, rows, d, rows_per_batch, mod_stride,
                                                              eps, (bf16*)dx, rinv);
   if (part) {
@@ -415,9 +480,9 @@ void swiglu_bwd(const void* gate_up, const void* dy, void* d_gate_up, long long 
 void qkv_post_fwd(const void* qkv, long long rows, int Hq, int Hkv, const float* cos_t, const float* sin_t,
                   int rope_rows, const void* gamma_q, const void* gamma_k, float eps, void* q, void* k, void* v,
                   cudaStream_t s) {
-  const long long warps = rows * (Hq + 2 * Hkv);
+  const long long warps = rows * ((Hq + 2 * Hkv + cb::QP_HEADS - 1) / cb::QP_HEADS);
   if (warps <= 0) return;
-  cb::qkv_post_fwd_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(
+  cb::qkv_post_fwd_kernel<<<(unsigned)std::min<long long>((warps + 7) / 8, 148 * 16), 256, 0, s>>>(
       (const bf16*)qkv, rows, Hq, Hkv, cos_t, sin_t, rope_rows > 0 ? rope_rows : 1, (const bf16*)gamma_q,
       (const bf16*)gamma_k, eps, (bf16*)q, (bf16*)k, (bf16*)v);
 }
@@ -430,7 +495,7 @@ void attn_bwd_delta(const void* dO, const void* O, float* delta, int B, int Sq, 
 }
 
 int qkv_post_bwd_blocks(long long rows, int Hq, int Hkv) {
-  const long long warps = rows * (Hq + 2 * Hkv);
+  const long long warps = rows * ((Hq + 2 * Hkv + cb::QP_HEADS - 1) / cb::QP_HEADS);
   return (int)std::max<long long>(1, std::min<long long>((warps + 7) / 8, 148 * 8));
 }
 

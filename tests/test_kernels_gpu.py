@@ -638,6 +638,28 @@ def test_qkv_post_autograd_on_own_kernels():
     ops.check_status()
 
 
+@pytest.mark.parametrize("rows,hq,hk", [(1, 1, 1), (9, 3, 1), (70, 5, 2), (1300, 7, 1)])
+def test_qkv_post_head_counts(rows, hq, hk):
+    """Heads that do not fill the last group of four, of one head and of several rows a warp. The norm weights' gradient comes out
+    the same every time."""
+    kern = torch.ops.cosmos_b200
+    torch.manual_seed(rows)
+    qkv, go = _rand(rows, hq + 2 * hk, 128), [_rand(rows, h, 128) for h in (hq, hk, hk)]
+    ang = torch.rand(rows, 64, device=DEV) * 6.0
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    gq, gk = ((1 + 0.1 * torch.randn(128, device=DEV)).bfloat16() for _ in range(2))
+    out = kern.qkv_post_fwd(qkv, hq, cos, sin, gq, gk, 1e-6)
+    f, gqf, gkf = (t.float().requires_grad_(True) for t in (qkv, gq, gk))
+    want = ref.mrope(f[:, :hq], cos, sin, gqf, 1e-6), ref.mrope(f[:, hq:hq + hk], cos, sin, gkf, 1e-6), f[:, hq + hk:]
+    torch.autograd.backward(want, [t.float() for t in go])
+    for x, y in zip(out, want):
+        assert ((x.float() - y).abs() <= 2 ** -8 * y.abs() + 1e-5).all()       # one rounding to bf16
+    d, part = kern.qkv_post_bwd(qkv, *go, cos, sin, gq, gk, 1e-6)
+    assert ((d.float() - f.grad).abs() <= 2 ** -8 * f.grad.abs() + 1e-5).all()
+    assert (part.sum(0)[0] - gqf.grad).abs().max() <= 1e-5 * rows * hq and (part.sum(0)[1] - gkf.grad).abs().max() <= 1e-5 * rows * hk
+    assert torch.equal(part, kern.qkv_post_bwd(qkv, *go, cos, sin, gq, gk, 1e-6)[1])
+
+
 def test_swiglu_and_gated_residual_autograd_on_own_kernels():
     from cosmos_b200.ops import autograd as own
     torch.manual_seed(33)
