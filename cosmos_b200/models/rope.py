@@ -77,11 +77,9 @@ def generator_positions(n_text: int, grid: Tuple[int, int, int], n_sound: int = 
     t, h, w = grid
     p_vid = grid_positions(t, h, w, start, device)
     out["text"], out["video"] = p_text, p_vid
-    after = next_start(p_vid) if p_vid.numel() else start
     if n_control:
-        p_ctl = grid_positions(t, h, w, start if share_temporal_with is not None else after, device)
-        out["control"] = p_ctl
-        after = max(after, next_start(p_ctl))
+        after = next_start(p_vid) if p_vid.numel() else start   # reads the ids back from the device
+        out["control"] = grid_positions(t, h, w, start if share_temporal_with is not None else after, device)
     if n_sound:
         ts = torch.linspace(0, max(t - 1, 0), n_sound, device=device).round().long() + start
         out["sound"] = torch.stack([ts, torch.full_like(ts, start), torch.full_like(ts, start)])

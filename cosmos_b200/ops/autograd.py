@@ -113,8 +113,12 @@ def attention(q, k, v, scale: Optional[float] = None, mask: int = MASK_FULL, n_a
 def _sum_to(t: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
     """Per-batch sums [B, d] -> the shape of the input they belong to ([B, d], [1, d] or [d])."""
     if like.numel() == t.shape[-1]:
-        t = t.sum(0)
+        t = _over_batch(t)
     return t.reshape(like.shape).to(like.dtype)
+
+
+def _over_batch(t: torch.Tensor) -> torch.Tensor:
+    return t[0] if t.shape[0] == 1 else t.sum(0)   # one entry needs no launch
 
 
 class AdaLNRMSNormFn(torch.autograd.Function):
@@ -133,7 +137,9 @@ class AdaLNRMSNormFn(torch.autograd.Function):
         x, gamma, shift, scale = ctx.saved_tensors
         dx, part = _k().rmsnorm_bwd(x, dy.contiguous(), gamma, scale, ctx.rpb, ctx.eps, True)
         sums = part.sum(1)  # [B, 3, d]
-        dgamma = sums[:, 2].sum(0).to(gamma.dtype) if (gamma is not None and ctx.needs_input_grad[1]) else None
+        if sums.shape[0] == 1 and scale.dtype == shift.dtype == x.dtype and (gamma is None or gamma.dtype == x.dtype):
+            sums = sums.to(x.dtype)   # one cast for the three
+        dgamma = _over_batch(sums[:, 2]).to(gamma.dtype) if (gamma is not None and ctx.needs_input_grad[1]) else None
         dshift = _sum_to(sums[:, 0], shift) if ctx.needs_input_grad[2] else None
         dscale = _sum_to(sums[:, 1], scale) if ctx.needs_input_grad[3] else None
         return dx, dgamma, dshift, dscale, None, None
@@ -187,6 +193,8 @@ class QKVPostFn(torch.autograd.Function):
         dv = z(hk) if dv is None else dv.contiguous()
         d_qkv, part = _k().qkv_post_bwd(qkv, dq, dk, dv, cos, sin, gq, gk, ctx.eps)
         sums = part.sum(0)
+        if gq is not None and gk is not None and gq.dtype == gk.dtype:
+            sums = sums.to(gq.dtype)   # one cast for both
         dgq = sums[0].to(gq.dtype) if (gq is not None and ctx.needs_input_grad[4]) else None
         dgk = sums[1].to(gk.dtype) if (gk is not None and ctx.needs_input_grad[5]) else None
         return d_qkv, None, None, None, dgq, dgk, None
