@@ -251,7 +251,9 @@ class TPDecoder(StepDecoder):
         """Consumes self.tokens / self.lens (device), writes self.next_tokens and advances lens."""
         b = self.tokens.shape[0]
         # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
-        if self.embed.is_cuda and self.embed.dtype == torch.bfloat16 and ops.get_backend() != "library" and self.cfg.d_model % 8 == 0:
+        e = self.embed   # rows that 16-byte accesses take
+        if e.is_cuda and e.dtype == torch.bfloat16 and ops.get_backend() != "library" and e.stride(1) == 1 \
+                and e.shape[1] % 8 == 0 and e.stride(0) % 8 == 0 and e.data_ptr() % 16 == 0:
             x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
                                                                     self.page_size, self.tokens, self.embed)
         else:
