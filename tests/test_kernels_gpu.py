@@ -576,6 +576,44 @@ def test_greedy_pick(b, v, stride):
     assert torch.equal(nxt, (x.float().max(dim=-1)[1] + 3).clamp(max=5))
 
 
+def test_early_launches_under_capture():
+    """Kernels that start behind the end of the one before them, as nodes of a graph: behind a copy, behind a kernel of torch, as the first
+    node of a joined side stream and behind one another. Each replay sees what that replay's kernels wrote."""
+    x, w1, w2, gam = _rand(300, 1024), _rand(1024, 1024) * 0.05, _rand(1024, 1024) * 0.05, _rand(1024)
+    src = _rand(300, 1024)
+
+    def work(side):
+        x.copy_(src)                                           # a copy, then a norm
+        h, _ = ops.rmsnorm(x, gam, 1e-6)
+        a = ops.gemm(h, w1)                                    # on CTA pairs
+        y = ops.gemm(a, w2, None, ops.EPI_GATED_RESID, x, None, 300)
+        cur = torch.cuda.current_stream()
+        side.wait_stream(cur)
+        with torch.cuda.stream(side):
+            z = ops.gemm(y[:16], w1)                           # single CTAs, split-K, first on its stream
+        cur.wait_stream(side)
+        q = ops.gemm(y, w1).view(1, 300, 8, 128)
+        o, _ = ops.attention(q, q[:, :, :2], q[:, :, 2:4])
+        return ops.rmsnorm((o.view(300, 1024) @ w2.t()) * 2, gam, 1e-6)[0], z
+
+    side, cap = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(cap):
+        work(side)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=cap):
+            out = work(side)
+    for seed in range(3):
+        torch.manual_seed(seed)
+        src.copy_(torch.randn(300, 1024, device=DEV))
+        g.replay()
+        got = [t.clone() for t in out]
+        want = work(side)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    ops.check_status()
+
+
 def _grads_close(own_in, ref_in, names, atol=4e-2, rtol=4e-2):
     for a, b, n in zip(own_in, ref_in, names):
         assert a.grad is not None, f"no gradient for {n}"
