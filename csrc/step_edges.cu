@@ -11,7 +11,7 @@ namespace cb {
 
 // cos, sin [S, half] of pos[axis(i)][s] * theta^(-2 i / head_dim), the angle in fp64 as the positions of long videos need. Axis of
 // frequency i: T, H, W, T, H, W, ... while H (below h3) and W (below w3) last, then T. The frequencies are worked out once
-// per block, before the positions are waited for. Prefill of 333 tokens: 14 kernels, about 45 us, are one of 4.
+// per block, before the positions are waited for. It was 14 kernels of 1 - 4 us; with it a prefill of 333 tokens takes 1066 us, without 1134.
 constexpr int ROPE_HALF_MAX = 256;
 
 __global__ void __launch_bounds__(256)
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeB
 }
 
 // next[b] = the smallest index of the row's largest logit (NaN counts as the largest), plus `first`, at most `limit`. A cluster of eight
-// blocks per row: one block alone takes 11 us for 152 k logits.
+// blocks per row, so that one sequence's 152 k logits are read by eight SMs.
 struct Best {
   float v;
   int i;
