@@ -35,9 +35,11 @@ rope_tables_kernel(const long long* __restrict__ pos, int S, int half, double th
 
 // One block per sequence: rotary tables of its position, the cache slot of the new token, its embedding, and the length moved on.
 // Ids are compared with their limits before they become addresses; a bad one is reported and row 0 stands in for it.
+// The kernels behind may start only once this one's wait is over: the layers' GEMMs request weights ahead of their own waits, so
+// everything that ran before the step (which may have written these weights) must be complete when the first of them starts.
 __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeBeginArgs a) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const int b = blockIdx.x, tid = threadIdx.x;
   const long long pos = a.lens[b];
   const float rpos = (float)(a.pos_delta ? pos + a.pos_delta[b] : pos);
