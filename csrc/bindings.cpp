@@ -565,7 +565,9 @@ std::tuple<Tensor, Tensor> dm_modulation_bwd(const c10::List<c10::optional<Tenso
     keep[i] = aligned_rows(*t);
     g[i] = keep[i].data_ptr();
   }
-  Tensor dt = at::empty({B, 6 * d}, like.options()), dtable = at::empty({6, d}, like.options());
+  Tensor dt = at::empty({B, 6 * d}, like.options());
+  if (B == 0) return {dt, at::zeros({6, d}, like.options())};   // the sum over no entries
+  Tensor dtable = at::empty({6, d}, like.options());
   cosmos::dm_modulation_bwd(g, dt.data_ptr(), dtable.data_ptr(), (int)B, (int)d, cur_stream());
   return {dt, dtable};
 }

@@ -513,6 +513,21 @@ def test_dm_modulation(b, d, unused):
     assert ((tab1.grad - tab2.grad).abs() <= 2 ** -7 * tab2.grad.abs()).all()
 
 
+def test_dm_modulation_of_an_empty_batch():
+    """The table's gradient is the sum over no entries. Deterministic algorithms fill new memory with NaN, so that a result that
+    nobody wrote shows."""
+    from cosmos_b200.models.mot import dm_modulation
+    t, tab = torch.empty(0, 6 * 64, device=DEV, dtype=torch.bfloat16).requires_grad_(True), _rand(6, 64).requires_grad_(True)
+    rows = dm_modulation(t, tab)
+    assert all(r.shape == (0, 64) for r in rows)
+    torch.use_deterministic_algorithms(True)
+    try:
+        torch.autograd.backward(rows, [torch.empty_like(r) for r in rows])
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert t.grad.shape == t.shape and tab.grad.shape == tab.shape and not tab.grad.any()
+
+
 @pytest.mark.parametrize("b,one,n,rows,h", [(1, False, 1, 3, 2), (2, True, 77, 317, 8), (3, False, 5, 5, 1), (2, False, 0, 4, 2)])
 @pytest.mark.parametrize("form", ["contiguous", "view of a projection", "odd start"])
 def test_copy_prefix(b, one, n, rows, h, form):
