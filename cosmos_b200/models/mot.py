@@ -247,8 +247,9 @@ def dm_modulation(t_mod: torch.Tensor, mod_table: torch.Tensor) -> List[torch.Te
     -> six [B, d] tensors: shift1, scale1, gate1, shift2, scale2, gate2."""
     b = t_mod.shape[0]
     d = mod_table.shape[-1]
-    if t_mod.dtype == mod_table.dtype and d % 8 == 0 and t_mod.dim() == 2 and mod_table.dim() == 2:
-        # one kernel forward and one backward, with the roundings of the expressions below
+    if (t_mod.dtype == mod_table.dtype and t_mod.device == mod_table.device and d % 8 == 0 and d > 0 and t_mod.dim() == 2
+            and mod_table.shape == (6, d) and b <= 65535 and ops._plain(t_mod, mod_table)):
+        # one kernel forward and one backward, with the roundings of the expressions below, which take every other form
         if ops._use_cuda(t_mod, mod_table):
             return list(torch.ops.cosmos_b200.dm_modulation(t_mod, mod_table).unbind(0))
         if ops._train_cuda(t_mod, mod_table):

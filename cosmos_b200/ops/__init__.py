@@ -14,6 +14,8 @@ from pathlib import Path
 from typing import Optional, Tuple
 
 import torch
+from torch.autograd import forward_ad
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from . import reference as ref
 from .reference import (EPI_GATED_RESID, EPI_PLAIN, EPI_QKV_ROPE, EPI_SWIGLU, MASK_CAUSAL, MASK_FULL,
@@ -100,6 +102,14 @@ def _train_cuda(t: torch.Tensor, *others) -> bool:
             "cosmos_b200 kernel library is not available on this GPU host "
             f"({_load_error}); run `python -m cosmos_b200.ops._build`")
     return True
+
+
+def _plain(*tensors) -> bool:
+    """True when nothing looks through the operations on these tensors: no forward-mode level, functorch transform, tracing,
+    compilation or dispatch mode, and no tensor subclass. The kernels' ops are opaque to those; expressions are not."""
+    return (not torch.compiler.is_compiling() and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
+            and forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and torch._C._get_tracing_state() is None and _get_current_dispatch_mode() is None)
 
 
 class _Counted:

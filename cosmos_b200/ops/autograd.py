@@ -201,15 +201,18 @@ class QKVPostFn(torch.autograd.Function):
 
 
 class ModulationFn(torch.autograd.Function):
-    """t_mod [B, 6d] + table [6, d] -> six [B, d] tensors."""
+    """t_mod [B, 6d] + table [6, d] -> six [B, d] tensors (of one storage, but no views of another: they can be changed in place)."""
 
     @staticmethod
     def forward(ctx, t_mod, table):
         ctx.like, ctx.shape = table.new_empty(0), (t_mod.shape[0], table.shape[1])
-        return _k().dm_modulation(t_mod, table).unbind(0)
+        return tuple(_k().dm_modulation_rows(t_mod, table))
 
     @staticmethod
     def backward(ctx, *grads):
+        if torch.is_grad_enabled():   # a graph of this backward is wanted
+            g = torch.stack(grads, dim=1)
+            return g.reshape(g.shape[0], -1), g.float().sum(0).to(g.dtype)
         return _k().dm_modulation_bwd(list(grads), ctx.like, *ctx.shape)
 
 

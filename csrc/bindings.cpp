@@ -544,10 +544,20 @@ Tensor dm_modulation(const Tensor& t_mod, const Tensor& table) {
   check_bf16_cuda(t_mod, "t_mod"); check_bf16_cuda(table, "table");
   c10::cuda::CUDAGuard guard(t_mod.device());
   TORCH_CHECK(t_mod.dim() == 2 && table.dim() == 2 && table.size(0) == 6 && t_mod.size(1) == 6 * table.size(1), "t_mod [B, 6d] and table [6, d] expected");
+  TORCH_CHECK(t_mod.device() == table.device(), "t_mod and table must be on one device");
   const Tensor tm = aligned_rows(t_mod), tb = aligned_rows(table);
   Tensor out = at::empty({6, t_mod.size(0), table.size(1)}, t_mod.options());
   cosmos::dm_modulation(tm.data_ptr(), tb.data_ptr(), out.data_ptr(), (int)t_mod.size(0), (int)table.size(1), cur_stream());
   return out;
+}
+
+// The same as six tensors [B, d] that share a storage and are no views
+std::vector<Tensor> dm_modulation_rows(const Tensor& t_mod, const Tensor& table) {
+  const Tensor all = dm_modulation(t_mod, table);
+  const int64_t B = all.size(1), d = all.size(2);
+  std::vector<Tensor> rows;
+  for (int64_t i = 0; i < 6; ++i) rows.push_back(at::empty({0}, all.options()).set_(all.storage(), i * B * d, {B, d}, {d, 1}));
+  return rows;
 }
 
 // Gradients of the six rows ([B, d], or none) -> those of t_mod [B, 6d] and of the table [6, d]
@@ -1612,6 +1622,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_bwd_delta", &attn_bwd_delta);
   m.def("dm_modulation", &dm_modulation);
+  m.def("dm_modulation_rows", &dm_modulation_rows);
   m.def("rope_tables", &make_rope_tables);
   m.def("decode_begin", &decode_begin);
   m.def("greedy_pick", &greedy_pick);

@@ -528,6 +528,54 @@ def test_dm_modulation_of_an_empty_batch():
     assert t.grad.shape == t.shape and tab.grad.shape == tab.shape and not tab.grad.any()
 
 
+def _modulation_expressions(t, tab):
+    b, d = t.shape[0], tab.shape[-1]
+    m = (t.view(b, 6, d).float() + tab.float()[None]).to(t.dtype)
+    return [m[:, i].contiguous() for i in range(6)]
+
+
+@pytest.mark.parametrize("b", [1, 3])
+def test_dm_modulation_under_transforms(b):
+    """What looks through the operations sees the expressions: forward mode, functorch, fake tensors, a second derivative."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.autograd import forward_ad as fw
+    from cosmos_b200.models.mot import dm_modulation
+    t, tab, dt, dtab = _rand(b, 6 * 16), _rand(6, 16), _rand(b, 6 * 16), _rand(6, 16)
+    with fw.dual_level():
+        got = [fw.unpack_dual(x).tangent for x in dm_modulation(fw.make_dual(t, dt), fw.make_dual(tab, dtab))]
+    assert all(torch.equal(x, y) for x, y in zip(got, _modulation_expressions(dt, dtab)))
+    vm = torch.func.vmap(lambda x: tuple(dm_modulation(x, tab)))(torch.stack([t, dt]))
+    assert all(torch.equal(x[1], y) for x, y in zip(vm, _modulation_expressions(dt, tab)))
+    want = torch.func.vjp(lambda x, y: torch.stack(_modulation_expressions(x, y)), t, tab)[1](_rand(6, b, 16).fill_(0.5))
+    got = torch.func.vjp(lambda x, y: torch.stack(dm_modulation(x, y)), t, tab)[1](_rand(6, b, 16).fill_(0.5))
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+    with FakeTensorMode():
+        rows = dm_modulation(torch.empty(b, 96, device=DEV, dtype=torch.bfloat16), torch.empty(6, 16, device=DEV, dtype=torch.bfloat16))
+        assert all(r.shape == (b, 16) for r in rows)
+    second = []
+    for f in (dm_modulation, _modulation_expressions):
+        p, q = t.clone().requires_grad_(True), tab.clone().requires_grad_(True)
+        first = torch.autograd.grad(sum((r * r).sum() for r in f(p, q)), (p, q), create_graph=True)
+        second.append(first + torch.autograd.grad(sum((x * x).sum() for x in first), (p, q)))
+    assert all(torch.equal(x, y) for x, y in zip(*second))
+
+
+def test_dm_modulation_of_other_forms():
+    from cosmos_b200.models.mot import dm_modulation
+    t, one = _rand(2, 6 * 16), _rand(1, 16)
+    assert all(torch.equal(x, y) for x, y in zip(dm_modulation(t, one), _modulation_expressions(t, one)))   # one row for all six
+    with pytest.raises(RuntimeError):
+        dm_modulation(t, _rand(6, 16).cpu())
+    assert all(r.shape == (2, 0) for r in dm_modulation(_rand(2, 0), _rand(6, 0)))
+    p, q = t.clone().requires_grad_(True), _rand(6, 16).requires_grad_(True)
+    rows = dm_modulation(p, q)
+    rows[1].mul_(3)                       # rows of their own: the others do not see it
+    torch.stack(rows).sum().backward()
+    want = torch.ones(2, 6, 16, device=DEV)
+    want[:, 1] = 3
+    assert torch.equal(p.grad.float(), want.view(2, 96)) and torch.equal(q.grad.float(), want.sum(0))
+
+
 @pytest.mark.parametrize("b,one,n,rows,h", [(1, False, 1, 3, 2), (2, True, 77, 317, 8), (3, False, 5, 5, 1), (2, False, 0, 4, 2)])
 @pytest.mark.parametrize("form", ["contiguous", "view of a projection", "odd start"])
 def test_copy_prefix(b, one, n, rows, h, form):
