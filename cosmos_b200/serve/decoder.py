@@ -57,7 +57,9 @@ class StepDecoder:
         if self.sampling is not None:
             self._sample(logits)                     # global ids across the vocab shards, into self.next_tokens
             return
-        if self.tp == 1 and logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and ops.get_backend() != "library":
+        nxt = self.next_tokens
+        if (self.tp == 1 and ops._use_cuda(logits) and logits.dim() == 2 and logits.stride(1) == 1 and 0 < logits.shape[1] and b <= 65535
+                and nxt.dtype == torch.long and nxt.device == logits.device and nxt.shape == (logits.shape[0],) and nxt.is_contiguous()):
             torch.ops.cosmos_b200.greedy_pick(logits, 0, self.cfg.vocab_size - 1, self.next_tokens)
             return
         val, idx = logits.float().max(dim=-1)
@@ -251,9 +253,7 @@ class TPDecoder(StepDecoder):
         """Consumes self.tokens / self.lens (device), writes self.next_tokens and advances lens."""
         b = self.tokens.shape[0]
         # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
-        e = self.embed   # rows that 16-byte accesses take
-        if e.is_cuda and e.dtype == torch.bfloat16 and ops.get_backend() != "library" and e.stride(1) == 1 \
-                and e.shape[1] % 8 == 0 and e.stride(0) % 8 == 0 and e.data_ptr() % 16 == 0:
+        if self._begins_on_kernel():
             x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
                                                                     self.page_size, self.tokens, self.embed)
         else:
@@ -261,7 +261,7 @@ class TPDecoder(StepDecoder):
         # Programmatic dependent launch for the layer kernels: each one's set-up, and the GEMMs' first weight tiles,
         # may overlap the tail of the kernel before it. Batch 1 over 1500 tokens, eight layers: 1080 -> 1050 us; batch 32 over 8448:
         # 2475 -> 2465. COSMOS_DECODE_PDL=0 turns it off.
-        pdl = self.device.type == "cuda" and ops.get_backend() != "library" and os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
+        pdl = ops._use_cuda(self.embed) and os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
         if pdl:
             torch.ops.cosmos_b200.set_pdl(True)
         try:
@@ -270,6 +270,22 @@ class TPDecoder(StepDecoder):
             if pdl:
                 torch.ops.cosmos_b200.set_pdl(False)
         self._finish_step(logits, b)
+
+    def _begins_on_kernel(self) -> bool:
+        """Whether `decode_begin` takes the state as it is: vectors of its integer types, and embeddings of whole 16-byte vectors. The
+        expressions of `_begin_step` take any."""
+        e, tab, b = self.embed, self.table, self.tokens.shape[0]
+        if not ops._use_cuda(e):
+            return False
+
+        def vector(t, dtype, n):
+            return t is None or (t.device == e.device and t.dtype == dtype and t.shape == (n,) and t.is_contiguous())
+
+        return (e.dim() == 2 and e.shape[0] > 0 and e.stride(1) == 1 and e.shape[1] % 8 == 0 and e.stride(0) % 8 == 0 and e.data_ptr() % 16 == 0
+                and vector(self.lens, torch.int32, b) and vector(self.tokens, torch.long, b) and vector(self.step_inc, torch.int32, b)
+                and vector(self.pos_delta, torch.long, b) and vector(self.inv_freq, torch.float32, self.inv_freq.numel())
+                and tab.device == e.device and tab.dtype == torch.int32 and tab.dim() == 2 and tab.shape[0] == b and tab.shape[1] > 0
+                and tab.stride(1) == 1)
 
     def _begin_step(self):
         """The embeddings, rotary tables and cache slots of the step's tokens, and the lengths moved on."""

@@ -49,3 +49,61 @@ def test_eager_step_behind_a_kernel_that_writes_a_weight(batch, d, inner):
         torch.cuda.synchronize()
         dec.step()
         assert torch.equal(got, dec.last_logits)
+
+
+def _logits_and_tokens(dec, steps=2):
+    out = []
+    for _ in range(steps):
+        dec.step()
+        out += [dec.last_logits.clone(), dec.next_tokens.clone().long(), dec.lens.clone().long()]
+    return out
+
+
+@pytest.mark.parametrize("name,dtype,forms", [
+    ("tokens", torch.int32, ("tokens",)), ("step_inc", torch.long, ()), ("pos_delta", torch.int32, ()), ("next_tokens", torch.int32, ("next_tokens",)),
+    ("step_inc", torch.int32, ("scalar",)), ("next_tokens", torch.long, ("strided",)), ("inv_freq", torch.float32, ("strided",))])
+def test_step_takes_its_state_in_other_forms(name, dtype, forms):
+    """State that the kernels at both ends of a step do not take: the same logits and tokens as with theirs."""
+    dec, same = _decoder(3), _decoder(3)
+    for d in (dec, same):
+        d.step_inc = torch.ones(3, dtype=torch.int32, device=DEV)
+        d.pos_delta = torch.tensor([0, -3, -40], device=DEV)
+    t = getattr(dec, name).to(dtype)
+    if "scalar" in forms:
+        t = t[0]
+    if "strided" in forms:
+        t = torch.stack([t, t], dim=-1)[..., 0]
+    setattr(dec, name, t)
+    for x, y in zip(_logits_and_tokens(dec), _logits_and_tokens(same)):
+        # the kernel's rotary tables may differ from torch's in the last bits, which bf16 sums over two layers hardly show
+        assert torch.equal(x, y) if x.dtype == torch.long else (x.float() - y.float()).norm() <= 1e-2 * y.float().norm()
+
+
+def test_first_own_op_of_a_program_is_a_step(monkeypatch):
+    """The step loads the kernel library itself: nothing before it may have."""
+    import cosmos_b200.serve.paged as paged
+    monkeypatch.setattr(paged.ops, "load_extension", lambda **kw: False)
+    dec = _decoder(1)
+    monkeypatch.undo()
+    calls = []
+    load = ops.load_extension
+    monkeypatch.setattr(ops, "load_extension", lambda *a, **kw: calls.append(1) or load(*a, **kw))
+    real = ops.rmsnorm
+    seen = []
+    monkeypatch.setattr(ops, "rmsnorm", lambda *a, **kw: seen.append(len(calls)) or real(*a, **kw))
+    dec.step()
+    assert seen and seen[0] > 0
+
+
+def test_step_in_fp32_needs_no_kernel_library(monkeypatch):
+    """A decoder of another type runs on the plain definitions, on a host without the library too."""
+    cfg = get_model_config("tiny128", n_layers=1)
+    dec = TPDecoder(cfg, 1, 0, None, DEV, page_size=16, max_batch=2, max_len=64, dtype=torch.float32)
+    assert all(dec.cache.reserve(i, 28) for i in range(2))
+    dec.table, dec.max_len = dec.cache.tables([0, 1])[0], 28
+    dec.lens, dec.tokens = torch.full((2,), 20, dtype=torch.int32, device=DEV), torch.tensor([5, 9], device=DEV)
+    dec.next_tokens = torch.zeros_like(dec.tokens)
+    switched = []
+    monkeypatch.setattr(torch.ops.cosmos_b200, "set_pdl", lambda on: switched.append(on))
+    dec.step()
+    assert not switched and dec.last_logits.isfinite().all()
