@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeB
     a.sin_t[(long long)b * a.half + i] = sinf(ang);
   }
   long long tok = a.tokens[b];
+  if (tok < 0) tok += a.vocab;   // as an index of torch: -1 is the last row
   if (tok < 0 || tok >= a.vocab) {
     if (tid == 0) atomicCAS(a.status, 0, ST_BAD_INDEX | (SITE_STACK_TOKEN << 8));
     tok = 0;

@@ -107,3 +107,10 @@ def test_step_in_fp32_needs_no_kernel_library(monkeypatch):
     monkeypatch.setattr(torch.ops.cosmos_b200, "set_pdl", lambda on: switched.append(on))
     dec.step()
     assert not switched and dec.last_logits.isfinite().all()
+
+
+def test_step_counts_negative_token_ids_from_the_end():
+    dec = _decoder(4)
+    dec.tokens = torch.tensor([-1, 0, -dec.cfg.vocab_size, 7], device=DEV)
+    x = torch.ops.cosmos_b200.decode_begin(dec.lens, None, None, dec.inv_freq, dec.table, dec.page_size, dec.tokens, dec.embed)[0]
+    assert torch.equal(x, dec.embed[dec.tokens])
