@@ -255,7 +255,7 @@ class TPDecoder(StepDecoder):
         # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
         if self._begins_on_kernel():
             x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
-                                                                    self.page_size, self.tokens, self.embed)
+                                                                    self.page_size, self.tokens, self.embed, self.cache.k[0].shape[0])
         else:
             x, cos, sin, slots = self._begin_step()
         # Programmatic dependent launch for the layer kernels: each one's set-up, and the GEMMs' first weight tiles,

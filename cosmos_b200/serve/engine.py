@@ -293,6 +293,8 @@ class BatchEngine:
             self._retire(r, "length")
 
     def _retire(self, r: Request, reason: str) -> None:
+        if self.device.type == "cuda":
+            ops.check_status()   # raises where a kernel reported a failure: nothing of this request is handed out then
         s = r.slot
         r.finish_reason, r.t_done = reason, time.time()
         self.dec.cache.release(r.rid)

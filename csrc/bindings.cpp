@@ -499,9 +499,11 @@ std::tuple<Tensor, Tensor> make_rope_tables(const Tensor& pos, int64_t head_dim,
   return {c, sn};
 }
 
-// What a decode step needs before its layers: (x [B, d], cos, sin [B, half], slots [B]); advances `lens`.
+// What a decode step needs before its layers: (x [B, d], cos, sin [B, half], slots [B]); advances `lens`. `num_pages`: of the cache,
+// 0 = the table's page ids have no upper limit.
 std::tuple<Tensor, Tensor, Tensor, Tensor> decode_begin(const Tensor& lens, const OptT& inc, const OptT& pos_delta, const Tensor& inv_freq,
-                                                        const Tensor& table, int64_t page_size, const Tensor& tokens, const Tensor& embed) {
+                                                        const Tensor& table, int64_t page_size, const Tensor& tokens, const Tensor& embed,
+                                                        int64_t num_pages) {
   check_bf16_cuda(embed, "embed");
   c10::cuda::CUDAGuard guard(embed.device());
   const int64_t B = lens.numel(), d = embed.size(1), half = inv_freq.numel();
@@ -524,6 +526,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> decode_begin(const Tensor& lens, cons
   a.status = status_tensor(embed.get_device()).data_ptr<int>();
   a.table_stride = table.stride(0); a.embed_stride = embed.stride(0);
   a.B = (int)B; a.half = (int)half; a.pages = (int)table.size(1); a.page_size = (int)page_size; a.d = (int)d; a.vocab = (int)embed.size(0);
+  a.num_pages = (int)num_pages;
   cosmos::decode_begin(a, cur_stream());
   return {x, c, sn, slots};
 }
@@ -1624,7 +1627,8 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("dm_modulation", &dm_modulation);
   m.def("dm_modulation_rows", &dm_modulation_rows);
   m.def("rope_tables", &make_rope_tables);
-  m.def("decode_begin", &decode_begin);
+  m.def("decode_begin(Tensor lens, Tensor? inc, Tensor? pos_delta, Tensor inv_freq, Tensor table, int page_size, Tensor tokens, Tensor embed, "
+        "int num_pages=0) -> (Tensor, Tensor, Tensor, Tensor)", &decode_begin);
   m.def("greedy_pick", &greedy_pick);
   m.def("dm_modulation_bwd", &dm_modulation_bwd);
   m.def("copy_prefix", &copy_prefix);

@@ -186,11 +186,12 @@ struct DecodeBeginArgs {
   const long long* tokens;      // [B]
   const void* embed;            // [vocab, d] bf16, row stride embed_stride
   float *cos_t, *sin_t;         // [B, half]
-  long long* slots;             // [B]
+  long long* slots;             // [B]; -1: the cache has no place for the token
   void* x;                      // [B, d] bf16
   int* status;
   long long table_stride, embed_stride;
   int B, half, pages, page_size, d, vocab;
+  int num_pages;                // of the cache; 0: not known
 };
 void decode_begin(const DecodeBeginArgs& a, cudaStream_t s);
 // next[b] = min(first + smallest index of the largest of logits[b][0 .. V), limit); bf16, row stride ld

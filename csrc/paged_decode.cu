@@ -392,7 +392,7 @@ decode_qkv_post_kernel(const bf16* __restrict__ qkv, int B, int Hq, int Hkv, con
     dst = q_out + ((long long)b * Hq + h) * 128;
   } else {
     const long long slot = slots[b];
-    if (!COSMOS_INDEX_OK(slot, SITE_DECODE_POST_SLOT)) return;  // whole warp: b and h are warp-uniform
+    if (!COSMOS_INDEX_OK(slot, SITE_DECODE_POST_SLOT) || slot < 0) return;  // no place (decode_begin); b and h are warp-uniform
     const long long page = slot / page_size;
     const int off = (int)(slot - page * page_size);
     const int hk = (h - Hq) % Hkv;

@@ -34,7 +34,9 @@ rope_tables_kernel(const long long* __restrict__ pos, int S, int half, double th
 }
 
 // One block per sequence: rotary tables of its position, the cache slot of the new token, its embedding, and the length moved on.
-// Ids are compared with their limits before they become addresses; a bad one is reported and row 0 stands in for it.
+// Ids are compared with their limits before they become addresses, and a bad one is reported. Row 0 stands in for a bad token. A
+// position past the table's row, and a page that is none of the cache's (unused entries are -1), give slot -1, for which the
+// layers store nothing, and the length stays where it is, inside the row, so that attention reads no further either.
 // The kernels behind may start only once this one's wait is over: the layers' GEMMs request weights ahead of their own waits, so
 // everything that ran before the step (which may have written these weights) must be complete when the first of them starts.
 __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeBeginArgs a) {
@@ -59,13 +61,15 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeB
   for (int i = tid; i < a.d / 8; i += 256) dst[i] = src[i];
   __syncthreads();   // everybody has read the length
   if (tid == 0) {
-    long long page = pos / a.page_size;
-    if (page < 0 || page >= a.pages) {
-      atomicCAS(a.status, 0, ST_BAD_INDEX | (SITE_DECODE_POST_SLOT << 8));
-      page = 0;
+    const long long room = (long long)a.pages * a.page_size;
+    long long slot = -1;
+    if (pos >= 0 && pos < room) {
+      const int page = a.table[b * a.table_stride + pos / a.page_size];
+      if (page >= 0 && (a.num_pages <= 0 || page < a.num_pages)) slot = (long long)page * a.page_size + pos % a.page_size;
     }
-    a.slots[b] = (long long)a.table[b * a.table_stride + page] * a.page_size + pos % a.page_size;
-    a.lens[b] = (int)pos + (a.inc ? a.inc[b] : 1);
+    if (slot < 0) atomicCAS(a.status, 0, ST_BAD_INDEX | (SITE_DECODE_POST_SLOT << 8));
+    a.slots[b] = slot;
+    a.lens[b] = (int)(slot < 0 ? min(max(pos, 0ll), room) : pos + (a.inc ? a.inc[b] : 1));
   }
 }
 

@@ -114,3 +114,62 @@ def test_step_counts_negative_token_ids_from_the_end():
     dec.tokens = torch.tensor([-1, 0, -dec.cfg.vocab_size, 7], device=DEV)
     x = torch.ops.cosmos_b200.decode_begin(dec.lens, None, None, dec.inv_freq, dec.table, dec.page_size, dec.tokens, dec.embed)[0]
     assert torch.equal(x, dec.embed[dec.tokens])
+
+
+@pytest.mark.parametrize("bad", ["length past the row", "far past it", "negative length", "unused entry", "page beyond the cache", "token"])
+def test_step_without_a_place_for_its_token_stores_nothing(bad):
+    """One sequence of three has a bad length, table entry or token. It is reported; its keys and values are not stored, the others' are;
+    the lengths stay inside the table."""
+    dec = _decoder(3)
+    room = dec.table.shape[1] * dec.page_size
+    lens = torch.tensor([40, 32, 47], dtype=torch.int32, device=DEV)   # the second one's next token begins a page
+    if bad == "unused entry":
+        dec.table[1, 32 // dec.page_size] = -1
+    elif bad == "page beyond the cache":
+        dec.table[1, 32 // dec.page_size] = dec.cache.k[0].shape[0]
+    elif bad == "token":
+        dec.tokens[1] = dec.cfg.vocab_size
+    else:
+        lens[1] = {"length past the row": room, "far past it": 2 ** 31 - 1, "negative length": -5}[bad]
+    dec.lens = lens.clone()
+    before = [(k.clone(), v.clone()) for k, v in zip(dec.cache.k, dec.cache.v)]
+    slots = torch.ops.cosmos_b200.decode_begin(lens.clone(), None, None, dec.inv_freq, dec.table, dec.page_size, dec.tokens, dec.embed,
+                                               dec.cache.k[0].shape[0])[3].tolist()
+    with pytest.raises(RuntimeError, match="index out of range at " + ("decoder stack token" if bad == "token" else "decode_qkv_post slot")):
+        ops.check_status()
+    assert [s < 0 for s in slots] == [False, bad != "token", False]
+    want = {"length past the row": room, "far past it": room, "negative length": 0, "token": 33}.get(bad, 32)
+    if bad in ("far past it", "negative length"):   # no state that a sequence gets into: up to the first layer's store
+        x, cos, sin, at = torch.ops.cosmos_b200.decode_begin(dec.lens, None, None, dec.inv_freq, dec.table, dec.page_size, dec.tokens,
+                                                             dec.embed, dec.cache.k[0].shape[0])
+        p = dec.layers[0]
+        ops.gemm_decode_qkv_post(x, p["wqkv"], dec.hq, cos, sin, p["q_norm"], p["k_norm"], 1e-6, at, dec.cache.k[0], dec.cache.v[0])
+    else:
+        dec.max_len = room
+        dec.step()
+    with pytest.raises(RuntimeError, match="index out of range"):
+        ops.check_status()
+    assert dec.lens.tolist() == [41, want, 48]
+    for li, pair in enumerate(before):
+        for old, new in zip(pair, (dec.cache.k[li], dec.cache.v[li])):
+            for s in slots:
+                if s >= 0:
+                    assert li > 0 or not torch.equal(old[s // 16, :, s % 16], new[s // 16, :, s % 16])
+                    old[s // 16, :, s % 16] = new[s // 16, :, s % 16]
+            assert torch.equal(old, new)
+
+
+def test_engine_hands_out_nothing_after_a_report():
+    """A request whose next page is taken away: the engine raises before the request is finished."""
+    from cosmos_b200.models.mot import MoTModel
+    from cosmos_b200.serve.engine import BatchEngine
+    cfg = get_model_config("tiny128", n_layers=1)
+    model = MoTModel(cfg, dtype=torch.bfloat16, device=DEV)
+    eng = BatchEngine(model, max_batch=2, max_len=64, page_size=16)
+    r = eng.submit(list(range(1, 16)), max_new_tokens=4)
+    eng.step()                                # the prompt and one token: a page is full
+    assert int(eng.dec.lens[r.slot]) == 16
+    eng.dec.table[r.slot, 1] = -1
+    with pytest.raises(RuntimeError, match="index out of range"):
+        eng.run_until_done()
+    assert r.rid not in eng.finished
