@@ -31,9 +31,11 @@ def rope_tables(pos: torch.Tensor, head_dim: int, theta: float, section: Sequenc
                 ) -> Tuple[torch.Tensor, torch.Tensor]:
     """pos [3, S] (t, h, w) -> cos, sin [S, head_dim/2] fp32 (rotate-half convention)."""
     half = head_dim // 2
-    if pos.is_cuda and pos.dtype == torch.long and pos.dim() == 2 and pos.shape[0] == 3 and head_dim <= 512 and ops.get_backend() != "library" and ops.load_extension():
-        assert sum(section) == half, f"mrope_section {section} must sum to {half}"
-        return torch.ops.cosmos_b200.rope_tables(pos, head_dim, float(theta), int(section[1]), int(section[2]))
+    st, sh, sw = section
+    if (pos.is_cuda and pos.dtype == torch.long and pos.dim() == 2 and pos.shape[0] == 3 and head_dim <= 512 and min(sh, sw) >= 0
+            and isinstance(theta, (int, float)) and ops._plain(pos) and ops.get_backend() != "library" and ops.load_extension()):
+        assert st + sh + sw == half, f"mrope_section {section} must sum to {half}"
+        return torch.ops.cosmos_b200.rope_tables(pos, head_dim, float(theta), int(sh), int(sw))
     inv_freq = 1.0 / (theta ** (torch.arange(0, half, dtype=torch.float64, device=pos.device) * 2.0 / head_dim))
     axis = axis_of_frequency(half, section, pos.device)   # filled on the device: a copy from the host would wait for the stream
     p = pos.to(torch.float64)[axis, :]            # [half, S]

@@ -488,7 +488,7 @@ Tensor aligned_rows(const Tensor& t) {   // contiguous, and 16-byte aligned: a v
 
 // cos, sin [S, half] of pos [3, S] (see rope.py)
 std::tuple<Tensor, Tensor> make_rope_tables(const Tensor& pos, int64_t head_dim, double theta, int64_t sh, int64_t sw) {
-  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.dim() == 2 && pos.size(0) == 3 && head_dim % 2 == 0 && head_dim <= 512,
+  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.dim() == 2 && pos.size(0) == 3 && head_dim >= 0 && head_dim <= 512,
               "rope_tables: int64 positions [3, S] on the GPU");
   c10::cuda::CUDAGuard guard(pos.device());
   const Tensor p = pos.contiguous();

@@ -606,6 +606,28 @@ def test_rope_tables(n, theta, section):
             assert (x.cpu() - y).abs().max() <= 2 ** -24
 
 
+@pytest.mark.parametrize("head_dim,section", [(129, (24, 20, 20)), (7, (3, 0, 0)), (6, (1, 1, 1)), (600, (100, 100, 100)), (1, (0, 0, 0))])
+def test_rope_tables_of_other_sizes(head_dim, section):
+    """Odd head sizes (half of them has a frequency), sizes above the kernel's, none at all: as the expressions on the CPU."""
+    from cosmos_b200.models import rope
+    pos = torch.arange(33).expand(3, -1)
+    for x, y in zip(rope.rope_tables(pos.cuda(), head_dim, 1.0e4, section), rope.rope_tables(pos, head_dim, 1.0e4, section)):
+        assert x.shape == y.shape and (x.cpu() - y).abs().le(2 ** -24).all()
+
+
+def test_rope_tables_other_forms():
+    from cosmos_b200.models import rope
+    pos = torch.arange(9, device=DEV).expand(3, -1)
+    want = rope.rope_tables(pos, 6, 1.0e4, (1, 1, 1))
+    got = torch.func.vmap(lambda p: rope.rope_tables(p, 6, 1.0e4, (1, 1, 1)))(torch.stack([pos, pos + 1]))
+    tensor = rope.rope_tables(pos, 6, torch.tensor(1.0e4, dtype=torch.float64, device=DEV), (1, 1, 1))
+    for x, y, z in zip(got, want, tensor):
+        assert (x[0] - y).abs().max() <= 2 ** -24 and (z - y).abs().max() <= 2 ** -24
+    for bad in ((3,), (1, 2), (1, 1, 1, 0)):    # three sections, whatever they add up to
+        with pytest.raises(ValueError):
+            rope.rope_tables(pos, 6, 1.0e4, bad)
+
+
 @pytest.mark.parametrize("b,d,page,delta,inc", [(1, 64, 16, False, False), (3, 4096, 32, True, True), (70, 1032, 16, True, False)])
 def test_decode_begin(b, d, page, delta, inc):
     from types import SimpleNamespace
