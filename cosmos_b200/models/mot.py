@@ -201,7 +201,9 @@ class WorkspaceAttn(AttnContext):
         n_pre = 0 if prefix is None else prefix[0].shape[1]
         qb, kb, vb, routes = self._buffers(b, s, n_pre, cfg, h)
         if prefix is not None:
-            if all(t.device == kb.device and t.dtype == kb.dtype and t.dim() == 4 for t in prefix):
+            # one launch for both; a prefix that is spread over the heads or cast stays with the copies
+            if ops._use_cuda(kb) and all(t.device == kb.device and t.dtype == kb.dtype and t.shape[:1] in ((1,), (b,))
+                                         and t.shape[1:] == (n_pre, *kb.shape[2:]) for t in prefix):
                 torch.ops.cosmos_b200.copy_prefix(prefix[0], prefix[1], kb, vb)
             else:
                 kb[:, :n_pre].copy_(prefix[0])

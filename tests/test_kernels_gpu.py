@@ -594,6 +594,24 @@ def test_copy_prefix(b, one, n, rows, h, form):
     assert torch.equal(kb, wk) and torch.equal(vb, wv)
 
 
+@pytest.mark.parametrize("form", ["one head", "fp32", "keys alone of one head"])
+def test_workspace_prefix_of_other_forms(form):
+    """Prefixes that the copies into the workspace spread over the heads or cast: the keys and values that `attend` gets."""
+    from cosmos_b200.config import get_model_config
+    from cosmos_b200.models.mot import WorkspaceAttn
+    cfg = get_model_config("tiny128")
+    b, s, n, hk, hd = 2, 5, 3, cfg.n_kv_heads, cfg.head_dim
+    h, w = _rand(b, s, cfg.d_model), _rand(cfg.q_dim + 2 * cfg.kv_dim, cfg.d_model, scale=0.05)
+    ang = torch.rand(s, 64, device=DEV)
+    norm = torch.ones(hd, device=DEV, dtype=torch.bfloat16)
+    wide, one = (_rand(b, n, hk, hd), _rand(b, n, hk, hd)), (_rand(b, n, 1, hd), _rand(b, n, 1, hd))
+    prefix = {"one head": one, "fp32": (wide[0].float(), wide[1].float()), "keys alone of one head": (one[0], wide[1])}[form]
+    with torch.no_grad():
+        _, k, v = WorkspaceAttn().qkv_project(h, w, ang.cos(), ang.sin(), norm, norm, cfg, prefix=prefix)
+    for got, p in ((k, prefix[0]), (v, prefix[1])):
+        assert got.shape == (b, n + s, hk, hd) and torch.equal(got[:, :n], p.bfloat16().expand(b, n, hk, hd))
+
+
 @pytest.mark.parametrize("n,theta,section", [(1, 5.0e5, (24, 20, 20)), (333, 1.0e4, (24, 20, 20)), (2001, 5.0e6, (10, 11, 11))])
 def test_rope_tables(n, theta, section):
     """The bits of the expressions in fp64, for positions up to a million and in any layout."""
