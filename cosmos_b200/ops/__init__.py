@@ -8,6 +8,7 @@ a CUDA bf16 tensor raises.
 """
 from __future__ import annotations
 
+import contextlib
 import math
 import os
 from pathlib import Path
@@ -110,6 +111,20 @@ def _plain(*tensors) -> bool:
     return (not torch.compiler.is_compiling() and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
             and forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
             and torch._C._get_tracing_state() is None and _get_current_dispatch_mode() is None)
+
+
+@contextlib.contextmanager
+def launch_overlap(level: int):
+    """What this thread's launches inside the block may overlap with the kernel before them: 0 nothing, 1 the kernels' set-up (the
+    default), 2 the first weight tiles of GEMMs as well, for the layers of a decode step (csrc/kernels.h)."""
+    if not _loaded:
+        yield
+        return
+    before = torch.ops.cosmos_b200.launch_overlap(level)
+    try:
+        yield
+    finally:
+        torch.ops.cosmos_b200.launch_overlap(before)
 
 
 class _Counted:

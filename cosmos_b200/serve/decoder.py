@@ -251,25 +251,22 @@ class TPDecoder(StepDecoder):
 
     def _step_impl(self) -> None:
         """Consumes self.tokens / self.lens (device), writes self.next_tokens and advances lens."""
-        b = self.tokens.shape[0]
-        # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
-        if self._begins_on_kernel():
-            x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
-                                                                    self.page_size, self.tokens, self.embed, self.cache.k[0].shape[0])
-        else:
-            x, cos, sin, slots = self._begin_step()
-        # Programmatic dependent launch for the layer kernels: each one's set-up, and the GEMMs' first weight tiles,
-        # may overlap the tail of the kernel before it. Batch 1 over 1500 tokens, eight layers: 1080 -> 1050 us; batch 32 over 8448:
-        # 2475 -> 2465. COSMOS_DECODE_PDL=0 turns it off.
-        pdl = ops._use_cuda(self.embed) and os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
-        if pdl:
-            torch.ops.cosmos_b200.set_pdl(True)
-        try:
-            logits = self._forward_layers(x, cos, sin, slots)
-        finally:
-            if pdl:
-                torch.ops.cosmos_b200.set_pdl(False)
-        self._finish_step(logits, b)
+        begins = self._begins_on_kernel()   # loads the library
+        # Programmatic dependent launch: the kernels' set-up, and around the layers the GEMMs' first weight tiles, may overlap the tail
+        # of the kernel before. Batch 1 over 1500 tokens, eight layers, set-up alone and both: 1080 -> 1050 us; batch 32 over 8448:
+        # 2475 -> 2465. At TP 2 and 4 both against none took 8.96 -> 8.77 and 5.80 -> 5.45 ms before norms and reductions
+        # were launched early. COSMOS_DECODE_PDL=0: nothing in the step overlaps.
+        overlap = os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
+        with ops.launch_overlap(1 if overlap else 0):
+            # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)
+            if begins:
+                x, cos, sin, slots = torch.ops.cosmos_b200.decode_begin(self.lens, self.step_inc, self.pos_delta, self.inv_freq, self.table,
+                                                                        self.page_size, self.tokens, self.embed, self.cache.k[0].shape[0])
+            else:
+                x, cos, sin, slots = self._begin_step()
+            with ops.launch_overlap(2 if overlap else 0):
+                logits = self._forward_layers(x, cos, sin, slots)
+            self._finish_step(logits, x.shape[0])
 
     def _begins_on_kernel(self) -> bool:
         """Whether `decode_begin` takes the state as it is: vectors of its integer types, and embeddings of whole 16-byte vectors. The

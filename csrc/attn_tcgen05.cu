@@ -600,7 +600,7 @@ static void launch_attn(int nc, dim3 grid, const CUtensorMap& tq, const cb::KVMa
   at[0].val.clusterDim.x = nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch.cuh
   at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = 2;
+  cfg.attrs = at; cfg.numAttrs = cosmos::early_on() ? 2 : 1;
   if (nc == 2) {
     static bool configured = false;
     if (!configured) {

@@ -1385,7 +1385,10 @@ Tensor silu_selftest(int64_t first, int64_t count, const Tensor& like) {
   cosmos::silu_selftest((uint32_t)first, count / 16, reinterpret_cast<unsigned long long*>(differ.data_ptr<int64_t>()), cur_stream());
   return differ;
 }
-void set_pdl(bool on) { cosmos::set_pdl(on); }
+int64_t launch_overlap(int64_t level) {
+  TORCH_CHECK(level >= 0 && level <= 2, "launch_overlap: level 0, 1 or 2");
+  return cosmos::set_launch_overlap((int)level);
+}
 void attn_set_cta_pair(bool on) { cosmos::attn_set_cta_pair(on); }
 void attn_set_exp_emulation(int64_t v) { attn_exp_emu() = (int)v; }
 void attn_set_debug(int64_t v) { attn_debug() = (int)v; }
@@ -1669,7 +1672,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("gemm_pick_tile", &gemm_pick_tile);
   m.def("gemm_set_debug", &gemm_set_debug);
   m.def("gemm_pick_k_splits", &gemm_pick_k_splits);
-  m.def("set_pdl", &set_pdl);
+  m.def("launch_overlap", &launch_overlap);
   m.def("sample_topk", &sample_topk);
   m.def("sample_pick_", &sample_pick_);
   m.def("attn_set_cta_pair", &attn_set_cta_pair);

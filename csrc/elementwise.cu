@@ -457,9 +457,14 @@ __global__ void __launch_bounds__(256) copy_prefix_kernel(const cosmos::PrefixAr
 
 namespace cosmos {
 
-static thread_local bool g_pdl = false;   // a GEMM of another thread may have a B that a kernel before it writes
-void set_pdl(bool on) { g_pdl = on; }
-bool pdl_on() { return g_pdl; }
+static thread_local int g_overlap = 1;   // a GEMM of another thread may have a B that a kernel before it writes
+int set_launch_overlap(int level) {
+  const int before = g_overlap;
+  g_overlap = level;
+  return before;
+}
+bool early_on() { return g_overlap >= 1; }
+bool pdl_on() { return g_overlap >= 2; }
 
 static void check_d(int d, const char* who) {
   if (d % 8 != 0 || d <= 0)

@@ -1217,7 +1217,7 @@ static void launch(const CUtensorMap* maps, const cb::GemmGroup& g, int units, i
   at[0].val.clusterDim.x = NC; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = g.p[0].tile_map ? 1 : 2;
+  cfg.attrs = at; cfg.numAttrs = g.p[0].tile_map || !early_on() ? 1 : 2;
   cudaLaunchKernelEx(&cfg, cb::gemm_bf16_kernel<EPI, NC, NW>, maps[0], maps[1], maps[2], maps[3], g);
 }
 

@@ -24,12 +24,14 @@ enum AttnMask : int {
 
 namespace cosmos {
 
-// Programmatic dependent launch. GEMMs, split-K reductions, row norms and attention over contiguous keys are always launched so
-// that their set-up overlaps the tail of the kernel before them. While this is on, the other kernels of a decode step (QKV
-// post-processing, paged attention and its merge, all-reduce + norm) are too, and GEMMs on single CTAs read their first weight
-// tiles ahead; the caller turns it on around a decode step (where the GEMMs' B operands are weights) and off afterwards.
-void set_pdl(bool on);   // for the calling thread
-bool pdl_on();
+// Programmatic dependent launch: what may overlap the tail of the kernel before it, for launches of the calling thread.
+// 0: nothing. 1 (as a thread begins): GEMMs, split-K reductions, row norms, attention over contiguous keys and the small kernels at
+// both ends of a step are launched so that their set-up does. 2: so are the other kernels of a decode step (QKV post-processing,
+// paged attention and its merge, all-reduce + norm), and GEMMs on single CTAs read their first weight tiles ahead; the caller sets
+// it around the layers of a decode step, where the GEMMs' B operands are weights. Returns the former level.
+int set_launch_overlap(int level);
+bool early_on();   // level >= 1
+bool pdl_on();     // level 2
 
 struct GemmArgs {
   const void* A = nullptr;  // [M, K] bf16, row stride lda

@@ -1,7 +1,7 @@
 // Kernel launches with the programmatic-serialization attribute: the kernel's blocks may start, and set themselves up, while the
 // kernel before it in the stream still runs. Only for kernels whose every thread executes `pdl_wait()` before it touches anything
-// that a predecessor wrote, or ends. `launch_early` always sets the attribute, for kernels that neither wait for a peer nor read
-// a weight before that point; `launch_pdl` while `cosmos::pdl_on()`.
+// that a predecessor wrote, or ends. `launch_early` sets the attribute while `cosmos::early_on()` (unless the caller wants no
+// overlap), for kernels that neither wait for a peer nor read a weight before that point; `launch_pdl` while `cosmos::pdl_on()`.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -34,7 +34,7 @@ inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 }
 template <typename... KArgs, typename... Args>
 inline void launch_early(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-  launch_with(true, kern, grid, block, smem, stream, args...);
+  launch_with(early_on(), kern, grid, block, smem, stream, args...);
 }
 
 }  // namespace cosmos

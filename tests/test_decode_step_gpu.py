@@ -103,10 +103,11 @@ def test_step_in_fp32_needs_no_kernel_library(monkeypatch):
     dec.table, dec.max_len = dec.cache.tables([0, 1])[0], 28
     dec.lens, dec.tokens = torch.full((2,), 20, dtype=torch.int32, device=DEV), torch.tensor([5, 9], device=DEV)
     dec.next_tokens = torch.zeros_like(dec.tokens)
-    switched = []
-    monkeypatch.setattr(torch.ops.cosmos_b200, "set_pdl", lambda on: switched.append(on))
+    monkeypatch.setattr(ops, "_loaded", False)
+    monkeypatch.setattr(ops, "load_extension", lambda *a, **kw: False)
+    monkeypatch.setattr(torch.ops, "cosmos_b200", None)
     dec.step()
-    assert not switched and dec.last_logits.isfinite().all()
+    assert dec.last_logits.isfinite().all()
 
 
 def test_step_counts_negative_token_ids_from_the_end():
@@ -173,3 +174,26 @@ def test_engine_hands_out_nothing_after_a_report():
     with pytest.raises(RuntimeError, match="index out of range"):
         eng.run_until_done()
     assert r.rid not in eng.finished
+
+
+@pytest.mark.parametrize("setting", ["0", "1"])
+def test_programmatic_edges_of_a_captured_step(setting, monkeypatch):
+    """COSMOS_DECODE_PDL=0 leaves no launch of the step, first and last kernel included, that may start before its predecessor ends.
+    The same logits with and without."""
+    from cuda.bindings import runtime
+    monkeypatch.setenv("COSMOS_DECODE_PDL", setting)
+    dec, same = _decoder(2), _decoder(2)
+    monkeypatch.setenv("COSMOS_DECODE_PDL", "1")
+    same.step()
+    monkeypatch.setenv("COSMOS_DECODE_PDL", setting)
+    dec.step()
+    assert torch.equal(dec.last_logits, same.last_logits)
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g), torch.no_grad():
+        dec._step_impl()
+    raw = runtime.cudaGraph_t(g.raw_cuda_graph())
+    n = runtime.cudaGraphGetEdges_v2(raw)[-1]
+    data = runtime.cudaGraphGetEdges_v2(raw, n)[3]
+    early = sum(d.type == int(runtime.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for d in data)
+    assert n > 15 and (early == 0 if setting == "0" else early > 15), (n, early)
+    assert torch.ops.cosmos_b200.launch_overlap(1) == 1    # the thread's own level again
