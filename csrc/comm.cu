@@ -356,13 +356,14 @@ __global__ void __launch_bounds__(256)
 allreduce_norm_kernel(const long long* bufs, const bf16* mc, bf16* own, const long long* pads, int rank, int world,
                       int slot, int* counters, const float* __restrict__ partial, int k_splits, int M, int N,
                       const bf16* __restrict__ R, const bf16* __restrict__ gamma, float eps, bf16* __restrict__ X,
-                      bf16* __restrict__ H, int* status) {
+                      bf16* __restrict__ H, int* status, int early) {
   __shared__ float red[8];
   __shared__ int e_s;
   const int tid = threadIdx.x;
   const int nvec = N >> 3;
   constexpr int MAXJ = 4;  // 256 threads x 4 vectors x 8 = 8192 columns
-  pdl_launch_dependents();
+  // `early`, set around the layers of a decode step: elsewhere no kernel takes SMs while this one still waits for its peers
+  if (early) pdl_launch_dependents();
   pdl_wait();
   if (partial) {
     for (int m = blockIdx.x; m < M; m += gridDim.x) {
@@ -572,11 +573,11 @@ void allreduce_norm(const long long* bufs_dev, const void* mc, void* own, const 
   if (mc)
     launch_pdl(cb::allreduce_norm_kernel<true>, dim3(blocks), dim3(256), 0, s, bufs_dev, (const bf16*)mc, (bf16*)own,
                pads_dev, rank, world, slot, counters, partial, k_splits, M, N, (const bf16*)R, (const bf16*)gamma, eps,
-               (bf16*)X, (bf16*)H, status);
+               (bf16*)X, (bf16*)H, status, pdl_on() ? 1 : 0);
   else
     launch_pdl(cb::allreduce_norm_kernel<false>, dim3(blocks), dim3(256), 0, s, bufs_dev, (const bf16*)nullptr,
                (bf16*)own, pads_dev, rank, world, slot, counters, partial, k_splits, M, N, (const bf16*)R,
-               (const bf16*)gamma, eps, (bf16*)X, (bf16*)H, status);
+               (const bf16*)gamma, eps, (bf16*)X, (bf16*)H, status, pdl_on() ? 1 : 0);
 }
 
 void sum_partials_gated_residual(const void* part, int n_part, long long rows, int d, const void* R, const void* gate,

@@ -44,3 +44,11 @@ def test_the_start_of_a_decode_step_is_a_full_dependency(name):
     complete, so the step's first kernel lets them start behind its wait."""
     body = KERNELS[name]
     assert body.index("pdl_wait()") < body.index("pdl_launch_dependents()")
+
+
+def test_kernels_that_wait_for_a_peer_trigger_on_request_only():
+    """Outside the layers of a decode step nothing starts behind a kernel that still waits for its peers."""
+    waiting = [name for name, body in KERNELS.items() if "barrier_device" in body and "pdl_launch_dependents" in body]
+    assert waiting == ["allreduce_norm_kernel"]
+    for name in waiting:
+        assert re.search(r"if \(early\) pdl_launch_dependents\(\);", KERNELS[name]) and KERNELS[name].count("pdl_launch_dependents") == 1
