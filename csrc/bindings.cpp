@@ -1385,6 +1385,14 @@ Tensor silu_selftest(int64_t first, int64_t count, const Tensor& like) {
   cosmos::silu_selftest((uint32_t)first, count / 16, reinterpret_cast<unsigned long long*>(differ.data_ptr<int64_t>()), cur_stream());
   return differ;
 }
+// The same for the silu of the convolutions: [results that differ in bf16, in fp32 (magnitudes below 80), largest distance there]
+Tensor conv_silu_selftest(int64_t first, int64_t count, const Tensor& like) {
+  TORCH_CHECK(like.is_cuda() && first >= 0 && count >= 0 && count % 16 == 0 && first + count <= (1ll << 32), "bad range of values");
+  c10::cuda::CUDAGuard guard(like.device());
+  Tensor differ = at::zeros({3}, like.options().dtype(at::kLong));
+  cosmos::conv_silu_selftest((uint32_t)first, count / 16, reinterpret_cast<unsigned long long*>(differ.data_ptr<int64_t>()), cur_stream());
+  return differ;
+}
 int64_t launch_overlap(int64_t level) {
   TORCH_CHECK(level >= 0 && level <= 2, "launch_overlap: level 0, 1 or 2");
   return cosmos::set_launch_overlap((int)level);
@@ -1680,6 +1688,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("attn_set_debug", &attn_set_debug);
   m.def("bounds_check_selftest", &bounds_check_selftest);
   m.def("silu_selftest", &silu_selftest);
+  m.def("conv_silu_selftest", &conv_silu_selftest);
   m.def("rs_adamw", &rs_adamw);
   m.def("grad_sq_list", &grad_sq_list);
   m.def("adamw_list", &adamw_list);

@@ -118,25 +118,28 @@ __device__ __forceinline__ void cv_swap_halves(const uint32_t (&pk)[8], int lane
   odd = o ? make_uint4(pk[4], pk[5], pk[6], pk[7]) : make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-// silu(z) = z / (1 + exp(-z)) of 16 values given as their negatives, rounded to bf16. The quotient is z times an approximate
-// reciprocal, refined once by its residual (of all 2^32 fp32 values, two then differ from the division's, in their last bit);
-// negatives of value and reciprocal let every step be a packed instruction. Beyond 80, where the exponential leaves its range,
-// and for infinities the division itself.
+// silu(z) = z / (1 + exp(-z)) of two values given as their negatives: z times an approximate reciprocal, with one step of iterative
+// refinement by the residual (silu16 in common.cuh takes two); negatives of value and reciprocal let every step be a packed
+// instruction. For magnitudes below 80. Of all 2^32 values two differ from the division's result, in their last bit, and none
+// once it is rounded to bf16 (conv_silu_selftest).
+__device__ __forceinline__ float2 cv_silu2(uint64_t zn) {
+  const float2 t = unpack2(mul2(zn, pack2(1.4426950408889634f, 1.4426950408889634f)));
+  const uint64_t den = add2(pack2(ex2(t.x), ex2(t.y)), pack2(1.f, 1.f));
+  const float2 d = unpack2(den);
+  float r0, r1;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d.y));
+  const uint64_t rn = pack2(r0, r1), q = mul2(zn, rn);
+  return unpack2(fma2(fma2(q, den, zn), rn, q));
+}
+// 16 of them rounded to bf16. Beyond 80, where the exponential leaves its range, and for infinities the division itself.
 __device__ __forceinline__ void cv_silu16(const uint64_t (&zn)[8], uint32_t (&out)[8]) {
-  const uint64_t log2e = pack2(1.4426950408889634f, 1.4426950408889634f), one = pack2(1.f, 1.f);
   float top = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const float2 z = unpack2(zn[k]);
     top = fmaxf(top, fmaxf(fabsf(z.x), fabsf(z.y)));
-    const float2 t = unpack2(mul2(zn[k], log2e));
-    const uint64_t den = add2(pack2(ex2(t.x), ex2(t.y)), one);
-    const float2 d = unpack2(den);
-    float r0, r1;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d.y));
-    const uint64_t rn = pack2(r0, r1), q = mul2(zn[k], rn);
-    const float2 y = unpack2(fma2(fma2(q, den, zn[k]), rn, q));
+    const float2 y = cv_silu2(zn[k]);
     out[k] = pack_bf16(y.x, y.y);
   }
   if (top >= 80.f) {
@@ -970,6 +973,44 @@ conv_pack_rgb_kernel(const T* __restrict__ src, long long c_stride, uint4* __res
   }
 }
 
+// Values with the bit patterns first .. first + 16 n - 1 against the division: [0] how many results differ in bf16, [1] in fp32 where
+// no value of 80 or more takes the division, [2] by how many spacings of fp32 at most.
+__global__ void __launch_bounds__(256)
+conv_silu_selftest_kernel(uint32_t first, long long n, unsigned long long* differ) {
+  unsigned long long bad16 = 0, bad32 = 0, far = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    uint64_t zn[8];
+    uint32_t o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t g = first + (uint32_t)(i * 16) + 2 * k;
+      zn[k] = pack2(-__uint_as_float(g), -__uint_as_float(g + 1));
+    }
+    cv_silu16(zn, o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float2 z = unpack2(zn[k]), y = cv_silu2(zn[k]);
+      const float got[2] = {y.x, y.y}, neg[2] = {z.x, z.y};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float want = -neg[e] / (1.f + __expf(neg[e])), stored = e ? bf16hi(o[k]) : bf16lo(o[k]);
+        const float rounded = bf16lo(pack_bf16(want, 0.f));
+        bad16 += stored != rounded && !(isnan(stored) && isnan(rounded));
+        if (fabsf(neg[e]) < 80.f && got[e] != want) {
+          ++bad32;
+          const long long d = llabs((long long)__float_as_int(got[e]) - __float_as_int(want));
+          far = max(far, (unsigned long long)d);
+        }
+      }
+    }
+  }
+  if (bad16) atomicAdd(differ, bad16);
+  if (bad32) {
+    atomicAdd(differ + 1, bad32);
+    atomicMax(differ + 2, far);
+  }
+}
+
 }  // namespace cb
 
 // ====================================================================== host
@@ -1227,6 +1268,10 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   maps[5] = rows_map(a.w, a.n_out, k_cols, p.mma_n / 2);
   if (R == 2) conv_dispatch<2>(maps, p, s);
   else conv_dispatch<1>(maps, p, s);
+}
+
+void conv_silu_selftest(uint32_t first, long long n, unsigned long long* differ, cudaStream_t s) {
+  if (n > 0) cb::conv_silu_selftest_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, s>>>(first, n, differ);
 }
 
 void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, int n, int h, int w, cudaStream_t s) {

@@ -279,6 +279,8 @@ struct ConvArgs {
   int* status = nullptr;
 };
 void conv3d_fused(const ConvArgs& a, cudaStream_t s);
+// Compares the convolutions' silu with the division for the 16 n values whose bit patterns follow `first`; adds to differ[3] (device).
+void conv_silu_selftest(uint32_t first, long long n, unsigned long long* differ, cudaStream_t s);
 // src [3, n, h, w] planes (fp32 or bf16) -> dst [n, h + 2, w + 2, 64]: the 9 spatial taps x 3 channels as 27 channels
 void conv_pack_rgb(const void* src, int is_f32, long long c_stride, void* dst, int n, int h, int w, cudaStream_t s);
 

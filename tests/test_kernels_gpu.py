@@ -1709,6 +1709,12 @@ def test_silu_of_the_swiglu_epilogue_is_the_division(first):
     assert torch.ops.cosmos_b200.silu_selftest(first, 2 ** 30, torch.empty(0, device=DEV)).item() == 0
 
 
+def test_silu_of_the_convolutions_is_the_division_in_bf16():
+    """Every fp32 value: no bf16 result differs from the division's; in fp32 two do, by one spacing."""
+    got = sum(torch.ops.cosmos_b200.conv_silu_selftest(i * 2 ** 30, 2 ** 30, torch.empty(0, device=DEV)) for i in range(4)).tolist()
+    assert got[0] == 0 and got[1] <= 2 and got[2] <= got[1]
+
+
 @pytest.mark.parametrize("m", [5, 300])
 @pytest.mark.parametrize("n", [8, 24, 40, 264])
 @pytest.mark.parametrize("shift", [1, 4])
