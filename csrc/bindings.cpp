@@ -1376,6 +1376,9 @@ void gemm_set_debug(int64_t bits) { cosmos::gemm_set_debug((int)bits); }
 int64_t gemm_pick_k_splits(int64_t M, int64_t N, int64_t K, int64_t epi) {
   return cosmos::gemm_pick_k_splits((int)M, (int)N, (int)K, (int)epi);
 }
+int64_t gemm_pick_split_ctas(int64_t M, int64_t N, int64_t K, int64_t epi) {
+  return cosmos::gemm_pick_split_ctas((int)M, (int)N, (int)K, (int)epi);
+}
 // The number of gates among the `count` bit patterns from `first` on (`count` a multiple of 16) whose silu in the SwiGLU epilogue
 // is not the division's.
 Tensor silu_selftest(int64_t first, int64_t count, const Tensor& like) {
@@ -1680,6 +1683,7 @@ TORCH_LIBRARY(cosmos_b200, m) {
   m.def("gemm_pick_tile", &gemm_pick_tile);
   m.def("gemm_set_debug", &gemm_set_debug);
   m.def("gemm_pick_k_splits", &gemm_pick_k_splits);
+  m.def("gemm_pick_split_ctas", &gemm_pick_split_ctas);
   m.def("launch_overlap", &launch_overlap);
   m.def("sample_topk", &sample_topk);
   m.def("sample_pick_", &sample_pick_);

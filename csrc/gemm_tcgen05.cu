@@ -1458,6 +1458,21 @@ void gemm_bf16_grouped(const GemmArgs* args, int n, cudaStream_t stream) {
     launch_epi<1>(args[0].epi, maps, g, g.total, limit, stream);
 }
 
+// CTAs of a split-K launch's tiles. More than one 128-row tile (a serving batch of 256): CTA pairs, so that each CTA stages half of the
+// weight tile. The split count was chosen for single CTAs, so pairs can need a second, mostly empty round where those have one:
+// 257 - 384 rows of a 4096-wide projection in three splits are 96 items on 74 pairs, or 144 on 148 CTAs whose k-block takes 1.4 times
+// as long (see pick_tile). 333 x 4096 x 4096 with the reduction 36 us on pairs, 30 on single CTAs; 333 x 4096 x 12288 67 and 54.
+static int split_ctas(int M, int N, int k_splits, int epi) {
+  if (!pair_enabled() || epi == EPI_SWIGLU || M <= cb::BM) return 1;
+  if (g_tile_ctas) return g_tile_ctas;
+  auto rounds = [&](int c) {
+    const long long items = (long long)((M + cb::BM * c - 1) / (cb::BM * c)) * ((N + cb::BN - 1) / cb::BN) * k_splits;
+    return (items + sm_count() / c - 1) / (sm_count() / c);
+  };
+  return rounds(2) * 1.0 <= rounds(1) * 1.4 ? 2 : 1;
+}
+int gemm_pick_split_ctas(int M, int N, int K, int epi) { return split_ctas(M, N, gemm_pick_k_splits(M, N, K, epi), epi); }
+
 void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (a.M <= 0 || a.N <= 0) return;
   if (a.k_splits <= 1 && !a.partial_only) {
@@ -1469,16 +1484,7 @@ void gemm_bf16(const GemmArgs& a, cudaStream_t stream) {
   if (!a.partial || a.N % 8 != 0) throw std::runtime_error("gemm_bf16: split-K needs a partial buffer and N % 8 == 0");
   cb::GemmGroup g{};
   CUtensorMap maps[4];
-  // More than one 128-row tile (a serving batch of 256): CTA pairs, so that each CTA stages half of the weight tile. The split
-  // count was chosen for single CTAs, so pairs can need a second, mostly empty round where those have one: 257 - 384 rows of a
-  // 4096-wide projection are 96 items on 74 pairs, or 144 on 148 CTAs whose k-block takes 1.4 times as long (see pick_tile).
-  // 333 x 4096 x 4096 with the reduction 36 us on pairs, 30 on single CTAs; 333 x 4096 x 12288 67 and 54.
-  auto rounds = [&](int c) {
-    const long long items = (long long)((a.M + cb::BM * c - 1) / (cb::BM * c)) * ((a.N + cb::BN - 1) / cb::BN) * a.k_splits;
-    return (items + sm_count() / c - 1) / (sm_count() / c);
-  };
-  const bool pairs = pair_enabled() && a.epi != EPI_SWIGLU && a.M > cb::BM && rounds(2) * 1.0 <= rounds(1) * 1.4;
-  const int nc = a.tile_map ? a.tile_m / cb::BM : pairs ? 2 : 1;
+  const int nc = a.tile_map ? a.tile_m / cb::BM : split_ctas(a.M, a.N, a.k_splits, a.epi);
   if (nc != 1 && nc != 2) throw std::runtime_error("gemm_bf16: tile rows must be 128 or 256");
   fill_problem(a, g.p[0], maps[0], maps[1], nc);
   const int k_blocks = (a.K + cb::BK - 1) / cb::BK;

@@ -82,6 +82,8 @@ struct GemmArgs {
 };
 // Split count that fills the machine for a skinny problem (1 = do not split).
 int gemm_pick_k_splits(int M, int N, int K, int epi);
+// CTAs of a tile (1 or 2) that a launch with that many splits uses.
+int gemm_pick_split_ctas(int M, int N, int K, int epi);
 // Debug knob for race hunting: at most `max_ctas` persistent CTAs per launch of a GEMM or a convolution (0 = one per SM).
 void gemm_set_grid_limit(int max_ctas);
 int gemm_grid_limit();

@@ -44,3 +44,16 @@ def test_paged_decode_split_choice(k):
     assert k.paged_decode_pick_splits(1, 8, 8448, 0) >= 8
     # a serving batch with short contexts: no split, no merge kernel
     assert k.paged_decode_pick_splits(256, 8, 416, 0) == 1
+
+
+@pytest.mark.parametrize("m,n,k_,epi,want", [
+    (128, 4096, 4096, ops.EPI_PLAIN, 1),           # one row tile
+    (256, 6144, 4096, ops.EPI_PLAIN, 2),           # 72 items on 74 pairs
+    (333, 4096, 4096, ops.EPI_GATED_RESID, 1),     # three splits: 96 items on 74 pairs, 144 on 148 CTAs
+    (333, 4096, 12288, ops.EPI_GATED_RESID, 1),
+    (384, 4096, 512, ops.EPI_GATED_RESID, 2),      # two splits: 64 items on 74 pairs
+    (385, 3072, 1024, ops.EPI_GATED_RESID, 2),     # 48 and 96
+    (200, 512, 4096, ops.EPI_SWIGLU, 1),           # has no pairs
+])
+def test_side_of_a_split_launch(k, m, n, k_, epi, want):
+    assert k.gemm_pick_split_ctas(m, n, k_, epi) == want

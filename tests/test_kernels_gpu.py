@@ -1667,20 +1667,24 @@ def test_gemm_wide_tiles(m, n, k):
         kern.gemm_set_tile(0, 0)
 
 
-@pytest.mark.parametrize("m,n,k", [(129, 4096, 512), (256, 768, 1024), (257, 4096, 768), (333, 4096, 1088), (384, 4096, 512), (385, 3072, 1024)])
-def test_gemm_split_on_pairs_and_single_ctas(m, n, k):
-    """Split-K launches of two to four row tiles, on the side that the number of rounds takes (pairs at 256 and 385 rows, single CTAs
-    at 257 to 384) and on the other: the same sums."""
+@pytest.mark.parametrize("m,n,k,side", [(129, 4096, 512, 2), (256, 768, 1024, 2), (257, 4096, 768, 1), (333, 4096, 1088, 1), (384, 4096, 512, 2),
+                                        (384, 4096, 768, 1), (385, 3072, 1024, 2)])
+def test_gemm_split_on_pairs_and_single_ctas(m, n, k, side):
+    """Split-K launches of two to four row tiles, on the side that the number of rounds takes (single CTAs at 257 to 384 rows of a
+    4096-wide projection in three splits, pairs elsewhere) and on either: the same sums."""
     kern = torch.ops.cosmos_b200
     assert kern.gemm_pick_k_splits(m, n, k, ops.EPI_GATED_RESID) > 1
+    assert kern.gemm_pick_split_ctas(m, n, k, ops.EPI_GATED_RESID) == side
     a, w, r = _rand(m, k), _rand(n, k) * 0.05, _rand(m, n)
     got = ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, None, m)
     _close(got, r.float() + a.float() @ w.float().t(), 3e-2, 2e-2, f"{m}x{n}x{k}")
-    kern.gemm_set_cta_pair(False)
     try:
-        assert torch.equal(got, ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, None, m))
+        for ctas in (1, 2):
+            kern.gemm_set_tile(ctas, 1)
+            assert kern.gemm_pick_split_ctas(m, n, k, ops.EPI_GATED_RESID) == ctas
+            assert torch.equal(got, ops.gemm(a, w, None, ops.EPI_GATED_RESID, r, None, m)), ctas
     finally:
-        kern.gemm_set_cta_pair(True)
+        kern.gemm_set_tile(0, 0)
     torch.cuda.synchronize()
     ops.check_status()
 
