@@ -1555,6 +1555,98 @@ def test_conv3d_chunk_is_conv3d_fused(t, cin, cout):
             assert torch.equal(k.conv3d_rgb_chunk(split(x).parts, x[:2].contiguous() if ctx else None, terms, rb, t), k.conv3d_rgb(x, terms, rb))
 
 
+@pytest.mark.parametrize("t", [1, 2, 5])
+@pytest.mark.parametrize("ctx", [True, False])
+@pytest.mark.parametrize("cin,cout", [(64, 64), (128, 32), (128, 128), (256, 256), (128, 320)])
+def test_conv3d_chunk_against_fp64(cin, cout, ctx, t):
+    """The form that the tokenizer calls (volumes in two tensors, context frames in a third or absent) against fp64 convolutions of the
+    same bf16 numbers, in every layout, and with one and three CTA pairs: the same bits. 2304 positions a frame are five tiles of 512
+    or nine of 256. Bound: one bf16 rounding (2^-9 relative) and fp32 sums of up to 6976 products, together below 2^-8 of the larger of the
+    result and 1."""
+    import torch.nn.functional as F
+    from cosmos_b200.models.vae_cuda import Volume
+    k = torch.ops.cosmos_b200
+    torch.manual_seed(t + cin + cout)
+    h, w = 34, 62
+    hp, wd = h + 2, w + 2
+    fused = cout in (64, 128, 256)
+
+    def full(c):
+        v = torch.zeros(t + 2, hp, wd, c, device=DEV, dtype=torch.bfloat16)
+        v[0 if ctx else 2:, 1:-1, 1:-1] = _rand(t + 2 if ctx else t, h, w, c)
+        return v
+
+    def split(v):
+        vol = Volume(t, v.shape[1:], DEV)
+        for lo, hi, part in vol.pieces():
+            part.copy_(v[2 + lo:2 + hi])
+        return vol.parts, v[:2].contiguous() if ctx else None
+
+    def new(frames, *shape):
+        vol = Volume(frames, (*shape, cout), DEV)
+        vol.body.fill_(7.0)
+        vol.tail.fill_(7.0)
+        return vol
+
+    def whole(vol):
+        return torch.cat([part for _, _, part in vol.pieces()])
+
+    def parity(v):
+        return torch.stack([v[:, i::2, j::2] for i in (0, 1) for j in (0, 1)], dim=1).contiguous()
+
+    def near(got, want):
+        assert got.shape == want.shape and ((got.double() - want).abs() <= 2 ** -8 * want.abs().clamp(min=1.0)).all()
+
+    x, res, sk = full(cin), full(cout), full(64)
+    wt, sw, b = _rand(cout, cin, 3, 3, 3, scale=1 / math.sqrt(27 * cin)), _rand(cout, 64, scale=0.125), torch.randn(cout, device=DEV)
+    g = _rand(cout) if fused else None
+    wp = wt.permute(0, 2, 3, 4, 1).reshape(cout, 27 * cin).contiguous()
+    ws = torch.cat([wp, sw], 1).contiguous()
+    terms, rb = _rand(9, 27 * 64, scale=0.02), torch.randn(3, device=DEV) * 0.1
+    x5 = x.permute(3, 0, 1, 2)[None].double()
+    conv = F.conv3d(x5, wt.double(), b.double())[0].permute(1, 2, 3, 0)                          # [t, h, w, cout]
+    down = F.conv3d(x5, wt.double(), b.double(), stride=(1, 2, 2))[0].permute(1, 2, 3, 0)
+    inner = lambda v: v[2:, 1:-1, 1:-1].double()  # noqa: E731
+    pad = lambda v: F.pad(v, (0, 0, 1, 1, 1, 1))  # noqa: E731
+    twice = lambda v: v.repeat_interleave(2, 1).repeat_interleave(2, 2)  # noqa: E731
+    xp, cx = split(x)
+    xs, cs = split(parity(x))
+    rp, sp = split(res)[0], split(sk)[0]
+
+    def run():
+        same, norm, s2d, up = new(t, hp, wd), new(t, hp, wd), new(t, 4, hp // 2, wd // 2), new(2 * t, 2 * h + 2, 2 * w + 2)
+        up1, dn, dnorm = new(2 * t - 1, 2 * h + 2, 2 * w + 2), new((t + 1) // 2, h // 2 + 2, w // 2 + 2), new((t + 1) // 2, h // 2 + 2, w // 2 + 2)
+        k.conv3d_chunk(xp, cx, wp, b, rp, [], same.parts, norm.parts if fused else [], g, 1e-6, 0, t, 0, 0)
+        k.conv3d_chunk(xp, cx, ws, b, [], sp, s2d.parts, [], None, 1e-6, 1, t, 0, 0)
+        k.conv3d_chunk(xp, cx, wp, b, rp, [], up.parts, [], None, 1e-6, 2, t, 1, 0)
+        k.conv3d_chunk(xp, cx, wp, b, rp, [], up1.parts, [], None, 1e-6, 2, t, 1, 1)
+        k.conv3d_chunk(xs, cs, wp, b, [], [], dn.parts, dnorm.parts if fused else [], g, 1e-6, 3, t, 0, 2)
+        out = [whole(v) for v in (same, norm, s2d, up, up1, dn, dnorm)]
+        return out + ([k.conv3d_rgb_chunk(split(x[..., :64].contiguous())[0], cx[..., :64].contiguous() if ctx else None, terms, rb, t)])
+
+    got = run()
+    plus = conv + inner(res)
+    near(got[0], pad(plus))
+    near(got[2], parity(pad(conv + inner(sk) @ sw.double().t())))
+    near(got[3], pad(twice(plus.repeat_interleave(2, 0))))
+    near(got[4], pad(twice(plus.repeat_interleave(2, 0)[1:])))
+    near(got[5], pad(down[::2]))
+    if fused:
+        for raw, n in ((got[0], got[1]), (got[5], got[6])):
+            y = raw.double()
+            near(n, F.silu(y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-6) * g.double()))
+    wo = terms.double().view(3, 3, 3, 3, 3, 64).sum(0).permute(0, 4, 1, 2, 3)
+    pix = ((F.conv3d(x5[:, :64], wo, rb.double())[0].clamp(-1, 1) + 1) * 127.5).permute(1, 2, 3, 0)
+    assert (got[7].double() - pix).abs().max() <= 0.5 + 1e-3
+    try:
+        for limit in (2, 6):
+            k.gemm_set_grid_limit(limit)
+            for i, (u, v) in enumerate(zip(run(), got)):
+                assert torch.equal(u, v), (limit, i)
+    finally:
+        k.gemm_set_grid_limit(0)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 10, 22)])
 def test_conv3d_of_colours(dtype, t, h, w):
