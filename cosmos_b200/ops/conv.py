@@ -2,7 +2,7 @@
 RMS-norm + SiLU. They run training through the tokenizer, every tokenizer whose channel widths are not multiples
 of 64, and the CPU path, and they are the oracle of the channels-last encoder and decoder. The inference hot path
 does not go through this module: `models/vae_cuda.py` runs encoder and decoder on the implicit-GEMM tcgen05 kernel
-(`torch.ops.cosmos_b200.conv3d_fused`, `conv3d_rgb`)."""
+(`torch.ops.cosmos_b200.conv3d_chunk`, `conv3d_rgb_chunk`)."""
 from __future__ import annotations
 
 from typing import Sequence, Tuple

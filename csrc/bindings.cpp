@@ -1040,47 +1040,20 @@ void conv3d_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const OptT
   conv_run(a, x0, w, bias, gamma, eps);
 }
 
-// The same on volumes [F, ...] whose first two frames are the context: x, resid, skip and the outputs, which are written from their
-// third frame on.
+// The same for callers that hold a clip in one tensor: volumes [F, ...] whose first two frames are the context (of x; those of resid
+// and skip are not read), outputs written from their third frame on.
 void conv3d_fused(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& resid, const OptT& skip, const OptT& out,
                   const OptT& out_norm, const OptT& gamma, double eps, int64_t mode, int64_t ma, int64_t mb) {
-  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
-  c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(mode >= 0 && mode <= 3, "conv3d_fused: unknown mode");
-  const bool down = mode == cosmos::CONV_OUT_DOWN;
-  TORCH_CHECK(x.is_contiguous() && x.dim() == (down ? 5 : 4) && (!down || x.size(1) == 4), "x must be a contiguous volume");
-  cosmos::ConvArgs a;
-  const int64_t F = x.size(0), Hp = x.size(down ? 2 : 1) * (down ? 2 : 1), Wp = x.size(down ? 3 : 2) * (down ? 2 : 1);
-  const int64_t C = x.size(-1), Cout = w.size(0);
-  TORCH_CHECK(F > 2, "x needs two context frames and at least one more");
-  TORCH_CHECK(F * Hp * Wp < (1ll << 31) - 2 * Hp * Wp, "volume too large for 32-bit row indices; use shorter temporal chunks");
-  a.frames = (int)F - 2; a.hp = (int)Hp; a.wp = (int)Wp; a.c = (int)C; a.n_out = (int)Cout; a.mode = (int)mode;
-  auto behind = [](const Tensor& t) { return static_cast<char*>(t.data_ptr()) + 2 * t.stride(0) * t.element_size(); };
-  a.ctx = x.data_ptr();
-  a.x = behind(x);
-  if (skip.has_value() && skip->defined()) {
-    check_bf16_cuda(*skip, "skip");
-    TORCH_CHECK(!down && skip->is_contiguous() && skip->dim() == 4 && skip->size(0) == F && skip->size(1) == Hp && skip->size(2) == Wp,
-                "skip must be a volume of x's size");
-    a.skip = behind(*skip); a.skip_c = (int)skip->size(3);
-  }
-  int64_t f_dst = 0;
-  std::vector<int64_t> shape = conv_mode(a, ma, mb, f_dst);
-  shape.insert(shape.begin(), f_dst + 2);
-  if (resid.has_value() && resid->defined()) {
-    check_bf16_cuda(*resid, "resid");
-    TORCH_CHECK(resid->is_contiguous() && resid->sizes() == at::IntArrayRef({F, Hp, Wp, Cout}), "resid must have x's padded size");
-    a.resid = behind(*resid);
-  }
-  auto output = [&](const OptT& t, const char* name) -> void* {
-    if (!t.has_value() || !t->defined()) return nullptr;
-    check_bf16_cuda(*t, name);
-    TORCH_CHECK(t->is_contiguous() && t->sizes() == at::IntArrayRef(shape), name, " has the wrong size for this mode");
-    return behind(*t);
+  TORCH_CHECK(x.is_contiguous() && x.dim() >= 4 && x.size(0) > 2, "x must be a contiguous volume of two context frames and at least one more");
+  const int64_t frames = x.size(0) - 2;
+  if (mode == cosmos::CONV_OUT_DOWN && ma >= frames) return;   // no frame is kept
+  auto behind = [](const OptT& t) -> std::vector<Tensor> {
+    if (!t.has_value() || !t->defined()) return {};
+    TORCH_CHECK(t->is_contiguous() && t->dim() >= 4 && t->size(0) > 2, "a contiguous volume behind two context frames expected");
+    return {t->slice(0, 2)};
   };
-  a.out = output(out, "out");
-  a.out_norm = output(out_norm, "out_norm");
-  conv_run(a, x, w, bias, gamma, eps);
+  const std::vector<Tensor> r = behind(resid), k = behind(skip), o = behind(out), n = behind(out_norm);
+  conv3d_chunk({x.slice(0, 2)}, x.slice(0, 0, 2), w, bias, r, k, o, n, gamma, eps, mode, frames, ma, mb);
 }
 
 // One convolution without fusions: out and resid [F, Hp, Wp, Cout]; the interior of the frames from `tpad` on is written, the border
@@ -1130,18 +1103,6 @@ Tensor conv_rgb(cosmos::ConvArgs& a, const Tensor& x, const Tensor& w, const Ten
   return out;
 }
 
-// x: [F, Hp, Wp, C], its first two frames the context
-Tensor conv3d_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
-  check_bf16_cuda(x, "x"); check_bf16_cuda(w, "w");
-  c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(0) > 2 && x.size(1) > 2 && x.size(2) > 2, "x must be a padded volume");
-  cosmos::ConvArgs a;
-  a.ctx = x.data_ptr();
-  a.x = static_cast<char*>(x.data_ptr()) + 2 * x.stride(0) * x.element_size();
-  a.frames = (int)x.size(0) - 2;
-  return conv_rgb(a, x, w, bias);
-}
-
 // x and ctx as conv3d_chunk takes them
 Tensor conv3d_rgb_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const Tensor& bias, int64_t frames) {
   check_bf16_cuda(w, "w");
@@ -1157,6 +1118,12 @@ Tensor conv3d_rgb_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, cons
     TORCH_CHECK(conv_volume({*ctx}, "ctx", frame, 2, a.ctx, none) == 2 && ctx->device() == w.device());
   }
   return conv_rgb(a, x0, w, bias);
+}
+
+// The same of a clip in one tensor [F, Hp, Wp, C], its first two frames the context
+Tensor conv3d_rgb(const Tensor& x, const Tensor& w, const Tensor& bias) {
+  TORCH_CHECK(x.dim() == 4 && x.is_contiguous() && x.size(0) > 2, "x must be a padded volume");
+  return conv3d_rgb_chunk({x.slice(0, 2)}, x.slice(0, 0, 2), w, bias, x.size(0) - 2);
 }
 
 // frames [3, n, h, w] (fp32 or bf16; channel stride free, the rest dense) -> dst [n, h + 2, w + 2, 64]
