@@ -253,9 +253,9 @@ class TPDecoder(StepDecoder):
         """Consumes self.tokens / self.lens (device), writes self.next_tokens and advances lens."""
         begins = self._begins_on_kernel()   # loads the library
         # Programmatic dependent launch: the kernels' set-up, and around the layers the GEMMs' first weight tiles, may overlap the tail
-        # of the kernel before. Batch 1 over 1500 tokens, eight layers, set-up alone and both: 1080 -> 1050 us; batch 32 over 8448:
-        # 2475 -> 2465. At TP 2 and 4 both against none took 8.96 -> 8.77 and 5.80 -> 5.45 ms before norms and reductions
-        # were launched early. COSMOS_DECODE_PDL=0: nothing in the step overlaps.
+        # of the kernel before. Nothing / set-up alone / both, eight layers: batch 1 over 1500 tokens 1092 / 1048 / 1022 us; batch 32
+        # over 8448 2448 / 2409 / 2388. At TP 2 and 4 both against nothing took 8.96 -> 8.77 and 5.80 -> 5.45 ms before norms and
+        # reductions were launched early. COSMOS_DECODE_PDL=0: nothing in the step overlaps.
         overlap = os.environ.get("COSMOS_DECODE_PDL", "1") == "1"
         with ops.launch_overlap(1 if overlap else 0):
             # attention sees the token being written; idle slots of a serving batch do not advance (step_inc)

@@ -3,9 +3,9 @@
 // their products are left out), and so may be a volume's last two frames, which are the next chunk's: what a chunk hands on is
 // neither copied nor holds the whole volume.
 //
-// A CTA pair (cta_group::2) computes R x 256 rows (positions of a frame) by up to 256 output channels. What
-// bounds such a kernel is the delivery of the operands from L2 into shared memory (about 45 B per clock and SM): a plain
-// implicit GEMM fetches a fresh 128-row tile of activations for each of the 27 taps. Here
+// A CTA pair (cta_group::2) computes R x 256 rows (positions of a frame) by up to 256 output channels. A plain implicit GEMM
+// fetches a fresh 128-row tile of activations for each of the 27 taps, more than L2 delivers into shared memory under the
+// products (60 - 80 B per clock and SM). Here
 //   * the three taps of one row of the filter read one staged tile of 128 R + 8 rows at row offsets 0, 1 and 2: the matrix
 //     descriptor starts in the middle of a swizzle atom (the swizzle is a function of the shared-memory address), so a tile
 //     crosses L2 -> shared memory 9 times and not 27;
@@ -14,7 +14,8 @@
 //   * activations and weights have rings of their own, so that a weight tile holds its slot for one product and an
 //     activation tile for three.
 // Per 64 channels, tap and 128 rows a CTA of the pair stages 5.6 KB of activations and 4 of weights at 128 output channels, where
-// a tile for each tap would take 16 and 8.
+// a tile for each tap would take 16 and 8. Wide layers are bound by the products at the power limit (figures below), narrow ones by
+// the epilogue (64 channels and less, conv_time_kernel), the first and the last by memory.
 //
 // A strided convolution reads its input split into the four parities of (row, column) ("s2d": [frames, 4, (H + 2) / 2,
 // (W + 2) / 2, C]), which the layer before it writes; each tap is then again a row offset, taps of equal column parity share
@@ -628,8 +629,8 @@ conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ C
   } else {
     // ---------------- epilogue: eight warps per row tile; tensor-memory lane quadrant = warp % 4, and the two warps of a
     // quadrant take every other group of 16 columns. The loops over these groups stay rolled: unrolled over 256 columns the
-    // code left the instruction cache and a tile took 67 us. Latency bounds what is left (the divisions of the SiLU most of
-    // all, which are exact so that the result is the separate norm kernel's), hence the number of warps.
+    // code left the instruction cache and a tile took 67 us. Latency bounds what is left (the chain of the SiLU most of all,
+    // though its quotient takes no division, cv_silu2), hence the number of warps.
     const int quad = warp & 3, half = ((warp - 2) >> 2) & 1, r = (warp - 2) >> 3;
     const int pair_id = 1 + r * 4 + quad;
     const float* bias = p.n_tiles == 1 ? gamma + CV_GAMMA / 4 : p.bias;

@@ -15,7 +15,7 @@
 
 namespace cb {
 
-constexpr int OPT_CHUNK = 8192;    // elements: 256 threads x 8 elements x 4 trips
+constexpr int OPT_CHUNK = 8192;    // elements: 256 threads x 4 elements x 8 trips, four of them in flight
 constexpr int OPT_THREADS = 256;
 constexpr int OPT_TRIPS = 4;
 

@@ -38,7 +38,8 @@ rope_tables_kernel(const long long* __restrict__ pos, int S, int half, double th
 // position past the table's row, and a page that is none of the cache's (unused entries are -1), give slot -1, for which the
 // layers store nothing, and the length stays where it is, inside the row, so that attention reads no further either.
 // The kernels behind may start only once this one's wait is over: the layers' GEMMs request weights ahead of their own waits, so
-// everything that ran before the step (which may have written these weights) must be complete when the first of them starts.
+// everything that ran before the step (which may have written these weights) must be complete when the first of them starts. In a
+// captured step the later trigger costs nothing that shows: batch 1 over 1500 tokens 993 us either way, batch 32 over 8448 2321 and 2322.
 __global__ void __launch_bounds__(256) decode_begin_kernel(const cosmos::DecodeBeginArgs a) {
   pdl_wait();
   pdl_launch_dependents();
