@@ -92,7 +92,12 @@ class _CLConvs:
         if vol.frames == 1:
             vol.tail[0].copy_(ctx[1]) if ctx is not None else vol.tail[0].zero_()
         cache[key] = vol.tail
-        return ctx
+        return ctx if ctx is not None or self.finite else torch.zeros_like(vol.tail)
+
+    def _finish(self) -> None:
+        """The kernel leaves out products with an absent context, which are zero as long as the weights are finite; otherwise zeros
+        stand in for it."""
+        self.finite = bool(torch.stack([w.isfinite().all() for w in self.w.values()]).all())
 
     def _volume(self, frames: int, *frame_shape, zero: bool = False) -> Volume:
         return Volume(frames, frame_shape, self.device, zero)
@@ -138,6 +143,8 @@ class CLDecoder(_CLConvs):
         assert wo.shape[0] == 3 and wo.shape[1] == 64, "the RGB head expects 64 input channels"
         self.w_out = _bf16_terms(wo.permute(0, 2, 3, 4, 1).reshape(3, 27 * 64))
         self.b_out = vae.dec_out.bias.data.float().contiguous()
+        self._finish()
+        self.finite = self.finite and bool(wo.isfinite().all())
 
     # ------------------------------------------------------------------ public
     @torch.no_grad()
@@ -261,6 +268,7 @@ class CLEncoder(_CLConvs):
         res("mid", vae.enc_mid)
         self.g["out"] = vae.enc_norm.gamma.data.to(torch.bfloat16).contiguous()
         self._add_conv("out", vae.enc_out)
+        self._finish()
 
     def _res(self, cache, name, x, n, **kw):
         """One residual block; x: its input, n: silu(rmsnorm(x))."""

@@ -999,7 +999,7 @@ std::vector<int64_t> conv_mode(cosmos::ConvArgs& a, int64_t ma, int64_t mb, int6
 
 // One convolution of a chunk. x: channels-last volume of padded frames [Hp, Wp, C] (C % 64 == 0), mode 3: of s2d frames [4, Hp / 2,
 // Wp / 2, C]; volumes (x, resid, skip and both outputs) as conv_volume takes them, empty lists for those that are absent; ctx: the
-// two frames before x, or none, which stands for zeros; w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only). Outputs (at
+// two frames before x, or none, which stands for zeros (with finite weights: their products are left out); w: [Cout, 27 C (+ Cskip)] or [Cout, 3 C] (taps in time only). Outputs (at
 // least one) are written border included. (ma, mb): mode 2 temporal doubling and first chunk, mode 3 first kept frame and frame step.
 void conv3d_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const OptT& bias, at::TensorList resid, at::TensorList skip,
                   at::TensorList out, at::TensorList out_norm, const OptT& gamma, double eps, int64_t mode, int64_t frames, int64_t ma,
@@ -1020,7 +1020,6 @@ void conv3d_chunk(at::TensorList x, const OptT& ctx, const Tensor& w, const OptT
   if (ctx.has_value() && ctx->defined()) {
     const void* none = nullptr;
     TORCH_CHECK(conv_volume({*ctx}, "ctx", frame, 2, a.ctx, none) == 2 && ctx->device() == w.device());
-    a.ctx_frames = 2;
   }
   if (!skip.empty()) {
     TORCH_CHECK(!down, "no skip input in this form");
@@ -1071,8 +1070,12 @@ void conv3d_cl(const Tensor& x, const Tensor& w, const OptT& bias, const OptT& r
   cosmos::ConvArgs a;
   a.keep_border = 1;
   const int64_t frame = Hp * Wp * x.element_size();
-  a.ctx_frames = (int)std::min<int64_t>(tpad, 2);
-  a.ctx = a.ctx_frames ? static_cast<char*>(x.data_ptr()) + (tpad - a.ctx_frames) * frame * C : nullptr;
+  Tensor first;   // frames that x does not have are zero
+  if (tpad < 2) {
+    first = at::zeros({2, Hp, Wp, C}, x.options());
+    if (tpad == 1) first.select(0, 1).copy_(x.select(0, 0));
+  }
+  a.ctx = tpad < 2 ? first.data_ptr() : static_cast<char*>(x.data_ptr()) + (tpad - 2) * frame * C;
   a.x = static_cast<char*>(x.data_ptr()) + tpad * frame * C;
   a.w = w.data_ptr();
   a.out = static_cast<char*>(out.data_ptr()) + tpad * frame * Cout;

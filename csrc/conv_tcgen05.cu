@@ -75,7 +75,7 @@ struct ConvParams {
   // rows: n_seg segments (frames of a strided convolution, else one) of seg_rows rows
   int n_seg, seg_rows, tiles_per_seg;
   int frame_rows;        // rows of an input frame
-  int ctx_shift;         // context tensor: place of its first frame before the volume's first, 2 or 1; 0: absent
+  int has_ctx;           // else the products with its two frames are left out
   int v_first, v_step;   // segment s begins at input frame v_first + s v_step (counted from the first context frame)
   int x_split, skip_split;
   int pw, plane;         // width and size of the plane that a segment's rows walk through
@@ -163,7 +163,7 @@ struct ConvSource {
 };
 __device__ __forceinline__ ConvSource conv_source(const ConvParams& p, int v, const CUtensorMap* ctx, const CUtensorMap* body,
                                                   const CUtensorMap* tail) {
-  if (v < 2) return {ctx, (v + p.ctx_shift - 2) * p.frame_rows};
+  if (v < 2) return {ctx, v * p.frame_rows};
   if (v - 2 < p.x_split) return {body, (v - 2) * p.frame_rows};
   return {tail, (v - 2 - p.x_split) * p.frame_rows};
 }
@@ -491,7 +491,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ C
               src = seg < p.skip_split ? ConvSource{&tmSkip, seg * p.frame_rows} : ConvSource{&tmSkipTail, (seg - p.skip_split) * p.frame_rows};
             } else {
               const int v = v0 + p.g[g].kt;
-              if (v < 2 && !p.ctx_shift) continue;
+              if (v < 2 && !p.has_ctx) continue;
               src = conv_source(p, v, &tmCtx, &tmBody, &tmTail);
               src.row += p.g[g].off;
             }
@@ -534,7 +534,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ C
           const int nc = min(CV_CHUNK, cblocks - c0);
           const int n_groups = ph ? 1 : p.n_groups;
           for (int g = 0; g < n_groups && ok; ++g) {
-            if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
+            if (!ph && v0 + p.g[g].kt < 2 && !p.has_ctx) continue;
             const int n_taps = ph ? 1 : p.g[g].n_taps;
             for (int i = 0; i < n_taps && ok; ++i) {
               const int x = (ph ? p.skip_kcol : p.g[g].tap[i] * cblocks * 64) + c0 * 64;
@@ -577,7 +577,7 @@ conv_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constant__ C
             const int nc = min(CV_CHUNK, cblocks - c0);
             const int n_groups = ph ? 1 : p.n_groups;
             for (int g = 0; g < n_groups && ok; ++g) {
-              if (!ph && v0 + p.g[g].kt < 2 && !p.ctx_shift) continue;
+              if (!ph && v0 + p.g[g].kt < 2 && !p.has_ctx) continue;
               const int n_taps = ph ? 1 : p.g[g].n_taps;
               int ia = ia0;
               uint32_t pha = pha0;
@@ -760,7 +760,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constan
       const int seg = t / p.tiles_per_seg, tile = t - seg * p.tiles_per_seg;
       const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
       const int local = tile * 512 + int(rank) * 256;
-      for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
+      for (int i = p.has_ctx ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
         const ConvSource src = conv_source(p, i, &tmCtx, &tmBody, &tmTail);
         for (int g = 0; g < p.n_groups && ok; ++g) {
           const int y = src.row + local + p.g[0].off + g * p.pw;
@@ -796,7 +796,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constan
       for (int t = first_tile; t < total && ok; t += tile_step) {
         const int seg = t / p.tiles_per_seg;
         const int j0 = seg * p.seg_frames, j1 = min(j0 + p.seg_frames, p.f_out);
-        for (int i = p.ctx_shift ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
+        for (int i = p.has_ctx ? j0 : max(j0, 2); i < j1 + 2 && ok; ++i) {
           const Step st = step_of(i, j0, j1, base);
           // a product of n frames has 2 n pieces along N, of which the even CTA holds the first n
           int x[3], y[3];
@@ -852,7 +852,7 @@ conv_time_kernel(const __grid_constant__ CUtensorMap tmCtx, const __grid_constan
           }
           const int n2 = st.n - st.n1;
           const uint32_t idesc1 = make_idesc_bf16(256, st.n1 * p.nt, 0, 0), idesc2 = make_idesc_bf16(256, n2 * p.nt, 0, 0);
-          const int n_groups = i < 2 && !p.ctx_shift ? 0 : p.n_groups;   // no frame there: zeros
+          const int n_groups = i < 2 && !p.has_ctx ? 0 : p.n_groups;   // no frame there
           for (int g = 0; g < n_groups && ok; ++g) {
             for (int c = 0; c < p.cblocks && ok; ++c) {
               if (!__all_sync(0xffffffffu, mbar_wait(full(ia), pha, abort_flag, p.status, ST_TIMEOUT_MMA))) { ok = false; break; }
@@ -1187,7 +1187,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
   p.up_first = a.up_first;
   p.status = a.status;
   p.frame_rows = (int)plane;
-  p.ctx_shift = a.ctx ? a.ctx_frames : 0;
+  p.has_ctx = a.ctx != nullptr;
   p.x_split = a.x_tail ? a.frames - 2 : a.frames;
   p.skip_split = a.skip_tail ? a.frames - 2 : a.frames;
   p.n_seg = a.f_out;
@@ -1204,7 +1204,7 @@ void conv3d_fused(const ConvArgs& a, cudaStream_t s) {
     if (!t) tail = body;
   };
   volume(maps[1], maps[2], a.x, a.x_tail, a.c);
-  maps[0] = a.ctx ? rows_map(a.ctx, a.ctx_frames * plane, a.c, box) : maps[1];
+  maps[0] = a.ctx ? rows_map(a.ctx, 2 * plane, a.c, box) : maps[1];
   if (has_skip) volume(maps[3], maps[4], a.skip, a.skip_tail, a.skip_c);
   else maps[3] = maps[4] = maps[1];
   const int stage_max = cb::CV_SMEM_MAX - 1024 - cb::CV_TAIL;

@@ -257,8 +257,7 @@ enum ConvOut : int {
 struct ConvArgs {
   const void* x = nullptr;      // [frames, hp, wp, c] (CONV_OUT_DOWN: [frames, 4, hp / 2, wp / 2, c])
   const void* x_tail = nullptr;
-  const void* ctx = nullptr;    // the ctx_frames (1 or 2) frames before x; those that are missing are zero
-  int ctx_frames = 2;
+  const void* ctx = nullptr;    // the two frames before x; none: zeros, whose products (with finite weights) are left out
   const void* w = nullptr;      // [n_out, 27 c (+ skip_c)], tap-major; taps_t_only: [n_out, 3 c]
   const float* bias = nullptr;  // [n_out]; pixels: [3]
   const void* resid = nullptr;  // added; layout of a CONV_OUT_SAME output

@@ -1647,6 +1647,40 @@ def test_conv3d_chunk_against_fp64(cin, cout, ctx, t):
         k.gemm_set_grid_limit(0)
 
 
+@pytest.mark.parametrize("cin,cout,tpad", [(64, 64, 0), (64, 128, 1), (128, 32, 1), (64, 256, 0), (64, 64, 2)])
+def test_conv3d_cl_of_weights_that_are_not_finite(cin, cout, tpad):
+    """An infinite weight of an early tap meets the zeros in front of the first frame: NaN, as in the definition, in that channel."""
+    import torch.nn.functional as F
+    torch.manual_seed(cin + cout)
+    x, wt = _rand(3, 8, 10, cin), _rand(cout, cin, 3, 3, 3, scale=0.02)
+    wt[5, 3, 0, 1, 1] = math.inf
+    out = torch.zeros(3, 8, 10, cout, device=DEV, dtype=torch.bfloat16)
+    wp = wt.permute(0, 2, 3, 4, 1).reshape(cout, 27 * cin).contiguous()
+    torch.ops.cosmos_b200.conv3d_cl(x, wp, None, None, out, tpad)
+    xf = F.pad(x.permute(3, 0, 1, 2)[None].float(), (0, 0, 0, 0, 2, 0))
+    want = F.conv3d(xf, wt.float())[0].permute(1, 2, 3, 0)[tpad:]
+    got = out[tpad:, 1:-1, 1:-1].float()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isfinite(), want.isfinite())
+    _close(got[..., :5], want[..., :5], 2e-2, 2e-2)
+
+
+@pytest.mark.parametrize("part", ["dec_in", "enc_in", "enc_mid"])
+def test_tokenizer_with_weights_that_are_not_finite(part):
+    """An infinite weight of an early tap: whatever a clip's first chunk has NaN in with a context of zeros, it has without one."""
+    from cosmos_b200.models.vae import CausalVideoVAE
+    from cosmos_b200.models.vae_cuda import CLDecoder, CLEncoder
+    torch.manual_seed(3)
+    vae = CausalVideoVAE(widths=(64, 64, 64, 64)).to(DEV)
+    conv = {"dec_in": vae.dec_in, "enc_in": vae.enc_in, "enc_mid": vae.enc_mid.c1}[part]
+    conv.weight.data[5, 1, 0, 1, 1] = math.inf
+    cl, key = CLDecoder(vae) if part == "dec_in" else CLEncoder(vae), "mid.c1" if part == "enc_mid" else "in"
+    x = cl._volume(1, 6, 6, 64, zero=True)
+    x.tail[1, 1:-1, 1:-1] = _rand(4, 4, 64)
+    out, _ = cl._conv({}, key, x)
+    assert out.tail[1, 1:-1, 1:-1, 5].isnan().all()
+    assert out.tail[1, 1:-1, 1:-1, 6].isfinite().all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("t,h,w", [(1, 8, 8), (3, 10, 22)])
 def test_conv3d_of_colours(dtype, t, h, w):
