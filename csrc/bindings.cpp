@@ -559,7 +559,11 @@ std::vector<Tensor> dm_modulation_rows(const Tensor& t_mod, const Tensor& table)
   const Tensor all = dm_modulation(t_mod, table);
   const int64_t B = all.size(1), d = all.size(2);
   std::vector<Tensor> rows;
-  for (int64_t i = 0; i < 6; ++i) rows.push_back(at::empty({0}, all.options()).set_(all.storage(), i * B * d, {B, d}, {d, 1}));
+  for (int64_t i = 0; i < 6; ++i) {   // by hand: empty() and set_() take the host 4 us more
+    rows.push_back(at::detail::make_tensor<c10::TensorImpl>(c10::Storage(all.storage()), all.key_set(), all.dtype()));
+    rows.back().unsafeGetTensorImpl()->set_storage_offset(i * B * d);
+    rows.back().unsafeGetTensorImpl()->set_sizes_contiguous({B, d});
+  }
   return rows;
 }
 
